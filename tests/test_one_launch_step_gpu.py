@@ -1,0 +1,62 @@
+"""The step in one launch (small grids of default tiling) against the step of
+three launches (a tiling set by the caller): the same bits."""
+import numpy as np
+import pytest
+
+from virs_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def _sim(shape, W, seed, storage, sections, n_rcv, rounding=capi.ROUND_NEAREST, tiling=None):
+    """Scattered walls and hard sources; soft sources and receivers on every
+    kind of voxel, several receivers on one voxel, some on the border."""
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = shape
+    n = nx * ny * nz
+    flags = np.zeros(n, np.uint8)
+    flags[rng.random(n) < 0.02] = 1
+    flags[rng.random(n) < 0.002] = 3
+    sim = capi.Simulation(capi.default_params(sponge_width=W, courant=1.0, boundary_form=1, storage=storage))
+    sim.set_grid(shape, 0.05, flags, rng.integers(0, 3, n).astype(np.uint8))
+    sim.classify()
+    one = np.stack([capi.design_octave_cascade(40000.0, a) for a in rng.uniform(0.1, 0.7, (3, 3))])
+    coef = np.concatenate([one] * 3, 1)[:, :sections]
+    sim.set_filters(coef.astype(np.float32), n_sections=sections)
+    x, y, z = np.meshgrid(np.arange(1, nx - 1), np.arange(1, ny - 1), np.arange(1, nz - 1), indexing="ij")
+    inner = ((z * ny + y) * nx + x).reshape(-1)
+    cls = sim.flags()[inner]
+    src = np.concatenate([rng.choice(inner[cls == f], min(2, int((cls == f).sum())), replace=False) for f in range(4)])
+    rcv = np.concatenate([src, src[:1], rng.choice(n, n_rcv)])
+    steps = 70
+    sim.set_sources(src, rng.standard_normal((src.size, steps)).astype(np.float32))
+    sim.set_receivers(rcv)
+    sim.set_hard_source(rng.standard_normal(20).astype(np.float32))
+    sim.set_rounding(rounding)
+    if tiling:
+        sim.set_tiling(*tiling)
+    sim.start(steps)
+    for k in (33, 1, 36):
+        sim.run(k)
+    out = sim.ir(), *sim.pressure(prev=True)
+    sim.close()
+    return out
+
+
+@pytest.mark.parametrize("shape,W,storage,sections,n_rcv,rounding", [
+    ((32, 32, 5), 1, capi.STORAGE_F32, 1, 4, 0),       # a plane is one block exactly
+    ((33, 31, 4), 2, capi.STORAGE_F32, 2, 4, 0),       # ... and a vector less or more
+    ((130, 17, 9), 3, capi.STORAGE_F32, 3, 300, 0),    # more probes than threads in a block
+    ((5, 4, 3), 1, capi.STORAGE_F32, 4, 4, 0),         # one inner plane
+    ((61, 50, 23), 8, capi.STORAGE_F32, 6, 4, 0),      # sections beyond the unrolled ones
+    ((61, 50, 23), 8, capi.STORAGE_BF16, 3, 4, 0),
+    ((70, 33, 19), 2, capi.STORAGE_F16, 1, 260, 0),
+    ((70, 33, 19), 2, capi.STORAGE_F16, 2, 4, 1),
+    ((37, 40, 12), 1, capi.STORAGE_BF16, 5, 4, 1),
+])
+def test_same_bits_as_three_launches(shape, W, storage, sections, n_rcv, rounding):
+    a = _sim(shape, W, 7, storage, sections, n_rcv, rounding)
+    b = _sim(shape, W, 7, storage, sections, n_rcv, rounding, tiling=(8, 0, 2))
+    assert np.abs(a[0]).max() > 0
+    for u, v in zip(a, b):
+        assert np.array_equal(u.view(np.uint32), v.view(np.uint32))

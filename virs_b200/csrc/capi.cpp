@@ -177,7 +177,9 @@ struct virs_sim {
     std::vector<uint64_t> rcv_ref;
     DevBuf ir;
     uint64_t ircap = 0;
-    DevBuf ctr;
+    DevBuf ctr;                    // two words: the step of buffer parity k reads word k and writes the next step's to the other
+    DevBuf probe;                  // sources and receivers for the one-launch step (kernels_fused.cu)
+    bool probe_ok = false;
     uint64_t steps_done = 0;
 
     // constants
@@ -188,6 +190,7 @@ struct virs_sim {
     // kernel variant: depth 0 = register-streaming kernel, 1..3 = TMA
     // kernel with that many planes in flight
     int tile_rows = 8, zc = 0, depth = 2;
+    bool tiling_set = false;       // by the caller or the autotuner
     CUtensorMap tmP[2], tmQ[2], tmC;
     DevBuf side;                   // {free, p, p^{n-1}} per boundary slot (TMA kernel -> boundary pass)
     int maps_rows = 0;             // tile rows the maps were built for (0 = none)
@@ -430,6 +433,7 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
     s->pair_nomem = false;
     // sources and receivers refer to voxel indices of the previous grid
     s->nsrc = s->nrcv = 0;
+    s->probe_ok = false;
     s->src_ref.clear();
     s->rcv_ref.clear();
     s->has_grid = true;
@@ -665,6 +669,42 @@ bool zero_masks_ready(const virs_sim *s)
     return s->depth > 0 && zero_masks_useful(s) && s->zm_rows == s->tile_rows && s->zm_zc == eff_planes(s);
 }
 
+// Single steps in one launch each (kernels_fused.cu) instead of stencil,
+// boundary pass and post kernel: on grids whose step is bound by latency.
+// Measured per step, three launches against one (sponge width 1 / 8):
+//   0.07 M voxels  FP32  9.2 / 9.2 against  3.4 / 3.7 us   BF16 9.9 / 10.0 against 3.7 / 3.6 us
+//   1.5 M               11.7 / 14.5          6.7 / 10.4         11.9 / 14.5          6.6 / 10.5
+//   7.8 M               28.6 / 55.4         24.7 / 48.5         25.6 / 48.8         22.1 / 47.0
+//   15.7 M              51.8 / 86.4         49.2 / 84.9         37.1 / 71.1         44.1 / 83.5
+// so the line lies at 16 M voxels in FP32 and 8 M in 16-bit storage.  A
+// tiling set by the caller names the stencil kernel; the stop rule and the
+// timing of the parts need the separate kernels.
+bool fused_on(const virs_sim *s)
+{
+    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 16u << 20 : 8u << 20;
+    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most;
+}
+
+// the probe list of the one-launch step: a probe on a border plane, which no
+// block covers and no step writes, goes to the first block
+virs_status build_probes(virs_sim *s)
+{
+    const uint32_t n = s->nsrc + s->nrcv, plane = s->px * s->ny;
+    std::vector<Probe> h(n);
+    for (uint32_t k = 0; k < n; ++k) {
+        const uint64_t d = to_dev(s, k < s->nsrc ? s->src_ref[k] : s->rcv_ref[k - s->nsrc]);
+        const uint32_t z = (uint32_t)(d / plane);
+        const bool in = z >= 1 && z + 1 < s->nz;
+        h[k] = {in ? z : 1u, in ? (uint32_t)(d % plane) : 0u, PROBE_NO_SLOT, (uint32_t)d};
+    }
+    VIRS_TRY(s->probe.alloc(std::max<uint32_t>(n, 1) * sizeof(Probe), "probes"));
+    if (n) VIRS_CUDA(copy_on(s->stream, s->probe.ptr, h.data(), n * sizeof(Probe), cudaMemcpyHostToDevice));
+    VIRS_CUDA(launch_probe_slots(s->probe.as<Probe>(), n, s->bpos.as<uint32_t>(), s->nb, s->stream));
+    s->probe_ok = true;
+    s->graph_dirty = true;
+    return VIRS_OK;
+}
+
 virs_status ready_to_run(virs_sim *s)
 {
     if (!s->has_grid) return fail(VIRS_E_STATE, "no grid: call virs_load_obj, virs_set_mesh or virs_set_grid");
@@ -674,8 +714,9 @@ virs_status ready_to_run(virs_sim *s)
         return fail(VIRS_E_ARG, "wall material " + std::to_string(s->max_wall_mat) + " has no filter (" +
                                     std::to_string(s->nmat) + " materials set)");
     if (!s->state.ptr) VIRS_TRY(alloc_states(s));
-    if (!s->ctr.ptr) VIRS_TRY(s->ctr.alloc(sizeof(uint32_t), "step counter"));
+    if (!s->ctr.ptr) VIRS_TRY(s->ctr.alloc(2 * sizeof(uint32_t), "step counter"));
     if (s->depth > 0 && s->maps_rows != s->tile_rows) VIRS_TRY(build_maps(s));
+    if (fused_on(s) && !s->probe_ok) VIRS_TRY(build_probes(s));
     if (s->depth > 0 && zero_masks_useful(s) && !zero_masks_ready(s)) {
         s->zm_rows = s->zm_zc = 0;
         VIRS_TRY(build_zero_masks(s, s->tile_rows, eff_planes(s), s->zmask));
@@ -713,7 +754,7 @@ StepArgs step_args(const virs_sim *s, int parity)
     a.state_out = nullptr;
     a.coef = s->coef.as<float>();
     a.hard = s->hard.as<float>();
-    a.ctr = s->ctr.as<uint32_t>();
+    a.ctr = s->ctr.as<uint32_t>() + parity;
     a.nb = s->nb;
     a.nhard = s->nhard;
     a.nsec = s->nsec;
@@ -746,7 +787,9 @@ PostArgs post_args(const virs_sim *s, int parity)
     a.sig = s->sig.as<float>();
     a.rcv = s->rcv.as<uint64_t>();
     a.ir = s->ir.as<float>();
-    a.ctr = s->ctr.as<uint32_t>();
+    a.ctr = s->ctr.as<uint32_t>() + parity;
+    a.ctr_out = s->ctr.as<uint32_t>() + (parity ^ 1);
+    a.probe = s->probe.as<Probe>();
     a.nsrc = s->nsrc;
     a.nrcv = s->nrcv;
     a.siglen = s->siglen;
@@ -783,6 +826,8 @@ cudaError_t launch_stencil_range(const virs_sim *s, int parity, cudaStream_t st,
 
 cudaError_t enqueue_step(const virs_sim *s, int parity, cudaStream_t st)
 {
+    if (fused_on(s))
+        return launch_fused(s->prm.storage, step_args(s, parity), post_args(s, parity), st);
     cudaError_t e = launch_stencil(s, parity, st);
     if (e != cudaSuccess) return e;
     e = launch_boundary(s->prm.storage, step_args(s, parity), BND_UPDATE, st);
@@ -897,18 +942,19 @@ StepArgs step_args_bufs(const virs_sim *s, int p, int q)
     return a;
 }
 
-PostArgs post_args_buf(const virs_sim *s, int q)
+PostArgs post_args_buf(const virs_sim *s, int q, int parity)
 {
-    PostArgs a = post_args(s, 0);
+    PostArgs a = post_args(s, parity);
     a.q = buf_ptr(s, q);
     return a;
 }
 
-// Two steps: p^n in buffer x, p^{n-1} in y; p^{n+1} to z, p^{n+2} to w.
+// Two steps from parity par: p^n in buffer x, p^{n-1} in y; p^{n+1} to z, p^{n+2} to w.
 // After k_pair_tma the first step is completed (boundary pass, post kernel);
 // then one launch runs the second step's boundary pass and recomputes its
 // provisional voxels, and the second post kernel follows.
-cudaError_t enqueue_pair(const virs_sim *s, int x, int y, int z, int w, cudaStream_t st, cudaEvent_t *ev = nullptr)
+cudaError_t enqueue_pair(const virs_sim *s, int par, int x, int y, int z, int w, cudaStream_t st,
+                         cudaEvent_t *ev = nullptr)
 {
     const int sto = s->prm.storage;
     StepArgs a = step_args_bufs(s, x, y);
@@ -920,12 +966,12 @@ cudaError_t enqueue_pair(const virs_sim *s, int x, int y, int z, int w, cudaStre
     if (ev) cudaEventRecord(ev[1], st);
     if (e == cudaSuccess) e = launch_boundary(sto, step_args_bufs(s, x, z), BND_UPDATE, st);
     if (ev) cudaEventRecord(ev[2], st);
-    if (e == cudaSuccess) e = launch_post(sto, post_args_buf(s, z), st);
+    if (e == cudaSuccess) e = launch_post(sto, post_args_buf(s, z, par), st);
     if (ev) cudaEventRecord(ev[3], st);
     if (e == cudaSuccess)
         e = launch_boundary_fix(sto, step_args_bufs(s, z, w), buf_ptr(s, x), s->plist.as<uint32_t>(), s->nplist, st);
     if (ev) cudaEventRecord(ev[4], st);
-    if (e == cudaSuccess) e = launch_post(sto, post_args_buf(s, w), st);
+    if (e == cudaSuccess) e = launch_post(sto, post_args_buf(s, w, par ^ 1), st);
     return e;
 }
 
@@ -933,8 +979,8 @@ cudaError_t enqueue_pair(const virs_sim *s, int x, int y, int z, int w, cudaStre
 // field[par] (p^n) and field[par ^ 1] (p^{n-1}) afterwards
 cudaError_t enqueue_quad(const virs_sim *s, int par, cudaStream_t st, cudaEvent_t *ev = nullptr)
 {
-    cudaError_t e = enqueue_pair(s, par, par ^ 1, 2 + (par ^ 1), 2 + par, st, ev);
-    if (e == cudaSuccess) e = enqueue_pair(s, 2 + par, 2 + (par ^ 1), par ^ 1, par, st, ev ? ev + 5 : nullptr);
+    cudaError_t e = enqueue_pair(s, par, par, par ^ 1, 2 + (par ^ 1), 2 + par, st, ev);
+    if (e == cudaSuccess) e = enqueue_pair(s, par, 2 + par, 2 + (par ^ 1), par ^ 1, par, st, ev ? ev + 5 : nullptr);
     return e;
 }
 
@@ -1454,6 +1500,7 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
     s->pm_rows = 0;
     s->pzm_zc = -1;
     s->pl_ok = false;
+    s->probe_ok = false;
     s->classified = true;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     return VIRS_OK;
@@ -1666,6 +1713,7 @@ VIRS_EXPORT virs_status virs_set_sources(virs_sim *s, uint32_t n, const uint64_t
     s->src_ref.assign(idx, idx + n);
     s->sig.release();
     s->pl_ok = false;
+    s->probe_ok = false;
     s->graph_dirty = true;
     ++s->gen;
     return VIRS_OK;
@@ -1688,6 +1736,7 @@ VIRS_EXPORT virs_status virs_set_receivers(virs_sim *s, uint32_t n, const uint64
     s->rcv_ref.assign(idx, idx + n);
     s->ir.release();
     s->ircap = 0;
+    s->probe_ok = false;
     s->graph_dirty = true;
     ++s->gen;
     return VIRS_OK;
@@ -1721,7 +1770,7 @@ VIRS_EXPORT virs_status virs_start_simulation(virs_sim *s, uint64_t steps)
     VIRS_CUDA(zero_on(s->stream, s->field[0].ptr, s->field[0].bytes));
     VIRS_CUDA(zero_on(s->stream, s->field[1].ptr, s->field[1].bytes));
     VIRS_CUDA(zero_on(s->stream, s->state.ptr, s->state.bytes));
-    VIRS_CUDA(zero_on(s->stream, s->ctr.ptr, 4));
+    VIRS_CUDA(zero_on(s->stream, s->ctr.ptr, s->ctr.bytes));
     if (s->stopbuf.ptr) VIRS_CUDA(zero_on(s->stream, s->stopbuf.ptr, s->stopbuf.bytes));
     s->stopped = false;
     s->slab_open = false;
@@ -2135,7 +2184,7 @@ VIRS_EXPORT virs_status virs_step(virs_sim *s, uint32_t step, int *keep_going, f
     VIRS_TRY(ensure_ir(s, (uint64_t)step + 1));
     cudaStream_t st = s->stream;
     // the reference uploads the source value every step (simulator_gpu.cu:250-258)
-    VIRS_CUDA(cudaMemcpyAsync(s->ctr.ptr, &step, 4, cudaMemcpyHostToDevice, st));
+    VIRS_CUDA(cudaMemcpyAsync(s->ctr.as<uint32_t>() + s->cur, &step, 4, cudaMemcpyHostToDevice, st));
     cudaError_t e = enqueue_step(s, s->cur, st);
     if (e != cudaSuccess) return cuda_fail(e, "step launch");
     s->cur ^= 1;
@@ -2392,6 +2441,7 @@ VIRS_EXPORT virs_status virs_set_tiling(virs_sim *s, int rows, int planes, int d
     s->tile_rows = rows ? rows : 8;
     s->zc = planes;
     s->depth = depth < 0 ? 2 : depth;
+    s->tiling_set = rows != 0 || planes != 0 || depth >= 0;
     s->maps_rows = 0;
     s->drop_graphs();
     return VIRS_OK;
@@ -2473,6 +2523,7 @@ struct TuneKey {
 struct TunePick {
     virs_tiling t{};
     int pair_steps = 1, pair_rows = 14, pair_zc = 0;
+    bool fused = false;            // single steps in one launch each
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, TunePick> g_tune;
@@ -2482,7 +2533,7 @@ virs_status reset_state(virs_sim *s)
     VIRS_CUDA(cudaMemsetAsync(s->field[0].ptr, 0, s->field[0].bytes, s->stream));
     VIRS_CUDA(cudaMemsetAsync(s->field[1].ptr, 0, s->field[1].bytes, s->stream));
     VIRS_CUDA(cudaMemsetAsync(s->state.ptr, 0, s->state.bytes, s->stream));
-    VIRS_CUDA(cudaMemsetAsync(s->ctr.ptr, 0, 4, s->stream));
+    VIRS_CUDA(cudaMemsetAsync(s->ctr.ptr, 0, s->ctr.bytes, s->stream));
     if (s->stopbuf.ptr) VIRS_CUDA(cudaMemsetAsync(s->stopbuf.ptr, 0, s->stopbuf.bytes, s->stream));
     s->stopped = false;
     if (s->ir.ptr) VIRS_CUDA(cudaMemsetAsync(s->ir.ptr, 0, s->ir.bytes, s->stream));
@@ -2530,7 +2581,7 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
         struct Cand {
             int d, r, pl;
         };
-        std::vector<Cand> sc;
+        std::vector<Cand> sc{{0, 0, 0}}; // the step as it runs without a tiling
         for (int d : {1, 2, 3})
             for (int r : {4, 8, 16})
                 for (int pl : {8, 16, 32, 64}) sc.push_back({d, r, pl});
@@ -2539,8 +2590,9 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
             const Cand &cd = sc[c < sc.size() ? c : 2 * sc.size() - 1 - c];
             const int d = cd.d, r = cd.r, pl = cd.pl;
             if (st != VIRS_OK) break;
-            s->tile_rows = r;
-            s->depth = d;
+            s->tiling_set = d > 0;
+            s->tile_rows = d > 0 ? r : 8;
+            s->depth = d > 0 ? d : 2;
             s->zc = pl;
             s->maps_rows = 0;
             if ((st = ready_to_run(s)) != VIRS_OK) break;
@@ -2563,7 +2615,8 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
             if ((st = check_err(s)) != VIRS_OK) break;
             if (ms / trial_steps < best_ms) {
                 best_ms = ms / trial_steps;
-                pick.t = {r, pl, d, ms / trial_steps};
+                pick.t = {s->tile_rows, pl, s->depth, ms / trial_steps};
+                pick.fused = d == 0;
             }
             if ((st = reset_state(s)) != VIRS_OK) break;
         }
@@ -2574,6 +2627,7 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
             s->tile_rows = pick.t.tile_rows;
             s->depth = pick.t.pipeline_depth;
             s->zc = pick.t.planes_per_block;
+            s->tiling_set = !pick.fused;
             s->maps_rows = 0;
             // Each candidate is timed twice, in forward and then reverse
             // order: a sustained load brings the GPU to its power cap within
@@ -2628,6 +2682,7 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
     s->tile_rows = pick.t.tile_rows;
     s->zc = pick.t.planes_per_block;
     s->depth = pick.t.pipeline_depth;
+    s->tiling_set = !pick.fused;
     s->maps_rows = 0;
     s->pair_steps = pick.pair_steps;
     s->pair_rows = pick.pair_rows;

@@ -113,13 +113,24 @@ struct StepArgs {
     double K, mix_y, mix_d, gain;
 };
 
+// a source or receiver voxel, for the kernel that does a whole step in one
+// launch (kernels_fused.cu): the block that writes the voxel handles it
+constexpr uint32_t PROBE_NO_SLOT = 0xffffffffu;
+struct Probe {
+    uint32_t z, off;        // plane, and offset in it, whose block owns the probe
+    uint32_t slot;          // the voxel's boundary slot, or PROBE_NO_SLOT
+    uint32_t pos;           // device position
+};
+
 struct PostArgs {
     void *q;                // p^{n+1}
     const uint64_t *src;    // device indices
     const float *sig;       // [nsrc][siglen] (scaled)
     const uint64_t *rcv;    // device indices
     float *ir;              // [nrcv][cap]
-    uint32_t *ctr;
+    const uint32_t *ctr;    // device step counter: read here,
+    uint32_t *ctr_out;      // ... and the next step's written here (the counter alternates between two words)
+    const Probe *probe;     // [nsrc] sources, then [nrcv] receivers
     uint32_t nsrc, nrcv;
     uint64_t siglen, cap;
     float inv_scale;
@@ -153,6 +164,9 @@ cudaError_t launch_post_batch(int storage, const BatchMember *mem, uint32_t nmem
 // kernel launchers (kernels_step.cu)
 cudaError_t launch_step(int storage, int tile_rows, const StepArgs &a, cudaStream_t s);
 cudaError_t launch_post(int storage, const PostArgs &a, cudaStream_t s);
+// a whole step in one launch (kernels_fused.cu)
+cudaError_t launch_fused(int storage, const StepArgs &a, const PostArgs &po, cudaStream_t s);
+cudaError_t launch_probe_slots(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, cudaStream_t s);
 // modes of the boundary pass (kernels_step.cu)
 enum { BND_UPDATE = 0, BND_KEEP = 1, BND_RECORD = 2 };
 cudaError_t launch_boundary(int storage, const StepArgs &a, int mode, cudaStream_t s);

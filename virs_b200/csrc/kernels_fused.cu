@@ -1,0 +1,282 @@
+// One launch per step for grids whose fields stay near the L2: the stencil,
+// the boundary pass and the sources and receivers together.
+//
+// On such grids a step of three launches (stencil, boundary pass, post) is
+// bound by latency: each kernel runs for a few microseconds, most of them
+// ramp-up, dependent loads and the gap to the next launch.  The three parts
+// do not need that order:
+//   * the boundary pass reads p^n, and p^{n-1} and the states of its own
+//     voxel, so it can run beside the stencil as long as the stencil stores
+//     nothing at boundary voxels (a vector that holds some is stored voxel
+//     by voxel);
+//   * a hard-source voxel takes its value in the stencil;
+//   * a soft source adds to, and a receiver reads, one voxel of p^{n+1}: the
+//     block that wrote it does that after its own barrier (the probe list
+//     says which block that is), so no grid-wide order is needed;
+//   * the step counter alternates between two words (step n reads word
+//     parity, writes the other), so no block has to be the last.
+// Blocks [0, gb) take 256 boundary slots each, the others 256 vectors of four
+// voxels of one plane.  The planes are walked as one row of
+// px * ny voxels: the y neighbours are px further on, no tile hangs over the
+// grid's edge, and what the row ends mix up are border voxels, whose result
+// is not kept.  Every load of a thread is independent of the others and
+// issued before any arithmetic: the latency is paid once.  One vector and
+// one plane per thread: two or four planes need 64 and 116 registers and
+// measured 5 to 60 % slower on rooms with a thick sponge layer (the boundary
+// slots share the kernel's occupancy).
+//
+// A 160x120x100 room with a sponge of 8 (0.64 M boundary slots): 17.4 us a
+// step in three launches, 10.6 us in this one; 48x40x36: 9.2 and 3.4 us.
+// From about eight million voxels on the fields come from HBM and the
+// kernels that stage planes ahead of their use win (fused_on in capi.cpp).
+//
+// Consecutive steps overlap at their ends (programmatic dependent launch):
+// a block loads what no step writes (codes, boundary positions, probes),
+// then waits for the previous step's grid.
+#include <type_traits>
+
+#include "step_voxel.cuh"
+
+namespace virs {
+namespace {
+
+using namespace step;
+
+constexpr int FB = 256;
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Four voxels of a row in one load: 16 bytes in FP32, 8 in 16-bit storage
+// (eight per thread would need 77 registers, too few warps for this kernel).
+constexpr int V = 4;
+template <typename T> struct Vec {
+    using Raw = std::conditional_t<sizeof(T) == 4, uint4, uint2>;
+    Raw v;
+    __device__ void load(const T *p) { v = *reinterpret_cast<const Raw *>(p); }
+    __device__ void zero() { v = Raw{}; }
+    __device__ void get(float (&r)[V]) const
+    {
+        const T *h = reinterpret_cast<const T *>(&v);
+#pragma unroll
+        for (int k = 0; k < V; ++k) r[k] = Io<T>::get(h[k]);
+    }
+};
+
+// rounded and stored; SR: stochastically, one hash per pair of voxels as in
+// st_sr (pos is a multiple of four, base is even)
+template <typename T, bool SR>
+__device__ __forceinline__ void put4(T *p, const float (&r)[V], uint64_t pos, uint64_t base, uint32_t key)
+{
+    typename Vec<T>::Raw raw;
+    T *h = reinterpret_cast<T *>(&raw);
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+        const uint32_t w = SR ? sr_word(pos + k, base, key) : 0u;
+        h[k] = SR ? Sr<T>::put(r[k], w & 0xffffu) : Io<T>::put(r[k]);
+        h[k + 1] = SR ? Sr<T>::put(r[k + 1], w >> 16) : Io<T>::put(r[k + 1]);
+    }
+    *reinterpret_cast<typename Vec<T>::Raw *>(p) = raw;
+}
+
+// which probes this block owns: those at boundary slots [lo, hi) (slots) or
+// those at offsets [lo, hi) of plane z
+struct Owned {
+    bool slots;
+    uint32_t lo, hi, z;
+    __device__ bool has(const Probe &p) const
+    {
+        return slots ? p.slot >= lo && p.slot < hi
+                     : p.slot == PROBE_NO_SLOT && p.z == z && p.off >= lo && p.off < hi;
+    }
+};
+
+__device__ __forceinline__ bool owns_any(const PostArgs &po, const Owned &o)
+{
+    bool mine = false;
+    const uint32_t n = po.nsrc + po.nrcv;
+    for (uint32_t k = threadIdx.x; k < n; k += FB) mine |= o.has(po.probe[k]);
+    return mine;
+}
+
+// sources and receivers at the voxels this block wrote, as post_body
+// (kernels_step.cu) does for all of them
+template <typename T> __device__ __forceinline__ void post_owned(const PostArgs &po, const Owned &o, bool mine)
+{
+    using IO = Io<T>;
+    if (!__syncthreads_or(mine)) return; // also: every store of this block is visible to it
+    T *Q = static_cast<T *>(po.q);
+    const uint32_t sn = *po.ctr;
+    const uint32_t k1 = po.sr ? sr_step_key(sn, 1u) : 0u;
+    for (uint32_t k = threadIdx.x; k < po.nsrc; k += FB) {
+        const Probe p = po.probe[k];
+        if (!o.has(p)) continue;
+        const float v = sn < po.siglen ? po.sig[(uint64_t)k * po.siglen + sn] : 0.f;
+        Q[p.pos] = put_rounded<T>(__fadd_rn(IO::get(Q[p.pos]), v), po.sr, p.pos, po.sr_base, k1);
+    }
+    __syncthreads();
+    if (sn >= po.cap) return;
+    for (uint32_t k = threadIdx.x; k < po.nrcv; k += FB) {
+        const Probe p = po.probe[po.nsrc + k];
+        if (o.has(p)) po.ir[(uint64_t)k * po.cap + sn] = __fmul_rn(IO::get(Q[p.pos]), po.inv_scale);
+    }
+}
+
+template <typename T, int MAXS, int MODE, bool SR>
+__device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &po, uint32_t blk, uint32_t gb, uint32_t gx)
+{
+    using IO = Io<T>;
+    const uint32_t tid = threadIdx.x;
+    if (blk < gb) {
+        const uint64_t s0 = (uint64_t)blk * FB + tid;
+        const Owned own{true, blk * FB, blk * FB + FB, 0u};
+        const bool mine = owns_any(po, own), act = s0 < a.nb;
+        BVox<T, MAXS> v;
+        if (act) bvox_site<T, MODE, MAXS>(a, s0, v);
+        pdl_wait();
+        if (act) {
+            bvox_values<T, MODE, MAXS>(a, s0, v);
+            bvox_update<T, MODE, MAXS>(a, s0, v);
+        }
+        if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
+        post_owned<T>(po, own, mine);
+        return;
+    }
+    const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
+    const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
+    const bool act = first + tid * V < plane;
+    const Owned own{false, first, first + FB * V, z};
+    const bool mine = owns_any(po, own);
+    // the last block of a plane repeats the plane's last vector, unstored
+    const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
+    Codes<V> code;
+    code.load(a.code + i);
+    pdl_wait();
+    if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
+
+    const T *P = static_cast<const T *>(a.p);
+    T *Q = static_cast<T *>(a.q);
+    Vec<T> c, zp, zm, yp, ym, q;
+    c.load(P + i);
+    zm.load(P + (i - plane));
+    zp.load(P + (i + plane));
+    ym.load(P + (i - a.px));
+    yp.load(P + (i + a.px));
+    q.load(Q + i);
+    const float left = IO::ld1(P + (i - 1u)), right = IO::ld1(P + (i + V));
+    const float2 c2dt2 = make_float2(a.c2dt2, a.c2dt2), inv_h2 = make_float2(a.inv_h2, a.inv_h2);
+    float fc[V], fzp[V], fzm[V], fyp[V], fym[V], fq[V], r[V];
+    c.get(fc);
+    zm.get(fzm);
+    zp.get(fzp);
+    ym.get(fym);
+    yp.get(fyp);
+    q.get(fq);
+    air_update(fc, left, right, fyp, fym, fzp, fzm, fq, c2dt2, inv_h2, r);
+    if (act) {
+        const uint32_t srk = SR ? sr_step_key(*po.ctr, 0u) : 0u;
+        if (!code.any()) {
+            put4<T, SR>(Q + i, r, i, a.sr_base, srk);
+        } else {
+            // voxel by voxel: border voxels keep their value, boundary
+            // voxels belong to the blocks of their slots; only air next to a
+            // wall outside a boundary layer takes the mirror rule
+            if (code.mirror()) {
+#pragma unroll
+                for (int j = 0; j < V; ++j)
+                    if (code.get(j) != 0u && code.get(j) < CODE_BND)
+                        r[j] = leapfrog((uint8_t)code.get(j), fc[j], j == V - 1 ? right : fc[j + 1],
+                                        j == 0 ? left : fc[j - 1], fyp[j], fym[j], fzp[j], fzm[j], fq[j], a.c2dt2,
+                                        a.inv_h2);
+            }
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const uint32_t cj = code.get(j);
+                if (cj == CODE_NONE || (cj & 0xC0u) == CODE_BND) continue;
+                float v = r[j];
+                if (cj == CODE_WALL) v = 0.f;
+                else if (cj == CODE_HARD) {
+                    const uint32_t sn = *po.ctr;
+                    v = sn < a.nhard ? a.hard[sn] : 0.f;
+                }
+                Q[i + j] = SR ? Sr<T>::put(v, sr_bits((uint64_t)i + j, a.sr_base, srk)) : IO::put(v);
+            }
+        }
+    }
+    post_owned<T>(po, own, mine);
+}
+
+template <typename T, int MAXS, int MODE, bool SR>
+__global__ void __launch_bounds__(FB) k_fused(const __grid_constant__ StepArgs a, const __grid_constant__ PostArgs po,
+                                              uint32_t gb, uint32_t gx)
+{
+    pdl_trigger();
+    fused_block<T, MAXS, MODE, SR>(a, po, blockIdx.x, gb, gx);
+}
+
+// the slot of each probe's voxel in the boundary list (ascending positions)
+__global__ void k_probe_slots(Probe *probe, uint32_t n, const uint32_t *__restrict bpos, uint64_t nb)
+{
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uint32_t pos = probe[k].pos;
+    uint64_t lo = 0, hi = nb;
+    while (lo < hi) {
+        const uint64_t mid = (lo + hi) / 2;
+        if (bpos[mid] < pos) lo = mid + 1;
+        else hi = mid;
+    }
+    probe[k].slot = lo < nb && bpos[lo] == pos ? (uint32_t)lo : PROBE_NO_SLOT;
+}
+
+template <typename K, typename... A> cudaError_t launch_pdl(K kern, unsigned grid, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(FB);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <typename T, int MODE, bool SR>
+cudaError_t fused_by_sections(const StepArgs &a, const PostArgs &po, cudaStream_t s)
+{
+    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB);
+    const uint32_t gx = (a.px * a.ny + FB * V - 1) / (FB * V);
+    const unsigned grid = gb + gx * (a.nz - 2);
+    if (a.nsec <= 1) return launch_pdl(k_fused<T, 1, MODE, SR>, grid, s, a, po, gb, gx);
+    if (a.nsec == 2) return launch_pdl(k_fused<T, 2, MODE, SR>, grid, s, a, po, gb, gx);
+    if (a.nsec <= 4) return launch_pdl(k_fused<T, 4, MODE, SR>, grid, s, a, po, gb, gx);
+    return launch_pdl(k_fused<T, 0, MODE, SR>, grid, s, a, po, gb, gx);
+}
+
+template <typename T> cudaError_t fused_16(const StepArgs &a, const PostArgs &po, cudaStream_t s)
+{
+    if (a.sr) return fused_by_sections<T, BND_UPDATE, true>(a, po, s);
+    return fused_by_sections<T, BND_UPDATE, false>(a, po, s);
+}
+
+} // namespace
+
+cudaError_t launch_fused(int storage, const StepArgs &a, const PostArgs &po, cudaStream_t s)
+{
+    switch (storage) {
+    case VIRS_STORAGE_F16: return fused_16<__half>(a, po, s);
+    case VIRS_STORAGE_BF16: return fused_16<__nv_bfloat16>(a, po, s);
+    default: return fused_by_sections<float, BND_UPDATE, false>(a, po, s);
+    }
+}
+
+cudaError_t launch_probe_slots(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    k_probe_slots<<<(n + 127) / 128, 128, 0, s>>>(probe, n, bpos, nb);
+    return cudaGetLastError();
+}
+
+} // namespace virs

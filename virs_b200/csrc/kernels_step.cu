@@ -28,7 +28,7 @@
 // bit-identical to the CPU oracle: the reference CUDA build contracts
 // s - 6*p and t + c2dt2*lap into fused multiply-adds and flushes subnormals
 // (--use_fast_math); this file is compiled with -ftz=true.
-#include "step_common.cuh"
+#include "step_voxel.cuh"
 
 namespace virs {
 namespace {
@@ -172,59 +172,6 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_step(const __grid
 //               slot kept in a.side (the adjoint's recomputation)
 //   BND_RECORD  the record only: no filters, nothing written to the fields
 //               (the adjoint step, on adjoint fields)
-// The loads of one boundary voxel (first part) and its update (second).
-template <typename T, int MAXS> struct BVox {
-    size_t i;
-    uint8_t c, nm;
-    float ce, qv, nb[6];
-    BState<MAXS> st;
-};
-
-template <typename T, int MODE, int MAXS>
-__device__ __forceinline__ void bvox_load(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
-{
-    using IO = Io<T>;
-    const size_t i = __ldg(a.bpos + slot);
-    const size_t sy = a.px, sz = (size_t)a.px * a.ny;
-    const T *P = static_cast<const T *>(a.p);
-    const T *Q = static_cast<const T *>(a.q);
-    v.i = i;
-    v.c = __ldg(a.bcode + slot);
-    v.nm = a.rigid ? __ldg(a.bnrm + slot) : 0;
-    v.ce = IO::get(P[i]);
-    v.qv = IO::get(Q[i]);
-    v.nb[0] = IO::get(P[i + 1]);
-    v.nb[1] = IO::get(P[i - 1]);
-    v.nb[2] = IO::get(P[i + sy]);
-    v.nb[3] = IO::get(P[i - sy]);
-    v.nb[4] = IO::get(P[i + sz]);
-    v.nb[5] = IO::get(P[i - sz]);
-    if (MODE != BND_RECORD && MAXS > 0) bload<MAXS>(a, slot, v.st);
-}
-
-template <typename T, int MODE, int MAXS>
-__device__ __forceinline__ void bvox_update(const StepArgs &a, uint64_t slot, const BVox<T, MAXS> &v)
-{
-    float r;
-    if (a.rigid) {
-        // fdtd_kernel_rigid_walls (simulator_gpu.cu:152-180): the air
-        // neighbours only (normals mask), p+ = (2 - l2 n) p - p- + the sum
-        // of (l2 * s) * p_nb over +x, -x, +y, -y, +z, -z with s = 1 for air;
-        // with the reference build's contractions
-        const float b1 = __fmaf_rn(-a.l2, (float)__popc(v.nm), 2.f);
-        r = __fmaf_rn(b1, v.ce, -v.qv);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) r = __fmaf_rn(__fmul_rn(a.l2, (v.nm & (1u << k)) ? 1.f : 0.f), v.nb[k], r);
-    } else {
-        r = leapfrog(v.c, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5], v.qv, a.c2dt2, a.inv_h2);
-    }
-    if (MODE != BND_UPDATE) a.side[slot] = make_float4(r, v.ce, v.qv, 0.f);
-    if (MODE == BND_RECORD) return;
-    r = MAXS > 0 ? bcompute<MAXS>(a, r, v.ce, v.qv, slot, v.st) : boundary_loop(a, r, v.ce, v.qv, slot);
-    static_cast<T *>(a.q)[v.i] =
-        put_rounded<T>(r, a.sr, v.i, a.sr_base, a.sr ? sr_step_key(*a.ctr, 0u) : 0u);
-}
-
 // The compacted boundary pass (simulator_gpu.cu:105-150), in list order.
 // The stencil kernels left these voxels untouched (p^{n-1} in place); the
 // pass gathers the seven p values from the p^n buffer (not written during
@@ -423,7 +370,7 @@ template <typename T> __device__ __forceinline__ void post_body(const PostArgs &
     __syncthreads();
     if (threadIdx.x == 0) {
         if (a.stop && a.nrcv && sn < a.cap) stop_rule(a, sn);
-        *a.ctr = sn + 1;
+        *a.ctr_out = sn + 1;
     }
 }
 

@@ -37,14 +37,13 @@
 
 #include <algorithm>
 
-#include "step_common.cuh"
+#include "step_voxel.cuh"
 
 namespace virs {
 namespace {
 
 using namespace step;
 
-constexpr unsigned FULL = 0xffffffffu;
 constexpr int TX = 128;
 // A waiting thread asks to be parked for up to WAIT_HINT_NS per try (it
 // resumes as soon as the stage's phase completes), so the waiting warp does
@@ -112,83 +111,6 @@ template <typename T, int TY> struct Stage {
     static constexpr uint32_t CBa = (CB + 127u) & ~127u;
     static constexpr uint32_t SB = PBa + QBa + CBa;
 };
-
-// the V cell codes of a thread (4 or 8 bytes)
-template <int V> struct Codes;
-// bytes with bit 7 clear and some other bit set: bit 7 of each byte of
-// ((w & 0x7f..) + 0x7f..) & ~w
-__device__ __forceinline__ uint32_t mirror_bytes(uint32_t w)
-{
-    return ((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) & ~w & 0x80808080u;
-}
-template <> struct Codes<4> {
-    uint32_t w;
-    __device__ void load(const unsigned char *p) { w = *reinterpret_cast<const uint32_t *>(p); }
-    __device__ void clear() { w = 0u; }
-    __device__ bool any() const { return w != 0u; }
-    __device__ uint32_t get(int k) const { return (w >> (8 * k)) & 0xffu; }
-    __device__ uint32_t mirror() const { return mirror_bytes(w); }
-    __device__ bool is_mirror(uint32_t m, int k) const { return (m >> (8 * k + 7)) & 1u; }
-};
-template <> struct Codes<8> {
-    uint2 w;
-    __device__ void load(const unsigned char *p) { w = *reinterpret_cast<const uint2 *>(p); }
-    __device__ void clear() { w = make_uint2(0u, 0u); }
-    __device__ bool any() const { return (w.x | w.y) != 0u; }
-    __device__ uint32_t get(int k) const { return ((k < 4 ? w.x : w.y) >> (8 * (k & 3))) & 0xffu; }
-    // the mirror bytes of the two words folded into one: bit 7 of byte k
-    // (k < 4) from w.x, bit 6 of byte k - 4 from w.y
-    __device__ uint32_t mirror() const { return mirror_bytes(w.x) | (mirror_bytes(w.y) >> 1); }
-    __device__ bool is_mirror(uint32_t m, int k) const { return (m >> (8 * (k & 3) + (k < 4 ? 7 : 6))) & 1u; }
-};
-
-// The update of one thread's V voxels of a plane: cc holds the centres,
-// left / right the x neighbours beyond the vector, ym / yp / zm / zp the y
-// and z neighbours, qv p^{n-1}.
-template <typename T>
-__device__ __forceinline__ void tile_update(const Codes<Lay<T>::V> &code, const float (&cc)[Lay<T>::V], float left,
-                                        float right, const float (&yp)[Lay<T>::V], const float (&ym)[Lay<T>::V],
-                                        const float (&zp)[Lay<T>::V], const float (&zm)[Lay<T>::V],
-                                        const float (&qv)[Lay<T>::V], float2 c2dt2, float2 inv_h2, float c2dt2s,
-                                        float inv_h2s, float (&r)[Lay<T>::V])
-{
-    constexpr int V = Lay<T>::V;
-    // every voxel as air without wall neighbours, the common case, two
-    // at a time ...
-#pragma unroll
-    for (int k = 0; k < V; k += 2) {
-        const float2 x2 = make_float2(__fadd_rn(cc[k + 1], k > 0 ? cc[k - 1] : left),
-                                      __fadd_rn(k + 2 < V ? cc[k + 2] : right, cc[k]));
-        const float2 o = leapfrog_air2(make_float2(cc[k], cc[k + 1]), x2, make_float2(yp[k], yp[k + 1]),
-                                       make_float2(ym[k], ym[k + 1]), make_float2(zp[k], zp[k + 1]),
-                                       make_float2(zm[k], zm[k + 1]), make_float2(qv[k], qv[k + 1]), c2dt2, inv_h2);
-        r[k] = o.x;
-        r[k + 1] = o.y;
-    }
-    // ... then the voxels with another code.  Walls take 0; border,
-    // hard-source and boundary voxels keep p^{n-1} (the post kernel
-    // writes the hard-source value, the boundary pass updates boundary
-    // voxels from the untouched p^n buffer): a test and a select per
-    // voxel, no divergence.  Only air next to a wall outside the
-    // boundary layer (a grid without a sponge layer) needs the update
-    // with the mirror rule; such codes have bit 7 clear and other bits
-    // set, found for four bytes at once.
-    if (__any_sync(FULL, code.any())) {
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            const uint32_t c = code.get(k);
-            if (c & CODE_BND) r[k] = c == CODE_WALL ? 0.f : qv[k];
-        }
-        const uint32_t mirror = code.mirror();
-        if (__any_sync(FULL, mirror != 0u)) {
-#pragma unroll
-            for (int k = 0; k < V; ++k)
-                if (code.is_mirror(mirror, k))
-                    r[k] = leapfrog((uint8_t)code.get(k), cc[k], k == V - 1 ? right : cc[k + 1],
-                                    k == 0 ? left : cc[k - 1], yp[k], ym[k], zp[k], zm[k], qv[k], c2dt2s, inv_h2s);
-        }
-    }
-}
 
 // waits for phase `parity` of *b for at most limit_ns; on timeout sets *err
 __device__ __forceinline__ bool bounded_wait(uint64_t *b, uint32_t parity, uint64_t limit_ns, int *err)
@@ -585,11 +507,7 @@ __device__ __forceinline__ void put_vec(float *p, const float (&r)[4])
 }
 template <typename H> __device__ __forceinline__ void put_vec(H *p, const float (&r)[8])
 {
-    uint4 v;
-    H *h = reinterpret_cast<H *>(&v);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) h[k] = Io<H>::put(r[k]);
-    *reinterpret_cast<uint4 *>(p) = v;
+    *reinterpret_cast<uint4 *>(p) = Io<H>::pack(r);
 }
 
 template <typename T, int TY, int L> struct PairTile {
