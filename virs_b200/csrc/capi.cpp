@@ -153,13 +153,14 @@ struct virs_sim {
 
     // boundary
     uint64_t nb = 0;
-    DevBuf bidx, bpos, bcode, bnrm, bmat, bw, state;
+    DevBuf bidx, bpos, bmeta, bnrm, bmat, bw, state;
+    DevBuf wtab;                   // BndWeight per squared distance to the wall
     DevBuf hpos;                   // hard-source voxel positions
     uint32_t nhpos = 0;
 
     // filters
     uint32_t nmat = 0, nsec = 0;
-    DevBuf coef;
+    DevBuf coef, coefp;            // [M][S][5], and each material's padded to 16-byte vectors
     bool filters_set = false;
 
     // sources / receivers
@@ -314,6 +315,19 @@ virs_status upload_hard(virs_sim *s)
     return VIRS_OK;
 }
 
+// the coefficients of s->nmat materials of s->nsec sections, in both layouts
+virs_status upload_filters(virs_sim *s, const float *k)
+{
+    const size_t per = (size_t)s->nsec * 5, pad = (per + 3) / 4 * 4;
+    std::vector<float> p(s->nmat * pad, 0.f);
+    for (size_t m = 0; m < s->nmat; ++m) std::copy_n(k + m * per, per, p.begin() + (ptrdiff_t)(m * pad));
+    VIRS_TRY(s->coef.alloc(s->nmat * per * sizeof(float), "filter coefficients"));
+    VIRS_TRY(s->coefp.alloc(p.size() * sizeof(float), "filter coefficients"));
+    VIRS_CUDA(copy_on(s->stream, s->coef.ptr, k, s->nmat * per * sizeof(float), cudaMemcpyHostToDevice));
+    VIRS_CUDA(copy_on(s->stream, s->coefp.ptr, p.data(), p.size() * sizeof(float), cudaMemcpyHostToDevice));
+    return VIRS_OK;
+}
+
 // reference default filter: RBJ high-pass 440 Hz, Q 0.1 at fs = 1/dt
 // (simulator.cpp:955-967)
 virs_status default_filters(virs_sim *s)
@@ -322,9 +336,28 @@ virs_status default_filters(virs_sim *s)
     rbj_highpass((float)s->fs, 440.f, 0.1f, 1.f, k);
     s->nmat = 1;
     s->nsec = 1;
-    VIRS_TRY(s->coef.alloc(5 * sizeof(float), "filter coefficients"));
-    VIRS_CUDA(copy_on(s->stream, s->coef.ptr, k, sizeof(k), cudaMemcpyHostToDevice));
+    VIRS_TRY(upload_filters(s, k));
     s->filters_set = true;
+    return VIRS_OK;
+}
+
+// the boundary correction's constants per sponge weight, with the kernel's
+// operations in their order (double, no contraction)
+virs_status build_weights(virs_sim *s, const std::vector<float> &w)
+{
+    std::vector<BndWeight> t(w.size());
+    const double K = (double)s->K, gain = (double)s->prm.boundary_gain;
+    for (size_t d = 0; d < w.size(); ++d) {
+        if (s->prm.boundary_form == VIRS_BOUNDARY_REFERENCE) {
+            t[d] = {(double)w[d], 0.0, 1.0, 1.0};
+            continue;
+        }
+        const double kgw = K * gain * (double)w[d];
+        const double ac = kgw * s->prm.mix_direct * 0.5;
+        t[d] = {kgw, ac, 1.0 + ac, 1.0 / (1.0 + ac)};
+    }
+    VIRS_TRY(s->wtab.alloc(t.size() * sizeof(BndWeight), "boundary weights"));
+    VIRS_CUDA(copy_on(s->stream, s->wtab.ptr, t.data(), t.size() * sizeof(BndWeight), cudaMemcpyHostToDevice));
     return VIRS_OK;
 }
 
@@ -411,7 +444,7 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
     compute_constants(s);
     // release the old grid first so that peak memory stays at one grid
     for (DevBuf *b : {&s->flags_raw, &s->wall_mat, &s->flags, &s->code, &s->normals, &s->bseg, &s->segnz, &s->field[0],
-                      &s->field[1], &s->bidx, &s->bpos, &s->bcode, &s->bnrm, &s->bmat, &s->bw, &s->state, &s->side, &s->hpos,
+                      &s->field[1], &s->bidx, &s->bpos, &s->bmeta, &s->bnrm, &s->bmat, &s->bw, &s->state, &s->side, &s->hpos,
                       &s->spare[0], &s->spare[1], &s->plist, &s->pzmask})
         b->release();
     const size_t ext = (size_t)s->px * ny * s->ext_nz;
@@ -746,13 +779,13 @@ StepArgs step_args(const virs_sim *s, int parity)
     a.l2 = s->l2;
     a.rigid = s->prm.rigid_walls ? 1 : 0;
     if (s->stop_rule) a.stop = s->stopbuf.as<uint32_t>();
-    a.bmat = s->bmat.as<uint8_t>();
-    a.bcode = s->bcode.as<uint8_t>();
+    a.bmeta = s->bmeta.as<uint32_t>();
+    a.wtab = s->wtab.as<BndWeight>();
     a.bnrm = s->bnrm.as<uint8_t>();
-    a.bw = s->bw.as<float>();
     a.state = s->state.as<float>();
     a.state_out = nullptr;
     a.coef = s->coef.as<float>();
+    a.coefp = s->coefp.as<float>();
     a.hard = s->hard.as<float>();
     a.ctr = s->ctr.as<uint32_t>() + parity;
     a.nb = s->nb;
@@ -1461,12 +1494,13 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
 
         std::vector<float> wt((size_t)W * W + 1);
         for (int d = 0; d <= W * W; ++d) wt[d] = sponge_weight(W, d);
+        VIRS_TRY(build_weights(s, wt));
         VIRS_TRY(wtab.alloc(wt.size() * 4, "sponge weights"));
         VIRS_CUDA(copy_on(s->stream, wtab.ptr, wt.data(), wt.size() * 4, cudaMemcpyHostToDevice));
         VIRS_TRY(s->bidx.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary indices"));
         VIRS_TRY(s->bpos.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary positions"));
         VIRS_TRY(s->bmat.alloc(std::max<uint64_t>(nb, 1), "boundary materials"));
-        VIRS_TRY(s->bcode.alloc(std::max<uint64_t>(nb, 1), "boundary codes"));
+        VIRS_TRY(s->bmeta.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary codes"));
         VIRS_TRY(s->bnrm.alloc(std::max<uint64_t>(nb, 1), "boundary normals"));
         VIRS_TRY(s->bw.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary weights"));
         VIRS_TRY(s->side.alloc(std::max<uint64_t>(nb, 1) * sizeof(float4), "boundary records"));
@@ -1481,7 +1515,7 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         cp.bmat = s->bmat.as<uint8_t>();
         cp.code = s->code.as<uint8_t>();
         cp.normals = s->normals.as<uint8_t>();
-        cp.bcode = s->bcode.as<uint8_t>();
+        cp.bmeta = s->bmeta.as<uint32_t>();
         cp.bnrm = s->bnrm.as<uint8_t>();
         cp.bw = s->bw.as<float>();
         cp.nx = s->nx;
@@ -1569,10 +1603,9 @@ VIRS_EXPORT virs_status virs_set_filters(virs_sim *s, uint32_t nm, uint32_t ns, 
         if (!std::isfinite(coeffs[i])) return fail(VIRS_E_ARG, "non-finite filter coefficient");
     VIRS_TRY(use_device(s));
     VIRS_TRY(wait_done(s));
-    VIRS_TRY(s->coef.alloc((size_t)nm * ns * 5 * 4, "filter coefficients"));
-    VIRS_CUDA(copy_on(s->stream, s->coef.ptr, coeffs, (size_t)nm * ns * 5 * 4, cudaMemcpyHostToDevice));
     s->nmat = nm;
     s->nsec = ns;
+    VIRS_TRY(upload_filters(s, coeffs));
     s->filters_set = true;
     s->graph_dirty = true;
     ++s->gen;
@@ -2750,7 +2783,7 @@ struct virs_batch {
     int dev = 0, storage = 0, rows = 8, depth = 2, planes = 0;
     bool persistent = false;
     uint64_t ntiles = 0, nbnd = 0;
-    uint32_t max_sections = 0;
+    int sections = 0;              // launch_boundary_batch
     DevBuf desc, err;
     // each member's zero-code masks for the batch's tiling
     std::deque<DevBuf> zmasks;
@@ -2796,7 +2829,7 @@ virs_status batch_build(virs_batch *b)
     b->zmasks.clear();
     std::vector<BatchMember> h(b->mem.size());
     uint64_t tiles = 0, bnd = 0;
-    b->max_sections = 0;
+    uint32_t min_sections = UINT32_MAX, max_sections = 0;
     const CUtensorMapDataType dt = b->storage == VIRS_STORAGE_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : b->storage == VIRS_STORAGE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                     : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -2834,13 +2867,15 @@ virs_status batch_build(virs_batch *b)
         m.first_bnd = bnd;
         tiles += (uint64_t)m.gx * m.gy * m.gz;
         bnd += s->nb;
-        b->max_sections = std::max(b->max_sections, s->nsec);
+        min_sections = std::min(min_sections, s->nsec);
+        max_sections = std::max(max_sections, s->nsec);
         b->gen[i] = s->gen;
     }
     VIRS_TRY(b->desc.alloc(h.size() * sizeof(BatchMember), "batch descriptors"));
     VIRS_CUDA(copy_on(b->stream, b->desc.ptr, h.data(), h.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
     b->ntiles = tiles;
     b->nbnd = bnd;
+    b->sections = max_sections > 4 ? 0 : min_sections == max_sections ? (int)max_sections : -4;
     return VIRS_OK;
 }
 
@@ -2852,7 +2887,7 @@ cudaError_t batch_enqueue(const virs_batch *b, int parity, cudaStream_t st)
         launch_step_tma_batch(b->storage, b->rows, b->depth, d, n, b->ntiles, parity, b->persistent, b->err.as<int>(), st,
                               sr_on(b->mem[0]));
     if (e != cudaSuccess) return e;
-    e = launch_boundary_batch(b->storage, d, n, b->nbnd, parity, b->max_sections, st);
+    e = launch_boundary_batch(b->storage, d, n, b->nbnd, parity, b->sections, st);
     if (e != cudaSuccess) return e;
     return launch_post_batch(b->storage, d, n, parity, st);
 }

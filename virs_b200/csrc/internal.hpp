@@ -80,6 +80,13 @@ constexpr int SEG = 128;              // voxels per boundary-prefix segment
 
 // ---- kernel argument blocks -------------------------------------------------
 
+// what the boundary correction needs of a sponge weight w: in the centered
+// form kgw = K gain w, a = kgw mix_d / 2, 1 + a and its reciprocal; in the
+// reference form w in the first member
+struct alignas(16) BndWeight {
+    double kgw, ac, den, rden;
+};
+
 struct StepArgs {
     float4 *side;           // per boundary slot {free, p, p^{n-1}, 0}, kept by the boundary pass for the adjoint
     const uint32_t *stop;   // nonzero *stop: the RMS stop rule has fired, the step does nothing (nullptr: off)
@@ -89,13 +96,13 @@ struct StepArgs {
     const uint8_t *code;
     const uint8_t *normals; // air-neighbour mask (rigid-wall update)
     const uint32_t *bpos;   // [nb] padded device index of each boundary slot
-    const uint8_t *bcode;   // [nb] cell code of each slot's voxel (read in slot order, not gathered)
+    const uint32_t *bmeta;  // [nb] per slot: cell code | material << 8 | squared wall distance << 16 (the entry of wtab)
+    const BndWeight *wtab;  // per squared distance to the wall
     const uint8_t *bnrm;    // [nb] air-neighbour mask of each slot's voxel (rigid-wall update)
-    const uint8_t *bmat;
-    const float *bw;
     float *state;           // X_q[n-1], X_q[n-2] of the cascade's input and section outputs (state_index)
     float *state_out;       // where the pass writes the states after the step (nullptr: in place, `state`)
     const float *coef;      // [M][S][5]
+    const float *coefp;     // the same, each material's 5 S values padded to 16-byte vectors
     const float *hard;      // per-step hard source values (scaled)
     const uint32_t *ctr;    // device step counter
     uint64_t nb;
@@ -157,8 +164,10 @@ struct alignas(64) BatchMember {
 };
 cudaError_t launch_step_tma_batch(int storage, int tile_rows, int depth, const BatchMember *mem, uint32_t nmem,
                                   uint64_t ntiles, int parity, bool persistent, int *err, cudaStream_t s, bool sr);
+// sections: every member's number of sections (1..4), -4 when they differ
+// but none has more than 4, 0 otherwise
 cudaError_t launch_boundary_batch(int storage, const BatchMember *mem, uint32_t nmem, uint64_t nbnd, int parity,
-                                  uint32_t max_sections, cudaStream_t s);
+                                  int sections, cudaStream_t s);
 cudaError_t launch_post_batch(int storage, const BatchMember *mem, uint32_t nmem, int parity, cudaStream_t s);
 
 // kernel launchers (kernels_step.cu)
@@ -246,7 +255,8 @@ struct CompactArgs {
     uint32_t *bpos;            // padded device index of each slot's voxel
     const uint8_t *code;       // padded cell codes and air-neighbour masks
     const uint8_t *normals;
-    uint8_t *bcode, *bnrm;     // ... copied per slot
+    uint8_t *bnrm;             // ... copied per slot, the code in
+    uint32_t *bmeta;           // code | material << 8 | squared distance << 16
     uint8_t *bmat;
     float *bw;
     uint32_t nx, ny, nz, px, spr;

@@ -177,7 +177,7 @@ __global__ void k_compact(const CompactArgs a)
     const uint64_t slot = (uint64_t)a.bseg[((size_t)z * ny + y) * a.spr + blockIdx.x] + before;
     a.bidx[slot] = (uint32_t)(((uint64_t)z * ny + y) * nx + x);
     a.bpos[slot] = (uint32_t)i;
-    a.bcode[slot] = a.code[i];
+    a.bmeta[slot] = (uint32_t)a.code[i] | (uint32_t)a.bmat_full[i] << 8 | (uint32_t)a.bd2_full[i] << 16;
     a.bnrm[slot] = a.normals[i];
     a.bmat[slot] = a.bmat_full[i];
     a.bw[slot] = a.wtab[a.bd2_full[i]];

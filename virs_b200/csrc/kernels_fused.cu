@@ -251,7 +251,8 @@ cudaError_t fused_by_sections(const StepArgs &a, const PostArgs &po, cudaStream_
     const unsigned grid = gb + gx * (a.nz - 2);
     if (a.nsec <= 1) return launch_pdl(k_fused<T, 1, MODE, SR>, grid, s, a, po, gb, gx);
     if (a.nsec == 2) return launch_pdl(k_fused<T, 2, MODE, SR>, grid, s, a, po, gb, gx);
-    if (a.nsec <= 4) return launch_pdl(k_fused<T, 4, MODE, SR>, grid, s, a, po, gb, gx);
+    if (a.nsec == 3) return launch_pdl(k_fused<T, 3, MODE, SR>, grid, s, a, po, gb, gx);
+    if (a.nsec == 4) return launch_pdl(k_fused<T, 4, MODE, SR>, grid, s, a, po, gb, gx);
     return launch_pdl(k_fused<T, 0, MODE, SR>, grid, s, a, po, gb, gx);
 }
 

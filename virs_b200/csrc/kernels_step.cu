@@ -424,7 +424,8 @@ void boundary_by_sections(uint32_t ns, unsigned g, const StepArgs &a, cudaStream
 {
     if (MODE == BND_RECORD || ns <= 1) k_boundary<T, MODE, 1><<<g, BT, 0, s>>>(a);
     else if (ns == 2) k_boundary<T, MODE, 2><<<g, BT, 0, s>>>(a);
-    else if (ns <= 4) k_boundary<T, MODE, 4><<<g, BT, 0, s>>>(a);
+    else if (ns == 3) k_boundary<T, MODE, 3><<<g, BT, 0, s>>>(a);
+    else if (ns == 4) k_boundary<T, MODE, 4><<<g, BT, 0, s>>>(a);
     else k_boundary<T, MODE, 0><<<g, BT, 0, s>>>(a);
 }
 
@@ -438,11 +439,17 @@ template <typename T> void boundary_by_mode(int mode, uint32_t ns, unsigned g, c
 }
 
 template <typename T>
-void boundary_batch_by_sections(uint32_t maxs, unsigned g, const BatchMember *mem, uint32_t nmem, uint64_t nbnd,
+void boundary_batch_by_sections(int sections, unsigned g, const BatchMember *mem, uint32_t nmem, uint64_t nbnd,
                                 int parity, cudaStream_t s)
 {
-    if (maxs <= 4) k_boundary_batch<T, 4><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity);
-    else k_boundary_batch<T, 0><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity);
+    switch (sections) {
+    case 1: k_boundary_batch<T, 1><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    case 2: k_boundary_batch<T, 2><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    case 3: k_boundary_batch<T, 3><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    case 4: k_boundary_batch<T, 4><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    case -4: k_boundary_batch<T, -4><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    default: k_boundary_batch<T, 0><<<g, 256, 0, s>>>(mem, nmem, nbnd, parity); break;
+    }
 }
 
 } // namespace
@@ -456,7 +463,8 @@ void boundary_fix_t(const StepArgs &a, const void *pn, const uint32_t *list, uin
     const uint32_t ns = a.nsec;
     if (ns <= 1) k_boundary_fix<T, 1><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
     else if (ns == 2) k_boundary_fix<T, 2><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
-    else if (ns <= 4) k_boundary_fix<T, 4><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
+    else if (ns == 3) k_boundary_fix<T, 3><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
+    else if (ns == 4) k_boundary_fix<T, 4><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
     else k_boundary_fix<T, 0><<<g, BT, 0, s>>>(a, pn, list, nlist, gb);
 }
 } // namespace
@@ -486,16 +494,16 @@ cudaError_t launch_boundary(int storage, const StepArgs &a, int mode, cudaStream
 }
 
 cudaError_t launch_boundary_batch(int storage, const BatchMember *mem, uint32_t nmem, uint64_t nbnd, int parity,
-                                  uint32_t max_sections, cudaStream_t s)
+                                  int sections, cudaStream_t s)
 {
     if (nbnd == 0) return cudaSuccess;
     const unsigned g = (unsigned)((nbnd + 255) / 256);
     switch (storage) {
-    case VIRS_STORAGE_F16: boundary_batch_by_sections<__half>(max_sections, g, mem, nmem, nbnd, parity, s); break;
+    case VIRS_STORAGE_F16: boundary_batch_by_sections<__half>(sections, g, mem, nmem, nbnd, parity, s); break;
     case VIRS_STORAGE_BF16:
-        boundary_batch_by_sections<__nv_bfloat16>(max_sections, g, mem, nmem, nbnd, parity, s);
+        boundary_batch_by_sections<__nv_bfloat16>(sections, g, mem, nmem, nbnd, parity, s);
         break;
-    default: boundary_batch_by_sections<float>(max_sections, g, mem, nmem, nbnd, parity, s); break;
+    default: boundary_batch_by_sections<float>(sections, g, mem, nmem, nbnd, parity, s); break;
     }
     return cudaGetLastError();
 }

@@ -96,8 +96,8 @@ __device__ __forceinline__ void tile_update(const Codes<Io<T>::VEC> &code, const
 
 // The loads of one boundary voxel (first part) and its update (second).
 template <typename T, int MAXS> struct BVox {
-    size_t i;
-    uint8_t c, nm;
+    uint32_t i, meta; // device position; code, material and weight entry (StepArgs::bmeta)
+    uint8_t nm;
     float ce, qv, nb[6];
     BState<MAXS> st;
 };
@@ -107,7 +107,7 @@ template <typename T, int MODE, int MAXS>
 __device__ __forceinline__ void bvox_site(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
 {
     v.i = __ldg(a.bpos + slot);
-    v.c = __ldg(a.bcode + slot);
+    v.meta = __ldg(a.bmeta + slot);
     v.nm = a.rigid ? __ldg(a.bnrm + slot) : 0;
 }
 
@@ -116,8 +116,7 @@ template <typename T, int MODE, int MAXS>
 __device__ __forceinline__ void bvox_values(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
 {
     using IO = Io<T>;
-    const size_t i = v.i;
-    const size_t sy = a.px, sz = (size_t)a.px * a.ny;
+    const uint32_t i = v.i, sy = a.px, sz = a.px * a.ny;
     const T *P = static_cast<const T *>(a.p);
     const T *Q = static_cast<const T *>(a.q);
     v.ce = IO::get(P[i]);
@@ -128,7 +127,7 @@ __device__ __forceinline__ void bvox_values(const StepArgs &a, uint64_t slot, BV
     v.nb[3] = IO::get(P[i - sy]);
     v.nb[4] = IO::get(P[i + sz]);
     v.nb[5] = IO::get(P[i - sz]);
-    if (MODE != BND_RECORD && MAXS > 0) bload<MAXS>(a, slot, v.st);
+    if (MODE != BND_RECORD && MAXS != 0) bload<MAXS>(a, slot, v.st);
 }
 
 template <typename T, int MODE, int MAXS>
@@ -152,11 +151,12 @@ __device__ __forceinline__ void bvox_update(const StepArgs &a, uint64_t slot, co
 #pragma unroll
         for (int k = 0; k < 6; ++k) r = __fmaf_rn(__fmul_rn(a.l2, (v.nm & (1u << k)) ? 1.f : 0.f), v.nb[k], r);
     } else {
-        r = leapfrog(v.c, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5], v.qv, a.c2dt2, a.inv_h2);
+        r = leapfrog((uint8_t)v.meta, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5], v.qv, a.c2dt2, a.inv_h2);
     }
     if (MODE != BND_UPDATE) a.side[slot] = make_float4(r, v.ce, v.qv, 0.f);
     if (MODE == BND_RECORD) return;
-    r = MAXS > 0 ? bcompute<MAXS>(a, r, v.ce, v.qv, slot, v.st) : boundary_loop(a, r, v.ce, v.qv, slot);
+    if constexpr (MAXS != 0) r = bcompute<MAXS>(a, r, v.ce, v.qv, slot, v.meta, v.st);
+    else r = boundary_loop(a, r, v.ce, v.qv, slot, v.meta);
     static_cast<T *>(a.q)[v.i] =
         put_rounded<T>(r, a.sr, v.i, a.sr_base, a.sr ? sr_step_key(*a.ctr, 0u) : 0u);
 }
