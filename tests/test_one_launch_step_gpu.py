@@ -60,3 +60,47 @@ def test_same_bits_as_three_launches(shape, W, storage, sections, n_rcv, roundin
     assert np.abs(a[0]).max() > 0
     for u, v in zip(a, b):
         assert np.array_equal(u.view(np.uint32), v.view(np.uint32))
+
+
+@pytest.mark.parametrize("storage,sections", [(capi.STORAGE_F32, (3, 3, 3)), (capi.STORAGE_F32, (1, 4, 2)),
+                                              (capi.STORAGE_BF16, (2, 6, 1)), (capi.STORAGE_F16, (1, 1, 1))])
+def test_small_batch_same_bits_as_three_launches(storage, sections):
+    """Members of different sizes, with equal and with different cascades."""
+    def members():
+        out = []
+        for k, (shape, s) in enumerate(zip(((40, 32, 5), (33, 31, 20), (5, 4, 3)), sections)):
+            rng = np.random.default_rng(k)
+            n = int(np.prod(shape))
+            flags = np.zeros(n, np.uint8)
+            flags[rng.random(n) < 0.03] = 1
+            flags[rng.random(n) < 0.002] = 3
+            sim = capi.Simulation(capi.default_params(sponge_width=1 + k, courant=1.0, boundary_form=1, storage=storage))
+            sim.set_grid(shape, 0.05, flags, rng.integers(0, 2, n).astype(np.uint8))
+            sim.classify()
+            coef = np.tile(np.stack([capi.design_octave_cascade(40000.0, a) for a in rng.uniform(0.1, 0.7, (2, 3))]),
+                           (1, 2, 1))[:, :s]
+            sim.set_filters(coef.astype(np.float32), n_sections=s)
+            mid = (shape[2] // 2 * shape[1] + shape[1] // 2) * shape[0] + shape[0] // 2
+            sim.set_sources([mid], rng.standard_normal((1, 70)).astype(np.float32))
+            sim.set_receivers([mid, mid - 1])
+            sim.start(70)
+            out.append(sim)
+        return out
+
+    got = []
+    for tiled in (False, True):
+        sims = members()
+        b = capi.Batch(sims)
+        if tiled:
+            b.set_tiling(8, 0, 2)
+        for k in (33, 37):
+            b.run(k)
+        b.synchronize()
+        got.append([(s.ir(), *s.pressure(prev=True)) for s in sims])
+        b.close()
+        for s in sims:
+            s.close()
+    for x, y in zip(*got):
+        assert np.abs(x[0]).max() > 0
+        for u, v in zip(x, y):
+            assert np.array_equal(u.view(np.uint32), v.view(np.uint32))

@@ -2782,6 +2782,9 @@ struct virs_batch {
     std::vector<uint64_t> gen;
     int dev = 0, storage = 0, rows = 8, depth = 2, planes = 0;
     bool persistent = false;
+    bool tiling_set = false, fused = false; // a step in one launch (kernels_fused.cu), through `table`
+    DevBuf table;
+    uint32_t nblocks = 0;
     uint64_t ntiles = 0, nbnd = 0;
     int sections = 0;              // launch_boundary_batch
     DevBuf desc, err;
@@ -2822,10 +2825,25 @@ virs_status batch_check(const virs_batch *b)
     return VIRS_OK;
 }
 
+// A step of the batch in one launch (kernels_fused.cu) when its members are
+// few or small.  Measured per step, three launches against one (sponge 1-2,
+// three sections): 0.6 M voxels in 4 rooms FP32 29.5 against 7.4 us, BF16
+// 33.6 against 7.1; 7.4 M in 8 rooms 57.5 against 52.9 and 55.5 against 41.4;
+// 26 M in 24 rooms 153 against 155 and 132 against 143.  The line lies at
+// 12 M voxels with the row padding.
+bool batch_fused(const virs_batch *b)
+{
+    size_t n = 0;
+    for (const virs_sim *s : b->mem) n += s->nvox;
+    return !b->tiling_set && n <= (12u << 20);
+}
+
 // descriptors of every member for the batch's tiling
 virs_status batch_build(virs_batch *b)
 {
     b->drop_graphs();
+    b->fused = batch_fused(b);
+    std::vector<uint2> table;
     b->zmasks.clear();
     std::vector<BatchMember> h(b->mem.size());
     uint64_t tiles = 0, bnd = 0;
@@ -2846,7 +2864,8 @@ virs_status batch_build(virs_batch *b)
         VIRS_TRY(encode(&m.mapC, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s->code.ptr, s, (uint32_t)tma_tile_x(), b->rows));
         const int zc = b->planes > 0 ? b->planes : (s->zc > 0 ? s->zc : default_planes(s->nz));
         const uint64_t *zm = nullptr;
-        if (zero_masks_useful(s)) {
+        if (b->fused && !s->probe_ok) VIRS_TRY(build_probes(s));
+        if (!b->fused && zero_masks_useful(s)) {
             b->zmasks.emplace_back();
             VIRS_TRY(build_zero_masks(s, b->rows, zc, b->zmasks.back()));
             zm = b->zmasks.back().as<uint64_t>();
@@ -2863,6 +2882,10 @@ virs_status batch_build(virs_batch *b)
         m.gx = (s->px + tma_tile_x() - 1) / tma_tile_x();
         m.gy = (s->ny + b->rows - 1) / b->rows;
         m.gz = (s->nz - 2 + zc - 1) / zc;
+        if (b->fused) {
+            const uint32_t n = (uint32_t)fused_blocks(s->px, s->ny, s->nz, s->nb);
+            for (uint32_t k = 0; k < n; ++k) table.push_back(make_uint2((uint32_t)i, k));
+        }
         m.first_tile = tiles;
         m.first_bnd = bnd;
         tiles += (uint64_t)m.gx * m.gy * m.gz;
@@ -2873,6 +2896,11 @@ virs_status batch_build(virs_batch *b)
     }
     VIRS_TRY(b->desc.alloc(h.size() * sizeof(BatchMember), "batch descriptors"));
     VIRS_CUDA(copy_on(b->stream, b->desc.ptr, h.data(), h.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
+    if (b->fused) {
+        VIRS_TRY(b->table.alloc(table.size() * sizeof(uint2), "batch block table"));
+        VIRS_CUDA(copy_on(b->stream, b->table.ptr, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        b->nblocks = (uint32_t)table.size();
+    }
     b->ntiles = tiles;
     b->nbnd = bnd;
     b->sections = max_sections > 4 ? 0 : min_sections == max_sections ? (int)max_sections : -4;
@@ -2883,6 +2911,9 @@ cudaError_t batch_enqueue(const virs_batch *b, int parity, cudaStream_t st)
 {
     const BatchMember *d = b->desc.as<BatchMember>();
     const uint32_t n = (uint32_t)b->mem.size();
+    if (b->fused)
+        return launch_fused_batch(b->storage, b->sections, d, b->table.as<uint2>(), b->nblocks, parity, st,
+                                  sr_on(b->mem[0]));
     cudaError_t e =
         launch_step_tma_batch(b->storage, b->rows, b->depth, d, n, b->ntiles, parity, b->persistent, b->err.as<int>(), st,
                               sr_on(b->mem[0]));
@@ -3022,6 +3053,7 @@ VIRS_EXPORT virs_status virs_batch_set_tiling(virs_batch *b, int rows, int plane
     b->rows = rows ? rows : 8;
     b->planes = planes;
     b->depth = depth < 0 ? 2 : depth;
+    b->tiling_set = rows != 0 || planes != 0 || depth >= 0;
     return batch_build(b);
 }
 
@@ -3039,7 +3071,7 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
     VIRS_CUDA(cudaEventCreate(&e0));
     VIRS_CUDA(cudaEventCreate(&e1));
     virs_tiling pick{8, 0, 2, 0.f};
-    bool pick_persistent = false;
+    bool pick_persistent = false, pick_tiled = false;
     float best_ms = 1e30f;
     virs_status st = VIRS_OK;
     // every candidate timed twice, in forward and then reverse order (the
@@ -3047,7 +3079,7 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
     struct Cand {
         int pers, d, r, pl;
     };
-    std::vector<Cand> cand;
+    std::vector<Cand> cand{{0, 0, 8, 0}}; // the step as it runs without a tiling
     for (int pers : {0, 1})
         for (int d : {1, 2, 3})
             for (int r : {4, 8, 16})
@@ -3056,8 +3088,9 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
         const Cand &cd = cand[c < cand.size() ? c : 2 * cand.size() - 1 - c];
         const int pers = cd.pers, d = cd.d, r = cd.r, pl = cd.pl;
         if (st != VIRS_OK) break;
+        b->tiling_set = d > 0;
         b->rows = r;
-        b->depth = d;
+        b->depth = d > 0 ? d : 2;
         b->planes = pl;
         b->persistent = pers != 0;
         if ((st = batch_build(b)) != VIRS_OK) break;
@@ -3074,8 +3107,9 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
         }
         if (ms < best_ms) {
             best_ms = ms;
-            pick = {r, pl, d, ms / trial_steps};
+            pick = {r, pl, b->depth, ms / trial_steps};
             pick_persistent = pers != 0;
+            pick_tiled = d > 0;
         }
         for (virs_sim *s : b->mem)
             if ((st = reset_state(s)) != VIRS_OK) break;
@@ -3087,6 +3121,7 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
     b->depth = pick.pipeline_depth;
     b->planes = pick.planes_per_block;
     b->persistent = pick_persistent;
+    b->tiling_set = pick_tiled;
     VIRS_TRY(batch_build(b));
     VIRS_TRY(virs_batch_synchronize(b));
     if (best) *best = pick;

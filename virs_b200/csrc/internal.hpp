@@ -170,6 +170,11 @@ cudaError_t launch_boundary_batch(int storage, const BatchMember *mem, uint32_t 
                                   int sections, cudaStream_t s);
 cudaError_t launch_post_batch(int storage, const BatchMember *mem, uint32_t nmem, int parity, cudaStream_t s);
 
+// the same in one launch (kernels_fused.cu): table[block] = {member, block of the member}
+cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks,
+                               int parity, cudaStream_t s, bool sr);
+uint64_t fused_blocks(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb); // blocks of one simulation's step
+
 // kernel launchers (kernels_step.cu)
 cudaError_t launch_step(int storage, int tile_rows, const StepArgs &a, cudaStream_t s);
 cudaError_t launch_post(int storage, const PostArgs &a, cudaStream_t s);

@@ -214,6 +214,31 @@ __global__ void __launch_bounds__(FB) k_fused(const __grid_constant__ StepArgs a
     fused_block<T, MAXS, MODE, SR>(a, po, blockIdx.x, gb, gx);
 }
 
+// Many simulations: a table gives each block its member and its number in
+// it; the block copies that member's arguments into shared memory once.
+// Both are constant over the steps and read before the wait.
+template <typename T, int MAXS, bool SR>
+__global__ void __launch_bounds__(FB) k_fused_batch(const BatchMember *__restrict mem, const uint2 *__restrict table,
+                                                    int parity)
+{
+    __shared__ StepArgs a;
+    __shared__ PostArgs po;
+    pdl_trigger();
+    const uint2 e = __ldg(table + blockIdx.x);
+    {
+        const uint32_t *sa = reinterpret_cast<const uint32_t *>(&mem[e.x].step[parity]);
+        const uint32_t *sp = reinterpret_cast<const uint32_t *>(&mem[e.x].post[parity]);
+        constexpr uint32_t na = sizeof(StepArgs) / 4, np = sizeof(PostArgs) / 4;
+        static_assert(na + np <= FB, "one word per thread");
+        const uint32_t t = threadIdx.x;
+        if (t < na) reinterpret_cast<uint32_t *>(&a)[t] = __ldg(sa + t);
+        else if (t < na + np) reinterpret_cast<uint32_t *>(&po)[t - na] = __ldg(sp + (t - na));
+    }
+    __syncthreads();
+    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB), gx = (a.px * a.ny + FB * V - 1) / (FB * V);
+    fused_block<T, MAXS, BND_UPDATE, SR>(a, po, e.y, gb, gx);
+}
+
 // the slot of each probe's voxel in the boundary list (ascending positions)
 __global__ void k_probe_slots(Probe *probe, uint32_t n, const uint32_t *__restrict bpos, uint64_t nb)
 {
@@ -229,7 +254,8 @@ __global__ void k_probe_slots(Probe *probe, uint32_t n, const uint32_t *__restri
     probe[k].slot = lo < nb && bpos[lo] == pos ? (uint32_t)lo : PROBE_NO_SLOT;
 }
 
-template <typename K, typename... A> cudaError_t launch_pdl(K kern, unsigned grid, cudaStream_t s, A... args)
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, cudaStream_t s, const A &...args)
 {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -240,7 +266,7 @@ template <typename K, typename... A> cudaError_t launch_pdl(K kern, unsigned gri
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 template <typename T, int MODE, bool SR>
@@ -270,6 +296,41 @@ cudaError_t launch_fused(int storage, const StepArgs &a, const PostArgs &po, cud
     case VIRS_STORAGE_F16: return fused_16<__half>(a, po, s);
     case VIRS_STORAGE_BF16: return fused_16<__nv_bfloat16>(a, po, s);
     default: return fused_by_sections<float, BND_UPDATE, false>(a, po, s);
+    }
+}
+
+namespace {
+template <typename T, bool SR>
+cudaError_t fused_batch_t(int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks, int parity,
+                          cudaStream_t s)
+{
+    switch (sections) {
+    case 1: return launch_pdl(k_fused_batch<T, 1, SR>, nblocks, s, mem, table, parity);
+    case 2: return launch_pdl(k_fused_batch<T, 2, SR>, nblocks, s, mem, table, parity);
+    case 3: return launch_pdl(k_fused_batch<T, 3, SR>, nblocks, s, mem, table, parity);
+    case 4: return launch_pdl(k_fused_batch<T, 4, SR>, nblocks, s, mem, table, parity);
+    case -4: return launch_pdl(k_fused_batch<T, -4, SR>, nblocks, s, mem, table, parity);
+    default: return launch_pdl(k_fused_batch<T, 0, SR>, nblocks, s, mem, table, parity);
+    }
+}
+} // namespace
+
+uint64_t fused_blocks(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb)
+{
+    return (nb + FB - 1) / FB + ((uint64_t)px * ny + FB * V - 1) / (FB * V) * (nz - 2);
+}
+
+cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks,
+                               int parity, cudaStream_t s, bool sr)
+{
+    switch (storage) {
+    case VIRS_STORAGE_F16:
+        return sr ? fused_batch_t<__half, true>(sections, mem, table, nblocks, parity, s)
+                  : fused_batch_t<__half, false>(sections, mem, table, nblocks, parity, s);
+    case VIRS_STORAGE_BF16:
+        return sr ? fused_batch_t<__nv_bfloat16, true>(sections, mem, table, nblocks, parity, s)
+                  : fused_batch_t<__nv_bfloat16, false>(sections, mem, table, nblocks, parity, s);
+    default: return fused_batch_t<float, false>(sections, mem, table, nblocks, parity, s);
     }
 }
 
