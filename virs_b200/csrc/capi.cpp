@@ -248,8 +248,7 @@ struct virs_sim {
         uint64_t steps = 0, nck = 0, gen = 0;
         uint32_t every = 0;
         bool ready = false;
-        DevBuf ckp, ckq, cks, segrec, segst, buf[2], ast, dbar, cq, grad, dl, gsig;
-        CUtensorMap mapP[2], mapQ[2];
+        DevBuf ckp, ckq, cks, segrec, segst, buf[2], ast, dbar, rr[2], grad, dl, gsig;
     } adj;
     bool fields_valid = true;      // false after virs_adjoint until the next start
     bool slab_open = false;        // virs_slab_step_begin ran, virs_slab_step_end not yet
@@ -860,7 +859,7 @@ cudaError_t launch_stencil_range(const virs_sim *s, int parity, cudaStream_t st,
 cudaError_t enqueue_step(const virs_sim *s, int parity, cudaStream_t st)
 {
     if (fused_on(s))
-        return launch_fused(s->prm.storage, step_args(s, parity), post_args(s, parity), st);
+        return launch_fused(s->prm.storage, BND_UPDATE, step_args(s, parity), post_args(s, parity), st);
     cudaError_t e = launch_stencil(s, parity, st);
     if (e != cudaSuccess) return e;
     e = launch_boundary(s->prm.storage, step_args(s, parity), BND_UPDATE, st);
@@ -3184,18 +3183,17 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     for (int k = 0; k < 2; ++k) VIRS_TRY(A.buf[k].alloc(fb, "adjoint field"));
     VIRS_TRY(A.ast.alloc(sba, "adjoint filter states"));
     VIRS_TRY(A.dbar.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms"));
-    VIRS_TRY(A.cq.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms"));
+    for (int k = 0; k < 2; ++k) VIRS_TRY(A.rr[k].alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms"));
     VIRS_TRY(A.grad.alloc(ncoef * sizeof(double), "coefficient gradients"));
     VIRS_TRY(A.dl.alloc(std::max<uint32_t>(s->nrcv, 1) * steps * 4, "loss gradient"));
     VIRS_TRY(A.gsig.alloc(std::max<uint32_t>(s->nsrc, 1) * steps * 4, "signal gradients"));
     if (s->nrcv) VIRS_CUDA(copy_on(s->stream, A.dl.ptr, dl_dir, (size_t)s->nrcv * steps * 4, cudaMemcpyHostToDevice));
-    const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    for (int k = 0; k < 2; ++k) {
-        VIRS_TRY(encode(&A.mapP[k], dt, 4, A.buf[k].ptr, s, (uint32_t)tma_box_width(VIRS_STORAGE_F32), s->tile_rows + 2));
-        VIRS_TRY(encode(&A.mapQ[k], dt, 4, A.buf[k].ptr, s, (uint32_t)tma_tile_x(), s->tile_rows));
-    }
     VIRS_TRY(ready_to_run(s));
-    int t = 0; // A.buf[t] holds T, A.buf[t ^ 1] holds RR
+    if (!s->probe_ok) VIRS_TRY(build_probes(s));
+    int t = 0; // A.buf[t] holds T, A.buf[t ^ 1] holds RR; A.rr[t] the RR of the boundary slots
+    VIRS_CUDA(launch_adj_inject(A.buf[t].as<float>(), s->code.as<uint8_t>(), s->rcv.as<uint64_t>(), s->nrcv,
+                                A.dl.as<float>(), steps, steps - 1, s->src.as<uint64_t>(), s->nsrc,
+                                A.gsig.as<float>(), steps, st));
     for (int64_t c = (int64_t)A.nck - 1; c >= 0; --c) {
         const uint64_t n0 = (uint64_t)c * every, n1 = std::min<uint64_t>(n0 + every, steps);
         // rebuild the segment: restore the checkpoint and run forward, keeping
@@ -3207,7 +3205,6 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
         VIRS_CUDA(launch_set_u32(s->ctr.as<uint32_t>(), (uint32_t)n0, st));
         for (uint64_t n = n0; n < n1; ++n) {
             const uint64_t k = n - n0;
-            cudaError_t e = launch_stencil(s, s->cur, st);
             // the boundary pass keeps its records straight in the segment's
             // slot k, and reads the states before the step from slot k and
             // writes those after it to slot k + 1 (the last step's to the
@@ -3217,40 +3214,33 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
             ka.state = reinterpret_cast<float *>(A.segst.as<char>() + k * sb);
             ka.state_out = k + 1 < every ? reinterpret_cast<float *>(A.segst.as<char>() + (k + 1) * sb)
                                          : s->state.as<float>();
-            if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, st);
-            if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, s->cur), st);
+            cudaError_t e;
+            if (fused_on(s)) {
+                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), st);
+            } else {
+                e = launch_stencil(s, s->cur, st);
+                if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, st);
+                if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, s->cur), st);
+            }
             if (e != cudaSuccess) return cuda_fail(e, "adjoint recomputation");
             s->cur ^= 1;
         }
         // reverse steps of the segment
         for (int64_t n = (int64_t)n1 - 1; n >= (int64_t)n0; --n) {
             const uint64_t k = (uint64_t)n - n0;
-            float *T = A.buf[t].as<float>(), *RR = A.buf[t ^ 1].as<float>();
-            cudaError_t e = launch_adj_inject(T, s->code.as<uint8_t>(), s->rcv.as<uint64_t>(), s->nrcv, A.dl.as<float>(),
-                                              steps, (uint64_t)n, s->src.as<uint64_t>(), s->nsrc, A.gsig.as<float>(),
-                                              steps, st);
-            if (e == cudaSuccess)
-                e = launch_adj_boundary(T, s->bidx.as<uint32_t>(), s->bmat.as<uint8_t>(), s->bw.as<float>(),
-                                        s->coef.as<float>(), A.segrec.as<float4>() + k * nb,
-                                        reinterpret_cast<const float *>(A.segst.as<char>() + k * sb), A.ast.as<float>(),
-                                        A.dbar.as<float>(), A.cq.as<float>(), A.grad.as<double>(), nb, s->nx, s->ny,
-                                        s->px, s->nsec, s->nmat, s->prm.boundary_form, (double)s->K,
-                                        s->prm.mix_filtered, s->prm.mix_direct, (double)s->prm.boundary_gain, st);
+            StepArgs a = step_args(s, 0);
+            cudaError_t e = launch_adj_boundary(a, A.buf[t].as<float>(), A.segrec.as<float4>() + k * nb,
+                                                reinterpret_cast<const float *>(A.segst.as<char>() + k * sb),
+                                                A.ast.as<float4>(), A.dbar.as<float>(), A.rr[t ^ 1].as<float>(),
+                                                A.grad.as<double>(), s->nmat, n + 1 < (int64_t)n1, st);
             if (e == cudaSuccess) {
-                StepArgs a = step_args(s, 0);
-                a.p = T;
-                a.q = RR;
+                a.p = A.buf[t].ptr;
+                a.q = A.buf[t ^ 1].ptr;
                 a.nhard = 0;
-                const TmaMaps m{&A.mapP[t], &A.mapQ[t ^ 1], &s->tmC};
-                e = launch_step_tma(VIRS_STORAGE_F32, s->tile_rows, s->depth, a, m, s->err.as<int>(), st);
-                if (e == cudaSuccess) e = launch_zero_at(RR, s->hpos.as<uint32_t>(), s->nhpos, st);
-                // the free value A F - RR at the boundary voxels, which the
-                // stencil left alone
-                if (e == cudaSuccess) e = launch_boundary(VIRS_STORAGE_F32, a, BND_RECORD, st);
+                const AdjPost po{s->probe.as<Probe>(), s->nsrc, s->nrcv, A.rr[t].as<float>(), A.dbar.as<float>(),
+                                 A.dl.as<float>(), A.gsig.as<float>(), steps, n - 1};
+                e = launch_adj_step(a, po, st);
             }
-            if (e == cudaSuccess)
-                e = launch_adj_fix(RR, T, s->bidx.as<uint32_t>(), s->side.as<float4>(), A.dbar.as<float>(),
-                                   A.cq.as<float>(), nb, s->nx, s->ny, s->px, st);
             if (e != cudaSuccess) return cuda_fail(e, "adjoint step");
             t ^= 1;
         }

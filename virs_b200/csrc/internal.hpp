@@ -179,10 +179,22 @@ uint64_t fused_blocks(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb); // bl
 cudaError_t launch_step(int storage, int tile_rows, const StepArgs &a, cudaStream_t s);
 cudaError_t launch_post(int storage, const PostArgs &a, cudaStream_t s);
 // a whole step in one launch (kernels_fused.cu)
-cudaError_t launch_fused(int storage, const StepArgs &a, const PostArgs &po, cudaStream_t s);
+// (mode BND_UPDATE, or BND_KEEP in FP32)
+cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, cudaStream_t s);
+// the adjoint's step (kernels_fused.cu): what its blocks need beyond StepArgs
+struct AdjPost {
+    const Probe *probe;     // as PostArgs
+    uint32_t nsrc, nrcv;
+    const float *rr, *dbar; // per boundary slot
+    const float *dl;        // [nrcv][stride] loss gradients
+    float *gsig;            // [nsrc][stride] signal gradients
+    uint64_t stride;
+    int64_t n;              // the next reverse step (-1: none)
+};
+cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, cudaStream_t s);
 cudaError_t launch_probe_slots(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, cudaStream_t s);
 // modes of the boundary pass (kernels_step.cu)
-enum { BND_UPDATE = 0, BND_KEEP = 1, BND_RECORD = 2 };
+enum { BND_UPDATE = 0, BND_KEEP = 1 };
 cudaError_t launch_boundary(int storage, const StepArgs &a, int mode, cudaStream_t s);
 int default_planes(uint32_t nz);
 
@@ -280,12 +292,10 @@ cudaError_t launch_hard_list(const uint8_t *code, uint64_t n, uint32_t *count, u
 cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv, uint32_t nrcv, const float *dl,
                               uint64_t dl_stride, uint64_t n, const uint64_t *src, uint32_t nsrc, float *gsig,
                               uint64_t gs_stride, cudaStream_t s);
-cudaError_t launch_adj_boundary(float *T, const uint32_t *bidx, const uint8_t *bmat, const float *bw, const float *coef,
-                                const float4 *rec, const float *fst, float *ast, float *dbar, float *cq, double *grad,
-                                uint64_t nb, uint32_t nx, uint32_t ny, uint32_t px, uint32_t nsec, uint32_t nmat,
-                                int form, double K, double mix_y, double mix_d, double gain, cudaStream_t s);
-cudaError_t launch_adj_fix(float *Tn, float *Tb, const uint32_t *bidx, const float4 *rec, const float *dbar,
-                           const float *cq, uint64_t nb, uint32_t nx, uint32_t ny, uint32_t px, cudaStream_t s);
+// f: the forward step's arguments; overlap: the kernel before on the stream
+// is launch_adj_step (nothing that wrote rec or fst)
+cudaError_t launch_adj_boundary(const StepArgs &f, float *T, const float4 *rec, const float *fst, float4 *ast,
+                                float *dbar, float *rr, double *grad, uint32_t nmat, bool overlap, cudaStream_t s);
 cudaError_t launch_set_u32(uint32_t *p, uint32_t v, cudaStream_t s);
 cudaError_t launch_zero_at(float *f, const uint32_t *pos, uint32_t n, cudaStream_t s);
 

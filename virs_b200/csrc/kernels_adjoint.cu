@@ -5,20 +5,25 @@
 // the filter states.  With T the adjoint of p^{n+1} and RR the negated
 // adjoint carried by p^n through its role as q of the next step, one
 // reverse step n is
-//   k_adj_inject     T[rcv] += dL/dIR_n ; dL/dsig_n = T[src]
 //   k_adj_boundary   at boundary voxels the correction and the biquad cascade
 //                    run transposed: F = T (reference form) or T/(1+a)
 //                    (centered form), the cascade's state adjoints and the
-//                    coefficient gradients (FP64), dbar = d(loss)/d(p - q)
-//   stencil          T' = A F - RR into RR's buffer: the forward stencil
-//                    kernel itself, since A (2 + lambda^2 * Laplacian with
+//                    coefficient gradients (FP64), dbar = d(loss)/d(p - q),
+//                    and the voxel's next RR' = F + dbar - cq, kept per slot
+//   k_adj_step       T' = A F - RR into RR's buffer, at boundary voxels
+//                    T'_b = A F_b - RR_b + dbar_b (kernels_fused.cu): the
+//                    forward stencil, since A (2 + lambda^2 * Laplacian with
 //                    mirrored walls and zero fixed voxels) is symmetric on
-//                    the updated voxels; hard-source voxels are given 0
-//   k_adj_fix        boundary voxels: T'_b = A F_b - RR_b + dbar_b (from the
-//                    stencil's record) and RR'_b = F_b + dbar_b - cq_b
-// and the buffers swap.  The forward values the cascade needs (p - q and
-// the states before step n) come from a recomputation of the segment from
-// the last checkpoint.
+//                    the updated voxels; hard-source voxels take 0.  Then, for
+//                    the next reverse step, T'[rcv] += dL/dIR and
+//                    dL/dsig = T'[src]
+// and the buffers swap.  k_adj_inject does the latter before the first step.
+// The forward values the cascade needs (p - q and the states before step n)
+// come from a recomputation of the segment from the last checkpoint.
+//
+// 128x128x96 voxels, 79 K slots of two sections: a reverse step was five
+// launches of 28.7 us and their gaps, two of 12 us in all now.
+#include "pdl.cuh"
 #include "step_common.cuh"
 
 namespace virs {
@@ -42,69 +47,53 @@ __global__ void k_adj_inject(float *T, const uint8_t *__restrict code, const uin
 
 struct AdjArgs {
     float *T;                  // adjoint field (p role)
-    const uint32_t *bidx;
-    const uint8_t *bmat;
-    const float *bw;
-    const float *coef;         // [M][S][5]
+    const uint32_t *bpos, *bmeta; // as StepArgs
+    const BndWeight *wtab;
+    const float *coef, *coefp; // [M][S][5], and padded to vectors (StepArgs)
     const float4 *rec;         // forward records of this step {free, p, q, 0}
     const float *fst;          // forward states before this step (the cascade's layout, state_index)
-    float *ast;                // state adjoints, four per section [S][4][nb]
-    float *dbar, *cq;          // per slot
+    float4 *ast;               // state adjoints, one vector per section [S][nb]
+    float *dbar, *rr;          // per slot: dbar, and the voxel's next RR
     double *grad;              // [M][S][5]
     uint64_t nb;
-    uint32_t nx, ny, px, nsec, ncoef;
+    uint32_t nsec, ncoef;
     int form;
-    double K, mix_y, mix_d, gain;
+    double kg, mix_y, mix_d;   // K * gain
 };
+
+// the transposed correction of one slot: the value F left in the adjoint
+// field, the cascade output's adjoint and what dbar and RR' take beyond it
+struct AdjCorr {
+    double fr, ybar, db, cq;
+};
+__device__ __forceinline__ AdjCorr adj_correct(const AdjArgs &a, float f, uint32_t meta)
+{
+    const BndWeight e = a.wtab[meta >> 16];
+    AdjCorr c;
+    if (a.form == VIRS_BOUNDARY_REFERENCE) {
+        const double kgw = a.kg * e.kgw; // the weight itself
+        c.fr = f;
+        c.ybar = -kgw * a.mix_y * f;
+        c.db = -kgw * a.mix_d * f;
+        c.cq = 0.0;
+    } else {
+        c.fr = quotient((double)f, e.den, e.rden);
+        c.ybar = -e.kgw * a.mix_y * c.fr;
+        c.db = 0.0;
+        c.cq = e.ac * c.fr;
+    }
+    return c;
+}
+// the slot's results: F into the field, dbar, and RR' = F + dbar - cq
+__device__ __forceinline__ void adj_store(const AdjArgs &a, uint64_t b, uint32_t pos, const AdjCorr &c, double yb)
+{
+    const float fr = (float)c.fr, db = (float)(c.db + yb), cq = (float)c.cq;
+    a.T[pos] = fr;
+    a.dbar[b] = db;
+    a.rr[b] = __fsub_rn(__fadd_rn(fr, db), cq);
+}
 
 constexpr int AB = 256;
-
-// The shuffle schedule of peer_sum for one lane, worked out once and used
-// for every sum of a slot: in round r the lane takes the value of lane
-// src[r] and adds it when bit r of `use` is set; `rounds` (at most five,
-// for a group of 32) is the same on every lane.
-struct PeerPlan {
-    int src[5];
-    unsigned use;
-    int rounds;
-};
-
-__device__ __forceinline__ PeerPlan peer_plan(unsigned peers)
-{
-    PeerPlan p;
-    p.use = 0u;
-    p.rounds = 0;
-    const int lane = (int)(threadIdx.x & 31u);
-    unsigned rank = __popc(peers & ((1u << lane) - 1u));
-    peers &= 0xfffffffeu << lane;
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-        p.src[r] = lane;
-        if (__any_sync(0xffffffffu, peers != 0u)) {
-            const int next = __ffs(peers);
-            if (next > 0) {
-                p.src[r] = next - 1;
-                p.use |= 1u << r;
-            }
-            peers &= __ballot_sync(0xffffffffu, (rank & 1u) == 0u);
-            rank >>= 1;
-            p.rounds = r + 1;
-        }
-    }
-    return p;
-}
-
-// peer_sum with a schedule from peer_plan
-__device__ __forceinline__ double plan_sum(const PeerPlan &p, double v)
-{
-#pragma unroll
-    for (int r = 0; r < 5; ++r)
-        if (r < p.rounds) {
-            const double u = __shfl_sync(0xffffffffu, v, p.src[r]);
-            if ((p.use >> r) & 1u) v += u;
-        }
-    return v;
-}
 
 // The sum of v over the lanes of a full warp that share this lane's key
 // (peers = __match_any_sync of the key), complete at the group's lowest
@@ -129,30 +118,17 @@ __device__ __forceinline__ double peer_sum(unsigned peers, double v)
 
 __global__ void __launch_bounds__(AB) k_adj_boundary(const AdjArgs a)
 {
+    pdl_trigger();
     extern __shared__ double gsm[]; // block partial sums of the coefficient gradients
     for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB) gsm[k] = 0.0;
     __syncthreads();
+    pdl_wait();
     const uint64_t b = (uint64_t)blockIdx.x * AB + threadIdx.x;
     if (b < a.nb) {
-        const uint32_t ref = a.bidx[b];
-        const uint32_t x = ref % a.nx, t = ref / a.nx, y = t % a.ny, z = t / a.ny;
-        const size_t i = ((size_t)z * a.ny + y) * a.px + x;
-        const float f = a.T[i];
-        const double w = (double)a.bw[b];
-        const double kgw = a.K * a.gain * w;
-        double fr, ybar, db = 0.0, cqv = 0.0;
-        if (a.form == VIRS_BOUNDARY_REFERENCE) {
-            fr = f;
-            ybar = -kgw * a.mix_y * f;
-            db = -kgw * a.mix_d * f;
-        } else {
-            const double ac = kgw * a.mix_d * 0.5;
-            fr = f / (1.0 + ac);
-            ybar = -kgw * a.mix_y * fr;
-            cqv = ac * fr;
-        }
+        const uint32_t pos = a.bpos[b], meta = a.bmeta[b];
+        const AdjCorr c = adj_correct(a, a.T[pos], meta);
         // forward inputs of every section at this step
-        const uint32_t S = a.nsec, m = a.bmat[b];
+        const uint32_t S = a.nsec, m = (meta >> 8) & 0xffu;
         const float *kc = a.coef + (uint64_t)m * S * 5;
         const float4 rec = a.rec[b];
         float xin[16];
@@ -173,13 +149,11 @@ __global__ void __launch_bounds__(AB) k_adj_boundary(const AdjArgs a)
         const bool full = __activemask() == 0xffffffffu;
         const unsigned peers = full ? __match_any_sync(0xffffffffu, m) : 0u;
         const bool lead = full && (int)(threadIdx.x & 31u) == __ffs(peers) - 1;
-        double yb = ybar;
+        double yb = c.ybar;
         for (int q = (int)S - 1; q >= 0; --q) {
             const float *kq = kc + 5 * q;
-            float *aq = a.ast + b;
-            const uint64_t o0 = (uint64_t)(4 * q + 0) * a.nb, o1 = (uint64_t)(4 * q + 1) * a.nb;
-            const uint64_t o2 = (uint64_t)(4 * q + 2) * a.nb, o3 = (uint64_t)(4 * q + 3) * a.nb;
-            const double yt = yb + (double)aq[o2];
+            const float4 aq = a.ast[(uint64_t)q * a.nb + b];
+            const double yt = yb + (double)aq.z;
             const double s0 = a.fst[state_index(2 * q, b, a.nb)], s1 = a.fst[state_index(2 * q + 1, b, a.nb)],
                          s2 = a.fst[state_index(2 * q + 2, b, a.nb)], s3 = a.fst[state_index(2 * q + 3, b, a.nb)];
             double *g = gsm + (uint64_t)(m * S + q) * 5;
@@ -194,145 +168,144 @@ __global__ void __launch_bounds__(AB) k_adj_boundary(const AdjArgs a)
 #pragma unroll
                 for (int j = 0; j < 5; ++j) atomicAdd(g + j, gv[j]);
             }
-            const double xbar = (double)kq[0] * yt + (double)aq[o0];
-            const double x1 = (double)kq[1] * yt + (double)aq[o1];
+            const double xbar = (double)kq[0] * yt + (double)aq.x;
+            const double x1 = (double)kq[1] * yt + (double)aq.y;
             const double x2 = (double)kq[2] * yt;
-            const double y1 = -(double)kq[3] * yt + (double)aq[o3];
+            const double y1 = -(double)kq[3] * yt + (double)aq.w;
             const double y2 = -(double)kq[4] * yt;
-            aq[o0] = (float)x1;
-            aq[o1] = (float)x2;
-            aq[o2] = (float)y1;
-            aq[o3] = (float)y2;
+            a.ast[(uint64_t)q * a.nb + b] = make_float4((float)x1, (float)x2, (float)y1, (float)y2);
             yb = xbar;
         }
-        db += yb;
-        a.T[i] = (float)fr;
-        a.dbar[b] = (float)db;
-        a.cq[b] = (float)cqv;
+        adj_store(a, b, pos, c, yb);
     }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB)
         if (gsm[k] != 0.0) atomicAdd(a.grad + k, gsm[k]);
 }
 
-constexpr int ABS = 128; // threads per block of k_adj_boundary_s: a few slots per SM at small sizes still fill it
-
-// The same for cascades of up to MAXS sections, unrolled: the forward
-// section inputs and the filter states stay in registers (the states are
-// read once, as the 16-byte groups of the cascade's layout).
-template <int MAXS> __global__ void __launch_bounds__(ABS) k_adj_boundary_s(const AdjArgs a)
+// The sums of v[0..N) over a warp (N a power of two): each exchange halves
+// the values a lane holds, so N values cost N - 1 + log2(32 / N) shuffles
+// instead of 5 N.  Returns the sum of value *idx, the same on every lane of
+// a group of 32 / N.
+template <int N> __device__ __forceinline__ double warp_sums(double (&v)[N], int *idx)
 {
-    constexpr int NG = (2 * (MAXS + 1) + 3) / 4;
-    extern __shared__ double gsm[]; // block partial sums of the coefficient gradients
-    for (uint32_t k = threadIdx.x; k < a.ncoef; k += ABS) gsm[k] = 0.0;
-    __syncthreads();
-    const uint64_t b = (uint64_t)blockIdx.x * ABS + threadIdx.x;
-    if (b < a.nb) {
-        const uint32_t ref = a.bidx[b];
-        const uint32_t S = a.nsec, m = a.bmat[b];
-        const float4 rec = a.rec[b];
-        const double w = (double)a.bw[b];
-        float h[4 * NG];
-        const float4 *st = reinterpret_cast<const float4 *>(a.fst) + b;
-        const uint32_t ng = (2u * (S + 1u) + 3u) / 4u;
+    const int lane = (int)(threadIdx.x & 31u);
+    int k = 0;
+    int n = N;
 #pragma unroll
-        for (int g = 0; g < NG; ++g)
-            if ((uint32_t)g < ng) {
-                const float4 v = st[(uint64_t)g * a.nb];
-                h[4 * g] = v.x;
-                h[4 * g + 1] = v.y;
-                h[4 * g + 2] = v.z;
-                h[4 * g + 3] = v.w;
-            }
-        const uint32_t x = ref % a.nx, t = ref / a.nx, y = t % a.ny, z = t / a.ny;
-        const size_t i = ((size_t)z * a.ny + y) * a.px + x;
-        const float f = a.T[i];
-        const double kgw = a.K * a.gain * w;
-        double fr, ybar, db = 0.0, cqv = 0.0;
-        if (a.form == VIRS_BOUNDARY_REFERENCE) {
-            fr = f;
-            ybar = -kgw * a.mix_y * f;
-            db = -kgw * a.mix_d * f;
-        } else {
-            const double ac = kgw * a.mix_d * 0.5;
-            fr = f / (1.0 + ac);
-            ybar = -kgw * a.mix_y * fr;
-            cqv = ac * fr;
-        }
-        // forward inputs of every section at this step
-        const float *kc = a.coef + (uint64_t)m * S * 5;
-        float xin[MAXS];
-        float in = __fsub_rn(rec.y, rec.z);
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n /= 2;
+            const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int q = 0; q < MAXS; ++q)
-            if (q < (int)S) {
-                const float *kq = kc + 5 * q;
-                xin[q] = in;
-                float yv = __fmaf_rn(kq[0], in, __fmul_rn(kq[1], h[2 * q]));
-                yv = __fmaf_rn(kq[2], h[2 * q + 1], yv);
-                yv = __fmaf_rn(-kq[3], h[2 * q + 2], yv);
-                in = __fmaf_rn(-kq[4], h[2 * q + 3], yv);
-            }
-        const bool full = __activemask() == 0xffffffffu;
-        const unsigned peers = full ? __match_any_sync(0xffffffffu, m) : 0u;
-        const bool lead = full && (int)(threadIdx.x & 31u) == __ffs(peers) - 1;
-        const PeerPlan plan = full ? peer_plan(peers) : PeerPlan{};
-        double yb = ybar;
-#pragma unroll
-        for (int q = MAXS - 1; q >= 0; --q)
-            if (q < (int)S) {
-                const float *kq = kc + 5 * q;
-                float *aq = a.ast + b;
-                const uint64_t o0 = (uint64_t)(4 * q + 0) * a.nb, o1 = (uint64_t)(4 * q + 1) * a.nb;
-                const uint64_t o2 = (uint64_t)(4 * q + 2) * a.nb, o3 = (uint64_t)(4 * q + 3) * a.nb;
-                const double yt = yb + (double)aq[o2];
-                double *g = gsm + (uint64_t)(m * S + q) * 5;
-                const double gv[5] = {yt * (double)xin[q], yt * (double)h[2 * q], yt * (double)h[2 * q + 1],
-                                      -yt * (double)h[2 * q + 2], -yt * (double)h[2 * q + 3]};
-                if (full) {
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) {
-                        const double v = plan_sum(plan, gv[j]);
-                        if (lead) atomicAdd(g + j, v);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) atomicAdd(g + j, gv[j]);
+            for (int j = 0; j < N / 2; ++j)
+                if (j < n) {
+                    const double give = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+                    v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
-                const double xbar = (double)kq[0] * yt + (double)aq[o0];
-                const double x1 = (double)kq[1] * yt + (double)aq[o1];
-                const double x2 = (double)kq[2] * yt;
-                const double y1 = -(double)kq[3] * yt + (double)aq[o3];
-                const double y2 = -(double)kq[4] * yt;
-                aq[o0] = (float)x1;
-                aq[o1] = (float)x2;
-                aq[o2] = (float)y1;
-                aq[o3] = (float)y2;
-                yb = xbar;
-            }
-        db += yb;
-        a.T[i] = (float)fr;
-        a.dbar[b] = (float)db;
-        a.cq[b] = (float)cqv;
+            k += up ? n : 0;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < a.ncoef; k += ABS)
-        if (gsm[k] != 0.0) atomicAdd(a.grad + k, gsm[k]);
+    *idx = k;
+    return v[0];
 }
 
-// boundary voxels after the stencil: T' (in RR's buffer) and the next RR
-// (in T's buffer)
-__global__ void k_adj_fix(float *Tn, float *Tb, const uint32_t *__restrict bidx, const float4 *__restrict rec,
-                          const float *__restrict dbar, const float *__restrict cq, uint64_t nb, uint32_t nx,
-                          uint32_t ny, uint32_t px)
+// Cascades of S = 1..4 sections, unrolled: the forward section inputs and
+// the filter states stay in registers.  What the forward recomputation and
+// the set-up wrote (records, states, positions) is read before the wait for
+// the kernel before; the launch that opens a segment does not overlap with
+// the recomputation (launch_adj_boundary).  The 5 S gradient terms of a
+// warp's slots are summed one material at a time, nearly always one or two
+// per warp.  A shuffle tree per term, records and states after the wait and
+// a double-precision division made it 15.4 us at 79 K slots of two sections,
+// 7.6 us now.
+template <int S> __global__ void __launch_bounds__(AB) k_adj_boundary_s(const __grid_constant__ AdjArgs a)
 {
-    const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const uint32_t ref = bidx[b];
-    const uint32_t x = ref % nx, t = ref / nx, y = t % ny, z = t / ny;
-    const size_t i = ((size_t)z * ny + y) * px + x;
-    Tn[i] = rec[b].x + dbar[b];
-    Tb[i] = Tb[i] + dbar[b] - cq[b];
+    constexpr int NG = (2 * (S + 1) + 3) / 4, NC = (5 * S + 3) / 4, NV = 5 * S;
+    constexpr int NP = NV <= 8 ? 8 : NV <= 16 ? 16 : 32;
+    extern __shared__ double gsm[]; // block partial sums of the coefficient gradients
+    pdl_trigger();
+    const uint64_t b = (uint64_t)blockIdx.x * AB + threadIdx.x;
+    const bool act = b < a.nb;
+    const uint64_t bl = act ? b : a.nb - 1; // idle lanes of the last block repeat its last slot, unstored
+    const uint32_t pos = __ldg(a.bpos + bl), meta = __ldg(a.bmeta + bl), m = (meta >> 8) & 0xffu;
+    const float4 rec = a.rec[bl];
+    float h[4 * NG], kc[4 * NC];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const float4 v = reinterpret_cast<const float4 *>(a.fst)[(uint64_t)g * a.nb + bl];
+        h[4 * g] = v.x;
+        h[4 * g + 1] = v.y;
+        h[4 * g + 2] = v.z;
+        h[4 * g + 3] = v.w;
+    }
+#pragma unroll
+    for (int g = 0; g < NC; ++g) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(a.coefp) + m * NC + g);
+        kc[4 * g] = v.x;
+        kc[4 * g + 1] = v.y;
+        kc[4 * g + 2] = v.z;
+        kc[4 * g + 3] = v.w;
+    }
+    for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB) gsm[k] = 0.0;
+    // forward inputs of every section at this step
+    float xin[S];
+    float in = __fsub_rn(rec.y, rec.z);
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+        xin[q] = in;
+        float yv = __fmaf_rn(kc[5 * q], in, __fmul_rn(kc[5 * q + 1], h[2 * q]));
+        yv = __fmaf_rn(kc[5 * q + 2], h[2 * q + 1], yv);
+        yv = __fmaf_rn(-kc[5 * q + 3], h[2 * q + 2], yv);
+        in = __fmaf_rn(-kc[5 * q + 4], h[2 * q + 3], yv);
+    }
+    pdl_wait();
+    float4 aq[S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) aq[q] = a.ast[(uint64_t)q * a.nb + bl];
+    const AdjCorr c = adj_correct(a, a.T[pos], meta);
+    double yb = c.ybar, gv[NP];
+#pragma unroll
+    for (int j = NV; j < NP; ++j) gv[j] = 0.0;
+#pragma unroll
+    for (int q = S - 1; q >= 0; --q) {
+        const double yt = yb + (double)aq[q].z;
+        gv[5 * q] = yt * (double)xin[q];
+        gv[5 * q + 1] = yt * (double)h[2 * q];
+        gv[5 * q + 2] = yt * (double)h[2 * q + 1];
+        gv[5 * q + 3] = -yt * (double)h[2 * q + 2];
+        gv[5 * q + 4] = -yt * (double)h[2 * q + 3];
+        const double xbar = (double)kc[5 * q] * yt + (double)aq[q].x;
+        const double x1 = (double)kc[5 * q + 1] * yt + (double)aq[q].y;
+        const double x2 = (double)kc[5 * q + 2] * yt;
+        const double y1 = -(double)kc[5 * q + 3] * yt + (double)aq[q].w;
+        const double y2 = -(double)kc[5 * q + 4] * yt;
+        aq[q] = make_float4((float)x1, (float)x2, (float)y1, (float)y2);
+        yb = xbar;
+    }
+    if (act) {
+#pragma unroll
+        for (int q = 0; q < S; ++q) a.ast[(uint64_t)q * a.nb + b] = aq[q];
+        adj_store(a, b, pos, c, yb);
+    }
+    __syncthreads(); // gsm is zero
+    unsigned left = __ballot_sync(0xffffffffu, act);
+    while (left) {
+        const uint32_t mm = __shfl_sync(0xffffffffu, m, __ffs(left) - 1);
+        const bool mine = act && m == mm;
+        left &= ~__ballot_sync(0xffffffffu, mine);
+        double v[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) v[j] = mine ? gv[j] : 0.0;
+        int idx;
+        const double sum = warp_sums<NP>(v, &idx);
+        if (idx < NV && (threadIdx.x & (32 / NP - 1)) == 0) atomicAdd(gsm + mm * NV + idx, sum);
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB)
+        if (gsm[k] != 0.0) atomicAdd(a.grad + k, gsm[k]);
 }
 
 } // namespace
@@ -345,46 +318,26 @@ cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_boundary(float *T, const uint32_t *bidx, const uint8_t *bmat, const float *bw, const float *coef,
-                                const float4 *rec, const float *fst, float *ast, float *dbar, float *cq, double *grad,
-                                uint64_t nb, uint32_t nx, uint32_t ny, uint32_t px, uint32_t nsec, uint32_t nmat,
-                                int form, double K, double mix_y, double mix_d, double gain, cudaStream_t s)
+cudaError_t launch_adj_boundary(const StepArgs &f, float *T, const float4 *rec, const float *fst, float4 *ast,
+                                float *dbar, float *rr, double *grad, uint32_t nmat, bool overlap, cudaStream_t s)
 {
-    if (nb == 0) return cudaSuccess;
-    AdjArgs a{T, bidx, bmat, bw, coef, rec, fst, ast, dbar, cq, grad, nb, nx, ny, px, nsec, nmat * nsec * 5, form,
-              K, mix_y, mix_d, gain};
+    if (f.nb == 0) return cudaSuccess;
+    const AdjArgs a{T, f.bpos, f.bmeta, f.wtab, f.coef, f.coefp, rec, fst, ast, dbar, rr, grad, f.nb, f.nsec,
+                    nmat * f.nsec * 5, f.form, f.K * f.gain, f.mix_y, f.mix_d};
     const size_t sm = (size_t)a.ncoef * sizeof(double);
-    const unsigned gs = (unsigned)((nb + ABS - 1) / ABS);
-    if (nsec <= 1) k_adj_boundary_s<1><<<gs, ABS, sm, s>>>(a);
-    else if (nsec == 2) k_adj_boundary_s<2><<<gs, ABS, sm, s>>>(a);
-    else if (nsec <= 4) k_adj_boundary_s<4><<<gs, ABS, sm, s>>>(a);
-    else k_adj_boundary<<<(unsigned)((nb + AB - 1) / AB), AB, sm, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_adj_fix(float *Tn, float *Tb, const uint32_t *bidx, const float4 *rec, const float *dbar,
-                           const float *cq, uint64_t nb, uint32_t nx, uint32_t ny, uint32_t px, cudaStream_t s)
-{
-    if (nb == 0) return cudaSuccess;
-    k_adj_fix<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(Tn, Tb, bidx, rec, dbar, cq, nb, nx, ny, px);
-    return cudaGetLastError();
-}
-
-namespace {
-__global__ void k_zero_at(float *f, const uint32_t *__restrict pos, uint32_t n)
-{
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) f[pos[k]] = 0.f;
-}
-} // namespace
-
-// the adjoint at the hard-source voxels is 0 (their forward value does not
-// depend on the field); the stencil leaves them alone
-cudaError_t launch_zero_at(float *f, const uint32_t *pos, uint32_t n, cudaStream_t s)
-{
-    if (n == 0) return cudaSuccess;
-    k_zero_at<<<(n + 255) / 256, 256, 0, s>>>(f, pos, n);
-    return cudaGetLastError();
+    const unsigned g = (unsigned)((f.nb + AB - 1) / AB);
+    const auto run = [&](void (*kern)(AdjArgs)) {
+        if (overlap) return launch_overlapped(kern, g, AB, sm, s, a);
+        kern<<<g, AB, sm, s>>>(a);
+        return cudaGetLastError();
+    };
+    switch (f.nsec) {
+    case 1: return run(k_adj_boundary_s<1>);
+    case 2: return run(k_adj_boundary_s<2>);
+    case 3: return run(k_adj_boundary_s<3>);
+    case 4: return run(k_adj_boundary_s<4>);
+    default: return run(k_adj_boundary);
+    }
 }
 
 namespace {

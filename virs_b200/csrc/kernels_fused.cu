@@ -35,6 +35,7 @@
 // then waits for the previous step's grid.
 #include <type_traits>
 
+#include "pdl.cuh"
 #include "step_voxel.cuh"
 
 namespace virs {
@@ -43,9 +44,6 @@ namespace {
 using namespace step;
 
 constexpr int FB = 256;
-
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Four voxels of a row in one load: 16 bytes in FP32, 8 in 16-bit storage
 // (eight per thread would need 77 registers, too few warps for this kernel).
@@ -122,38 +120,12 @@ template <typename T> __device__ __forceinline__ void post_owned(const PostArgs 
     }
 }
 
-template <typename T, int MAXS, int MODE, bool SR>
-__device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &po, uint32_t blk, uint32_t gb, uint32_t gx)
+// the four voxels at position i of a plane's row, after the wait; `act`
+// false: nothing stored
+template <typename T, bool SR>
+__device__ __forceinline__ void step_vec(const StepArgs &a, const Codes<V> &code, uint32_t i, uint32_t plane, bool act)
 {
     using IO = Io<T>;
-    const uint32_t tid = threadIdx.x;
-    if (blk < gb) {
-        const uint64_t s0 = (uint64_t)blk * FB + tid;
-        const Owned own{true, blk * FB, blk * FB + FB, 0u};
-        const bool mine = owns_any(po, own), act = s0 < a.nb;
-        BVox<T, MAXS> v;
-        if (act) bvox_site<T, MODE, MAXS>(a, s0, v);
-        pdl_wait();
-        if (act) {
-            bvox_values<T, MODE, MAXS>(a, s0, v);
-            bvox_update<T, MODE, MAXS>(a, s0, v);
-        }
-        if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
-        post_owned<T>(po, own, mine);
-        return;
-    }
-    const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
-    const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
-    const bool act = first + tid * V < plane;
-    const Owned own{false, first, first + FB * V, z};
-    const bool mine = owns_any(po, own);
-    // the last block of a plane repeats the plane's last vector, unstored
-    const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
-    Codes<V> code;
-    code.load(a.code + i);
-    pdl_wait();
-    if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
-
     const T *P = static_cast<const T *>(a.p);
     T *Q = static_cast<T *>(a.q);
     Vec<T> c, zp, zm, yp, ym, q;
@@ -174,7 +146,7 @@ __device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &p
     q.get(fq);
     air_update(fc, left, right, fyp, fym, fzp, fzm, fq, c2dt2, inv_h2, r);
     if (act) {
-        const uint32_t srk = SR ? sr_step_key(*po.ctr, 0u) : 0u;
+        const uint32_t srk = SR ? sr_step_key(*a.ctr, 0u) : 0u;
         if (!code.any()) {
             put4<T, SR>(Q + i, r, i, a.sr_base, srk);
         } else {
@@ -196,13 +168,46 @@ __device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &p
                 float v = r[j];
                 if (cj == CODE_WALL) v = 0.f;
                 else if (cj == CODE_HARD) {
-                    const uint32_t sn = *po.ctr;
+                    const uint32_t sn = *a.ctr;
                     v = sn < a.nhard ? a.hard[sn] : 0.f;
                 }
                 Q[i + j] = SR ? Sr<T>::put(v, sr_bits((uint64_t)i + j, a.sr_base, srk)) : IO::put(v);
             }
         }
     }
+}
+
+template <typename T, int MAXS, int MODE, bool SR>
+__device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &po, uint32_t blk, uint32_t gb, uint32_t gx)
+{
+    const uint32_t tid = threadIdx.x;
+    if (blk < gb) {
+        const uint64_t s0 = (uint64_t)blk * FB + tid;
+        const Owned own{true, blk * FB, blk * FB + FB, 0u};
+        const bool mine = owns_any(po, own), act = s0 < a.nb;
+        BVox<T, MAXS> v;
+        if (act) bvox_site<T, MAXS>(a, s0, v);
+        pdl_wait();
+        if (act) {
+            bvox_values<T, MAXS>(a, s0, v);
+            bvox_update<T, MODE, MAXS>(a, s0, v);
+        }
+        if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
+        post_owned<T>(po, own, mine);
+        return;
+    }
+    const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
+    const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
+    const bool act = first + tid * V < plane;
+    const Owned own{false, first, first + FB * V, z};
+    const bool mine = owns_any(po, own);
+    // the last block of a plane repeats the plane's last vector, unstored
+    const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
+    Codes<V> code;
+    code.load(a.code + i);
+    pdl_wait();
+    if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
+    step_vec<T, SR>(a, code, i, plane, act);
     post_owned<T>(po, own, mine);
 }
 
@@ -212,6 +217,62 @@ __global__ void __launch_bounds__(FB) k_fused(const __grid_constant__ StepArgs a
 {
     pdl_trigger();
     fused_block<T, MAXS, MODE, SR>(a, po, blockIdx.x, gb, gx);
+}
+
+// One step of the adjoint fields after the transposed correction
+// (kernels_adjoint.cu): the stencil T' = A F - RR (F in a.p, RR and then T'
+// in a.q), at a boundary slot T' = (the mirrored leapfrog on F with the
+// slot's own RR) + dbar, and on what a block wrote the sources' gradients
+// and the receivers' loss gradients of the next reverse step n (n < 0: none).
+// RR at boundary voxels lives in an array per slot (rr), not in the field, so
+// that no slot's RR is overwritten while its neighbours read F from the same
+// buffer.
+__global__ void __launch_bounds__(FB) k_adj_step(const __grid_constant__ StepArgs a, const __grid_constant__ AdjPost po,
+                                                 uint32_t gb, uint32_t gx)
+{
+    pdl_trigger();
+    const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+    Owned own;
+    bool mine = false;
+    const uint32_t np = po.n < 0 ? 0u : po.nsrc + po.nrcv;
+    if (blk < gb) {
+        const uint64_t s0 = (uint64_t)blk * FB + tid;
+        own = Owned{true, blk * FB, blk * FB + FB, 0u};
+        for (uint32_t k = tid; k < np; k += FB) mine |= own.has(po.probe[k]);
+        const bool act = s0 < a.nb;
+        BVox<float, 0> v;
+        if (act) bvox_site<float, 0>(a, s0, v);
+        pdl_wait();
+        if (act) {
+            bvox_values<float, 0>(a, s0, v);
+            const float r = leapfrog((uint8_t)v.meta, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5],
+                                     po.rr[s0], a.c2dt2, a.inv_h2);
+            static_cast<float *>(a.q)[v.i] = __fadd_rn(r, po.dbar[s0]);
+        }
+    } else {
+        const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
+        const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
+        const bool act = first + tid * V < plane;
+        own = Owned{false, first, first + FB * V, z};
+        for (uint32_t k = tid; k < np; k += FB) mine |= own.has(po.probe[k]);
+        const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
+        Codes<V> code;
+        code.load(a.code + i);
+        pdl_wait();
+        step_vec<float, false>(a, code, i, plane, act);
+    }
+    if (!__syncthreads_or(mine)) return;
+    float *T = static_cast<float *>(a.q);
+    for (uint32_t k = tid; k < po.nrcv; k += FB) {
+        const Probe p = po.probe[po.nsrc + k];
+        // a receiver on a voxel that no step updates reads a constant
+        if (own.has(p) && a.code[p.pos] < CODE_HARD) atomicAdd(T + p.pos, po.dl[(uint64_t)k * po.stride + (uint64_t)po.n]);
+    }
+    __syncthreads();
+    for (uint32_t k = tid; k < po.nsrc; k += FB) {
+        const Probe p = po.probe[k];
+        if (own.has(p)) po.gsig[(uint64_t)k * po.stride + (uint64_t)po.n] = T[p.pos];
+    }
 }
 
 // Many simulations: a table gives each block its member and its number in
@@ -257,16 +318,7 @@ __global__ void k_probe_slots(Probe *probe, uint32_t n, const uint32_t *__restri
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, cudaStream_t s, const A &...args)
 {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(FB);
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    return launch_overlapped(kern, grid, FB, 0, s, args...);
 }
 
 template <typename T, int MODE, bool SR>
@@ -290,13 +342,22 @@ template <typename T> cudaError_t fused_16(const StepArgs &a, const PostArgs &po
 
 } // namespace
 
-cudaError_t launch_fused(int storage, const StepArgs &a, const PostArgs &po, cudaStream_t s)
+cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, cudaStream_t s)
 {
     switch (storage) {
     case VIRS_STORAGE_F16: return fused_16<__half>(a, po, s);
     case VIRS_STORAGE_BF16: return fused_16<__nv_bfloat16>(a, po, s);
-    default: return fused_by_sections<float, BND_UPDATE, false>(a, po, s);
+    default:
+        return mode == BND_KEEP ? fused_by_sections<float, BND_KEEP, false>(a, po, s)
+                                : fused_by_sections<float, BND_UPDATE, false>(a, po, s);
     }
+}
+
+cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, cudaStream_t s)
+{
+    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB);
+    const uint32_t gx = (a.px * a.ny + FB * V - 1) / (FB * V);
+    return launch_pdl(k_adj_step, gb + gx * (a.nz - 2), s, a, po, gb, gx);
 }
 
 namespace {

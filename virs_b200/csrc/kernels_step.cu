@@ -170,8 +170,6 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_step(const __grid
 //   BND_UPDATE  leapfrog + filters, the result written to p^{n+1}
 //   BND_KEEP    the same, and the record {free value, p, p^{n-1}} of the
 //               slot kept in a.side (the adjoint's recomputation)
-//   BND_RECORD  the record only: no filters, nothing written to the fields
-//               (the adjoint step, on adjoint fields)
 // The compacted boundary pass (simulator_gpu.cu:105-150), in list order.
 // The stencil kernels left these voxels untouched (p^{n-1} in place); the
 // pass gathers the seven p values from the p^n buffer (not written during
@@ -185,8 +183,6 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_step(const __grid
 //   BND_UPDATE  the step
 //   BND_KEEP    the same, and the record {free value, p, p^{n-1}} of the
 //               slot kept in a.side (the adjoint's recomputation)
-//   BND_RECORD  the record only: no filters, nothing written to the fields
-//               (the adjoint step, on adjoint fields)
 constexpr int BT = 256;
 
 template <typename T, int MODE, int MAXS>
@@ -196,7 +192,7 @@ __global__ void __launch_bounds__(BT) k_boundary(const __grid_constant__ StepArg
     const uint64_t s0 = (uint64_t)blockIdx.x * BT + threadIdx.x;
     if (s0 >= a.nb) return;
     BVox<T, MAXS> v;
-    bvox_load<T, MODE, MAXS>(a, s0, v);
+    bvox_load<T, MAXS>(a, s0, v);
     bvox_update<T, MODE, MAXS>(a, s0, v);
 }
 
@@ -250,7 +246,7 @@ __global__ void __launch_bounds__(BT) k_boundary_fix(const __grid_constant__ Ste
         const uint64_t s0 = (uint64_t)blockIdx.x * BT + threadIdx.x;
         if (s0 >= a.nb) return;
         BVox<T, MAXS> v;
-        bvox_load<T, BND_UPDATE, MAXS>(a, s0, v);
+        bvox_load<T, MAXS>(a, s0, v);
         bvox_update<T, BND_UPDATE, MAXS>(a, s0, v);
         return;
     }
@@ -302,14 +298,14 @@ __global__ void __launch_bounds__(256) k_boundary_batch(const BatchMember *__res
         __syncthreads();
         if (g >= ntotal) return;
         BVox<T, MAXS> v;
-        bvox_load<T, BND_UPDATE, MAXS>(sa, g - sfirst, v);
+        bvox_load<T, MAXS>(sa, g - sfirst, v);
         bvox_update<T, BND_UPDATE, MAXS>(sa, g - sfirst, v);
         return;
     }
     if (g >= ntotal) return;
     const BatchMember &b = mem[batch_member_of(mem, m0, m1, g)];
     BVox<T, MAXS> v;
-    bvox_load<T, BND_UPDATE, MAXS>(b.step[parity], g - b.first_bnd, v);
+    bvox_load<T, MAXS>(b.step[parity], g - b.first_bnd, v);
     bvox_update<T, BND_UPDATE, MAXS>(b.step[parity], g - b.first_bnd, v);
 }
 
@@ -422,7 +418,7 @@ namespace {
 template <typename T, int MODE>
 void boundary_by_sections(uint32_t ns, unsigned g, const StepArgs &a, cudaStream_t s)
 {
-    if (MODE == BND_RECORD || ns <= 1) k_boundary<T, MODE, 1><<<g, BT, 0, s>>>(a);
+    if (ns <= 1) k_boundary<T, MODE, 1><<<g, BT, 0, s>>>(a);
     else if (ns == 2) k_boundary<T, MODE, 2><<<g, BT, 0, s>>>(a);
     else if (ns == 3) k_boundary<T, MODE, 3><<<g, BT, 0, s>>>(a);
     else if (ns == 4) k_boundary<T, MODE, 4><<<g, BT, 0, s>>>(a);
@@ -433,7 +429,6 @@ template <typename T> void boundary_by_mode(int mode, uint32_t ns, unsigned g, c
 {
     switch (mode) {
     case BND_KEEP: boundary_by_sections<T, BND_KEEP>(ns, g, a, s); break;
-    case BND_RECORD: boundary_by_sections<T, BND_RECORD>(ns, g, a, s); break;
     default: boundary_by_sections<T, BND_UPDATE>(ns, g, a, s); break;
     }
 }

@@ -298,17 +298,27 @@ __device__ __forceinline__ float2 leapfrog_air2(float2 ce, float2 x2, float2 yp,
 // does), then p+ -= K*(0.1*y + 0.9*d)*0.4 (times the sponge weight) in
 // double, or the centered form of the same correction.
 
+// num / den, correctly rounded, with rden the correctly rounded 1 / den and
+// den in [1, 2^1000]: num * rden and two corrections with the exact residual.
+// The last one is correctly rounded when the value before is within an ulp
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Infinities and NaN as the division gives
+// them.
+__device__ __forceinline__ double quotient(double num, double den, double rden)
+{
+    const double q0 = __dmul_rn(num, rden);
+    const double q1 = __fma_rn(__fma_rn(-q0, den, num), rden, q0);
+    const double q2 = __fma_rn(__fma_rn(-q1, den, num), rden, q1);
+    return fabs(q0) <= 1.7976931348623157e308 ? q2 : q0;
+}
+
 // The correction, given the cascade output y (double precision).  What it
 // needs of the sponge weight alone comes from the table of a.wtab (one entry
-// per squared distance, BndWeight in internal.hpp), the centered form's
-// quotient by 1 + a included: num / den is rounded from num * (1 / den) by
-// two corrections with the exact residual, which gives the correctly rounded
-// quotient when the reciprocal is correctly rounded and the next-to-last
-// value is within an ulp (P. Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", 1990).  With a division per voxel,
-// the weight as a float, and code, material and weight in three arrays, the
-// pass over 14.1 M slots (512x384x192, sponge 16, three sections) took 206 us
-// at 379 instructions per warp and 1.19 GB moved; 204 us now, 5.7 TB/s.
+// per squared distance, BndWeight in internal.hpp), the reciprocal of the
+// centered form's 1 + a included.  With a division per voxel, the weight as
+// a float, and code, material and weight in three arrays, the pass over
+// 14.1 M slots (512x384x192, sponge 16, three sections) took 206 us at 379
+// instructions per warp and 1.19 GB moved; 204 us now, 5.7 TB/s.
 __device__ __forceinline__ float correct(const StepArgs &a, float r, float d, float y, float qv, uint32_t meta)
 {
     const double2 *e = reinterpret_cast<const double2 *>(a.wtab + (meta >> 16));
@@ -323,10 +333,7 @@ __device__ __forceinline__ float correct(const StepArgs &a, float r, float d, fl
     const double kgw = e0.x, ac = e0.y, den = e1.x, rden = e1.y;
     const double num = __dadd_rn(__dsub_rn((double)r, __dmul_rn(kgw, __dmul_rn((double)y, a.mix_y))),
                                  __dmul_rn(ac, (double)qv));
-    const double q0 = __dmul_rn(num, rden);
-    const double q1 = __fma_rn(__fma_rn(-q0, den, num), rden, q0);
-    const double q2 = __fma_rn(__fma_rn(-q1, den, num), rden, q1);
-    return __double2float_rn(fabs(q0) <= 1.7976931348623157e308 ? q2 : q0); // infinities and NaN as the division gives them
+    return __double2float_rn(quotient(num, den, rden));
 }
 
 // Filter states.  In a cascade the output of section q is the input of

@@ -103,7 +103,7 @@ template <typename T, int MAXS> struct BVox {
 };
 
 // what no step writes: where the voxel is and its code
-template <typename T, int MODE, int MAXS>
+template <typename T, int MAXS>
 __device__ __forceinline__ void bvox_site(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
 {
     v.i = __ldg(a.bpos + slot);
@@ -111,8 +111,8 @@ __device__ __forceinline__ void bvox_site(const StepArgs &a, uint64_t slot, BVox
     v.nm = a.rigid ? __ldg(a.bnrm + slot) : 0;
 }
 
-// the pressures around it and its filter states
-template <typename T, int MODE, int MAXS>
+// the pressures around it and its filter states (MAXS == 0: not the states)
+template <typename T, int MAXS>
 __device__ __forceinline__ void bvox_values(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
 {
     using IO = Io<T>;
@@ -127,14 +127,14 @@ __device__ __forceinline__ void bvox_values(const StepArgs &a, uint64_t slot, BV
     v.nb[3] = IO::get(P[i - sy]);
     v.nb[4] = IO::get(P[i + sz]);
     v.nb[5] = IO::get(P[i - sz]);
-    if (MODE != BND_RECORD && MAXS != 0) bload<MAXS>(a, slot, v.st);
+    if constexpr (MAXS != 0) bload<MAXS>(a, slot, v.st);
 }
 
-template <typename T, int MODE, int MAXS>
+template <typename T, int MAXS>
 __device__ __forceinline__ void bvox_load(const StepArgs &a, uint64_t slot, BVox<T, MAXS> &v)
 {
-    bvox_site<T, MODE, MAXS>(a, slot, v);
-    bvox_values<T, MODE, MAXS>(a, slot, v);
+    bvox_site<T, MAXS>(a, slot, v);
+    bvox_values<T, MAXS>(a, slot, v);
 }
 
 template <typename T, int MODE, int MAXS>
@@ -154,7 +154,6 @@ __device__ __forceinline__ void bvox_update(const StepArgs &a, uint64_t slot, co
         r = leapfrog((uint8_t)v.meta, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5], v.qv, a.c2dt2, a.inv_h2);
     }
     if (MODE != BND_UPDATE) a.side[slot] = make_float4(r, v.ce, v.qv, 0.f);
-    if (MODE == BND_RECORD) return;
     if constexpr (MAXS != 0) r = bcompute<MAXS>(a, r, v.ce, v.qv, slot, v.meta, v.st);
     else r = boundary_loop(a, r, v.ce, v.qv, slot, v.meta);
     static_cast<T *>(a.q)[v.i] =
