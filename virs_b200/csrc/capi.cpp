@@ -11,6 +11,8 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <iterator>
+#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -47,20 +49,170 @@ virs_status cuda_fail(cudaError_t e, const char *what)
     return VIRS_E_CUDA;
 }
 
-virs_status DevBuf::alloc(size_t n, const char *what)
+// Freed device blocks kept for the next allocation of their size.  A program
+// that sets up room after room, or takes gradient after gradient, would
+// otherwise spend more time in cudaMalloc and cudaFree than on the GPU (33 of
+// each per room: 14 of 20 ms for a 320x240x160 one, 36 of 50 ms for a hall of
+// 403 M voxels).  Bounds: the blocks of a device total at most a sixteenth of
+// its memory (the oldest go first); an allocation that fails gives all of
+// them back and tries again; when the last handle on the device is destroyed,
+// the blocks go that nobody took since the last time that happened.  A block
+// enters only from a Recycle scope, whose owner has waited for the work that
+// used it; every access is under the mutex.
+namespace {
+struct DevPool {
+    struct Block {
+        void *ptr;
+        size_t size;
+        uint64_t age;
+    };
+    std::mutex mu;
+    std::list<Block> blocks; // oldest first
+    size_t cached = 0, limit = 0;
+    uint64_t age = 0;
+    int handles = 0;
+
+    void drop(std::list<Block>::iterator it)
+    {
+        cudaFree(it->ptr);
+        cached -= it->size;
+        blocks.erase(it);
+    }
+    void *take(size_t n, size_t *size)
+    {
+        auto best = blocks.end();
+        for (auto it = blocks.begin(); it != blocks.end(); ++it)
+            if (it->size >= n && it->size <= n + n / 8 && (best == blocks.end() || it->size < best->size)) best = it;
+        if (best == blocks.end()) return nullptr;
+        void *p = best->ptr;
+        *size = best->size;
+        cached -= best->size;
+        blocks.erase(best);
+        return p;
+    }
+    void put(void *p, size_t size)
+    {
+        if (limit == 0) {
+            size_t fr = 0, total = 0;
+            limit = cudaMemGetInfo(&fr, &total) == cudaSuccess ? std::max<size_t>(total / 16, 1) : 1;
+        }
+        if (size > limit) {
+            cudaFree(p);
+            return;
+        }
+        while (cached + size > limit) drop(blocks.begin());
+        blocks.push_back({p, size, age});
+        cached += size;
+    }
+};
+constexpr int MAX_DEV = 64;
+// never destroyed: a handle may outlive the statics of a library's unload
+DevPool *dev_pool()
 {
-    release();
+    static DevPool *pools = new DevPool[MAX_DEV];
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < MAX_DEV ? pools + dev : nullptr;
+}
+thread_local int g_recycle = 0;
+
+// device buffers released in this scope go to the pool; no work in flight
+// may use them
+struct Recycle {
+    Recycle() { ++g_recycle; }
+    ~Recycle() { --g_recycle; }
+    Recycle(const Recycle &) = delete;
+    Recycle &operator=(const Recycle &) = delete;
+};
+// scratch buffers of a function: declare Scratch, then the buffers, then
+// Scratch::End, which on every way out waits for the stream before the
+// buffers go to the pool
+struct Scratch {
+    bool on = false;
+    ~Scratch()
+    {
+        if (on) --g_recycle;
+    }
+    struct End {
+        Scratch &s;
+        cudaStream_t st;
+        ~End()
+        {
+            if (cudaStreamSynchronize(st) == cudaSuccess) {
+                s.on = true;
+                ++g_recycle;
+            }
+        }
+    };
+};
+
+// handles on a device: the last one's end ages the pool
+void pool_handle(int step)
+{
+    DevPool *p = dev_pool();
+    if (!p) return;
+    std::lock_guard<std::mutex> g(p->mu);
+    p->handles += step;
+    if (p->handles > 0 || step > 0) return;
+    for (auto it = p->blocks.begin(); it != p->blocks.end();) {
+        auto next = std::next(it);
+        if (it->age < p->age) p->drop(it);
+        it = next;
+    }
+    ++p->age;
+}
+} // namespace
+
+void DevBuf::release()
+{
+    if (ptr) {
+        DevPool *p = g_recycle ? dev_pool() : nullptr;
+        if (p) {
+            std::lock_guard<std::mutex> g(p->mu);
+            p->put(ptr, cap);
+        } else {
+            cudaFree(ptr);
+        }
+    }
+    ptr = nullptr;
+    bytes = cap = 0;
+}
+
+virs_status DevBuf::alloc(size_t n, const char *what, cudaStream_t st, bool zero)
+{
     if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc(&ptr, n);
-    if (e != cudaSuccess) {
-        ptr = nullptr;
-        cudaGetLastError();
-        return fail(VIRS_E_OOM, std::string("cudaMalloc of ") + std::to_string(n) + " bytes for " + what + " failed: " +
-                                    cudaGetErrorString(e));
+    if (!ptr || cap < n || cap > n + n / 2 + (1u << 20)) {
+        release();
+        // blocks of whole 512 bytes, large ones of 2 MiB as the driver maps them
+        const size_t unit = n >= (16u << 20) ? (2u << 20) : 512, size = (n + unit - 1) / unit * unit;
+        DevPool *p = dev_pool();
+        if (p) {
+            std::lock_guard<std::mutex> g(p->mu);
+            cap = size;
+            ptr = p->take(size, &cap);
+        }
+        if (!ptr) {
+            cap = size;
+            cudaError_t e = cudaMalloc(&ptr, size);
+            if (e != cudaSuccess && p) {
+                ptr = nullptr;
+                cudaGetLastError();
+                std::lock_guard<std::mutex> g(p->mu);
+                while (!p->blocks.empty()) p->drop(p->blocks.begin());
+                e = cudaMalloc(&ptr, size);
+            }
+            if (e != cudaSuccess) {
+                ptr = nullptr;
+                cap = 0;
+                cudaGetLastError();
+                return fail(VIRS_E_OOM, std::string("cudaMalloc of ") + std::to_string(n) + " bytes for " + what +
+                                            " failed: " + cudaGetErrorString(e));
+            }
+        }
     }
     bytes = n;
-    e = cudaMemsetAsync(ptr, 0, n, cudaStreamPerThread);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
+    if (!zero) return VIRS_OK;
+    cudaError_t e = cudaMemsetAsync(ptr, 0, n, st ? st : cudaStreamPerThread);
+    if (e == cudaSuccess && !st) e = cudaStreamSynchronize(cudaStreamPerThread);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemset");
     return VIRS_OK;
 }
@@ -181,6 +333,9 @@ struct virs_sim {
     DevBuf ctr;                    // two words: the step of buffer parity k reads word k and writes the next step's to the other
     DevBuf probe;                  // sources and receivers for the one-launch step (kernels_fused.cu)
     bool probe_ok = false;
+    uint64_t ctr_at = 0;           // the step the counter word of parity `cur` holds
+    mutable std::atomic<bool> waits{false}; // kernels with bounded waits queued since check_err
+    float *host_word = nullptr;    // pinned: virs_step's sample
     uint64_t steps_done = 0;
 
     // constants
@@ -224,7 +379,11 @@ struct virs_sim {
     // CUDA graphs for GRAPH_STEPS steps, one per parity of `cur`
     static constexpr int GRAPH_STEPS = 32;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    bool graph_dirty = true;
+    bool graph_dirty = true;       // something changed since the graphs were made
+    struct GraphKey {              // the arguments the graphs hold; what else they hold drops them when it changes
+        StepArgs step[2];
+        PostArgs post[2];
+    } graph_key;
     uint64_t gen = 0;              // bumped on every change of buffers or parameters
 
     // timing
@@ -242,6 +401,7 @@ struct virs_sim {
     uint64_t stop_step = 0;
 
     DevBuf energy_partial;
+    DevBuf post_sos, post_filt, post_res, post_peak; // workspaces of virs_postprocess_ir / _sinc
 
     // adjoint: checkpoints of a forward run and the reverse-pass buffers
     struct {
@@ -261,15 +421,20 @@ struct virs_sim {
         if (xdone) cudaEventDestroy(xdone);
         if (xstream) cudaStreamDestroy(xstream);
         if (stream) cudaStreamDestroy(stream);
+        if (host_word) cudaFreeHost(host_word);
     }
 
-    void drop_graphs()
+    void destroy_graphs()
     {
         for (auto &g : graph)
             if (g) {
                 cudaGraphExecDestroy(g);
                 g = nullptr;
             }
+    }
+    void drop_graphs()
+    {
+        destroy_graphs();
         graph_dirty = true;
         ++gen;
     }
@@ -306,7 +471,7 @@ virs_status upload_hard(virs_sim *s)
 {
     std::vector<float> v(s->hard_host.size());
     for (size_t i = 0; i < v.size(); ++i) v[i] = s->hard_host[i] * s->scale;
-    VIRS_TRY(s->hard.alloc(v.size() * sizeof(float), "hard source schedule"));
+    VIRS_TRY(s->hard.alloc(v.size() * sizeof(float), "hard source schedule", s->stream, false));
     if (!v.empty()) VIRS_CUDA(copy_on(s->stream, s->hard.ptr, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice));
     s->nhard = (uint32_t)v.size();
     s->graph_dirty = true;
@@ -320,8 +485,8 @@ virs_status upload_filters(virs_sim *s, const float *k)
     const size_t per = (size_t)s->nsec * 5, pad = (per + 3) / 4 * 4;
     std::vector<float> p(s->nmat * pad, 0.f);
     for (size_t m = 0; m < s->nmat; ++m) std::copy_n(k + m * per, per, p.begin() + (ptrdiff_t)(m * pad));
-    VIRS_TRY(s->coef.alloc(s->nmat * per * sizeof(float), "filter coefficients"));
-    VIRS_TRY(s->coefp.alloc(p.size() * sizeof(float), "filter coefficients"));
+    VIRS_TRY(s->coef.alloc(s->nmat * per * sizeof(float), "filter coefficients", s->stream, false));
+    VIRS_TRY(s->coefp.alloc(p.size() * sizeof(float), "filter coefficients", s->stream, false));
     VIRS_CUDA(copy_on(s->stream, s->coef.ptr, k, s->nmat * per * sizeof(float), cudaMemcpyHostToDevice));
     VIRS_CUDA(copy_on(s->stream, s->coefp.ptr, p.data(), p.size() * sizeof(float), cudaMemcpyHostToDevice));
     return VIRS_OK;
@@ -355,7 +520,7 @@ virs_status build_weights(virs_sim *s, const std::vector<float> &w)
         const double ac = kgw * s->prm.mix_direct * 0.5;
         t[d] = {kgw, ac, 1.0 + ac, 1.0 / (1.0 + ac)};
     }
-    VIRS_TRY(s->wtab.alloc(t.size() * sizeof(BndWeight), "boundary weights"));
+    VIRS_TRY(s->wtab.alloc(t.size() * sizeof(BndWeight), "boundary weights", s->stream, false));
     VIRS_CUDA(copy_on(s->stream, s->wtab.ptr, t.data(), t.size() * sizeof(BndWeight), cudaMemcpyHostToDevice));
     return VIRS_OK;
 }
@@ -447,13 +612,13 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
                       &s->spare[0], &s->spare[1], &s->plist, &s->pzmask})
         b->release();
     const size_t ext = (size_t)s->px * ny * s->ext_nz;
-    VIRS_TRY(s->flags_raw.alloc(ext, "flags"));
-    VIRS_TRY(s->wall_mat.alloc(ext, "wall materials"));
+    VIRS_TRY(s->flags_raw.alloc(ext, "flags", s->stream));
+    VIRS_TRY(s->wall_mat.alloc(ext, "wall materials", s->stream));
     if (flags) VIRS_TRY(h2d_rows(s->flags_raw.ptr, flags, 1, s, s->ext_nz));
     if (wmat) VIRS_TRY(h2d_rows(s->wall_mat.ptr, wmat, 1, s, s->ext_nz));
-    VIRS_TRY(s->flags.alloc(s->nvox, "classified flags"));
-    VIRS_TRY(s->field[0].alloc(s->nvox * s->storage_bytes(), "pressure field"));
-    VIRS_TRY(s->field[1].alloc(s->nvox * s->storage_bytes(), "pressure field"));
+    VIRS_TRY(s->flags.alloc(s->nvox, "classified flags", s->stream));
+    VIRS_TRY(s->field[0].alloc(s->nvox * s->storage_bytes(), "pressure field", s->stream));
+    VIRS_TRY(s->field[1].alloc(s->nvox * s->storage_bytes(), "pressure field", s->stream));
     s->cur = 0;
     s->nb = 0;
     s->steps_done = 0;
@@ -528,15 +693,17 @@ virs_status install_mesh(virs_sim *s, const Mesh &m, uint32_t part = 0, uint32_t
     std::memcpy(s->bmin, bmin, sizeof(bmin));
     if (ntri) {
         const size_t nvx = (size_t)s->px * s->ny * s->ext_nz; // the uploaded planes
+        Scratch scratch;
         DevBuf dv, dt, dm, dr, tri, la, lw, mx;
-        VIRS_TRY(dv.alloc(m.verts.size() * sizeof(float), "mesh vertices"));
-        VIRS_TRY(dt.alloc(m.tris.size() * sizeof(uint32_t), "mesh triangles"));
-        VIRS_TRY(dm.alloc(ntri * sizeof(int32_t), "triangle materials"));
-        VIRS_TRY(dr.alloc(std::max<size_t>(s->roles.size(), 1), "material roles"));
-        VIRS_TRY(tri.alloc(ntri * voxelize_tri_bytes(), "triangle table"));
-        VIRS_TRY(la.alloc(nvx * sizeof(uint32_t), "voxelisation marks"));
-        VIRS_TRY(lw.alloc(nvx * sizeof(uint32_t), "voxelisation marks"));
-        VIRS_TRY(mx.alloc(sizeof(uint32_t), "wall material maximum"));
+        Scratch::End end{scratch, s->stream};
+        VIRS_TRY(dv.alloc(m.verts.size() * sizeof(float), "mesh vertices", s->stream, false));
+        VIRS_TRY(dt.alloc(m.tris.size() * sizeof(uint32_t), "mesh triangles", s->stream, false));
+        VIRS_TRY(dm.alloc(ntri * sizeof(int32_t), "triangle materials", s->stream, false));
+        VIRS_TRY(dr.alloc(std::max<size_t>(s->roles.size(), 1), "material roles", s->stream, false));
+        VIRS_TRY(tri.alloc(ntri * voxelize_tri_bytes(), "triangle table", s->stream, false));
+        VIRS_TRY(la.alloc(nvx * sizeof(uint32_t), "voxelisation marks", s->stream));
+        VIRS_TRY(lw.alloc(nvx * sizeof(uint32_t), "voxelisation marks", s->stream));
+        VIRS_TRY(mx.alloc(sizeof(uint32_t), "wall material maximum", s->stream));
         VIRS_CUDA(copy_on(s->stream, dv.ptr, m.verts.data(), dv.bytes, cudaMemcpyHostToDevice));
         VIRS_CUDA(copy_on(s->stream, dt.ptr, m.tris.data(), dt.bytes, cudaMemcpyHostToDevice));
         VIRS_CUDA(copy_on(s->stream, dm.ptr, m.tri_mat.data(), dm.bytes, cudaMemcpyHostToDevice));
@@ -563,8 +730,7 @@ virs_status ensure_ir(virs_sim *s, uint64_t need)
     if (s->ircap && s->nrcv)
         VIRS_CUDA(copy2d_on(s->stream, nb.ptr, cap * sizeof(float), s->ir.ptr, s->ircap * sizeof(float),
                                s->ircap * sizeof(float), s->nrcv, cudaMemcpyDeviceToDevice));
-    std::swap(s->ir.ptr, nb.ptr);
-    std::swap(s->ir.bytes, nb.bytes);
+    s->ir.swap(nb);
     s->ircap = cap;
     s->graph_dirty = true;
     ++s->gen;
@@ -630,7 +796,7 @@ virs_status build_maps(virs_sim *s)
 // read and clear the device error flag of the bounded waits
 virs_status check_err(virs_sim *s)
 {
-    if (!s->err.ptr) return VIRS_OK;
+    if (!s->err.ptr || !s->waits.exchange(false)) return VIRS_OK;
     int e = 0;
     VIRS_CUDA(copy_on(s->stream, &e, s->err.ptr, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
@@ -729,7 +895,7 @@ virs_status build_probes(virs_sim *s)
         const bool in = z >= 1 && z + 1 < s->nz;
         h[k] = {in ? z : 1u, in ? (uint32_t)(d % plane) : 0u, PROBE_NO_SLOT, (uint32_t)d};
     }
-    VIRS_TRY(s->probe.alloc(std::max<uint32_t>(n, 1) * sizeof(Probe), "probes"));
+    VIRS_TRY(s->probe.alloc(std::max<uint32_t>(n, 1) * sizeof(Probe), "probes", s->stream, false));
     if (n) VIRS_CUDA(copy_on(s->stream, s->probe.ptr, h.data(), n * sizeof(Probe), cudaMemcpyHostToDevice));
     VIRS_CUDA(launch_probe_slots(s->probe.as<Probe>(), n, s->bpos.as<uint32_t>(), s->nb, s->stream));
     s->probe_ok = true;
@@ -837,6 +1003,7 @@ PostArgs post_args(const virs_sim *s, int parity)
 cudaError_t launch_stencil(const virs_sim *s, int parity, cudaStream_t st)
 {
     if (s->depth == 0) return launch_step(s->prm.storage, s->tile_rows, step_args(s, parity), st);
+    s->waits = true;
     const TmaMaps m{&s->tmP[parity], &s->tmQ[parity ^ 1], &s->tmC};
     return launch_step_tma(s->prm.storage, s->tile_rows, s->depth, step_args(s, parity), m, s->err.as<int>(), st);
 }
@@ -852,6 +1019,7 @@ cudaError_t launch_stencil_range(const virs_sim *s, int parity, cudaStream_t st,
                        s->zmi_zc == eff_planes(s);
     a.tzmask = inner ? s->zmask_in.as<uint64_t>() : nullptr;
     if (s->depth == 0) return launch_step(s->prm.storage, s->tile_rows, a, st);
+    s->waits = true;
     const TmaMaps m{&s->tmP[parity], &s->tmQ[parity ^ 1], &s->tmC};
     return launch_step_tma(s->prm.storage, s->tile_rows, s->depth, a, m, s->err.as<int>(), st);
 }
@@ -884,10 +1052,12 @@ virs_status build_pair_list(virs_sim *s)
 {
     cudaStream_t st = s->stream;
     const size_t nseg = mark_segments(s->nvox);
+    Scratch scratch;
     DevBuf mark, cnt, tmp, total;
+    Scratch::End end{scratch, st};
     VIRS_TRY(mark.alloc(s->nvox, "provisional-voxel marks"));
     VIRS_TRY(cnt.alloc(nseg * 4, "provisional-voxel counts"));
-    VIRS_TRY(tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch"));
+    VIRS_TRY(tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch", s->stream));
     VIRS_TRY(total.alloc(4, "provisional-voxel total"));
     VIRS_CUDA(cudaMemsetAsync(mark.ptr, 0, s->nvox, st));
     VIRS_CUDA(launch_pair_marks(s->code.as<uint8_t>(), s->px, s->ny, s->nz, s->bpos.as<uint32_t>(), s->nb,
@@ -993,6 +1163,7 @@ cudaError_t enqueue_pair(const virs_sim *s, int par, int x, int y, int z, int w,
     a.zc = s->pair_zc;
     if (zero_masks_useful(s) && s->pzm_zc == s->pair_zc) a.tzmask = s->pzmask.as<uint64_t>();
     const TmaMaps m{&s->pmP[x], &s->pmQ[y], &s->pmC};
+    s->waits = true;
     if (ev) cudaEventRecord(ev[0], st);
     cudaError_t e = launch_pair_tma(sto, s->pair_rows, a, m, buf_ptr(s, z), buf_ptr(s, w), s->err.as<int>(), st);
     if (ev) cudaEventRecord(ev[1], st);
@@ -1020,10 +1191,27 @@ cudaError_t enqueue_quad(const virs_sim *s, int par, cudaStream_t st, cudaEvent_
 // boundary pass, and the second one together with the fix-up
 uint64_t pair_launches(const virs_sim *s) { return 3 + (s->nb ? 1 : 0) + (s->nb || s->nplist ? 1 : 0); }
 
-virs_status build_graphs(virs_sim *s, cudaStream_t st)
+// the graph of parity par, made when it is first needed; graphs made before
+// stay while their kernels' arguments are the same (a simulation started
+// again in the same buffers)
+virs_status ready_graph(virs_sim *s, int par, cudaStream_t st)
 {
-    s->drop_graphs();
-    for (int par = 0; par < 2; ++par) {
+    if (s->graph_dirty) {
+        virs_sim::GraphKey key;
+        std::memset(&key, 0, sizeof(key));
+        for (int k = 0; k < 2; ++k) {
+            const StepArgs a = step_args(s, k);
+            const PostArgs p = post_args(s, k);
+            std::memcpy(&key.step[k], &a, sizeof(a));
+            std::memcpy(&key.post[k], &p, sizeof(p));
+        }
+        if (std::memcmp(&key, &s->graph_key, sizeof(key)) != 0) {
+            s->destroy_graphs();
+            std::memcpy(&s->graph_key, &key, sizeof(key));
+        }
+        s->graph_dirty = false;
+    }
+    if (!s->graph[par]) {
         cudaGraph_t g = nullptr;
         VIRS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
@@ -1041,7 +1229,6 @@ virs_status build_graphs(virs_sim *s, cudaStream_t st)
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
     }
-    s->graph_dirty = false;
     return VIRS_OK;
 }
 
@@ -1141,7 +1328,7 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
             constexpr uint64_t GQ = virs_sim::GRAPH_STEPS / 4;
             uint64_t q = 0;
             if (quads >= GQ) {
-                if (s->graph_dirty) VIRS_TRY(build_graphs(s, st));
+                VIRS_TRY(ready_graph(s, s->cur, st));
                 for (; q + GQ <= quads; q += GQ) VIRS_CUDA(cudaGraphLaunch(s->graph[s->cur], st));
             }
             for (; q < quads; ++q) {
@@ -1149,19 +1336,21 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
                 if (e != cudaSuccess) return cuda_fail(e, "two-step launch");
             }
         } else if (n >= (uint64_t)virs_sim::GRAPH_STEPS) {
-            if (s->graph_dirty) VIRS_TRY(build_graphs(s, st));
+            VIRS_TRY(ready_graph(s, s->cur, st)); // an even number of steps: the parity stays
             for (; i + virs_sim::GRAPH_STEPS <= n; i += virs_sim::GRAPH_STEPS)
-                VIRS_CUDA(cudaGraphLaunch(s->graph[s->cur ^ (int)(i & 1)], st));
+                VIRS_CUDA(cudaGraphLaunch(s->graph[s->cur], st));
         }
         for (uint64_t k = 0; k < n1 - i; ++k) {
             cudaError_t e = enqueue_step(s, s->cur ^ (int)((i + k) & 1), st);
             if (e != cudaSuccess) return cuda_fail(e, "step launch");
         }
     }
+    if (quads || !fused_on(s)) s->waits = true; // a replayed graph's kernels too
     const int cur0 = s->cur;
     const uint64_t done0 = s->steps_done;
     s->cur ^= (int)(n & 1);
     s->steps_done += n;
+    s->ctr_at += n;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     if (s->stop_rule) {
         // how many of the n steps ran before the rule fired
@@ -1174,6 +1363,7 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
             s->steps_done = (uint64_t)sb[1] + 1;
             s->stopped = true;
             s->stop_step = sb[1];
+            s->ctr_at = UINT64_MAX; // where the rule left it
             if (ran <= 4 * quads) VIRS_TRY(settle_pair_stop(s, cur0, ran, st));
         }
     }
@@ -1248,6 +1438,7 @@ VIRS_EXPORT virs_status virs_create(const virs_params *p, virs_sim **out)
     s->roles[1] = VIRS_ROLE_SOURCE;
     // simulator_gpu.cu:214-218: 10 for the first 10 steps
     s->hard_host.assign(10, 10.f);
+    pool_handle(1);
     *out = s.release();
     return VIRS_OK;
 }
@@ -1259,7 +1450,12 @@ VIRS_EXPORT virs_status virs_destroy(virs_sim *s)
     // the last work queued for the handle, on its own stream or a caller's
     if (s->done) cudaEventSynchronize(s->done);
     cudaStreamSynchronize(s->stream);
-    delete s;
+    if (s->xstream) cudaStreamSynchronize(s->xstream);
+    {
+        Recycle r;
+        delete s;
+    }
+    pool_handle(-1);
     return VIRS_OK;
 }
 
@@ -1413,12 +1609,14 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         // the sponge layer over every uploaded plane (for a slab, its halo
         // planes too), then only the kept planes
         const size_t nvc = (size_t)s->px * s->ny * s->ext_nz;
-        DevBuf k1, k2, bmat_full, bd2_full, segcnt_tmp, scan_tmp, total, wtab, flags_ext;
-        VIRS_TRY(k1.alloc(nvc * 4, "sponge scratch"));
-        VIRS_TRY(k2.alloc(nvc * 4, "sponge scratch"));
-        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch"));
-        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch"));
-        if (s->slab) VIRS_TRY(flags_ext.alloc(nvc, "sponge scratch"));
+        Scratch scratch;
+        DevBuf k1, k2, bmat_full, bd2_full, scan_tmp, total, wtab, flags_ext, bm, bd, cnt;
+        Scratch::End end{scratch, st};
+        VIRS_TRY(k1.alloc(nvc * 4, "sponge scratch", s->stream));
+        VIRS_TRY(k2.alloc(nvc * 4, "sponge scratch", s->stream));
+        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch", s->stream));
+        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch", s->stream));
+        if (s->slab) VIRS_TRY(flags_ext.alloc(nvc, "sponge scratch", s->stream));
         ClassifyArgs ca{};
         ca.flags_in = s->flags_raw.as<uint8_t>();
         ca.wall_mat = s->wall_mat.as<uint8_t>();
@@ -1433,30 +1631,24 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         ca.px = s->px;
         ca.W = W;
         VIRS_CUDA(launch_sponge(ca, st));
-        k1.release();
-        k2.release();
         if (s->slab) {
             // planes are contiguous: one copy per array
             const size_t off = (size_t)s->slab_drop * s->px * s->ny;
-            DevBuf bm, bd;
-            VIRS_TRY(bm.alloc(s->nvox, "sponge scratch"));
-            VIRS_TRY(bd.alloc(s->nvox * 2, "sponge scratch"));
+            VIRS_TRY(bm.alloc(s->nvox, "sponge scratch", s->stream));
+            VIRS_TRY(bd.alloc(s->nvox * 2, "sponge scratch", s->stream));
             VIRS_CUDA(cudaMemcpyAsync(s->flags.ptr, flags_ext.as<uint8_t>() + off, s->nvox, cudaMemcpyDeviceToDevice, st));
             VIRS_CUDA(cudaMemcpyAsync(bm.ptr, bmat_full.as<uint8_t>() + off, s->nvox, cudaMemcpyDeviceToDevice, st));
             VIRS_CUDA(cudaMemcpyAsync(bd.ptr, bd2_full.as<uint16_t>() + off, s->nvox * 2, cudaMemcpyDeviceToDevice, st));
             VIRS_CUDA(cudaStreamSynchronize(st));
-            std::swap(bmat_full.ptr, bm.ptr);
-            std::swap(bmat_full.bytes, bm.bytes);
-            std::swap(bd2_full.ptr, bd.ptr);
-            std::swap(bd2_full.bytes, bd.bytes);
-            flags_ext.release();
+            bmat_full.swap(bm);
+            bd2_full.swap(bd);
         }
 
         const size_t nseg = (size_t)s->spr * s->ny * s->nz;
-        VIRS_TRY(s->code.alloc(s->nvox, "cell codes"));
-        VIRS_TRY(s->normals.alloc(s->nvox, "normals"));
-        VIRS_TRY(s->bseg.alloc(nseg * 4, "boundary prefix"));
-        VIRS_TRY(s->segnz.alloc(nseg, "segment code flags"));
+        VIRS_TRY(s->code.alloc(s->nvox, "cell codes", s->stream));
+        VIRS_TRY(s->normals.alloc(s->nvox, "normals", s->stream));
+        VIRS_TRY(s->bseg.alloc(nseg * 4, "boundary prefix", s->stream));
+        VIRS_TRY(s->segnz.alloc(nseg, "segment code flags", s->stream));
         CodesArgs co{};
         co.flags = s->flags.as<uint8_t>();
         co.code = s->code.as<uint8_t>();
@@ -1470,21 +1662,20 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         co.spr = s->spr;
         VIRS_CUDA(launch_codes(co, st));
         {
-            DevBuf cnt;
-            VIRS_TRY(cnt.alloc(4, "hard-source count"));
+            VIRS_TRY(cnt.alloc(4, "hard-source count", s->stream));
             VIRS_CUDA(launch_hard_list(s->code.as<uint8_t>(), s->nvox, cnt.as<uint32_t>(), nullptr, 0, st));
             uint32_t nh = 0;
             VIRS_CUDA(cudaMemcpyAsync(&nh, cnt.ptr, 4, cudaMemcpyDeviceToHost, st));
             VIRS_CUDA(cudaStreamSynchronize(st));
-            VIRS_TRY(s->hpos.alloc(std::max<uint32_t>(nh, 1) * 4, "hard-source positions"));
+            VIRS_TRY(s->hpos.alloc(std::max<uint32_t>(nh, 1) * 4, "hard-source positions", s->stream));
             VIRS_CUDA(cudaMemsetAsync(cnt.ptr, 0, 4, st));
             VIRS_CUDA(launch_hard_list(s->code.as<uint8_t>(), s->nvox, cnt.as<uint32_t>(), s->hpos.as<uint32_t>(), nh,
                                        st));
             VIRS_CUDA(cudaStreamSynchronize(st));
             s->nhpos = nh;
         }
-        VIRS_TRY(scan_tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch"));
-        VIRS_TRY(total.alloc(4, "boundary count"));
+        VIRS_TRY(scan_tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch", s->stream));
+        VIRS_TRY(total.alloc(4, "boundary count", s->stream));
         VIRS_CUDA(launch_scan(s->bseg.as<uint32_t>(), nseg, scan_tmp.as<uint32_t>(), total.as<uint32_t>(), st));
         uint32_t nb = 0;
         VIRS_CUDA(cudaMemcpyAsync(&nb, total.ptr, 4, cudaMemcpyDeviceToHost, st));
@@ -1494,15 +1685,15 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         std::vector<float> wt((size_t)W * W + 1);
         for (int d = 0; d <= W * W; ++d) wt[d] = sponge_weight(W, d);
         VIRS_TRY(build_weights(s, wt));
-        VIRS_TRY(wtab.alloc(wt.size() * 4, "sponge weights"));
+        VIRS_TRY(wtab.alloc(wt.size() * 4, "sponge weights", s->stream));
         VIRS_CUDA(copy_on(s->stream, wtab.ptr, wt.data(), wt.size() * 4, cudaMemcpyHostToDevice));
-        VIRS_TRY(s->bidx.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary indices"));
-        VIRS_TRY(s->bpos.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary positions"));
-        VIRS_TRY(s->bmat.alloc(std::max<uint64_t>(nb, 1), "boundary materials"));
-        VIRS_TRY(s->bmeta.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary codes"));
-        VIRS_TRY(s->bnrm.alloc(std::max<uint64_t>(nb, 1), "boundary normals"));
-        VIRS_TRY(s->bw.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary weights"));
-        VIRS_TRY(s->side.alloc(std::max<uint64_t>(nb, 1) * sizeof(float4), "boundary records"));
+        VIRS_TRY(s->bidx.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary indices", s->stream));
+        VIRS_TRY(s->bpos.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary positions", s->stream));
+        VIRS_TRY(s->bmat.alloc(std::max<uint64_t>(nb, 1), "boundary materials", s->stream));
+        VIRS_TRY(s->bmeta.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary codes", s->stream));
+        VIRS_TRY(s->bnrm.alloc(std::max<uint64_t>(nb, 1), "boundary normals", s->stream));
+        VIRS_TRY(s->bw.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary weights", s->stream));
+        VIRS_TRY(s->side.alloc(std::max<uint64_t>(nb, 1) * sizeof(float4), "boundary records", s->stream));
         CompactArgs cp{};
         cp.flags = s->flags.as<uint8_t>();
         cp.bseg = s->bseg.as<uint32_t>();
@@ -1738,7 +1929,7 @@ VIRS_EXPORT virs_status virs_set_sources(virs_sim *s, uint32_t n, const uint64_t
     VIRS_TRY(wait_done(s));
     s->sig_host.assign(sig, sig + (size_t)n * len);
     s->sig_peak = peak;
-    VIRS_TRY(s->src.alloc(std::max<uint32_t>(n, 1) * 8, "source indices"));
+    VIRS_TRY(s->src.alloc(std::max<uint32_t>(n, 1) * 8, "source indices", s->stream, false));
     if (n) VIRS_CUDA(copy_on(s->stream, s->src.ptr, dev.data(), n * 8, cudaMemcpyHostToDevice));
     s->nsrc = n;
     s->siglen = len;
@@ -1762,7 +1953,7 @@ VIRS_EXPORT virs_status virs_set_receivers(virs_sim *s, uint32_t n, const uint64
     }
     VIRS_TRY(use_device(s));
     VIRS_TRY(wait_done(s));
-    VIRS_TRY(s->rcv.alloc(std::max<uint32_t>(n, 1) * 8, "receiver indices"));
+    VIRS_TRY(s->rcv.alloc(std::max<uint32_t>(n, 1) * 8, "receiver indices", s->stream, false));
     if (n) VIRS_CUDA(copy_on(s->stream, s->rcv.ptr, dev.data(), n * 8, cudaMemcpyHostToDevice));
     s->nrcv = n;
     s->rcv_ref.assign(idx, idx + n);
@@ -1779,7 +1970,7 @@ virs_status upload_signals(virs_sim *s)
 {
     std::vector<float> v(s->sig_host.size());
     for (size_t i = 0; i < v.size(); ++i) v[i] = s->sig_host[i] * s->scale;
-    VIRS_TRY(s->sig.alloc(std::max<size_t>(v.size(), 1) * 4, "source signals"));
+    VIRS_TRY(s->sig.alloc(std::max<size_t>(v.size(), 1) * 4, "source signals", s->stream, false));
     if (!v.empty()) VIRS_CUDA(copy_on(s->stream, s->sig.ptr, v.data(), v.size() * 4, cudaMemcpyHostToDevice));
     s->graph_dirty = true;
     ++s->gen;
@@ -1796,14 +1987,10 @@ VIRS_EXPORT virs_status virs_start_simulation(virs_sim *s, uint64_t steps)
     choose_scale(s);
     VIRS_TRY(upload_hard(s));
     VIRS_TRY(upload_signals(s));
-    s->ir.release();
-    s->ircap = 0;
-    VIRS_TRY(ensure_ir(s, std::max<uint64_t>(steps, 1)));
-    VIRS_CUDA(zero_on(s->stream, s->field[0].ptr, s->field[0].bytes));
-    VIRS_CUDA(zero_on(s->stream, s->field[1].ptr, s->field[1].bytes));
-    VIRS_CUDA(zero_on(s->stream, s->state.ptr, s->state.bytes));
-    VIRS_CUDA(zero_on(s->stream, s->ctr.ptr, s->ctr.bytes));
-    if (s->stopbuf.ptr) VIRS_CUDA(zero_on(s->stream, s->stopbuf.ptr, s->stopbuf.bytes));
+    s->ircap = std::max<uint64_t>(steps, 1024);
+    VIRS_TRY(s->ir.alloc(std::max<uint32_t>(s->nrcv, 1) * s->ircap * sizeof(float), "receiver samples", s->stream));
+    for (DevBuf *b : {&s->field[0], &s->field[1], &s->state, &s->ctr, &s->stopbuf})
+        if (b->ptr) VIRS_CUDA(cudaMemsetAsync(b->ptr, 0, b->bytes, s->stream));
     s->stopped = false;
     s->slab_open = false;
     s->cur = 0;
@@ -1811,7 +1998,9 @@ VIRS_EXPORT virs_status virs_start_simulation(virs_sim *s, uint64_t steps)
     s->out0.clear();
     s->rms_state = 0.f;
     s->fields_valid = true;
-    s->drop_graphs();
+    s->graph_dirty = true; // run_steps keeps the graphs if they still fit
+    ++s->gen;
+    s->ctr_at = 0;
     VIRS_CUDA(cudaStreamSynchronize(s->stream));
     VIRS_CUDA(cudaEventRecord(s->done, s->stream));
     return VIRS_OK;
@@ -1942,6 +2131,7 @@ cudaError_t slab_step(virs_sim *const *slabs, uint32_t n, size_t pb)
         if (e == cudaSuccess) {
             s->cur ^= 1;
             s->steps_done += 1;
+            s->ctr_at += 1;
             e = cudaEventRecord(s->done, s->stream);
         }
     }
@@ -1980,10 +2170,11 @@ virs_status slab_graph(virs_sim *const *slabs, uint32_t n, size_t pb, cudaGraphE
     VIRS_CUDA(evs.make(&fork));
     for (auto &j : join) VIRS_CUDA(evs.make(&j));
     std::vector<int> cur(n);
-    std::vector<uint64_t> done(n);
+    std::vector<uint64_t> done(n), ctr(n);
     for (uint32_t k = 0; k < n; ++k) {
         cur[k] = slabs[k]->cur;
         done[k] = slabs[k]->steps_done;
+        ctr[k] = slabs[k]->ctr_at;
     }
     VIRS_CUDA(cudaStreamBeginCapture(o, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaEventRecord(fork, o);
@@ -2006,6 +2197,7 @@ virs_status slab_graph(virs_sim *const *slabs, uint32_t n, size_t pb, cudaGraphE
     for (uint32_t k = 0; k < n; ++k) {
         slabs[k]->cur = cur[k];
         slabs[k]->steps_done = done[k];
+        slabs[k]->ctr_at = ctr[k];
     }
     cudaSetDevice(slabs[0]->prm.device);
     cudaGraph_t g = nullptr;
@@ -2046,6 +2238,8 @@ virs_status slab_graph_run(virs_sim *const *slabs, uint32_t n, cudaGraphExec_t e
         VIRS_CUDA(cudaStreamWaitEvent(s->xstream, after, 0));
         VIRS_CUDA(cudaEventRecord(s->done, s->stream));
         s->steps_done += times * SLAB_GRAPH_STEPS;
+        s->ctr_at += times * SLAB_GRAPH_STEPS;
+        s->waits = true;
     }
     return VIRS_OK;
 }
@@ -2161,6 +2355,7 @@ VIRS_EXPORT virs_status virs_slab_step_end(virs_sim *s, void *stream)
     VIRS_CUDA(launch_post(s->prm.storage, post_args(s, par), st));
     s->cur ^= 1;
     s->steps_done += 1;
+    s->ctr_at += 1;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     return VIRS_OK;
 }
@@ -2215,15 +2410,23 @@ VIRS_EXPORT virs_status virs_step(virs_sim *s, uint32_t step, int *keep_going, f
     VIRS_TRY(ready_to_run(s));
     VIRS_TRY(ensure_ir(s, (uint64_t)step + 1));
     cudaStream_t st = s->stream;
-    // the reference uploads the source value every step (simulator_gpu.cu:250-258)
-    VIRS_CUDA(cudaMemcpyAsync(s->ctr.as<uint32_t>() + s->cur, &step, 4, cudaMemcpyHostToDevice, st));
+    // the reference uploads the source value every step
+    // (simulator_gpu.cu:250-258); here the step number, unless the counter
+    // already stands there.  The sample comes back through pinned memory, so
+    // that the call waits once.
+    if (!s->host_word) VIRS_CUDA(cudaHostAlloc((void **)&s->host_word, sizeof(float), cudaHostAllocDefault));
+    if (s->ctr_at != step)
+        VIRS_CUDA(cudaMemcpyAsync(s->ctr.as<uint32_t>() + s->cur, &step, 4, cudaMemcpyHostToDevice, st));
+    s->ctr_at = UINT64_MAX;
     cudaError_t e = enqueue_step(s, s->cur, st);
     if (e != cudaSuccess) return cuda_fail(e, "step launch");
     s->cur ^= 1;
     s->steps_done = std::max<uint64_t>(s->steps_done, (uint64_t)step + 1);
-    float v = 0.f;
-    if (s->nrcv) VIRS_CUDA(cudaMemcpyAsync(&v, s->ir.as<float>() + step, 4, cudaMemcpyDeviceToHost, st));
+    s->ctr_at = (uint64_t)step + 1;
+    *s->host_word = 0.f;
+    if (s->nrcv) VIRS_CUDA(cudaMemcpyAsync(s->host_word, s->ir.as<float>() + step, 4, cudaMemcpyDeviceToHost, st));
     VIRS_CUDA(cudaStreamSynchronize(st));
+    const float v = *s->host_word;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     VIRS_TRY(check_err(s));
     if (sample) *sample = v;
@@ -2305,18 +2508,18 @@ VIRS_EXPORT virs_status virs_postprocess_ir(virs_sim *s, double rate, const doub
     // the simulation rate as the reference forms it: 1.f / dt in float
     const double sim_rate = (double)(1.f / s->dt);
     cudaStream_t st = s->stream;
-    DevBuf dsos, filt, res;
+    DevBuf &dsos = s->post_sos, &filt = s->post_filt, &res = s->post_res;
     const float *src = s->ir.as<float>();
     uint64_t stride = s->ircap;
     if (ns) {
-        VIRS_TRY(dsos.alloc((size_t)ns * 6 * sizeof(double), "post-processing sections"));
-        VIRS_TRY(filt.alloc((size_t)s->nrcv * steps * sizeof(float), "filtered receiver traces"));
+        VIRS_TRY(dsos.alloc((size_t)ns * 6 * sizeof(double), "post-processing sections", st, false));
+        VIRS_TRY(filt.alloc((size_t)s->nrcv * steps * sizeof(float), "filtered receiver traces", st, false));
         VIRS_CUDA(cudaMemcpyAsync(dsos.ptr, sos, (size_t)ns * 6 * sizeof(double), cudaMemcpyHostToDevice, st));
         VIRS_CUDA(launch_ir_sos(src, stride, steps, dsos.as<double>(), (int)ns, filt.as<float>(), steps, s->nrcv, st));
         src = filt.as<float>();
         stride = steps;
     }
-    VIRS_TRY(res.alloc((size_t)s->nrcv * len * sizeof(float), "resampled receiver traces"));
+    VIRS_TRY(res.alloc((size_t)s->nrcv * len * sizeof(float), "resampled receiver traces", st, false));
     VIRS_CUDA(launch_ir_resample(src, stride, steps, sim_rate, (float)rate, res.as<float>(), len, normalize ? 1 : 0,
                                  s->nrcv, st));
     VIRS_CUDA(cudaMemcpyAsync(out, res.ptr, (size_t)s->nrcv * len * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -2343,9 +2546,9 @@ VIRS_EXPORT virs_status virs_postprocess_ir_sinc(virs_sim *s, double rate, uint3
     VIRS_TRY(wait_done(s));
     VIRS_TRY(check_err(s));
     cudaStream_t st = s->stream;
-    DevBuf res, peak;
-    VIRS_TRY(res.alloc((size_t)s->nrcv * len * sizeof(float), "resampled receiver traces"));
-    if (normalize) VIRS_TRY(peak.alloc((size_t)s->nrcv * sizeof(uint32_t), "receiver peaks"));
+    DevBuf &res = s->post_res, &peak = s->post_peak;
+    VIRS_TRY(res.alloc((size_t)s->nrcv * len * sizeof(float), "resampled receiver traces", st, false));
+    if (normalize) VIRS_TRY(peak.alloc((size_t)s->nrcv * sizeof(uint32_t), "receiver peaks", st, false));
     VIRS_CUDA(launch_ir_sinc(s->ir.as<float>(), s->ircap, steps, 1.0 / (double)s->dt, rate, (int)half_taps, beta,
                              cutoff, res.as<float>(), len, normalize ? peak.as<uint32_t>() : nullptr, s->nrcv, st));
     VIRS_CUDA(cudaMemcpyAsync(out, res.ptr, (size_t)s->nrcv * len * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -2535,6 +2738,7 @@ VIRS_EXPORT virs_status virs_check_bounded_wait(virs_sim *s, uint32_t limit)
     VIRS_TRY(use_device(s));
     VIRS_TRY(wait_done(s));
     if (!s->err.ptr) VIRS_TRY(s->err.alloc(sizeof(int), "error flag"));
+    s->waits = true;
     VIRS_CUDA(launch_wait_probe(s->err.as<int>(), limit, s->stream));
     VIRS_CUDA(cudaStreamSynchronize(s->stream));
     return check_err(s);
@@ -2572,6 +2776,7 @@ virs_status reset_state(virs_sim *s)
     VIRS_CUDA(cudaStreamSynchronize(s->stream));
     s->cur = 0;
     s->steps_done = 0;
+    s->ctr_at = 0;
     s->out0.clear();
     s->rms_state = 0.f;
     return VIRS_OK;
@@ -2781,6 +2986,7 @@ struct virs_batch {
     std::vector<uint64_t> gen;
     int dev = 0, storage = 0, rows = 8, depth = 2, planes = 0;
     bool persistent = false;
+    bool waits = false;            // kernels with bounded waits queued since virs_batch_synchronize
     bool tiling_set = false, fused = false; // a step in one launch (kernels_fused.cu), through `table`
     DevBuf table;
     uint32_t nblocks = 0;
@@ -2954,6 +3160,7 @@ virs_status batch_steps(virs_batch *b, uint64_t n, cudaStream_t st, bool use_gra
         VIRS_CUDA(cudaEventRecord(s->done, s->stream));
         VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
     }
+    if (!b->fused) b->waits = true;
     const int cur = m0->cur;
     uint64_t i = 0;
     if (use_graph && n >= (uint64_t)virs_batch::GRAPH_STEPS) {
@@ -2968,6 +3175,7 @@ virs_status batch_steps(virs_batch *b, uint64_t n, cudaStream_t st, bool use_gra
     for (virs_sim *s : b->mem) {
         s->cur ^= (int)(n & 1);
         s->steps_done += n;
+        s->ctr_at += n;
         VIRS_CUDA(cudaEventRecord(s->done, st));
     }
     VIRS_CUDA(cudaEventRecord(b->done, st));
@@ -3012,7 +3220,10 @@ VIRS_EXPORT virs_status virs_batch_destroy(virs_batch *b)
 {
     if (!b) return VIRS_OK;
     cudaSetDevice(b->dev);
+    // the last run, on the batch's stream or a caller's
+    if (b->done) cudaEventSynchronize(b->done);
     cudaStreamSynchronize(b->stream);
+    Recycle r;
     delete b;
     return VIRS_OK;
 }
@@ -3032,6 +3243,8 @@ VIRS_EXPORT virs_status virs_batch_synchronize(virs_batch *b)
     if (!b) return fail(VIRS_E_ARG, "virs_batch_synchronize: null");
     VIRS_CUDA(cudaSetDevice(b->dev));
     VIRS_CUDA(cudaEventSynchronize(b->done));
+    if (!b->waits) return VIRS_OK;
+    b->waits = false;
     int e = 0;
     VIRS_CUDA(copy_on(b->stream, &e, b->err.ptr, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
@@ -3148,9 +3361,9 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
     A.every = every;
     A.nck = (steps + every - 1) / every;
     const size_t fb = s->nvox * 4, sb = state_bytes(s);
-    VIRS_TRY(A.ckp.alloc(A.nck * fb, "checkpoints"));
-    VIRS_TRY(A.ckq.alloc(A.nck * fb, "checkpoints"));
-    VIRS_TRY(A.cks.alloc(A.nck * sb, "checkpoints"));
+    VIRS_TRY(A.ckp.alloc(A.nck * fb, "checkpoints", s->stream, false));
+    VIRS_TRY(A.ckq.alloc(A.nck * fb, "checkpoints", s->stream, false));
+    VIRS_TRY(A.cks.alloc(A.nck * sb, "checkpoints", s->stream, false));
     VIRS_CUDA(cudaEventRecord(s->done, s->stream));
     VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
     for (uint64_t c = 0; c < A.nck; ++c) {
@@ -3178,15 +3391,15 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     // adjoints, four per section
     const size_t fb = s->nvox * 4, sb = state_bytes(s), sba = std::max<uint64_t>(nb, 1) * s->nsec * 4 * 4;
     const uint32_t ncoef = s->nmat * s->nsec * 5;
-    VIRS_TRY(A.segrec.alloc(every * std::max<uint64_t>(nb, 1) * sizeof(float4), "adjoint segment records"));
-    VIRS_TRY(A.segst.alloc(every * sb, "adjoint segment states"));
-    for (int k = 0; k < 2; ++k) VIRS_TRY(A.buf[k].alloc(fb, "adjoint field"));
-    VIRS_TRY(A.ast.alloc(sba, "adjoint filter states"));
-    VIRS_TRY(A.dbar.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms"));
-    for (int k = 0; k < 2; ++k) VIRS_TRY(A.rr[k].alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms"));
-    VIRS_TRY(A.grad.alloc(ncoef * sizeof(double), "coefficient gradients"));
-    VIRS_TRY(A.dl.alloc(std::max<uint32_t>(s->nrcv, 1) * steps * 4, "loss gradient"));
-    VIRS_TRY(A.gsig.alloc(std::max<uint32_t>(s->nsrc, 1) * steps * 4, "signal gradients"));
+    VIRS_TRY(A.segrec.alloc(every * std::max<uint64_t>(nb, 1) * sizeof(float4), "adjoint segment records", st, false));
+    VIRS_TRY(A.segst.alloc(every * sb, "adjoint segment states", st, false));
+    for (int k = 0; k < 2; ++k) VIRS_TRY(A.buf[k].alloc(fb, "adjoint field", st));
+    VIRS_TRY(A.ast.alloc(sba, "adjoint filter states", st));
+    VIRS_TRY(A.dbar.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms", st));
+    for (int k = 0; k < 2; ++k) VIRS_TRY(A.rr[k].alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms", st));
+    VIRS_TRY(A.grad.alloc(ncoef * sizeof(double), "coefficient gradients", st));
+    VIRS_TRY(A.dl.alloc(std::max<uint32_t>(s->nrcv, 1) * steps * 4, "loss gradient", st, false));
+    VIRS_TRY(A.gsig.alloc(std::max<uint32_t>(s->nsrc, 1) * steps * 4, "signal gradients", st));
     if (s->nrcv) VIRS_CUDA(copy_on(s->stream, A.dl.ptr, dl_dir, (size_t)s->nrcv * steps * 4, cudaMemcpyHostToDevice));
     VIRS_TRY(ready_to_run(s));
     if (!s->probe_ok) VIRS_TRY(build_probes(s));
@@ -3252,6 +3465,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
         VIRS_CUDA(copy_on(s->stream, grad_signal, A.gsig.ptr, (size_t)s->nsrc * steps * 4, cudaMemcpyDeviceToHost));
     // the fields now hold an intermediate forward state
     s->fields_valid = false;
+    s->ctr_at = UINT64_MAX;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     return VIRS_OK;
 }

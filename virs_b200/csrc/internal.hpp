@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstddef>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda.h>
@@ -46,20 +47,27 @@ inline uint32_t state_groups(uint32_t nsec) { return (2u * (nsec + 1u) + 3u) / 4
 
 // ---- device buffer -----------------------------------------------------------
 
+// alloc keeps the buffer's memory when it is large enough (the caller has
+// waited for the work that uses it).  The contents are zero on return, or,
+// with a stream, from that point of the stream on; `zero` false: whatever
+// the memory held.  release gives the memory to CUDA, or, inside a Recycle
+// scope, to the pool of freed blocks (capi.cpp).
 struct DevBuf {
     void *ptr = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;       // as asked for
+    size_t cap = 0;         // the block's size
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
-    void release()
+    void release();
+    virs_status alloc(size_t n, const char *what, cudaStream_t st = nullptr, bool zero = true);
+    void swap(DevBuf &o)
     {
-        if (ptr) cudaFree(ptr);
-        ptr = nullptr;
-        bytes = 0;
+        std::swap(ptr, o.ptr);
+        std::swap(bytes, o.bytes);
+        std::swap(cap, o.cap);
     }
-    virs_status alloc(size_t n, const char *what);   // zero-filled
     template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
 
