@@ -616,7 +616,7 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
     VIRS_TRY(s->wall_mat.alloc(ext, "wall materials", s->stream));
     if (flags) VIRS_TRY(h2d_rows(s->flags_raw.ptr, flags, 1, s, s->ext_nz));
     if (wmat) VIRS_TRY(h2d_rows(s->wall_mat.ptr, wmat, 1, s, s->ext_nz));
-    VIRS_TRY(s->flags.alloc(s->nvox, "classified flags", s->stream));
+    VIRS_TRY(s->flags.alloc(s->nvox, "classified flags", s->stream, false));
     VIRS_TRY(s->field[0].alloc(s->nvox * s->storage_bytes(), "pressure field", s->stream));
     VIRS_TRY(s->field[1].alloc(s->nvox * s->storage_bytes(), "pressure field", s->stream));
     s->cur = 0;
@@ -702,7 +702,10 @@ virs_status install_mesh(virs_sim *s, const Mesh &m, uint32_t part = 0, uint32_t
         VIRS_TRY(dr.alloc(std::max<size_t>(s->roles.size(), 1), "material roles", s->stream, false));
         VIRS_TRY(tri.alloc(ntri * voxelize_tri_bytes(), "triangle table", s->stream, false));
         VIRS_TRY(la.alloc(nvx * sizeof(uint32_t), "voxelisation marks", s->stream));
-        VIRS_TRY(lw.alloc(nvx * sizeof(uint32_t), "voxelisation marks", s->stream));
+        bool source = false;
+        for (int32_t k : m.tri_mat)
+            source = source || (k >= 0 && (size_t)k < s->roles.size() && s->roles[(size_t)k] == VIRS_ROLE_SOURCE);
+        if (source) VIRS_TRY(lw.alloc(nvx * sizeof(uint32_t), "voxelisation marks", s->stream));
         VIRS_TRY(mx.alloc(sizeof(uint32_t), "wall material maximum", s->stream));
         VIRS_CUDA(copy_on(s->stream, dv.ptr, m.verts.data(), dv.bytes, cudaMemcpyHostToDevice));
         VIRS_CUDA(copy_on(s->stream, dt.ptr, m.tris.data(), dt.bytes, cudaMemcpyHostToDevice));
@@ -1610,21 +1613,24 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         // planes too), then only the kept planes
         const size_t nvc = (size_t)s->px * s->ny * s->ext_nz;
         Scratch scratch;
-        DevBuf k1, k2, bmat_full, bd2_full, scan_tmp, total, wtab, flags_ext, bm, bd, cnt;
+        DevBuf bits, near2, live, bmat_full, bd2_full, scan_tmp, total, wtab, flags_ext, bm, bd, cnt;
         Scratch::End end{scratch, st};
-        VIRS_TRY(k1.alloc(nvc * 4, "sponge scratch", s->stream));
-        VIRS_TRY(k2.alloc(nvc * 4, "sponge scratch", s->stream));
-        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch", s->stream));
-        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch", s->stream));
-        if (s->slab) VIRS_TRY(flags_ext.alloc(nvc, "sponge scratch", s->stream));
+        // written where they are read: no zero fill
+        VIRS_TRY(bits.alloc(nvc / 8, "sponge scratch", st, false));
+        VIRS_TRY(near2.alloc(nvc * 2, "sponge scratch", st, false));
+        VIRS_TRY(live.alloc(sponge_live_tiles(s->px, s->ny, s->ext_nz), "sponge scratch", st, false));
+        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch", st, false));
+        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch", st, false));
+        if (s->slab) VIRS_TRY(flags_ext.alloc(nvc, "sponge scratch", st, false));
         ClassifyArgs ca{};
         ca.flags_in = s->flags_raw.as<uint8_t>();
         ca.wall_mat = s->wall_mat.as<uint8_t>();
         ca.flags_out = (s->slab ? flags_ext : s->flags).as<uint8_t>();
         ca.bmat_full = bmat_full.as<uint8_t>();
         ca.bd2_full = bd2_full.as<uint16_t>();
-        ca.k1 = k1.as<uint32_t>();
-        ca.k2 = k2.as<uint32_t>();
+        ca.bits = bits.as<uint32_t>();
+        ca.near2 = near2.as<uint16_t>();
+        ca.live = live.as<uint8_t>();
         ca.nx = s->nx;
         ca.ny = s->ny;
         ca.nz = s->ext_nz;
@@ -1634,8 +1640,8 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         if (s->slab) {
             // planes are contiguous: one copy per array
             const size_t off = (size_t)s->slab_drop * s->px * s->ny;
-            VIRS_TRY(bm.alloc(s->nvox, "sponge scratch", s->stream));
-            VIRS_TRY(bd.alloc(s->nvox * 2, "sponge scratch", s->stream));
+            VIRS_TRY(bm.alloc(s->nvox, "sponge scratch", st, false));
+            VIRS_TRY(bd.alloc(s->nvox * 2, "sponge scratch", st, false));
             VIRS_CUDA(cudaMemcpyAsync(s->flags.ptr, flags_ext.as<uint8_t>() + off, s->nvox, cudaMemcpyDeviceToDevice, st));
             VIRS_CUDA(cudaMemcpyAsync(bm.ptr, bmat_full.as<uint8_t>() + off, s->nvox, cudaMemcpyDeviceToDevice, st));
             VIRS_CUDA(cudaMemcpyAsync(bd.ptr, bd2_full.as<uint16_t>() + off, s->nvox * 2, cudaMemcpyDeviceToDevice, st));
@@ -1645,10 +1651,10 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         }
 
         const size_t nseg = (size_t)s->spr * s->ny * s->nz;
-        VIRS_TRY(s->code.alloc(s->nvox, "cell codes", s->stream));
-        VIRS_TRY(s->normals.alloc(s->nvox, "normals", s->stream));
-        VIRS_TRY(s->bseg.alloc(nseg * 4, "boundary prefix", s->stream));
-        VIRS_TRY(s->segnz.alloc(nseg, "segment code flags", s->stream));
+        VIRS_TRY(s->code.alloc(s->nvox, "cell codes", st, false));
+        VIRS_TRY(s->normals.alloc(s->nvox, "normals", st, false));
+        VIRS_TRY(s->bseg.alloc(nseg * 4, "boundary prefix", st, false));
+        VIRS_TRY(s->segnz.alloc(nseg, "segment code flags", st, false));
         CodesArgs co{};
         co.flags = s->flags.as<uint8_t>();
         co.code = s->code.as<uint8_t>();
@@ -1660,42 +1666,38 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         co.nz = s->nz;
         co.px = s->px;
         co.spr = s->spr;
+        // {hard-source voxels, boundary voxels}, read back together
+        VIRS_TRY(total.alloc(8, "voxel counts", st));
+        co.nhard = total.as<uint32_t>();
         VIRS_CUDA(launch_codes(co, st));
-        {
-            VIRS_TRY(cnt.alloc(4, "hard-source count", s->stream));
-            VIRS_CUDA(launch_hard_list(s->code.as<uint8_t>(), s->nvox, cnt.as<uint32_t>(), nullptr, 0, st));
-            uint32_t nh = 0;
-            VIRS_CUDA(cudaMemcpyAsync(&nh, cnt.ptr, 4, cudaMemcpyDeviceToHost, st));
-            VIRS_CUDA(cudaStreamSynchronize(st));
-            VIRS_TRY(s->hpos.alloc(std::max<uint32_t>(nh, 1) * 4, "hard-source positions", s->stream));
-            VIRS_CUDA(cudaMemsetAsync(cnt.ptr, 0, 4, st));
+        VIRS_TRY(scan_tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch", st, false));
+        VIRS_CUDA(launch_scan(s->bseg.as<uint32_t>(), nseg, scan_tmp.as<uint32_t>(), total.as<uint32_t>() + 1, st));
+        uint32_t counts[2] = {0, 0};
+        VIRS_CUDA(cudaMemcpyAsync(counts, total.ptr, 8, cudaMemcpyDeviceToHost, st));
+        VIRS_CUDA(cudaStreamSynchronize(st));
+        const uint32_t nh = counts[0], nb = counts[1];
+        s->nb = nb;
+        s->nhpos = nh;
+        VIRS_TRY(s->hpos.alloc(std::max<uint32_t>(nh, 1) * 4, "hard-source positions", st));
+        if (nh) {
+            VIRS_TRY(cnt.alloc(4, "hard-source count", st));
             VIRS_CUDA(launch_hard_list(s->code.as<uint8_t>(), s->nvox, cnt.as<uint32_t>(), s->hpos.as<uint32_t>(), nh,
                                        st));
-            VIRS_CUDA(cudaStreamSynchronize(st));
-            s->nhpos = nh;
         }
-        VIRS_TRY(scan_tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch", s->stream));
-        VIRS_TRY(total.alloc(4, "boundary count", s->stream));
-        VIRS_CUDA(launch_scan(s->bseg.as<uint32_t>(), nseg, scan_tmp.as<uint32_t>(), total.as<uint32_t>(), st));
-        uint32_t nb = 0;
-        VIRS_CUDA(cudaMemcpyAsync(&nb, total.ptr, 4, cudaMemcpyDeviceToHost, st));
-        VIRS_CUDA(cudaStreamSynchronize(st));
-        s->nb = nb;
 
         std::vector<float> wt((size_t)W * W + 1);
         for (int d = 0; d <= W * W; ++d) wt[d] = sponge_weight(W, d);
         VIRS_TRY(build_weights(s, wt));
         VIRS_TRY(wtab.alloc(wt.size() * 4, "sponge weights", s->stream));
         VIRS_CUDA(copy_on(s->stream, wtab.ptr, wt.data(), wt.size() * 4, cudaMemcpyHostToDevice));
-        VIRS_TRY(s->bidx.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary indices", s->stream));
-        VIRS_TRY(s->bpos.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary positions", s->stream));
-        VIRS_TRY(s->bmat.alloc(std::max<uint64_t>(nb, 1), "boundary materials", s->stream));
-        VIRS_TRY(s->bmeta.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary codes", s->stream));
-        VIRS_TRY(s->bnrm.alloc(std::max<uint64_t>(nb, 1), "boundary normals", s->stream));
-        VIRS_TRY(s->bw.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary weights", s->stream));
-        VIRS_TRY(s->side.alloc(std::max<uint64_t>(nb, 1) * sizeof(float4), "boundary records", s->stream));
+        VIRS_TRY(s->bidx.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary indices", st, false));
+        VIRS_TRY(s->bpos.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary positions", st, false));
+        VIRS_TRY(s->bmat.alloc(std::max<uint64_t>(nb, 1), "boundary materials", st, false));
+        VIRS_TRY(s->bmeta.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary codes", st, false));
+        VIRS_TRY(s->bnrm.alloc(std::max<uint64_t>(nb, 1), "boundary normals", st, false));
+        VIRS_TRY(s->bw.alloc(std::max<uint64_t>(nb, 1) * 4, "boundary weights", st, false));
+        VIRS_TRY(s->side.alloc(std::max<uint64_t>(nb, 1) * sizeof(float4), "boundary records", st, false));
         CompactArgs cp{};
-        cp.flags = s->flags.as<uint8_t>();
         cp.bseg = s->bseg.as<uint32_t>();
         cp.bmat_full = bmat_full.as<uint8_t>();
         cp.bd2_full = bd2_full.as<uint16_t>();
@@ -1713,7 +1715,7 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         cp.nz = s->nz;
         cp.px = s->px;
         cp.spr = s->spr;
-        VIRS_CUDA(launch_compact(cp, st));
+        VIRS_CUDA(launch_compact(cp, nb, st));
         VIRS_CUDA(cudaStreamSynchronize(st));
     }
     s->state.release();

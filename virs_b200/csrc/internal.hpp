@@ -249,13 +249,16 @@ struct ClassifyArgs {
     const uint8_t *flags_in;   // padded
     const uint8_t *wall_mat;   // padded
     uint8_t *flags_out;        // padded
-    uint8_t *bmat_full;        // padded scratch
-    uint16_t *bd2_full;        // padded scratch
-    uint32_t *k1, *k2;         // padded scratch
+    uint8_t *bmat_full;        // padded scratch, set at boundary voxels
+    uint16_t *bd2_full;        // padded scratch, set at boundary voxels
+    uint32_t *bits;            // padded voxels / 32 words: walls
+    uint16_t *near2;           // padded: the nearest wall in the plane
+    uint8_t *live;             // sponge_live_tiles(): tiles of near2 with any
     uint32_t nx, ny, nz, px;
     int W;
 };
 cudaError_t launch_sponge(const ClassifyArgs &a, cudaStream_t s);
+size_t sponge_live_tiles(uint32_t px, uint32_t ny, uint32_t nz);
 
 struct CodesArgs {
     const uint8_t *flags;      // padded, classified
@@ -263,6 +266,7 @@ struct CodesArgs {
     uint8_t *normals;          // padded
     uint32_t *segcnt;          // [nseg]
     uint8_t *segnz;            // [nseg] 1 if the segment holds a non-zero code
+    uint32_t *nhard;           // hard-source voxels (zeroed by the caller)
     uint32_t nx, ny, nz, px, spr;
 };
 cudaError_t launch_codes(const CodesArgs &a, cudaStream_t s);
@@ -271,7 +275,6 @@ size_t scan_tmp_words(size_t n);
 cudaError_t launch_scan(uint32_t *data, size_t n, uint32_t *tmp, uint32_t *total, cudaStream_t s);
 
 struct CompactArgs {
-    const uint8_t *flags;      // padded, classified
     const uint32_t *bseg;
     const uint8_t *bmat_full;
     const uint16_t *bd2_full;
@@ -286,7 +289,7 @@ struct CompactArgs {
     float *bw;
     uint32_t nx, ny, nz, px, spr;
 };
-cudaError_t launch_compact(const CompactArgs &a, cudaStream_t s);
+cudaError_t launch_compact(const CompactArgs &a, uint32_t total, cudaStream_t s); // total: slots of all segments
 // per tile of a rows x zc tiling of the TMA stencil: bit j set when the codes
 // of the plane in stage j are all zero (kernels_classify.cu)
 // (planes [zb, ze) in chunks of zc: 1 and nz - 1 for a whole step)

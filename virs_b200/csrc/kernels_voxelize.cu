@@ -18,7 +18,7 @@
 // leaves the wall material alone.  So the flag comes from the last wall or
 // source triangle that hits the voxel and the wall material from the last
 // wall triangle: two maxima per voxel give exactly that, in any order of
-// execution.
+// execution (one is enough for a mesh without sources).
 //
 // This file is compiled with -fmad=false and without flush-to-zero: every
 // float expression is evaluated as written in IEEE single precision, as on
@@ -148,26 +148,43 @@ __global__ void __launch_bounds__(256) k_tri_sweep(const Tri *__restrict tris, u
             if (!overlap(g, (float)i, (float)j, (float)k)) continue;
             const size_t idx = ((size_t)(k - zw) * ny + (size_t)j) * px + (size_t)i;
             atomicMax(last_any + idx, (uint32_t)(t + 1));
-            if (role != VIRS_ROLE_SOURCE) atomicMax(last_wall + idx, (uint32_t)(t + 1));
+            if (last_wall && role != VIRS_ROLE_SOURCE) atomicMax(last_wall + idx, (uint32_t)(t + 1));
         }
     }
 }
 
-__global__ void k_resolve(const Tri *__restrict tris, const uint32_t *__restrict last_any,
-                          const uint32_t *__restrict last_wall, uint64_t n, uint8_t *__restrict flags,
-                          uint8_t *__restrict wall_mat, uint32_t *__restrict max_mat)
+// four voxels per thread; nothing is written where no triangle passes
+// (flags and materials are zero).  last_wall == nullptr: no triangle is a
+// source, so the last one is the last wall.  0.93 ms for 403 M voxels with a
+// voxel per thread and two arrays, 0.40 now.
+__global__ void __launch_bounds__(256) k_resolve(const Tri *__restrict tris, const uint4 *__restrict last_any,
+                                                 const uint4 *__restrict last_wall, uint64_t n4,
+                                                 uint32_t *__restrict flags, uint32_t *__restrict wall_mat,
+                                                 uint32_t *__restrict max_mat)
 {
     uint32_t mx = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t a = last_any[i], w = last_wall[i];
-        if (a) flags[i] = tris[a - 1].role == VIRS_ROLE_SOURCE ? 3 : 1;
-        if (w) {
-            const uint32_t r = tris[w - 1].role;
-            wall_mat[i] = (uint8_t)r;
-            mx = r > mx ? r : mx;
+    const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i < n4) {
+        const uint4 a = __ldg(last_any + i);
+        if (a.x | a.y | a.z | a.w) {
+            const uint4 w = last_wall ? __ldg(last_wall + i) : a;
+            const uint32_t A[4] = {a.x, a.y, a.z, a.w}, W[4] = {w.x, w.y, w.z, w.w};
+            uint32_t f = 0, m = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (A[c]) f |= (tris[A[c] - 1].role == VIRS_ROLE_SOURCE ? 3u : 1u) << (8 * c);
+                if (W[c]) {
+                    const uint32_t r = tris[W[c] - 1].role;
+                    m |= (r & 0xffu) << (8 * c);
+                    mx = r > mx ? r : mx;
+                }
+            }
+            flags[i] = f;
+            wall_mat[i] = m;
         }
     }
-    if (mx) atomicMax(max_mat, mx);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (mx && (threadIdx.x & 31) == 0) atomicMax(max_mat, mx);
 }
 
 } // namespace
@@ -191,8 +208,10 @@ cudaError_t launch_voxelize(const float *verts, const uint32_t *tris, const int3
     const unsigned gy = ntri < 64 ? 256u : (ntri < 1024 ? 16u : 1u);
     k_tri_sweep<<<dim3(gx, gy), 256, 0, s>>>(T, ntri, px, ny, (int)zw, last_any, last_wall);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const uint64_t n = (uint64_t)px * ny * nzl;
-    k_resolve<<<1184, 256, 0, s>>>(T, last_any, last_wall, n, flags, wall_mat, max_mat);
+    const uint64_t n4 = (uint64_t)px * ny * nzl / 4; // px is a multiple of 32
+    k_resolve<<<(unsigned)((n4 + 255) / 256), 256, 0, s>>>(
+        T, reinterpret_cast<const uint4 *>(last_any), reinterpret_cast<const uint4 *>(last_wall), n4,
+        reinterpret_cast<uint32_t *>(flags), reinterpret_cast<uint32_t *>(wall_mat), max_mat);
     return cudaGetLastError();
 }
 
