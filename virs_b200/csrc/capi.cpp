@@ -366,6 +366,7 @@ struct virs_sim {
     // plist holds the voxels whose second step is provisional (pl_ok: built
     // for the current codes and sources)
     int pair_steps = 1, pair_rows = 14, pair_zc = 0;
+    bool pair_auto = false;        // the caller left the tile to the library (pair_tile)
     DevBuf spare[2];
     CUtensorMap pmP[4], pmQ[4], pmC;
     int pm_rows = 0;
@@ -1049,6 +1050,35 @@ bool pair_on(const virs_sim *s)
            s->nz >= 3;
 }
 
+// The two-step kernel's tile: the caller's, or, when the caller left rows and
+// planes to the library, 16 rows and as many planes as leave about four
+// blocks per SM, 16 to 60 (the zero-code masks cover the 64 stages of 60
+// planes).  Per step in FP32, 14 rows over all planes against this rule:
+// 1024x768x512 856 and 770 us, 701x517x333 271 and 251, 512x300x200 109 and
+// 79, 254x259x325 161 and 72.
+struct PairTile {
+    int rows, zc;
+};
+PairTile pair_tile(const virs_sim *s)
+{
+    if (!s->pair_auto) return {s->pair_rows, s->pair_zc};
+    const uint64_t ix = (uint64_t)pair_tile_x(s->prm.storage);
+    const uint64_t tiles = (s->px + ix - 1) / ix * ((s->ny + 13) / 14);
+    const uint64_t zc = (uint64_t)(s->nz - 2) * tiles / (4ull * (uint64_t)sm_count(s->prm.device));
+    return {16, (int)std::min<uint64_t>(std::max<uint64_t>(zc, 16), 60)};
+}
+
+// Whether a run takes its groups of four steps two at a time.  With the tile
+// left to the library, only where that is the faster way to the same bits:
+// not on grids whose single steps take one launch each (150x140x130: 10 us a
+// step against 20), and not in 16-bit storage, where the two-step kernel is
+// bound by issue (the hall 528 against 650 us, 701x517x333 186 against 230).
+// The timing of the parts takes two steps as asked.
+bool pairs_pay(const virs_sim *s)
+{
+    return !s->pair_auto || s->timing || (s->prm.storage == VIRS_STORAGE_F32 && !fused_on(s));
+}
+
 // the voxels whose p^{n+2} the two-step kernel leaves provisional, for the
 // current codes, boundary list and sources (kernels_classify.cu)
 virs_status build_pair_list(virs_sim *s)
@@ -1093,8 +1123,9 @@ virs_status ready_pairs(virs_sim *s)
             s->drop_graphs();
             return VIRS_OK;
         }
-    if (s->pm_rows != s->pair_rows) {
-        const int rows = s->pair_rows;
+    const PairTile tile = pair_tile(s);
+    if (s->pm_rows != tile.rows) {
+        const int rows = tile.rows;
         const CUtensorMapDataType dt = s->prm.storage == VIRS_STORAGE_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                        : s->prm.storage == VIRS_STORAGE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                             : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1109,16 +1140,16 @@ virs_status ready_pairs(virs_sim *s)
         s->pzm_zc = -1;
         s->drop_graphs();
     }
-    if (zero_masks_useful(s) && s->pzm_zc != s->pair_zc) {
+    if (zero_masks_useful(s) && s->pzm_zc != tile.zc) {
         const uint32_t ix = (uint32_t)pair_tile_x(s->prm.storage), v = (uint32_t)(16 / s->storage_bytes());
-        const uint32_t rows = (uint32_t)s->pair_rows, zc = s->pair_zc > 0 ? (uint32_t)s->pair_zc : s->nz - 2;
+        const uint32_t rows = (uint32_t)tile.rows, zc = tile.zc > 0 ? (uint32_t)tile.zc : s->nz - 2;
         const uint32_t gx = (s->px + ix - 1) / ix, gy = (s->ny + rows - 3) / (rows - 2);
         const uint32_t gz = (s->nz - 2 + zc - 1) / zc;
         VIRS_TRY(s->pzmask.alloc((size_t)gx * gy * gz * 8, "two-step zero-code masks"));
         VIRS_CUDA(launch_pair_zero_masks(s->segnz.as<uint8_t>(), s->px, s->ny, s->nz, s->spr, rows, zc, ix, v, gx, gy,
                                          gz, s->pzmask.as<uint64_t>(), s->stream));
         VIRS_CUDA(cudaStreamSynchronize(s->stream));
-        s->pzm_zc = s->pair_zc;
+        s->pzm_zc = tile.zc;
         s->drop_graphs();
     }
     if (!s->pl_ok) VIRS_TRY(build_pair_list(s));
@@ -1163,12 +1194,13 @@ cudaError_t enqueue_pair(const virs_sim *s, int par, int x, int y, int z, int w,
 {
     const int sto = s->prm.storage;
     StepArgs a = step_args_bufs(s, x, y);
-    a.zc = s->pair_zc;
-    if (zero_masks_useful(s) && s->pzm_zc == s->pair_zc) a.tzmask = s->pzmask.as<uint64_t>();
+    const PairTile tile = pair_tile(s);
+    a.zc = tile.zc;
+    if (zero_masks_useful(s) && s->pzm_zc == tile.zc) a.tzmask = s->pzmask.as<uint64_t>();
     const TmaMaps m{&s->pmP[x], &s->pmQ[y], &s->pmC};
     s->waits = true;
     if (ev) cudaEventRecord(ev[0], st);
-    cudaError_t e = launch_pair_tma(sto, s->pair_rows, a, m, buf_ptr(s, z), buf_ptr(s, w), s->err.as<int>(), st);
+    cudaError_t e = launch_pair_tma(sto, tile.rows, a, m, buf_ptr(s, z), buf_ptr(s, w), s->err.as<int>(), st);
     if (ev) cudaEventRecord(ev[1], st);
     if (e == cudaSuccess) e = launch_boundary(sto, step_args_bufs(s, x, z), BND_UPDATE, st);
     if (ev) cudaEventRecord(ev[2], st);
@@ -1218,7 +1250,7 @@ virs_status ready_graph(virs_sim *s, int par, cudaStream_t st)
         cudaGraph_t g = nullptr;
         VIRS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
-        if (pair_on(s))
+        if (pair_on(s) && pairs_pay(s))
             for (int i = 0; i < virs_sim::GRAPH_STEPS / 4 && e == cudaSuccess; ++i) e = enqueue_quad(s, par, st);
         else
             for (int i = 0; i < virs_sim::GRAPH_STEPS && e == cudaSuccess; ++i) e = enqueue_step(s, par ^ (i & 1), st);
@@ -1266,7 +1298,7 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
     // with two steps per pass, whole groups of four steps go through the
     // spare buffers and back; the remaining n % 4 are single steps
     uint64_t quads = 0;
-    if (pair_on(s) && n >= 4) {
+    if (pair_on(s) && pairs_pay(s) && n >= 4) {
         VIRS_TRY(ready_pairs(s));
         if (pair_on(s)) {
             quads = n / 4;
@@ -2696,6 +2728,7 @@ VIRS_EXPORT virs_status virs_set_time_blocking(virs_sim *s, int steps_per_pass, 
     s->pair_steps = steps_per_pass;
     s->pair_rows = tile_rows ? tile_rows : 14;
     s->pair_zc = planes;
+    s->pair_auto = steps_per_pass == 2 && tile_rows == 0 && planes == 0;
     s->pm_rows = 0;
     s->pair_nomem = false;
     if (steps_per_pass == 1) {
@@ -2880,6 +2913,7 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
                 const int pl = cand[c < cand.size() ? c : 2 * cand.size() - 1 - c].second;
                 if (st != VIRS_OK) break;
                 s->pair_steps = 2;
+                s->pair_auto = false;
                 s->pair_rows = r;
                 s->pair_zc = pl;
                 s->pm_rows = 0;
@@ -2926,6 +2960,7 @@ VIRS_EXPORT virs_status virs_autotune(virs_sim *s, uint32_t trial_steps, virs_ti
     s->pair_steps = pick.pair_steps;
     s->pair_rows = pick.pair_rows;
     s->pair_zc = pick.pair_zc;
+    s->pair_auto = false;
     s->pm_rows = 0;
     if (pick.pair_steps == 1) {
         s->spare[0].release();
