@@ -61,18 +61,19 @@ template <typename T> struct Vec {
     }
 };
 
-// rounded and stored; SR: stochastically, one hash per pair of voxels as in
-// st_sr (pos is a multiple of four, base is even)
+// rounded and stored; SR: stochastically (pos is a multiple of four)
 template <typename T, bool SR>
 __device__ __forceinline__ void put4(T *p, const float (&r)[V], uint64_t pos, uint64_t base, uint32_t key)
 {
     typename Vec<T>::Raw raw;
-    T *h = reinterpret_cast<T *>(&raw);
+    if constexpr (SR) {
+        uint32_t v[2];
+        sr_pack<T>(r, pos, base, key, v);
+        raw = make_uint2(v[0], v[1]);
+    } else {
+        T *h = reinterpret_cast<T *>(&raw);
 #pragma unroll
-    for (int k = 0; k < V; k += 2) {
-        const uint32_t w = SR ? sr_word(pos + k, base, key) : 0u;
-        h[k] = SR ? Sr<T>::put(r[k], w & 0xffffu) : Io<T>::put(r[k]);
-        h[k + 1] = SR ? Sr<T>::put(r[k + 1], w >> 16) : Io<T>::put(r[k + 1]);
+        for (int k = 0; k < V; ++k) h[k] = Io<T>::put(r[k]);
     }
     *reinterpret_cast<typename Vec<T>::Raw *>(p) = raw;
 }

@@ -166,32 +166,57 @@ __device__ __forceinline__ uint32_t sr_bits(uint64_t pos, uint64_t base, uint32_
 
 // FP32 pattern rounded stochastically to the kept bits of T (truncated,
 // exactly representable in T), or to nearest where stated above
-__device__ __forceinline__ __nv_bfloat16 sr_bf16(float f, uint32_t r16)
-{
-    uint32_t u = __float_as_uint(f);
-    if ((u & 0x7fffffffu) < 0x7f7f0000u) {
-        u = (u + r16) & 0xffff0000u;
-        return __ushort_as_bfloat16((unsigned short)(u >> 16));
-    }
-    return __float2bfloat16_rn(f);
-}
-
-__device__ __forceinline__ __half sr_f16(float f, uint32_t r16)
-{
-    const uint32_t u = __float_as_uint(f), a = u & 0x7fffffffu;
-    if (a >= 0x38800000u && a < 0x477fe000u) return __float2half_rn(__uint_as_float((u + (r16 & 0x1fffu)) & ~0x1fffu));
-    return __float2half_rn(f);
-}
-
 template <typename T> struct Sr;
 template <> struct Sr<float> {
     __device__ static float put(float f, uint32_t) { return f; }
 };
 template <> struct Sr<__nv_bfloat16> {
-    __device__ static __nv_bfloat16 put(float f, uint32_t r16) { return sr_bf16(f, r16); }
+    // larger magnitudes and non-finite values round to nearest
+    __device__ static bool plain(uint32_t u) { return (u & 0x7fffffffu) >= 0x7f7f0000u; }
+    __device__ static __nv_bfloat16 put(float f, uint32_t r16)
+    {
+        const uint32_t u = __float_as_uint(f);
+        return plain(u) ? __float2bfloat16_rn(f) : __ushort_as_bfloat16((unsigned short)((u + r16) >> 16));
+    }
+    // V values with the random words of their pairs, packed: the truncation
+    // is the choice of the upper halves; one test for the whole vector
+    template <int V> __device__ static void put_vec(const float (&r)[V], const uint32_t (&w)[V / 2], uint32_t (&out)[V / 2])
+    {
+        uint32_t top = 0;
+#pragma unroll
+        for (int k = 0; k < V; ++k) top = max(top, __float_as_uint(r[k]) & 0x7fffffffu);
+        if (plain(top)) {
+#pragma unroll
+            for (int k = 0; k < V; k += 2)
+                out[k / 2] = (uint32_t)__bfloat16_as_ushort(put(r[k], w[k / 2] & 0xffffu)) |
+                             (uint32_t)__bfloat16_as_ushort(put(r[k + 1], w[k / 2] >> 16)) << 16;
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < V; k += 2)
+            out[k / 2] = __byte_perm(__float_as_uint(r[k]) + (w[k / 2] & 0xffffu),
+                                     __float_as_uint(r[k + 1]) + (w[k / 2] >> 16), 0x7632);
+    }
 };
 template <> struct Sr<__half> {
-    __device__ static __half put(float f, uint32_t r16) { return sr_f16(f, r16); }
+    // in FP16's normal range: truncated to its ten bits after adding 13
+    // random ones (then converted exactly); the others round to nearest in
+    // the conversion
+    __device__ static float cut(float f, uint32_t r16)
+    {
+        const uint32_t u = __float_as_uint(f);
+        const bool in = (u & 0x7fffffffu) - 0x38800000u < 0x477fe000u - 0x38800000u;
+        return __uint_as_float(in ? (u + (r16 & 0x1fffu)) & ~0x1fffu : u);
+    }
+    __device__ static __half put(float f, uint32_t r16) { return __float2half_rn(cut(f, r16)); }
+    template <int V> __device__ static void put_vec(const float (&r)[V], const uint32_t (&w)[V / 2], uint32_t (&out)[V / 2])
+    {
+#pragma unroll
+        for (int k = 0; k < V; k += 2) {
+            const __half2 h = __floats2half2_rn(cut(r[k], w[k / 2]), cut(r[k + 1], w[k / 2] >> 16));
+            out[k / 2] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
 };
 
 // a store of one value: to nearest, or stochastic with `key` (sr != 0)
@@ -201,23 +226,26 @@ __device__ __forceinline__ T put_rounded(float f, int sr, uint64_t pos, uint64_t
     return sr ? Sr<T>::put(f, sr_bits(pos, base, key)) : Io<T>::put(f);
 }
 
-// a stochastic store of one 16-byte vector of V values starting at the
-// (even) padded position pos0: one hash per voxel pair
+// V values from the even padded position pos0 on (base is even too),
+// rounded stochastically and packed: one hash per voxel pair
+template <typename T, int V>
+__device__ __forceinline__ void sr_pack(const float (&r)[V], uint64_t pos0, uint64_t base, uint32_t key, uint32_t (&out)[V / 2])
+{
+    const uint32_t pair = (uint32_t)((pos0 + base) >> 1);
+    uint32_t w[V / 2];
+#pragma unroll
+    for (int k = 0; k < V / 2; ++k) w[k] = mix32((pair + (uint32_t)k) ^ key);
+    Sr<T>::put_vec(r, w, out);
+}
+
+// a stochastic store of one 16-byte vector
 template <typename T>
 __device__ __forceinline__ void st_sr(T *p, const float (&r)[Io<T>::VEC], uint64_t pos0, uint64_t base, uint32_t key)
 {
-    constexpr int V = Io<T>::VEC;
-    if constexpr (V == 8) {
-        uint4 v;
-        uint32_t *w32 = reinterpret_cast<uint32_t *>(&v);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t w = sr_word(pos0 + 2 * k, base, key);
-            const T lo = Sr<T>::put(r[2 * k], w & 0xffffu), hi = Sr<T>::put(r[2 * k + 1], w >> 16);
-            w32[k] = (uint32_t)*reinterpret_cast<const unsigned short *>(&lo) |
-                     ((uint32_t)*reinterpret_cast<const unsigned short *>(&hi) << 16);
-        }
-        __stcs(reinterpret_cast<uint4 *>(p), v);
+    if constexpr (Io<T>::VEC == 8) {
+        uint32_t v[4];
+        sr_pack<T>(r, pos0, base, key, v);
+        __stcs(reinterpret_cast<uint4 *>(p), make_uint4(v[0], v[1], v[2], v[3]));
     } else {
         Io<T>::st(p, r);
     }
