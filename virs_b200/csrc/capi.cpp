@@ -332,6 +332,7 @@ struct virs_sim {
     uint64_t ircap = 0;
     DevBuf ctr;                    // two words: the step of buffer parity k reads word k and writes the next step's to the other
     DevBuf probe;                  // sources and receivers for the one-launch step (kernels_fused.cu)
+    FusedGeo geo{};
     bool probe_ok = false;
     uint64_t ctr_at = 0;           // the step the counter word of parity `cur` holds
     mutable std::atomic<bool> waits{false}; // kernels with bounded waits queued since check_err
@@ -384,6 +385,7 @@ struct virs_sim {
     struct GraphKey {              // the arguments the graphs hold; what else they hold drops them when it changes
         StepArgs step[2];
         PostArgs post[2];
+        FusedGeo geo;
     } graph_key;
     uint64_t gen = 0;              // bumped on every change of buffers or parameters
 
@@ -871,37 +873,54 @@ bool zero_masks_ready(const virs_sim *s)
     return s->depth > 0 && zero_masks_useful(s) && s->zm_rows == s->tile_rows && s->zm_zc == eff_planes(s);
 }
 
+// stochastic rounding of the 16-bit stores, and its key offset: a slab's
+// voxels take the keys of the same voxels of the whole grid
+bool sr_on(const virs_sim *s) { return s->rounding == VIRS_ROUND_STOCHASTIC && s->prm.storage != VIRS_STORAGE_F32; }
+uint64_t sr_base(const virs_sim *s) { return s->slab ? (s->slab_lo - 1) * (uint64_t)s->ny * s->px : 0; }
+
 // Single steps in one launch each (kernels_fused.cu) instead of stencil,
-// boundary pass and post kernel: on grids whose step is bound by latency.
-// Measured per step, three launches against one (sponge width 1 / 8):
-//   0.07 M voxels  FP32  9.2 / 9.2 against  3.4 / 3.7 us   BF16 9.9 / 10.0 against 3.7 / 3.6 us
-//   1.5 M               11.7 / 14.5          6.7 / 10.4         11.9 / 14.5          6.6 / 10.5
-//   7.8 M               28.6 / 55.4         24.7 / 48.5         25.6 / 48.8         22.1 / 47.0
-//   15.7 M              51.8 / 86.4         49.2 / 84.9         37.1 / 71.1         44.1 / 83.5
-// so the line lies at 16 M voxels in FP32 and 8 M in 16-bit storage.  A
-// tiling set by the caller names the stencil kernel; the stop rule and the
-// timing of the parts need the separate kernels.
+// boundary pass and post kernel: on grids whose step is bound by latency, and
+// as far up as the boundary slots' gathers find their lines in the L2 beside
+// the stencil.  Measured per step, three launches against one (sponge width
+// 1 / 4 / 16, three sections; the first two rows 1 / 8, two sections):
+//   0.07 M voxels FP32   8.6 /   9.3 against   3.2 /   3.6 us   BF16  10.0 / 10.1 against 3.1 / 3.5 us
+//   3.7 M               18.9 /  26.3           9.5 /  18.3            17.5 / 24.0         9.2 / 17.6
+//   24 M                79.1 /  99.5 / 169    66.7 /  87.9 / 163     63.0 / 82.2 / 152   59.4 / 78.9 / 152
+//   38 M               103.4 / 131.4 / 235    95.2 / 128.5 / 241     80.7 / 110  / 213   81.8 / 116  / 226
+//   60 M               169.6 / 203.4 / 344   158.1 / 195.2 / 343    121   / 155  / 294  137   / 175  / 321
+//   118 M              296.2 / 345.9 / 570   290.9 / 353.0 / 588    192   / 242  / 457  252   / 320  / 550
+// so the line lies at 64 M voxels in FP32, 24 M in 16-bit storage, 20 M with
+// stochastic rounding (24 M: 70.5 against 71.5 us), and at 8 M boundary slots
+// (24 M voxels, sponge 16: 7.6 M slots; 38 M: 10.7 M), whose states stream
+// better through a kernel of their own.  A tiling set by the
+// caller names the stencil kernel; the stop rule and the timing of the parts
+// need the separate kernels.
 bool fused_on(const virs_sim *s)
 {
-    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 16u << 20 : 8u << 20;
-    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most;
+    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 64u << 20 : sr_on(s) ? 20u << 20 : 24u << 20;
+    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most && s->nb <= (8u << 20);
 }
 
-// the probe list of the one-launch step: a probe on a border plane, which no
-// block covers and no step writes, goes to the first block
+// the probes and block flags of the one-launch step, pl as fused_geo; `buf`
+// holds the probes, then a flag per block
+virs_status make_probes(const virs_sim *s, int pl, DevBuf &buf, FusedGeo *geo)
+{
+    const uint32_t n = s->nsrc + s->nrcv;
+    FusedGeo g = fused_geo(s->px, s->ny, s->nz, s->nb, sm_count(s->prm.device), pl);
+    std::vector<Probe> h(n);
+    for (uint32_t k = 0; k < n; ++k)
+        h[k] = {0u, (uint32_t)to_dev(s, k < s->nsrc ? s->src_ref[k] : s->rcv_ref[k - s->nsrc])};
+    VIRS_TRY(buf.alloc(n * sizeof(Probe) + g.blocks, "probes", s->stream));
+    g.has_probe = buf.as<uint8_t>() + n * sizeof(Probe);
+    if (n) VIRS_CUDA(copy_on(s->stream, buf.ptr, h.data(), n * sizeof(Probe), cudaMemcpyHostToDevice));
+    VIRS_CUDA(launch_probe_blocks(buf.as<Probe>(), n, s->bpos.as<uint32_t>(), s->nb, s->px * s->ny, s->nz, g,
+                                  buf.as<uint8_t>() + n * sizeof(Probe), s->stream));
+    *geo = g;
+    return VIRS_OK;
+}
 virs_status build_probes(virs_sim *s)
 {
-    const uint32_t n = s->nsrc + s->nrcv, plane = s->px * s->ny;
-    std::vector<Probe> h(n);
-    for (uint32_t k = 0; k < n; ++k) {
-        const uint64_t d = to_dev(s, k < s->nsrc ? s->src_ref[k] : s->rcv_ref[k - s->nsrc]);
-        const uint32_t z = (uint32_t)(d / plane);
-        const bool in = z >= 1 && z + 1 < s->nz;
-        h[k] = {in ? z : 1u, in ? (uint32_t)(d % plane) : 0u, PROBE_NO_SLOT, (uint32_t)d};
-    }
-    VIRS_TRY(s->probe.alloc(std::max<uint32_t>(n, 1) * sizeof(Probe), "probes", s->stream, false));
-    if (n) VIRS_CUDA(copy_on(s->stream, s->probe.ptr, h.data(), n * sizeof(Probe), cudaMemcpyHostToDevice));
-    VIRS_CUDA(launch_probe_slots(s->probe.as<Probe>(), n, s->bpos.as<uint32_t>(), s->nb, s->stream));
+    VIRS_TRY(make_probes(s, 0, s->probe, &s->geo));
     s->probe_ok = true;
     s->graph_dirty = true;
     return VIRS_OK;
@@ -928,11 +947,6 @@ virs_status ready_to_run(virs_sim *s)
     }
     return VIRS_OK;
 }
-
-// stochastic rounding of the 16-bit stores, and its key offset: a slab's
-// voxels take the keys of the same voxels of the whole grid
-bool sr_on(const virs_sim *s) { return s->rounding == VIRS_ROUND_STOCHASTIC && s->prm.storage != VIRS_STORAGE_F32; }
-uint64_t sr_base(const virs_sim *s) { return s->slab ? (s->slab_lo - 1) * (uint64_t)s->ny * s->px : 0; }
 
 StepArgs step_args(const virs_sim *s, int parity)
 {
@@ -1031,7 +1045,7 @@ cudaError_t launch_stencil_range(const virs_sim *s, int parity, cudaStream_t st,
 cudaError_t enqueue_step(const virs_sim *s, int parity, cudaStream_t st)
 {
     if (fused_on(s))
-        return launch_fused(s->prm.storage, BND_UPDATE, step_args(s, parity), post_args(s, parity), st);
+        return launch_fused(s->prm.storage, BND_UPDATE, step_args(s, parity), post_args(s, parity), s->geo, st);
     cudaError_t e = launch_stencil(s, parity, st);
     if (e != cudaSuccess) return e;
     e = launch_boundary(s->prm.storage, step_args(s, parity), BND_UPDATE, st);
@@ -1240,6 +1254,7 @@ virs_status ready_graph(virs_sim *s, int par, cudaStream_t st)
             std::memcpy(&key.step[k], &a, sizeof(a));
             std::memcpy(&key.post[k], &p, sizeof(p));
         }
+        if (fused_on(s)) std::memcpy(&key.geo, &s->geo, sizeof(s->geo));
         if (std::memcmp(&key, &s->graph_key, sizeof(key)) != 0) {
             s->destroy_graphs();
             std::memcpy(&s->graph_key, &key, sizeof(key));
@@ -3031,7 +3046,7 @@ struct virs_batch {
     int sections = 0;              // launch_boundary_batch
     DevBuf desc, err;
     // each member's zero-code masks for the batch's tiling
-    std::deque<DevBuf> zmasks;
+    std::deque<DevBuf> zmasks, probes;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -3068,16 +3083,22 @@ virs_status batch_check(const virs_batch *b)
 }
 
 // A step of the batch in one launch (kernels_fused.cu) when its members are
-// few or small.  Measured per step, three launches against one (sponge 1-2,
-// three sections): 0.6 M voxels in 4 rooms FP32 29.5 against 7.4 us, BF16
-// 33.6 against 7.1; 7.4 M in 8 rooms 57.5 against 52.9 and 55.5 against 41.4;
-// 26 M in 24 rooms 153 against 155 and 132 against 143.  The line lies at
-// 12 M voxels with the row padding.
+// small (their rows fill few of the stencil's 128-voxel tiles) or few.
+// Measured per step, three launches against one (sponge 1-2, three sections):
+//   4 rooms, 0.6 M voxels in all    FP32  29.5 against   6.3 us   BF16  33.6 against   6.1 us
+//   12, 2.9 M                             44.0            23.0           46.7            21.3
+//   24, 26 M (1.1 M each)                148             124            127             111
+//   100, 97 M (0.97 M each)              548             498            444             449
+//   30, 50 M (1.7 M each)                281             266            244             241
+//   20, 86 M (4.3 M each)                341             346            281             313
+// so the line lies at 3 M voxels per member in FP32, 1.5 M in 16-bit storage
+// (row padding included), and at 12 M in all for fewer, larger members.
 bool batch_fused(const virs_batch *b)
 {
     size_t n = 0;
     for (const virs_sim *s : b->mem) n += s->nvox;
-    return !b->tiling_set && n <= (12u << 20);
+    const size_t each = b->storage == VIRS_STORAGE_F32 ? 3u << 20 : 3u << 19;
+    return !b->tiling_set && n <= std::max<size_t>(12u << 20, each * b->mem.size());
 }
 
 // descriptors of every member for the batch's tiling
@@ -3087,6 +3108,7 @@ virs_status batch_build(virs_batch *b)
     b->fused = batch_fused(b);
     std::vector<uint2> table;
     b->zmasks.clear();
+    b->probes.clear();
     std::vector<BatchMember> h(b->mem.size());
     uint64_t tiles = 0, bnd = 0;
     uint32_t min_sections = UINT32_MAX, max_sections = 0;
@@ -3106,7 +3128,11 @@ virs_status batch_build(virs_batch *b)
         VIRS_TRY(encode(&m.mapC, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s->code.ptr, s, (uint32_t)tma_tile_x(), b->rows));
         const int zc = b->planes > 0 ? b->planes : (s->zc > 0 ? s->zc : default_planes(s->nz));
         const uint64_t *zm = nullptr;
-        if (b->fused && !s->probe_ok) VIRS_TRY(build_probes(s));
+        if (b->fused) {
+            b->probes.emplace_back();
+            VIRS_TRY(make_probes(s, 2, b->probes.back(), &m.geo));
+            VIRS_CUDA(cudaStreamSynchronize(s->stream));
+        }
         if (!b->fused && zero_masks_useful(s)) {
             b->zmasks.emplace_back();
             VIRS_TRY(build_zero_masks(s, b->rows, zc, b->zmasks.back()));
@@ -3119,14 +3145,14 @@ virs_status batch_build(virs_batch *b)
             m.step[par].tzmask = zm; // the batch's tiling, not the member's own
             m.post[par] = post_args(s, par);
             m.post[par].stop = nullptr;
+            if (b->fused) m.post[par].probe = b->probes.back().as<Probe>();
         }
         m.bidx = s->bidx.as<uint32_t>();
         m.gx = (s->px + tma_tile_x() - 1) / tma_tile_x();
         m.gy = (s->ny + b->rows - 1) / b->rows;
         m.gz = (s->nz - 2 + zc - 1) / zc;
         if (b->fused) {
-            const uint32_t n = (uint32_t)fused_blocks(s->px, s->ny, s->nz, s->nb);
-            for (uint32_t k = 0; k < n; ++k) table.push_back(make_uint2((uint32_t)i, k));
+            for (uint32_t k = 0; k < m.geo.blocks; ++k) table.push_back(make_uint2((uint32_t)i, k));
         }
         m.first_tile = tiles;
         m.first_bnd = bnd;
@@ -3466,7 +3492,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
                                          : s->state.as<float>();
             cudaError_t e;
             if (fused_on(s)) {
-                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), st);
+                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), s->geo, st);
             } else {
                 e = launch_stencil(s, s->cur, st);
                 if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, st);
@@ -3489,7 +3515,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
                 a.nhard = 0;
                 const AdjPost po{s->probe.as<Probe>(), s->nsrc, s->nrcv, A.rr[t].as<float>(), A.dbar.as<float>(),
                                  A.dl.as<float>(), A.gsig.as<float>(), steps, n - 1};
-                e = launch_adj_step(a, po, st);
+                e = launch_adj_step(a, po, s->geo, st);
             }
             if (e != cudaSuccess) return cuda_fail(e, "adjoint step");
             t ^= 1;

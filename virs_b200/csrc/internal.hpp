@@ -128,12 +128,17 @@ struct StepArgs {
     double K, mix_y, mix_d, gain;
 };
 
-// a source or receiver voxel, for the kernel that does a whole step in one
-// launch (kernels_fused.cu): the block that writes the voxel handles it
-constexpr uint32_t PROBE_NO_SLOT = 0xffffffffu;
+// The kernel that does a whole step in one launch (kernels_fused.cu): its
+// blocks, and a source or receiver voxel, handled by the block that writes it.
+struct FusedGeo {
+    uint32_t gb, gx;        // boundary blocks; stencil blocks per plane (or pair of planes)
+    uint32_t magic;         // ceil(2^32 / gx), or 0
+    uint32_t pl;            // planes and slots per thread: 1 or 2
+    uint32_t blocks;
+    const uint8_t *has_probe; // [blocks]
+};
 struct Probe {
-    uint32_t z, off;        // plane, and offset in it, whose block owns the probe
-    uint32_t slot;          // the voxel's boundary slot, or PROBE_NO_SLOT
+    uint32_t blk;           // the block that handles it
     uint32_t pos;           // device position
 };
 
@@ -165,6 +170,7 @@ struct alignas(64) BatchMember {
     CUtensorMap mapC;       // cell codes
     StepArgs step[2];       // per parity: p = field[parity], q = field[parity ^ 1]
     PostArgs post[2];
+    FusedGeo geo;           // step in one launch: the member's blocks
     const uint32_t *bidx;
     uint64_t first_tile;    // index of this member's first tile in the batch
     uint64_t first_bnd;     // index of this member's first boundary voxel
@@ -181,14 +187,17 @@ cudaError_t launch_post_batch(int storage, const BatchMember *mem, uint32_t nmem
 // the same in one launch (kernels_fused.cu): table[block] = {member, block of the member}
 cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks,
                                int parity, cudaStream_t s, bool sr);
-uint64_t fused_blocks(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb); // blocks of one simulation's step
 
 // kernel launchers (kernels_step.cu)
 cudaError_t launch_step(int storage, int tile_rows, const StepArgs &a, cudaStream_t s);
 cudaError_t launch_post(int storage, const PostArgs &a, cudaStream_t s);
 // a whole step in one launch (kernels_fused.cu)
 // (mode BND_UPDATE, or BND_KEEP in FP32)
-cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, cudaStream_t s);
+// fused_geo: the blocks for a grid, pl (1, 2) planes per thread or 0: by size;
+// launch_probe_blocks fills the probes' blocks and the flags (zeroed before)
+FusedGeo fused_geo(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb, int sms, int pl);
+cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, const FusedGeo &g,
+                         cudaStream_t s);
 // the adjoint's step (kernels_fused.cu): what its blocks need beyond StepArgs
 struct AdjPost {
     const Probe *probe;     // as PostArgs
@@ -199,8 +208,9 @@ struct AdjPost {
     uint64_t stride;
     int64_t n;              // the next reverse step (-1: none)
 };
-cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, cudaStream_t s);
-cudaError_t launch_probe_slots(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, cudaStream_t s);
+cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, const FusedGeo &g, cudaStream_t s);
+cudaError_t launch_probe_blocks(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, uint32_t plane,
+                                uint32_t nz, const FusedGeo &g, uint8_t *has_probe, cudaStream_t s);
 // modes of the boundary pass (kernels_step.cu)
 enum { BND_UPDATE = 0, BND_KEEP = 1 };
 cudaError_t launch_boundary(int storage, const StepArgs &a, int mode, cudaStream_t s);

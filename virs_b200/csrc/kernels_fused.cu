@@ -15,24 +15,24 @@
 //     says which block that is), so no grid-wide order is needed;
 //   * the step counter alternates between two words (step n reads word
 //     parity, writes the other), so no block has to be the last.
-// Blocks [0, gb) take 256 boundary slots each, the others 256 vectors of four
-// voxels of one plane.  The planes are walked as one row of
+// Blocks [0, gb) take 256 * PL boundary slots each, the others 256 vectors of
+// four voxels of PL consecutive planes.  The planes are walked as one row of
 // px * ny voxels: the y neighbours are px further on, no tile hangs over the
 // grid's edge, and what the row ends mix up are border voxels, whose result
 // is not kept.  Every load of a thread is independent of the others and
-// issued before any arithmetic: the latency is paid once.  One vector and
-// one plane per thread: two or four planes need 64 and 116 registers and
-// measured 5 to 60 % slower on rooms with a thick sponge layer (the boundary
-// slots share the kernel's occupancy).
-//
-// A 160x120x100 room with a sponge of 8 (0.64 M boundary slots): 17.4 us a
-// step in three launches, 10.6 us in this one; 48x40x36: 9.2 and 3.4 us.
-// From about eight million voxels on the fields come from HBM and the
-// kernels that stage planes ahead of their use win (fused_on in capi.cpp).
+// issued before any arithmetic: the latency is paid once.  Two planes and two
+// slots per thread (PL = 2) share the block's fixed costs and a plane of
+// loads; one (PL = 1) where that would leave SMs idle (fused_geo).
 //
 // Consecutive steps overlap at their ends (programmatic dependent launch):
-// a block loads what no step writes (codes, boundary positions, probes),
-// then waits for the previous step's grid.
+// a block loads what no step writes (codes, boundary positions, its probe
+// flag), then waits for the previous step's grid.
+//
+// 160x120x100 voxels with a sponge of 8 (0.64 M boundary slots): 17.4 us a
+// step in three launches, 10.4 with one plane and slot per thread, 9.4 now;
+// 300x200x130 with a sponge of 1: 28.6, 24.4 and 20.2.  Where the lines to the
+// staged kernels lie: fused_on and batch_fused in capi.cpp.
+#include <algorithm>
 #include <type_traits>
 
 #include "pdl.cuh"
@@ -78,38 +78,33 @@ __device__ __forceinline__ void put4(T *p, const float (&r)[V], uint64_t pos, ui
     *reinterpret_cast<typename Vec<T>::Raw *>(p) = raw;
 }
 
-// which probes this block owns: those at boundary slots [lo, hi) (slots) or
-// those at offsets [lo, hi) of plane z
-struct Owned {
-    bool slots;
-    uint32_t lo, hi, z;
-    __device__ bool has(const Probe &p) const
-    {
-        return slots ? p.slot >= lo && p.slot < hi
-                     : p.slot == PROBE_NO_SLOT && p.z == z && p.off >= lo && p.off < hi;
-    }
+// the block with number blk: a boundary block or one of the stencil's
+struct Site {
+    uint32_t bx, z;
 };
-
-__device__ __forceinline__ bool owns_any(const PostArgs &po, const Owned &o)
+__device__ __forceinline__ Site stencil_site(uint32_t blk, const FusedGeo &g)
 {
-    bool mine = false;
-    const uint32_t n = po.nsrc + po.nrcv;
-    for (uint32_t k = threadIdx.x; k < n; k += FB) mine |= o.has(po.probe[k]);
-    return mine;
+    const uint32_t s = blk - g.gb, bz = g.magic ? __umulhi(s, g.magic) : s / g.gx;
+    return {s - bz * g.gx, 1u + bz * g.pl};
 }
 
-// sources and receivers at the voxels this block wrote, as post_body
-// (kernels_step.cu) does for all of them
-template <typename T> __device__ __forceinline__ void post_owned(const PostArgs &po, const Owned &o, bool mine)
+// the probe list towards the L1 of a block that will go through it
+__device__ __forceinline__ void prefetch_probes(const Probe *probe, uint32_t n)
+{
+    if (threadIdx.x < n) asm volatile("prefetch.global.L1 [%0];" ::"l"(probe + threadIdx.x));
+}
+
+// Sources and receivers at the voxels this block wrote, as post_body
+// (kernels_step.cu) does for all of them; only blocks with a probe come here.
+template <typename T> __device__ __forceinline__ void post_owned(const PostArgs &po, uint32_t blk, uint32_t sn)
 {
     using IO = Io<T>;
-    if (!__syncthreads_or(mine)) return; // also: every store of this block is visible to it
+    __syncthreads(); // every store of this block is visible to it
     T *Q = static_cast<T *>(po.q);
-    const uint32_t sn = *po.ctr;
     const uint32_t k1 = po.sr ? sr_step_key(sn, 1u) : 0u;
     for (uint32_t k = threadIdx.x; k < po.nsrc; k += FB) {
         const Probe p = po.probe[k];
-        if (!o.has(p)) continue;
+        if (p.blk != blk) continue;
         const float v = sn < po.siglen ? po.sig[(uint64_t)k * po.siglen + sn] : 0.f;
         Q[p.pos] = put_rounded<T>(__fadd_rn(IO::get(Q[p.pos]), v), po.sr, p.pos, po.sr_base, k1);
     }
@@ -117,107 +112,156 @@ template <typename T> __device__ __forceinline__ void post_owned(const PostArgs 
     if (sn >= po.cap) return;
     for (uint32_t k = threadIdx.x; k < po.nrcv; k += FB) {
         const Probe p = po.probe[po.nsrc + k];
-        if (o.has(p)) po.ir[(uint64_t)k * po.cap + sn] = __fmul_rn(IO::get(Q[p.pos]), po.inv_scale);
+        if (p.blk == blk) po.ir[(uint64_t)k * po.cap + sn] = __fmul_rn(IO::get(Q[p.pos]), po.inv_scale);
     }
 }
 
-// the four voxels at position i of a plane's row, after the wait; `act`
-// false: nothing stored
-template <typename T, bool SR>
-__device__ __forceinline__ void step_vec(const StepArgs &a, const Codes<V> &code, uint32_t i, uint32_t plane, bool act)
+// out of line for PL = 2, whose registers it would take
+template <typename T> __device__ __noinline__ void post_owned_call(const PostArgs &po, uint32_t blk)
+{
+    post_owned<T>(po, blk, *po.ctr);
+}
+
+// the loads of the PL vectors at plane offset o of planes z .. z + PL - 1 (the
+// last block of an odd number of planes repeats its first plane, unstored)
+template <typename T, int PL> struct StencilVecs {
+    uint32_t i[PL];        // positions
+    Codes<V> code[PL];
+    Vec<T> c[PL + 2], yp[PL], ym[PL], q[PL]; // c: planes z - 1 .. z + PL
+    float left[PL], right[PL];
+
+    __device__ __forceinline__ void site(const StepArgs &a, uint32_t z, uint32_t o, uint32_t plane)
+    {
+#pragma unroll
+        for (int k = 0; k < PL; ++k) {
+            i[k] = (z + k < a.nz - 1u ? z + k : z) * plane + o;
+            code[k].load(a.code + i[k]);
+        }
+    }
+    __device__ __forceinline__ void values(const StepArgs &a, uint32_t plane)
+    {
+        using IO = Io<T>;
+        const T *P = static_cast<const T *>(a.p);
+        const T *Q = static_cast<const T *>(a.q);
+        c[0].load(P + (i[0] - plane));
+        c[1].load(P + i[0]);
+#pragma unroll
+        for (int k = 0; k < PL; ++k) {
+            const T *p = P + i[k];
+            c[k + 2].load(p + plane); // the plane after an unstored one: as the one after the first
+            ym[k].load(p - a.px);
+            yp[k].load(p + a.px);
+            q[k].load(Q + i[k]);
+            left[k] = IO::ld1(p - 1);
+            right[k] = IO::ld1(p + V);
+        }
+    }
+};
+
+template <typename T, int PL, bool SR>
+__device__ __forceinline__ void stencil_update(const StepArgs &a, const StencilVecs<T, PL> &s, bool act, uint32_t z)
 {
     using IO = Io<T>;
-    const T *P = static_cast<const T *>(a.p);
     T *Q = static_cast<T *>(a.q);
-    Vec<T> c, zp, zm, yp, ym, q;
-    c.load(P + i);
-    zm.load(P + (i - plane));
-    zp.load(P + (i + plane));
-    ym.load(P + (i - a.px));
-    yp.load(P + (i + a.px));
-    q.load(Q + i);
-    const float left = IO::ld1(P + (i - 1u)), right = IO::ld1(P + (i + V));
     const float2 c2dt2 = make_float2(a.c2dt2, a.c2dt2), inv_h2 = make_float2(a.inv_h2, a.inv_h2);
-    float fc[V], fzp[V], fzm[V], fyp[V], fym[V], fq[V], r[V];
-    c.get(fc);
-    zm.get(fzm);
-    zp.get(fzp);
-    ym.get(fym);
-    yp.get(fyp);
-    q.get(fq);
-    air_update(fc, left, right, fyp, fym, fzp, fzm, fq, c2dt2, inv_h2, r);
-    if (act) {
-        const uint32_t srk = SR ? sr_step_key(*a.ctr, 0u) : 0u;
+    const uint32_t srk = SR ? sr_step_key(*a.ctr, 0u) : 0u;
+#pragma unroll
+    for (int k = 0; k < PL; ++k) {
+        if (k > 0 && z + k >= a.nz - 1u) break;
+        const Codes<V> &code = s.code[k];
+        const uint32_t i = s.i[k];
+        const float left = s.left[k], right = s.right[k];
+        float fc[V], fzp[V], fzm[V], fyp[V], fym[V], fq[V], r[V];
+        s.c[k].get(fzm);
+        s.c[k + 1].get(fc);
+        s.c[k + 2].get(fzp);
+        s.ym[k].get(fym);
+        s.yp[k].get(fyp);
+        s.q[k].get(fq);
+        air_update(fc, left, right, fyp, fym, fzp, fzm, fq, c2dt2, inv_h2, r);
+        if (!act) continue;
         if (!code.any()) {
             put4<T, SR>(Q + i, r, i, a.sr_base, srk);
-        } else {
-            // voxel by voxel: border voxels keep their value, boundary
-            // voxels belong to the blocks of their slots; only air next to a
-            // wall outside a boundary layer takes the mirror rule
-            if (code.mirror()) {
+            continue;
+        }
+        // voxel by voxel: border voxels keep their value, boundary voxels
+        // belong to the blocks of their slots; only air next to a wall
+        // outside a boundary layer takes the mirror rule
+        if (code.mirror()) {
 #pragma unroll
-                for (int j = 0; j < V; ++j)
-                    if (code.get(j) != 0u && code.get(j) < CODE_BND)
-                        r[j] = leapfrog((uint8_t)code.get(j), fc[j], j == V - 1 ? right : fc[j + 1],
-                                        j == 0 ? left : fc[j - 1], fyp[j], fym[j], fzp[j], fzm[j], fq[j], a.c2dt2,
-                                        a.inv_h2);
-            }
+            for (int j = 0; j < V; ++j)
+                if (code.get(j) != 0u && code.get(j) < CODE_BND)
+                    r[j] = leapfrog((uint8_t)code.get(j), fc[j], j == V - 1 ? right : fc[j + 1],
+                                    j == 0 ? left : fc[j - 1], fyp[j], fym[j], fzp[j], fzm[j], fq[j], a.c2dt2, a.inv_h2);
+        }
 #pragma unroll
-            for (int j = 0; j < V; ++j) {
-                const uint32_t cj = code.get(j);
-                if (cj == CODE_NONE || (cj & 0xC0u) == CODE_BND) continue;
-                float v = r[j];
-                if (cj == CODE_WALL) v = 0.f;
-                else if (cj == CODE_HARD) {
-                    const uint32_t sn = *a.ctr;
-                    v = sn < a.nhard ? a.hard[sn] : 0.f;
-                }
-                Q[i + j] = SR ? Sr<T>::put(v, sr_bits((uint64_t)i + j, a.sr_base, srk)) : IO::put(v);
+        for (int j = 0; j < V; ++j) {
+            const uint32_t cj = code.get(j);
+            if (cj == CODE_NONE || (cj & 0xC0u) == CODE_BND) continue;
+            float v = r[j];
+            if (cj == CODE_WALL) v = 0.f;
+            else if (cj == CODE_HARD) {
+                const uint32_t sn = *a.ctr;
+                v = sn < a.nhard ? a.hard[sn] : 0.f;
             }
+            Q[i + j] = SR ? Sr<T>::put(v, sr_bits((uint64_t)i + j, a.sr_base, srk)) : IO::put(v);
         }
     }
 }
 
-template <typename T, int MAXS, int MODE, bool SR>
-__device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &po, uint32_t blk, uint32_t gb, uint32_t gx)
+template <typename T, int PL, int MAXS, int MODE, bool SR>
+__device__ __forceinline__ void fused_block(const StepArgs &a, const PostArgs &po, uint32_t blk, const FusedGeo &g)
 {
     const uint32_t tid = threadIdx.x;
-    if (blk < gb) {
-        const uint64_t s0 = (uint64_t)blk * FB + tid;
-        const Owned own{true, blk * FB, blk * FB + FB, 0u};
-        const bool mine = owns_any(po, own), act = s0 < a.nb;
-        BVox<T, MAXS> v;
-        if (act) bvox_site<T, MAXS>(a, s0, v);
-        pdl_wait();
-        if (act) {
-            bvox_values<T, MAXS>(a, s0, v);
-            bvox_update<T, MODE, MAXS>(a, s0, v);
+    const bool probes = __ldg(g.has_probe + blk) != 0;
+    uint32_t sn = 0;
+    if (blk < g.gb) {
+        BVox<T, MAXS> v[PL];
+        bool act[PL];
+#pragma unroll
+        for (int k = 0; k < PL; ++k) {
+            const uint64_t s = ((uint64_t)blk * PL + k) * FB + tid;
+            act[k] = s < a.nb;
+            if (act[k]) bvox_site<T, MAXS>(a, s, v[k]);
         }
-        if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
-        post_owned<T>(po, own, mine);
-        return;
+        if (PL == 1 && probes) prefetch_probes(po.probe, po.nsrc + po.nrcv);
+        pdl_wait();
+        if (PL == 1 && probes) sn = *po.ctr;
+#pragma unroll
+        for (int k = 0; k < PL; ++k)
+            if (act[k]) bvox_values<T, MAXS>(a, ((uint64_t)blk * PL + k) * FB + tid, v[k]);
+#pragma unroll
+        for (int k = 0; k < PL; ++k)
+            if (act[k]) bvox_update<T, MODE, MAXS>(a, ((uint64_t)blk * PL + k) * FB + tid, v[k]);
+    } else {
+        const Site st = stencil_site(blk, g);
+        const uint32_t plane = a.px * a.ny, o = (st.bx * FB + tid) * V;
+        const bool act = o < plane;
+        StencilVecs<T, PL> s;
+        s.site(a, st.z, act ? o : plane - V, plane); // the last block of a plane repeats its last vector, unstored
+        if (PL == 1 && probes) prefetch_probes(po.probe, po.nsrc + po.nrcv);
+        pdl_wait();
+        if (PL == 1 && probes) sn = *po.ctr;
+        s.values(a, plane);
+        stencil_update<T, PL, SR>(a, s, act, st.z);
     }
-    const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
-    const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
-    const bool act = first + tid * V < plane;
-    const Owned own{false, first, first + FB * V, z};
-    const bool mine = owns_any(po, own);
-    // the last block of a plane repeats the plane's last vector, unstored
-    const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
-    Codes<V> code;
-    code.load(a.code + i);
-    pdl_wait();
     if (blk == 0 && tid == 0) *po.ctr_out = *po.ctr + 1u;
-    step_vec<T, SR>(a, code, i, plane, act);
-    post_owned<T>(po, own, mine);
+    if (probes) {
+        if constexpr (PL == 1) post_owned<T>(po, blk, sn);
+        else post_owned_call<T>(po, blk);
+    }
 }
 
-template <typename T, int MAXS, int MODE, bool SR>
-__global__ void __launch_bounds__(FB) k_fused(const __grid_constant__ StepArgs a, const __grid_constant__ PostArgs po,
-                                              uint32_t gb, uint32_t gx)
+// blocks per SM the register allocation must allow
+template <int PL> constexpr int fused_min_blocks() { return PL == 1 ? 5 : 4; }
+
+template <typename T, int PL, int MAXS, int MODE, bool SR>
+__global__ void __launch_bounds__(FB, fused_min_blocks<PL>()) k_fused(const __grid_constant__ StepArgs a,
+                                                                      const __grid_constant__ PostArgs po,
+                                                                      const __grid_constant__ FusedGeo g)
 {
     pdl_trigger();
-    fused_block<T, MAXS, MODE, SR>(a, po, blockIdx.x, gb, gx);
+    fused_block<T, PL, MAXS, MODE, SR>(a, po, blockIdx.x, g);
 }
 
 // One step of the adjoint fields after the transposed correction
@@ -228,51 +272,59 @@ __global__ void __launch_bounds__(FB) k_fused(const __grid_constant__ StepArgs a
 // RR at boundary voxels lives in an array per slot (rr), not in the field, so
 // that no slot's RR is overwritten while its neighbours read F from the same
 // buffer.
-__global__ void __launch_bounds__(FB) k_adj_step(const __grid_constant__ StepArgs a, const __grid_constant__ AdjPost po,
-                                                 uint32_t gb, uint32_t gx)
+template <int PL>
+__global__ void __launch_bounds__(FB, fused_min_blocks<PL>()) k_adj_step(const __grid_constant__ StepArgs a,
+                                                                         const __grid_constant__ AdjPost po,
+                                                                         const __grid_constant__ FusedGeo g)
 {
     pdl_trigger();
     const uint32_t tid = threadIdx.x, blk = blockIdx.x;
-    Owned own;
-    bool mine = false;
-    const uint32_t np = po.n < 0 ? 0u : po.nsrc + po.nrcv;
-    if (blk < gb) {
-        const uint64_t s0 = (uint64_t)blk * FB + tid;
-        own = Owned{true, blk * FB, blk * FB + FB, 0u};
-        for (uint32_t k = tid; k < np; k += FB) mine |= own.has(po.probe[k]);
-        const bool act = s0 < a.nb;
-        BVox<float, 0> v;
-        if (act) bvox_site<float, 0>(a, s0, v);
+    const bool probes = po.n >= 0 && __ldg(g.has_probe + blk) != 0;
+    if (blk < g.gb) {
+        BVox<float, 0> v[PL];
+        bool act[PL];
+#pragma unroll
+        for (int k = 0; k < PL; ++k) {
+            const uint64_t s = ((uint64_t)blk * PL + k) * FB + tid;
+            act[k] = s < a.nb;
+            if (act[k]) bvox_site<float, 0>(a, s, v[k]);
+        }
         pdl_wait();
-        if (act) {
-            bvox_values<float, 0>(a, s0, v);
-            const float r = leapfrog((uint8_t)v.meta, v.ce, v.nb[0], v.nb[1], v.nb[2], v.nb[3], v.nb[4], v.nb[5],
-                                     po.rr[s0], a.c2dt2, a.inv_h2);
-            static_cast<float *>(a.q)[v.i] = __fadd_rn(r, po.dbar[s0]);
+#pragma unroll
+        for (int k = 0; k < PL; ++k)
+            if (act[k]) bvox_values<float, 0>(a, 0, v[k]);
+#pragma unroll
+        for (int k = 0; k < PL; ++k) {
+            const uint64_t s = ((uint64_t)blk * PL + k) * FB + tid;
+            if (!act[k]) continue;
+            const BVox<float, 0> &x = v[k];
+            const float r = leapfrog((uint8_t)x.meta, x.ce, x.nb[0], x.nb[1], x.nb[2], x.nb[3], x.nb[4], x.nb[5],
+                                     po.rr[s], a.c2dt2, a.inv_h2);
+            static_cast<float *>(a.q)[x.i] = __fadd_rn(r, po.dbar[s]);
         }
     } else {
-        const uint32_t s = blk - gb, bz = s / gx, bx = s - bz * gx;
-        const uint32_t plane = a.px * a.ny, z = (uint32_t)a.zb + bz, first = bx * FB * V;
-        const bool act = first + tid * V < plane;
-        own = Owned{false, first, first + FB * V, z};
-        for (uint32_t k = tid; k < np; k += FB) mine |= own.has(po.probe[k]);
-        const uint32_t i = z * plane + (act ? first + tid * V : plane - V);
-        Codes<V> code;
-        code.load(a.code + i);
+        const Site st = stencil_site(blk, g);
+        const uint32_t plane = a.px * a.ny, o = (st.bx * FB + tid) * V;
+        const bool act = o < plane;
+        StencilVecs<float, PL> s;
+        s.site(a, st.z, act ? o : plane - V, plane);
         pdl_wait();
-        step_vec<float, false>(a, code, i, plane, act);
+        s.values(a, plane);
+        stencil_update<float, PL, false>(a, s, act, st.z);
     }
-    if (!__syncthreads_or(mine)) return;
+    if (!probes) return;
+    __syncthreads();
     float *T = static_cast<float *>(a.q);
     for (uint32_t k = tid; k < po.nrcv; k += FB) {
         const Probe p = po.probe[po.nsrc + k];
         // a receiver on a voxel that no step updates reads a constant
-        if (own.has(p) && a.code[p.pos] < CODE_HARD) atomicAdd(T + p.pos, po.dl[(uint64_t)k * po.stride + (uint64_t)po.n]);
+        if (p.blk == blk && a.code[p.pos] < CODE_HARD)
+            atomicAdd(T + p.pos, po.dl[(uint64_t)k * po.stride + (uint64_t)po.n]);
     }
     __syncthreads();
     for (uint32_t k = tid; k < po.nsrc; k += FB) {
         const Probe p = po.probe[k];
-        if (own.has(p)) po.gsig[(uint64_t)k * po.stride + (uint64_t)po.n] = T[p.pos];
+        if (p.blk == blk) po.gsig[(uint64_t)k * po.stride + (uint64_t)po.n] = T[p.pos];
     }
 }
 
@@ -280,40 +332,49 @@ __global__ void __launch_bounds__(FB) k_adj_step(const __grid_constant__ StepArg
 // it; the block copies that member's arguments into shared memory once.
 // Both are constant over the steps and read before the wait.
 template <typename T, int MAXS, bool SR>
-__global__ void __launch_bounds__(FB) k_fused_batch(const BatchMember *__restrict mem, const uint2 *__restrict table,
-                                                    int parity)
+__global__ void __launch_bounds__(FB, fused_min_blocks<2>()) k_fused_batch(const BatchMember *__restrict mem,
+                                                                           const uint2 *__restrict table, int parity)
 {
     __shared__ StepArgs a;
     __shared__ PostArgs po;
+    __shared__ FusedGeo g;
     pdl_trigger();
     const uint2 e = __ldg(table + blockIdx.x);
     {
         const uint32_t *sa = reinterpret_cast<const uint32_t *>(&mem[e.x].step[parity]);
         const uint32_t *sp = reinterpret_cast<const uint32_t *>(&mem[e.x].post[parity]);
-        constexpr uint32_t na = sizeof(StepArgs) / 4, np = sizeof(PostArgs) / 4;
-        static_assert(na + np <= FB, "one word per thread");
+        const uint32_t *sg = reinterpret_cast<const uint32_t *>(&mem[e.x].geo);
+        constexpr uint32_t na = sizeof(StepArgs) / 4, np = sizeof(PostArgs) / 4, ng = sizeof(FusedGeo) / 4;
+        static_assert(na + np + ng <= FB, "one word per thread");
         const uint32_t t = threadIdx.x;
         if (t < na) reinterpret_cast<uint32_t *>(&a)[t] = __ldg(sa + t);
         else if (t < na + np) reinterpret_cast<uint32_t *>(&po)[t - na] = __ldg(sp + (t - na));
+        else if (t < na + np + ng) reinterpret_cast<uint32_t *>(&g)[t - na - np] = __ldg(sg + (t - na - np));
     }
     __syncthreads();
-    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB), gx = (a.px * a.ny + FB * V - 1) / (FB * V);
-    fused_block<T, MAXS, BND_UPDATE, SR>(a, po, e.y, gb, gx);
+    fused_block<T, 2, MAXS, BND_UPDATE, SR>(a, po, e.y, g);
 }
 
-// the slot of each probe's voxel in the boundary list (ascending positions)
-__global__ void k_probe_slots(Probe *probe, uint32_t n, const uint32_t *__restrict bpos, uint64_t nb)
+// The block of each probe's voxel: its slot's (a binary search in the
+// ascending boundary positions), else its plane's; a probe on a border plane,
+// which no block covers and no step writes, goes to the first block.
+__global__ void k_probe_blocks(Probe *probe, uint32_t n, const uint32_t *__restrict bpos, uint64_t nb, uint32_t plane,
+                               uint32_t nz, const FusedGeo g, uint8_t *has_probe)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const uint32_t pos = probe[k].pos;
+    const uint32_t pos = probe[k].pos, z = pos / plane;
     uint64_t lo = 0, hi = nb;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) / 2;
         if (bpos[mid] < pos) lo = mid + 1;
         else hi = mid;
     }
-    probe[k].slot = lo < nb && bpos[lo] == pos ? (uint32_t)lo : PROBE_NO_SLOT;
+    uint32_t blk = 0;
+    if (lo < nb && bpos[lo] == pos) blk = (uint32_t)(lo / (FB * g.pl));
+    else if (z >= 1 && z < nz - 1) blk = g.gb + (z - 1) / g.pl * g.gx + (pos - z * plane) / (FB * V);
+    probe[k].blk = blk;
+    has_probe[blk] = 1;
 }
 
 template <typename... P, typename... A>
@@ -322,46 +383,30 @@ cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, cudaStream_t s, const 
     return launch_overlapped(kern, grid, FB, 0, s, args...);
 }
 
-template <typename T, int MODE, bool SR>
-cudaError_t fused_by_sections(const StepArgs &a, const PostArgs &po, cudaStream_t s)
+template <typename T, int PL, int MODE, bool SR>
+cudaError_t fused_by_sections(const StepArgs &a, const PostArgs &po, const FusedGeo &g, cudaStream_t s)
 {
-    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB);
-    const uint32_t gx = (a.px * a.ny + FB * V - 1) / (FB * V);
-    const unsigned grid = gb + gx * (a.nz - 2);
-    if (a.nsec <= 1) return launch_pdl(k_fused<T, 1, MODE, SR>, grid, s, a, po, gb, gx);
-    if (a.nsec == 2) return launch_pdl(k_fused<T, 2, MODE, SR>, grid, s, a, po, gb, gx);
-    if (a.nsec == 3) return launch_pdl(k_fused<T, 3, MODE, SR>, grid, s, a, po, gb, gx);
-    if (a.nsec == 4) return launch_pdl(k_fused<T, 4, MODE, SR>, grid, s, a, po, gb, gx);
-    return launch_pdl(k_fused<T, 0, MODE, SR>, grid, s, a, po, gb, gx);
-}
-
-template <typename T> cudaError_t fused_16(const StepArgs &a, const PostArgs &po, cudaStream_t s)
-{
-    if (a.sr) return fused_by_sections<T, BND_UPDATE, true>(a, po, s);
-    return fused_by_sections<T, BND_UPDATE, false>(a, po, s);
-}
-
-} // namespace
-
-cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, cudaStream_t s)
-{
-    switch (storage) {
-    case VIRS_STORAGE_F16: return fused_16<__half>(a, po, s);
-    case VIRS_STORAGE_BF16: return fused_16<__nv_bfloat16>(a, po, s);
-    default:
-        return mode == BND_KEEP ? fused_by_sections<float, BND_KEEP, false>(a, po, s)
-                                : fused_by_sections<float, BND_UPDATE, false>(a, po, s);
+    switch (a.nsec) {
+    case 1: return launch_pdl(k_fused<T, PL, 1, MODE, SR>, g.blocks, s, a, po, g);
+    case 2: return launch_pdl(k_fused<T, PL, 2, MODE, SR>, g.blocks, s, a, po, g);
+    case 3: return launch_pdl(k_fused<T, PL, 3, MODE, SR>, g.blocks, s, a, po, g);
+    case 4: return launch_pdl(k_fused<T, PL, 4, MODE, SR>, g.blocks, s, a, po, g);
+    default: return launch_pdl(k_fused<T, PL, 0, MODE, SR>, g.blocks, s, a, po, g);
     }
 }
 
-cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, cudaStream_t s)
+template <typename T, int MODE, bool SR>
+cudaError_t fused_by_planes(const StepArgs &a, const PostArgs &po, const FusedGeo &g, cudaStream_t s)
 {
-    const uint32_t gb = (uint32_t)((a.nb + FB - 1) / FB);
-    const uint32_t gx = (a.px * a.ny + FB * V - 1) / (FB * V);
-    return launch_pdl(k_adj_step, gb + gx * (a.nz - 2), s, a, po, gb, gx);
+    return g.pl == 1 ? fused_by_sections<T, 1, MODE, SR>(a, po, g, s) : fused_by_sections<T, 2, MODE, SR>(a, po, g, s);
 }
 
-namespace {
+template <typename T> cudaError_t fused_16(const StepArgs &a, const PostArgs &po, const FusedGeo &g, cudaStream_t s)
+{
+    if (a.sr) return fused_by_planes<T, BND_UPDATE, true>(a, po, g, s);
+    return fused_by_planes<T, BND_UPDATE, false>(a, po, g, s);
+}
+
 template <typename T, bool SR>
 cudaError_t fused_batch_t(int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks, int parity,
                           cudaStream_t s)
@@ -375,11 +420,38 @@ cudaError_t fused_batch_t(int sections, const BatchMember *mem, const uint2 *tab
     default: return launch_pdl(k_fused_batch<T, 0, SR>, nblocks, s, mem, table, parity);
     }
 }
+
 } // namespace
 
-uint64_t fused_blocks(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb)
+FusedGeo fused_geo(uint32_t px, uint32_t ny, uint32_t nz, uint64_t nb, int sms, int pl)
 {
-    return (nb + FB - 1) / FB + ((uint64_t)px * ny + FB * V - 1) / (FB * V) * (nz - 2);
+    FusedGeo g{};
+    const uint64_t plane = (uint64_t)px * ny;
+    g.gx = (uint32_t)((plane + FB * V - 1) / (FB * V));
+    const uint64_t one = (uint64_t)g.gx * (nz - 2) + (nb + FB - 1) / FB;
+    g.pl = pl ? (uint32_t)pl : one <= 5ull * (uint64_t)sms ? 1u : 2u;
+    g.gb = (uint32_t)((nb + FB * g.pl - 1) / (FB * g.pl));
+    const uint64_t st = (uint64_t)g.gx * ((nz - 2 + g.pl - 1) / g.pl);
+    g.blocks = (uint32_t)(g.gb + st);
+    // s / gx as a multiplication: exact for s * gx below 2^32
+    g.magic = g.gx > 1 && st * g.gx < (1ull << 32) ? (uint32_t)(((1ull << 32) + g.gx - 1) / g.gx) : 0u;
+    return g;
+}
+
+cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArgs &po, const FusedGeo &g, cudaStream_t s)
+{
+    switch (storage) {
+    case VIRS_STORAGE_F16: return fused_16<__half>(a, po, g, s);
+    case VIRS_STORAGE_BF16: return fused_16<__nv_bfloat16>(a, po, g, s);
+    default:
+        return mode == BND_KEEP ? fused_by_planes<float, BND_KEEP, false>(a, po, g, s)
+                                : fused_by_planes<float, BND_UPDATE, false>(a, po, g, s);
+    }
+}
+
+cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, const FusedGeo &g, cudaStream_t s)
+{
+    return g.pl == 1 ? launch_pdl(k_adj_step<1>, g.blocks, s, a, po, g) : launch_pdl(k_adj_step<2>, g.blocks, s, a, po, g);
 }
 
 cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks,
@@ -396,10 +468,11 @@ cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem
     }
 }
 
-cudaError_t launch_probe_slots(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, cudaStream_t s)
+cudaError_t launch_probe_blocks(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, uint32_t plane,
+                                uint32_t nz, const FusedGeo &g, uint8_t *has_probe, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    k_probe_slots<<<(n + 127) / 128, 128, 0, s>>>(probe, n, bpos, nb);
+    k_probe_blocks<<<(n + 127) / 128, 128, 0, s>>>(probe, n, bpos, nb, plane, nz, g, has_probe);
     return cudaGetLastError();
 }
 
