@@ -336,7 +336,7 @@ struct virs_sim {
     bool probe_ok = false;
     uint64_t ctr_at = 0;           // the step the counter word of parity `cur` holds
     mutable std::atomic<bool> waits{false}; // kernels with bounded waits queued since check_err
-    float *host_word = nullptr;    // pinned: virs_step's sample
+    float *host_word = nullptr, *host_word_dev = nullptr; // pinned: virs_step's sample
     uint64_t steps_done = 0;
 
     // constants
@@ -1042,15 +1042,16 @@ cudaError_t launch_stencil_range(const virs_sim *s, int parity, cudaStream_t st,
     return launch_step_tma(s->prm.storage, s->tile_rows, s->depth, a, m, s->err.as<int>(), st);
 }
 
-cudaError_t enqueue_step(const virs_sim *s, int parity, cudaStream_t st)
+cudaError_t enqueue_step(const virs_sim *s, int parity, cudaStream_t st, float *host0 = nullptr)
 {
-    if (fused_on(s))
-        return launch_fused(s->prm.storage, BND_UPDATE, step_args(s, parity), post_args(s, parity), s->geo, st);
+    PostArgs po = post_args(s, parity);
+    po.host0 = host0;
+    if (fused_on(s)) return launch_fused(s->prm.storage, BND_UPDATE, step_args(s, parity), po, s->geo, st);
     cudaError_t e = launch_stencil(s, parity, st);
     if (e != cudaSuccess) return e;
     e = launch_boundary(s->prm.storage, step_args(s, parity), BND_UPDATE, st);
     if (e != cudaSuccess) return e;
-    return launch_post(s->prm.storage, post_args(s, parity), st);
+    return launch_post(s->prm.storage, po, st);
 }
 
 // ---- two steps per pass -------------------------------------------------------
@@ -2461,21 +2462,24 @@ VIRS_EXPORT virs_status virs_step(virs_sim *s, uint32_t step, int *keep_going, f
     cudaStream_t st = s->stream;
     // the reference uploads the source value every step
     // (simulator_gpu.cu:250-258); here the step number, unless the counter
-    // already stands there.  The sample comes back through pinned memory, so
-    // that the call waits once.
-    if (!s->host_word) VIRS_CUDA(cudaHostAlloc((void **)&s->host_word, sizeof(float), cudaHostAllocDefault));
+    // already stands there.  The kernel that records receiver 0's sample
+    // stores it into pinned host memory as well, so that the call waits once
+    // and copies nothing.
+    if (!s->host_word) {
+        VIRS_CUDA(cudaHostAlloc((void **)&s->host_word, sizeof(float), cudaHostAllocMapped));
+        VIRS_CUDA(cudaHostGetDevicePointer((void **)&s->host_word_dev, s->host_word, 0));
+    }
     if (s->ctr_at != step)
         VIRS_CUDA(cudaMemcpyAsync(s->ctr.as<uint32_t>() + s->cur, &step, 4, cudaMemcpyHostToDevice, st));
     s->ctr_at = UINT64_MAX;
-    cudaError_t e = enqueue_step(s, s->cur, st);
+    *s->host_word = 0.f;
+    cudaError_t e = enqueue_step(s, s->cur, st, s->host_word_dev);
     if (e != cudaSuccess) return cuda_fail(e, "step launch");
     s->cur ^= 1;
     s->steps_done = std::max<uint64_t>(s->steps_done, (uint64_t)step + 1);
     s->ctr_at = (uint64_t)step + 1;
-    *s->host_word = 0.f;
-    if (s->nrcv) VIRS_CUDA(cudaMemcpyAsync(s->host_word, s->ir.as<float>() + step, 4, cudaMemcpyDeviceToHost, st));
     VIRS_CUDA(cudaStreamSynchronize(st));
-    const float v = *s->host_word;
+    const float v = *(volatile float *)s->host_word;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     VIRS_TRY(check_err(s));
     if (sample) *sample = v;
@@ -3039,9 +3043,8 @@ struct virs_batch {
     int dev = 0, storage = 0, rows = 8, depth = 2, planes = 0;
     bool persistent = false;
     bool waits = false;            // kernels with bounded waits queued since virs_batch_synchronize
-    bool tiling_set = false, fused = false; // a step in one launch (kernels_fused.cu), through `table`
-    DevBuf table;
-    uint32_t nblocks = 0;
+    bool tiling_set = false, fused = false; // a step in one launch (kernels_fused.cu) per 64 members: `launches`
+    std::vector<FusedBatch> launches[2]; // per parity
     uint64_t ntiles = 0, nbnd = 0;
     int sections = 0;              // launch_boundary_batch
     DevBuf desc, err;
@@ -3085,11 +3088,11 @@ virs_status batch_check(const virs_batch *b)
 // A step of the batch in one launch (kernels_fused.cu) when its members are
 // small (their rows fill few of the stencil's 128-voxel tiles) or few.
 // Measured per step, three launches against one (sponge 1-2, three sections):
-//   4 rooms, 0.6 M voxels in all    FP32  29.5 against   6.3 us   BF16  33.6 against   6.1 us
-//   12, 2.9 M                             44.0            23.0           46.7            21.3
-//   24, 26 M (1.1 M each)                148             124            127             111
-//   100, 97 M (0.97 M each)              548             498            444             449
-//   30, 50 M (1.7 M each)                281             266            244             241
+//   4 rooms, 0.6 M voxels in all    FP32  29.5 against   6.3 us   BF16  33.6 against   6.2 us
+//   12, 2.9 M                             44.0            22.0           46.9            21.3
+//   24, 26 M (1.1 M each)                148             111            127             109
+//   100, 97 M (0.97 M each)              551             454            448             445
+//   30, 50 M (1.7 M each)                286             242            246             241
 //   20, 86 M (4.3 M each)                341             346            281             313
 // so the line lies at 3 M voxels per member in FP32, 1.5 M in 16-bit storage
 // (row padding included), and at 12 M in all for fewer, larger members.
@@ -3106,7 +3109,7 @@ virs_status batch_build(virs_batch *b)
 {
     b->drop_graphs();
     b->fused = batch_fused(b);
-    std::vector<uint2> table;
+    for (auto &l : b->launches) l.clear();
     b->zmasks.clear();
     b->probes.clear();
     std::vector<BatchMember> h(b->mem.size());
@@ -3128,9 +3131,10 @@ virs_status batch_build(virs_batch *b)
         VIRS_TRY(encode(&m.mapC, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, s->code.ptr, s, (uint32_t)tma_tile_x(), b->rows));
         const int zc = b->planes > 0 ? b->planes : (s->zc > 0 ? s->zc : default_planes(s->nz));
         const uint64_t *zm = nullptr;
+        FusedGeo geo{};
         if (b->fused) {
             b->probes.emplace_back();
-            VIRS_TRY(make_probes(s, 2, b->probes.back(), &m.geo));
+            VIRS_TRY(make_probes(s, 2, b->probes.back(), &geo));
             VIRS_CUDA(cudaStreamSynchronize(s->stream));
         }
         if (!b->fused && zero_masks_useful(s)) {
@@ -3151,9 +3155,16 @@ virs_status batch_build(virs_batch *b)
         m.gx = (s->px + tma_tile_x() - 1) / tma_tile_x();
         m.gy = (s->ny + b->rows - 1) / b->rows;
         m.gz = (s->nz - 2 + zc - 1) / zc;
-        if (b->fused) {
-            for (uint32_t k = 0; k < m.geo.blocks; ++k) table.push_back(make_uint2((uint32_t)i, k));
-        }
+        if (b->fused)
+            for (int par = 0; par < 2; ++par) {
+                auto &l = b->launches[par];
+                if (i % FUSED_MEMBERS == 0) l.emplace_back(FusedBatch{});
+                FusedBatch &f = l.back();
+                f.first[f.n] = f.blocks;
+                f.m[f.n] = {m.step[par], m.post[par], geo};
+                f.blocks += geo.blocks;
+                ++f.n;
+            }
         m.first_tile = tiles;
         m.first_bnd = bnd;
         tiles += (uint64_t)m.gx * m.gy * m.gz;
@@ -3164,11 +3175,6 @@ virs_status batch_build(virs_batch *b)
     }
     VIRS_TRY(b->desc.alloc(h.size() * sizeof(BatchMember), "batch descriptors"));
     VIRS_CUDA(copy_on(b->stream, b->desc.ptr, h.data(), h.size() * sizeof(BatchMember), cudaMemcpyHostToDevice));
-    if (b->fused) {
-        VIRS_TRY(b->table.alloc(table.size() * sizeof(uint2), "batch block table"));
-        VIRS_CUDA(copy_on(b->stream, b->table.ptr, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-        b->nblocks = (uint32_t)table.size();
-    }
     b->ntiles = tiles;
     b->nbnd = bnd;
     b->sections = max_sections > 4 ? 0 : min_sections == max_sections ? (int)max_sections : -4;
@@ -3179,9 +3185,13 @@ cudaError_t batch_enqueue(const virs_batch *b, int parity, cudaStream_t st)
 {
     const BatchMember *d = b->desc.as<BatchMember>();
     const uint32_t n = (uint32_t)b->mem.size();
-    if (b->fused)
-        return launch_fused_batch(b->storage, b->sections, d, b->table.as<uint2>(), b->nblocks, parity, st,
-                                  sr_on(b->mem[0]));
+    if (b->fused) {
+        for (const FusedBatch &f : b->launches[parity]) {
+            const cudaError_t e = launch_fused_batch(b->storage, b->sections, f, st, sr_on(b->mem[0]));
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     cudaError_t e =
         launch_step_tma_batch(b->storage, b->rows, b->depth, d, n, b->ntiles, parity, b->persistent, b->err.as<int>(), st,
                               sr_on(b->mem[0]));

@@ -148,6 +148,7 @@ struct PostArgs {
     const float *sig;       // [nsrc][siglen] (scaled)
     const uint64_t *rcv;    // device indices
     float *ir;              // [nrcv][cap]
+    float *host0;           // receiver 0's sample goes here too (pinned host memory; nullptr: not)
     const uint32_t *ctr;    // device step counter: read here,
     uint32_t *ctr_out;      // ... and the next step's written here (the counter alternates between two words)
     const Probe *probe;     // [nsrc] sources, then [nrcv] receivers
@@ -170,7 +171,6 @@ struct alignas(64) BatchMember {
     CUtensorMap mapC;       // cell codes
     StepArgs step[2];       // per parity: p = field[parity], q = field[parity ^ 1]
     PostArgs post[2];
-    FusedGeo geo;           // step in one launch: the member's blocks
     const uint32_t *bidx;
     uint64_t first_tile;    // index of this member's first tile in the batch
     uint64_t first_bnd;     // index of this member's first boundary voxel
@@ -184,9 +184,21 @@ cudaError_t launch_boundary_batch(int storage, const BatchMember *mem, uint32_t 
                                   int sections, cudaStream_t s);
 cudaError_t launch_post_batch(int storage, const BatchMember *mem, uint32_t nmem, int parity, cudaStream_t s);
 
-// the same in one launch (kernels_fused.cu): table[block] = {member, block of the member}
-cudaError_t launch_fused_batch(int storage, int sections, const BatchMember *mem, const uint2 *table, uint32_t nblocks,
-                               int parity, cudaStream_t s, bool sr);
+// the same in one launch (kernels_fused.cu), up to FUSED_MEMBERS members per
+// launch, as kernel parameters
+constexpr uint32_t FUSED_MEMBERS = 64;
+struct FusedMember {
+    StepArgs step;
+    PostArgs post;
+    FusedGeo geo;
+};
+struct FusedBatch {
+    uint32_t n, blocks;
+    uint32_t first[FUSED_MEMBERS]; // a member's first block
+    FusedMember m[FUSED_MEMBERS];
+};
+static_assert(sizeof(FusedBatch) <= 32764, "kernel parameter space");
+cudaError_t launch_fused_batch(int storage, int sections, const FusedBatch &b, cudaStream_t s, bool sr);
 
 // kernel launchers (kernels_step.cu)
 cudaError_t launch_step(int storage, int tile_rows, const StepArgs &a, cudaStream_t s);

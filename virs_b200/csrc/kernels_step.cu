@@ -361,8 +361,11 @@ template <typename T> __device__ __forceinline__ void post_body(const PostArgs &
     }
     __syncthreads();
     if (sn < a.cap)
-        for (uint32_t r = threadIdx.x; r < a.nrcv; r += blockDim.x)
-            a.ir[(uint64_t)r * a.cap + sn] = __fmul_rn(IO::get(Q[a.rcv[r]]), a.inv_scale);
+        for (uint32_t r = threadIdx.x; r < a.nrcv; r += blockDim.x) {
+            const float v = __fmul_rn(IO::get(Q[a.rcv[r]]), a.inv_scale);
+            a.ir[(uint64_t)r * a.cap + sn] = v;
+            if (r == 0 && a.host0) *a.host0 = v;
+        }
     __syncthreads();
     if (threadIdx.x == 0) {
         if (a.stop && a.nrcv && sn < a.cap) stop_rule(a, sn);
