@@ -1066,11 +1066,10 @@ bool pair_on(const virs_sim *s)
 }
 
 // The two-step kernel's tile: the caller's, or, when the caller left rows and
-// planes to the library, 16 rows and as many planes as leave about four
-// blocks per SM, 16 to 60 (the zero-code masks cover the 64 stages of 60
-// planes).  Per step in FP32, 14 rows over all planes against this rule:
-// 1024x768x512 856 and 770 us, 701x517x333 271 and 251, 512x300x200 109 and
-// 79, 254x259x325 161 and 72.
+// planes to the library, 14 rows and as many planes as leave about four
+// blocks per SM, 16 to 42 (the zero-code masks cover 64 stages).  Per step in
+// FP32, all planes against this rule: 1024x768x512 792 and 685 us,
+// 701x517x333 266 and 232, 512x384x192 129 and 88; 16 rows 725, 233 and 89.
 struct PairTile {
     int rows, zc;
 };
@@ -1078,24 +1077,25 @@ PairTile pair_tile(const virs_sim *s)
 {
     if (!s->pair_auto) return {s->pair_rows, s->pair_zc};
     const uint64_t ix = (uint64_t)pair_tile_x(s->prm.storage);
-    const uint64_t tiles = (s->px + ix - 1) / ix * ((s->ny + 13) / 14);
+    const uint64_t tiles = (s->px + ix - 1) / ix * ((s->ny + 11) / 12);
     const uint64_t zc = (uint64_t)(s->nz - 2) * tiles / (4ull * (uint64_t)sm_count(s->prm.device));
-    return {16, (int)std::min<uint64_t>(std::max<uint64_t>(zc, 16), 60)};
+    return {14, (int)std::min<uint64_t>(std::max<uint64_t>(zc, 16), 42)};
 }
 
 // Whether a run takes its groups of four steps two at a time.  With the tile
-// left to the library, only where that is the faster way to the same bits:
-// not on grids whose single steps take one launch each (150x140x130: 10 us a
-// step against 20), and not in 16-bit storage, where the two-step kernel is
-// bound by issue (the hall 528 against 650 us, 701x517x333 186 against 230).
-// The timing of the parts takes two steps as asked.
+// left to the library, only where that is the faster way to the same bits: in
+// FP32 above 28 M voxels (per step, one launch a step against two steps per
+// pass: 24 M 66.7 and 66 us, 38 M 95.0 and 88.3, 60 M 159 and 143), not in
+// 16-bit storage, where the two-step kernel is bound by issue (the hall 515
+// against 600 us, 701x517x333 187 against 211).  The timing of the parts
+// takes two steps as asked.
 bool pairs_pay(const virs_sim *s)
 {
-    return !s->pair_auto || s->timing || (s->prm.storage == VIRS_STORAGE_F32 && !fused_on(s));
+    return !s->pair_auto || s->timing || (s->prm.storage == VIRS_STORAGE_F32 && (!fused_on(s) || s->nvox > (28u << 20)));
 }
 
 // the voxels whose p^{n+2} the two-step kernel leaves provisional, for the
-// current codes, boundary list and sources (kernels_classify.cu)
+// current codes and sources (kernels_classify.cu)
 virs_status build_pair_list(virs_sim *s)
 {
     cudaStream_t st = s->stream;
@@ -1108,7 +1108,7 @@ virs_status build_pair_list(virs_sim *s)
     VIRS_TRY(tmp.alloc(scan_tmp_words(nseg) * 4, "scan scratch", s->stream));
     VIRS_TRY(total.alloc(4, "provisional-voxel total"));
     VIRS_CUDA(cudaMemsetAsync(mark.ptr, 0, s->nvox, st));
-    VIRS_CUDA(launch_pair_marks(s->code.as<uint8_t>(), s->px, s->ny, s->nz, s->bpos.as<uint32_t>(), s->nb,
+    VIRS_CUDA(launch_pair_marks(s->code.as<uint8_t>(), s->px, s->ny, s->nz,
                                 s->hpos.as<uint32_t>(), s->nhpos, s->src.as<uint64_t>(), s->nsrc, mark.as<uint8_t>(),
                                 cnt.as<uint32_t>(), st));
     VIRS_CUDA(launch_scan(cnt.as<uint32_t>(), nseg, tmp.as<uint32_t>(), total.as<uint32_t>(), st));
@@ -1201,9 +1201,15 @@ PostArgs post_args_buf(const virs_sim *s, int q, int parity)
 }
 
 // Two steps from parity par: p^n in buffer x, p^{n-1} in y; p^{n+1} to z, p^{n+2} to w.
-// After k_pair_tma the first step is completed (boundary pass, post kernel);
-// then one launch runs the second step's boundary pass and recomputes its
-// provisional voxels, and the second post kernel follows.
+// The first step's boundary pass comes first: it reads p^n and its own
+// voxels' p^{n-1}, and leaves their p^{n+1} in y, where the two-step kernel
+// keeps what it finds at boundary voxels, so that its second step sees the
+// final p^{n+1} around them.  (y is not read again.)  After the kernel the
+// post kernel completes the first step; then one launch runs the second
+// step's boundary pass and recomputes the voxels at and next to sources, and
+// the second post kernel follows.  With the boundary pass after the kernel,
+// every neighbour of a boundary voxel had to be recomputed: 201 us per two
+// steps of the 1024x768x512 hall for that launch, 99 now.
 cudaError_t enqueue_pair(const virs_sim *s, int par, int x, int y, int z, int w, cudaStream_t st,
                          cudaEvent_t *ev = nullptr)
 {
@@ -1215,9 +1221,10 @@ cudaError_t enqueue_pair(const virs_sim *s, int par, int x, int y, int z, int w,
     const TmaMaps m{&s->pmP[x], &s->pmQ[y], &s->pmC};
     s->waits = true;
     if (ev) cudaEventRecord(ev[0], st);
-    cudaError_t e = launch_pair_tma(sto, tile.rows, a, m, buf_ptr(s, z), buf_ptr(s, w), s->err.as<int>(), st);
+    cudaError_t e = launch_boundary(sto, step_args_bufs(s, x, y), BND_UPDATE, st);
     if (ev) cudaEventRecord(ev[1], st);
-    if (e == cudaSuccess) e = launch_boundary(sto, step_args_bufs(s, x, z), BND_UPDATE, st);
+    if (e == cudaSuccess)
+        e = launch_pair_tma(sto, tile.rows, a, m, buf_ptr(s, z), buf_ptr(s, w), s->err.as<int>(), st);
     if (ev) cudaEventRecord(ev[2], st);
     if (e == cudaSuccess) e = launch_post(sto, post_args_buf(s, z, par), st);
     if (ev) cudaEventRecord(ev[3], st);
@@ -1332,8 +1339,8 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
             double ms = 0, bms = 0;
             for (uint64_t p = 0; p < 2 * quads && err == cudaSuccess; ++p) {
                 float t = 0, b1 = 0, b2 = 0;
-                err = cudaEventElapsedTime(&t, ev[5 * p], ev[5 * p + 1]);
-                if (err == cudaSuccess) err = cudaEventElapsedTime(&b1, ev[5 * p + 1], ev[5 * p + 2]);
+                err = cudaEventElapsedTime(&b1, ev[5 * p], ev[5 * p + 1]);
+                if (err == cudaSuccess) err = cudaEventElapsedTime(&t, ev[5 * p + 1], ev[5 * p + 2]);
                 if (err == cudaSuccess) err = cudaEventElapsedTime(&b2, ev[5 * p + 3], ev[5 * p + 4]);
                 ms += t;
                 bms += (double)b1 + b2;

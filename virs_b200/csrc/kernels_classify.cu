@@ -553,13 +553,13 @@ cudaError_t launch_pair_zero_masks(const uint8_t *segnz, uint32_t px, uint32_t n
 
 // ---- voxels whose second step of a two-step pass is provisional --------------
 //
-// The two-step stencil computes p^{n+2} from p^{n+1} before the boundary
-// pass and the post kernel have changed p^{n+1} at boundary voxels and
-// sources.  The p^{n+2} of every voxel the stencil updates (air or mirror
-// code: bit 7 clear) that is such a voxel or its face neighbour must be
-// recomputed afterwards.  k_pair_mark marks them, k_mark_count counts the
-// marks of each 1024-voxel segment, and after an exclusive scan of the
-// counts k_mark_list writes their positions in ascending order.
+// The two-step stencil computes p^{n+2} from p^{n+1} before the post kernel
+// has changed p^{n+1} at the sources.  The p^{n+2} of every voxel the stencil
+// updates (air or mirror code: bit 7 clear) that is a source or its face
+// neighbour must be recomputed afterwards.  k_pair_mark marks them,
+// k_mark_count counts the marks of each 1024-voxel segment, and after an
+// exclusive scan of the counts k_mark_list writes their positions in
+// ascending order.
 namespace {
 constexpr int MARK_B = 1024;
 
@@ -577,12 +577,12 @@ __device__ __forceinline__ void mark_around(const uint8_t *__restrict code, uint
 }
 
 __global__ void k_pair_mark(const uint8_t *__restrict code, uint32_t px, uint32_t ny, uint32_t nz,
-                            const uint32_t *__restrict bpos, uint64_t nb, const uint32_t *__restrict hpos, uint32_t nh,
-                            const uint64_t *__restrict src, uint32_t nsrc, uint8_t *mark)
+                            const uint32_t *__restrict hpos, uint32_t nh, const uint64_t *__restrict src,
+                            uint32_t nsrc, uint8_t *mark)
 {
-    const uint64_t n = nb + nh + nsrc;
+    const uint64_t n = (uint64_t)nh + nsrc;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t v = i < nb ? (uint64_t)bpos[i] : i < nb + nh ? (uint64_t)hpos[i - nb] : src[i - nb - nh];
+        const uint64_t v = i < nh ? (uint64_t)hpos[i] : src[i - nh];
         mark_around(code, mark, v, px, ny, nz);
     }
 }
@@ -607,15 +607,15 @@ __global__ void __launch_bounds__(MARK_B) k_mark_list(const uint8_t *__restrict 
 
 size_t mark_segments(uint64_t nvox) { return (size_t)((nvox + MARK_B - 1) / MARK_B); }
 
-cudaError_t launch_pair_marks(const uint8_t *code, uint32_t px, uint32_t ny, uint32_t nz, const uint32_t *bpos,
-                              uint64_t nb, const uint32_t *hpos, uint32_t nh, const uint64_t *src, uint32_t nsrc,
+cudaError_t launch_pair_marks(const uint8_t *code, uint32_t px, uint32_t ny, uint32_t nz, const uint32_t *hpos,
+                              uint32_t nh, const uint64_t *src, uint32_t nsrc,
                               uint8_t *mark, uint32_t *cnt, cudaStream_t s)
 {
     const uint64_t nvox = (uint64_t)px * ny * nz;
-    if (nb + nh + nsrc) {
-        const uint64_t n = nb + nh + nsrc;
+    if (nh + nsrc) {
+        const uint64_t n = (uint64_t)nh + nsrc;
         const unsigned g = (unsigned)std::min<uint64_t>((n + 255) / 256, 148ull * 16);
-        k_pair_mark<<<g, 256, 0, s>>>(code, px, ny, nz, bpos, nb, hpos, nh, src, nsrc, mark);
+        k_pair_mark<<<g, 256, 0, s>>>(code, px, ny, nz, hpos, nh, src, nsrc, mark);
     }
     k_mark_count<<<(unsigned)mark_segments(nvox), MARK_B, 0, s>>>(mark, nvox, cnt);
     return cudaGetLastError();

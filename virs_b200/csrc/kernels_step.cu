@@ -200,9 +200,8 @@ __global__ void __launch_bounds__(BT) k_boundary(const __grid_constant__ StepArg
 // its boundary pass and the recomputation of its provisional voxels, in one
 // launch.  Blocks [0, gb) take boundary slots as k_boundary does; the others
 // take entries of the provisional-voxel list: air and mirror voxels at or
-// next to a voxel whose p^{n+1} the first step's boundary pass or post
-// kernel changed, whose p^{n+2} the two-step kernel computed from the
-// provisional p^{n+1}.  They are recomputed from the final p^{n+1} (a.p) and
+// next to a source, whose p^{n+1} the first step's post kernel changed, and
+// whose p^{n+2} the two-step kernel computed from the provisional p^{n+1}.  They are recomputed from the final p^{n+1} (a.p) and
 // p^n (pn) with leapfrog(code, ...), which is bit-identical to the air
 // update for code 0 and is the mirror update for the others.  Both parts
 // read p^{n+1} and write disjoint voxels of p^{n+2} (a.q): boundary voxels,

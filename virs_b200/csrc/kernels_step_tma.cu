@@ -474,13 +474,16 @@ cudaError_t launch_batch1(int rows, int depth, const BatchMember *mem, uint32_t 
 // hard-source and border voxels keep the previous value in both steps, as
 // in k_step_tma.
 //
-// Voxels whose p^{n+1} changes after the stencil (boundary voxels, by the
-// boundary pass; hard and soft sources, by the post kernel) make the
-// p^{n+2} of their air neighbours (and of a soft source itself) provisional:
-// k_boundary_fix (kernels_step.cu) recomputes those from the final p^{n+1}
-// in the launch of the second boundary pass, so two steps through this
-// kernel give the results of two single steps bit for bit.  The fields are read once and written once per
-// two steps: four buffers, p^n and p^{n-1} in, p^{n+1} and p^{n+2} out.
+// The first step's boundary pass runs before this kernel and leaves the
+// p^{n+1} of the boundary voxels in the p^{n-1} buffer, where "keep the
+// previous value" finds it.  Voxels whose p^{n+1} changes after the stencil
+// (hard and soft sources, by the post kernel) make the p^{n+2} of their air
+// neighbours (and of a soft source itself) provisional: k_boundary_fix
+// (kernels_step.cu) recomputes those from the final p^{n+1} in the launch of
+// the second boundary pass, so two steps through this kernel give the
+// results of two single steps bit for bit.  The fields are read once and
+// written once per two steps: four buffers, p^n and p^{n-1} in, p^{n+1} and
+// p^{n+2} out.
 //
 // The code box is TX + 16 bytes wide with its x origin rounded down to 16
 // bytes (a TMA copy of 8-bit elements must start on a 16-byte boundary).
