@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(LB) k_ir_resample(const float *__restrict in, 
 // a lane's next tap follows from the last by the rotation by 32 taps, except
 // near tau = 0, where its relative error would matter.  8 channels, 4000 to
 // 5049 samples, 490 taps: 1463 us with the series, a sine and a division per
-// tap and channel, one output per thread; 49 us in this form (two chains of half the length, odd and
-// even powers, took 52: the FP64 rate bounds it, not the chain).
+// tap and channel, one output per thread; 46 us in this form (two chains of
+// half the length, odd and even powers, were no faster: the FP64 rate bounds
+// it, not the chain).
 constexpr int CH = 8;            // channels per warp
 constexpr int SINC_TERMS = 128;  // of the series (beta <= 50 needs 80)
 struct SincArgs {
@@ -152,7 +153,13 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
                                                 const __grid_constant__ SincArgs a, float *__restrict out,
                                                 uint64_t out_len, uint32_t channels, uint32_t *__restrict peak)
 {
-    const int lane = threadIdx.x & 31;
+    // the series' coefficients, two per load (indexed reads of the parameters
+    // are served one at a time: 49 us)
+    __shared__ double2 cf[SINC_TERMS / 2];
+    for (int j = threadIdx.x; j < SINC_TERMS / 2; j += RB)
+        cf[j] = make_double2(2 * j < a.terms ? a.c[2 * j] : 0.0, 2 * j + 1 < a.terms ? a.c[2 * j + 1] : 0.0);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, pairs = (a.terms + 1) / 2;
     const uint64_t k = (uint64_t)blockIdx.x * (RB / 32) + threadIdx.x / 32;
     if (k >= out_len) return; // the whole warp
     const uint32_t c0 = blockIdx.y * CH, nc = min(channels - c0, (uint32_t)CH);
@@ -173,8 +180,12 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
         sn = s2;
         if (!(fabs(u) < 1.0)) continue;
         const double v = 1.0 - u * u;
-        double w = a.c[a.terms - 1];
-        for (int j = a.terms - 2; j >= 0; --j) w = fma(w, v, a.c[j]);
+        double w = 0.0;
+#pragma unroll 4
+        for (int j = pairs - 1; j >= 0; --j) {
+            const double2 c = cf[j];
+            w = fma(fma(w, v, c.y), v, c.x);
+        }
         w *= tau == 0.0 ? a.fc2 : s / (M_PI * tau);
         const float *fn = f + (uint64_t)n;
 #pragma unroll
