@@ -93,7 +93,7 @@ __device__ __forceinline__ void adj_store(const AdjArgs &a, uint64_t b, uint32_t
     a.rr[b] = __fsub_rn(__fadd_rn(fr, db), cq);
 }
 
-constexpr int AB = 256;
+constexpr int AB = 128;
 
 // The sum of v over the lanes of a full warp that share this lane's key
 // (peers = __match_any_sync of the key), complete at the group's lowest
