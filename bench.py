@@ -98,7 +98,7 @@ def stencil_roofline(r, storage: str):
     f32 = storage == "f32"
     if r.get("time_blocking", {}).get("active"):
         return (PAIR_F32 if f32 else PAIR_16, 2, "k_pair_tma<%s> (two steps per pass; then the boundary passes, "
-                "post kernels and the fix-up of the voxels next to boundary voxels and sources)" % KERNEL_TYPES[storage],
+                "post kernels and the fix-up of the voxels next to sources)" % KERNEL_TYPES[storage],
                 ROOT / "profiles" / "k_pair_tma_dram_traffic.txt")
     return (BYTES_F32 if f32 else BYTES_16, 1,
             "k_step_tma<%s> (stencil; boundary voxels in a separate list pass)" % KERNEL_TYPES[storage],
@@ -596,7 +596,7 @@ def run_virs(args):
                                "effective bandwidth above the bytes moved" % (upd, steps_per_launch),
             "boundary_pass_ms": r32.get("boundary_ms"),
             "boundary_pass_note": ("per step: a two-step pass's two boundary launches (the second also recomputes "
-                                   "the voxels next to boundary voxels and sources), halved" if steps_per_launch == 2
+                                   "the voxels next to sources), halved" if steps_per_launch == 2
                                    else "per step"),
         },
         "e2e": {

@@ -390,13 +390,12 @@ virs_status virs_set_tiling(virs_sim *sim, int tile_rows, int planes_per_block, 
  * and virs_run_host advance whole groups of four steps two at a time: one
  * kernel reads p^n and p^{n-1} once and writes p^{n+1} and p^{n+2}, over two
  * more field buffers allocated on first use (a grid for which they do not fit
- * runs single steps).  The voxels next to boundary voxels and sources are
- * recomputed after the first step is complete, so the results are
- * bit-identical to single steps.  tile_rows 12, 14, 16 or 32 (0 = 14; with
+ * runs single steps).  The voxels next to sources are recomputed after the
+ * first step is complete, so the results are bit-identical to single steps.  tile_rows 12, 14, 16 or 32 (0 = 14; with
  * 12, 14 and 16 rows 4, 3 and 2 planes are in flight), planes per block
  * 0 = all.  With both 0 the library chooses the tile, and takes single steps
- * where they are faster (small grids, 16-bit storage).  Off (1) by default; not used with the register-streaming
- * kernel (pipeline depth 0).  With the device stop rule, a run that stops
+ * where they are faster (FP32 below 28 M voxels, 16-bit storage).  Off (1) by
+ * default; not used with the register-streaming kernel (pipeline depth 0).  With the device stop rule, a run that stops
  * inside a group of four steps leaves the stop step's fields in the usual
  * buffers, as single steps do.  *active tells whether the current settings
  * allow two steps per pass. */
