@@ -104,3 +104,32 @@ def test_small_batch_same_bits_as_three_launches(storage, sections):
         assert np.abs(x[0]).max() > 0
         for u, v in zip(x, y):
             assert np.array_equal(u.view(np.uint32), v.view(np.uint32))
+
+
+@pytest.mark.parametrize("n_rcv", [1, 3])
+def test_first_one_launch_step_on_a_callers_stream(n_rcv):
+    """The probes of the one-launch step are made inside the run (the timing
+    of the parts, on at the start, did not need them) and the run takes
+    another stream than the handle's."""
+    import torch
+    shape, steps = (150, 90, 40), 64
+    n = int(np.prod(shape))
+    mid = (20 * 90 + 45) * 150 + 75
+    out = []
+    for late in (False, True):
+        sim = capi.Simulation(capi.default_params(sponge_width=1, courant=1.0, boundary_form=1))
+        sim.set_grid(shape, 0.05, np.zeros(n, np.uint8), np.zeros(n, np.uint8))
+        sim.classify()
+        sim.set_sources([mid], np.random.default_rng(3).standard_normal((1, steps)).astype(np.float32))
+        sim.set_receivers([mid + k for k in range(n_rcv)])
+        sim.set_timing(late)
+        sim.start(steps)
+        sim.set_timing(False)
+        st = torch.cuda.Stream()
+        sim.run(steps, st.cuda_stream if late else None)
+        sim.synchronize()
+        out.append((sim.ir(), *sim.pressure(prev=True)))
+        sim.close()
+    assert np.abs(out[0][0]).max() > 0
+    for u, v in zip(*out):
+        assert np.array_equal(u.view(np.uint32), v.view(np.uint32))

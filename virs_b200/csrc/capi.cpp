@@ -921,6 +921,7 @@ virs_status make_probes(const virs_sim *s, int pl, DevBuf &buf, FusedGeo *geo)
 virs_status build_probes(virs_sim *s)
 {
     VIRS_TRY(make_probes(s, 0, s->probe, &s->geo));
+    VIRS_CUDA(cudaStreamSynchronize(s->stream)); // the run may take a caller's stream
     s->probe_ok = true;
     s->graph_dirty = true;
     return VIRS_OK;
