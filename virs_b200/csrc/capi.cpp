@@ -297,7 +297,8 @@ struct virs_sim {
     // the owned planes and a ghost plane each side) starts slab_drop planes
     // into them.  For a whole grid ext_nz == nz and slab_drop == 0.
     bool slab = false;
-    cudaStream_t xstream = nullptr;    // virs_slab_run: the ghost-plane pulls, beside the interior stencil
+    cudaStream_t xstream = nullptr;    // virs_slab_run: the ghost-plane pulls, beside the interior stencil;
+                                       // virs_adjoint: the recomputation, beside the reverse steps
     cudaEvent_t xdone = nullptr;       // ... and their completion
     int rounding = VIRS_ROUND_NEAREST; // of the 16-bit stores (virs_set_rounding)
     uint32_t ext_nz = 0, slab_drop = 0;
@@ -411,7 +412,8 @@ struct virs_sim {
         uint64_t steps = 0, nck = 0, gen = 0;
         uint32_t every = 0;
         bool ready = false;
-        DevBuf ckp, ckq, cks, segrec, segst, buf[2], ast, dbar, rr[2], grad, dl, gsig;
+        DevBuf ckp, ckq, cks, segrec[2], segst[2], buf[2], ast, dbar, rr[2], grad, dl, gsig;
+        cudaEvent_t built[2] = {}, used[2] = {}; // a segment's buffers are filled, and read
     } adj;
     bool fields_valid = true;      // false after virs_adjoint until the next start
     bool slab_open = false;        // virs_slab_step_begin ran, virs_slab_step_end not yet
@@ -422,6 +424,8 @@ struct virs_sim {
         slab_graph.reset();
         if (done) cudaEventDestroy(done);
         if (xdone) cudaEventDestroy(xdone);
+        for (cudaEvent_t e : {adj.built[0], adj.built[1], adj.used[0], adj.used[1]})
+            if (e) cudaEventDestroy(e);
         if (xstream) cudaStreamDestroy(xstream);
         if (stream) cudaStreamDestroy(stream);
         if (host_word) cudaFreeHost(host_word);
@@ -3462,6 +3466,47 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
     return VIRS_OK;
 }
 
+namespace {
+// Whether a segment is recomputed beside the reverse steps of the segment
+// after it, on a second stream with a second set of segment buffers (`extra`
+// bytes).  On small grids both chains are bound by latency (128x128x96, 256
+// steps, 64 or 16 to a segment: a gradient 6.44 -> 5.60 and 7.10 -> 5.62 ms;
+// 80x64x60 2.37 -> 1.95, 170x120x110 with 0.5 M slots 9.67 -> 9.3); on large ones little is left
+// to gain (400x300x250 19.07 -> 18.82) and the buffers grow, hence the 1 GiB.
+// Without the memory for them the two take turns in one stream.
+bool adj_beside(virs_sim *s, size_t extra)
+{
+    auto &A = s->adj;
+    if (A.nck < 2 || extra > (1u << 30)) return false;
+    const uint64_t every = A.every;
+    if (A.segrec[1].alloc(every * std::max<uint64_t>(s->nb, 1) * sizeof(float4), "adjoint segment records", s->stream,
+                          false) != VIRS_OK ||
+        A.segst[1].alloc(every * state_bytes(s), "adjoint segment states", s->stream, false) != VIRS_OK) {
+        A.segrec[1].release();
+        A.segst[1].release();
+        return false;
+    }
+    if (!s->xstream && cudaStreamCreateWithFlags(&s->xstream, cudaStreamNonBlocking) != cudaSuccess) {
+        s->xstream = nullptr;
+        return false;
+    }
+    for (cudaEvent_t *e : {&A.built[0], &A.built[1], &A.used[0], &A.used[1]})
+        if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) {
+            *e = nullptr;
+            return false;
+        }
+    return true;
+}
+// on every way out nothing is left on the second stream
+struct AdjBeside {
+    cudaStream_t st;
+    ~AdjBeside()
+    {
+        if (st) cudaStreamSynchronize(st);
+    }
+};
+} // namespace
+
 VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *grad_coef, float *grad_signal)
 {
     if (!s || !dl_dir) return fail(VIRS_E_ARG, "virs_adjoint: null argument");
@@ -3476,8 +3521,9 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     // adjoints, four per section
     const size_t fb = s->nvox * 4, sb = state_bytes(s), sba = std::max<uint64_t>(nb, 1) * s->nsec * 4 * 4;
     const uint32_t ncoef = s->nmat * s->nsec * 5;
-    VIRS_TRY(A.segrec.alloc(every * std::max<uint64_t>(nb, 1) * sizeof(float4), "adjoint segment records", st, false));
-    VIRS_TRY(A.segst.alloc(every * sb, "adjoint segment states", st, false));
+    const size_t rb = every * std::max<uint64_t>(nb, 1) * sizeof(float4);
+    VIRS_TRY(A.segrec[0].alloc(rb, "adjoint segment records", st, false));
+    VIRS_TRY(A.segst[0].alloc(every * sb, "adjoint segment states", st, false));
     for (int k = 0; k < 2; ++k) VIRS_TRY(A.buf[k].alloc(fb, "adjoint field", st));
     VIRS_TRY(A.ast.alloc(sba, "adjoint filter states", st));
     VIRS_TRY(A.dbar.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms", st));
@@ -3488,6 +3534,13 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     if (s->nrcv) VIRS_CUDA(copy_on(s->stream, A.dl.ptr, dl_dir, (size_t)s->nrcv * steps * 4, cudaMemcpyHostToDevice));
     VIRS_TRY(ready_to_run(s));
     if (!s->probe_ok) VIRS_TRY(build_probes(s));
+    const bool beside = adj_beside(s, rb + every * sb);
+    AdjBeside both{beside ? s->xstream : nullptr};
+    cudaStream_t rst = beside ? s->xstream : st; // the recomputation's stream
+    if (beside) {
+        VIRS_CUDA(cudaEventRecord(A.used[0], st));
+        VIRS_CUDA(cudaStreamWaitEvent(rst, A.used[0], 0));
+    }
     int t = 0; // A.buf[t] holds T, A.buf[t ^ 1] holds RR; A.rr[t] the RR of the boundary slots
     VIRS_CUDA(launch_adj_inject(A.buf[t].as<float>(), s->code.as<uint8_t>(), s->rcv.as<uint64_t>(), s->nrcv,
                                 A.dl.as<float>(), steps, steps - 1, s->src.as<uint64_t>(), s->nsrc,
@@ -3496,11 +3549,15 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
         const uint64_t n0 = (uint64_t)c * every, n1 = std::min<uint64_t>(n0 + every, steps);
         // rebuild the segment: restore the checkpoint and run forward, keeping
         // the states before every step and the stencil's boundary records
+        const int w = beside ? (int)(c & 1) : 0;
+        float4 *segrec = A.segrec[w].as<float4>();
+        char *segst = A.segst[w].as<char>();
         s->cur = 0;
-        VIRS_CUDA(cudaMemcpyAsync(s->field[0].ptr, A.ckp.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, st));
-        VIRS_CUDA(cudaMemcpyAsync(s->field[1].ptr, A.ckq.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, st));
-        VIRS_CUDA(cudaMemcpyAsync(A.segst.ptr, A.cks.as<char>() + c * sb, sb, cudaMemcpyDeviceToDevice, st));
-        VIRS_CUDA(launch_set_u32(s->ctr.as<uint32_t>(), (uint32_t)n0, st));
+        if (beside && c + 2 < (int64_t)A.nck) VIRS_CUDA(cudaStreamWaitEvent(rst, A.used[w], 0));
+        VIRS_CUDA(cudaMemcpyAsync(s->field[0].ptr, A.ckp.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
+        VIRS_CUDA(cudaMemcpyAsync(s->field[1].ptr, A.ckq.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
+        VIRS_CUDA(cudaMemcpyAsync(segst, A.cks.as<char>() + c * sb, sb, cudaMemcpyDeviceToDevice, rst));
+        VIRS_CUDA(launch_set_u32(s->ctr.as<uint32_t>(), (uint32_t)n0, rst));
         for (uint64_t n = n0; n < n1; ++n) {
             const uint64_t k = n - n0;
             // the boundary pass keeps its records straight in the segment's
@@ -3508,27 +3565,30 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
             // writes those after it to slot k + 1 (the last step's to the
             // handle's own states)
             StepArgs ka = step_args(s, s->cur);
-            ka.side = A.segrec.as<float4>() + k * nb;
-            ka.state = reinterpret_cast<float *>(A.segst.as<char>() + k * sb);
-            ka.state_out = k + 1 < every ? reinterpret_cast<float *>(A.segst.as<char>() + (k + 1) * sb)
-                                         : s->state.as<float>();
+            ka.side = segrec + k * nb;
+            ka.state = reinterpret_cast<float *>(segst + k * sb);
+            ka.state_out = k + 1 < every ? reinterpret_cast<float *>(segst + (k + 1) * sb) : s->state.as<float>();
             cudaError_t e;
             if (fused_on(s)) {
-                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), s->geo, st);
+                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), s->geo, rst);
             } else {
-                e = launch_stencil(s, s->cur, st);
-                if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, st);
-                if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, s->cur), st);
+                e = launch_stencil(s, s->cur, rst);
+                if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, rst);
+                if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, s->cur), rst);
             }
             if (e != cudaSuccess) return cuda_fail(e, "adjoint recomputation");
             s->cur ^= 1;
+        }
+        if (beside) {
+            VIRS_CUDA(cudaEventRecord(A.built[w], rst));
+            VIRS_CUDA(cudaStreamWaitEvent(st, A.built[w], 0));
         }
         // reverse steps of the segment
         for (int64_t n = (int64_t)n1 - 1; n >= (int64_t)n0; --n) {
             const uint64_t k = (uint64_t)n - n0;
             StepArgs a = step_args(s, 0);
-            cudaError_t e = launch_adj_boundary(a, A.buf[t].as<float>(), A.segrec.as<float4>() + k * nb,
-                                                reinterpret_cast<const float *>(A.segst.as<char>() + k * sb),
+            cudaError_t e = launch_adj_boundary(a, A.buf[t].as<float>(), segrec + k * nb,
+                                                reinterpret_cast<const float *>(segst + k * sb),
                                                 A.ast.as<float4>(), A.dbar.as<float>(), A.rr[t ^ 1].as<float>(),
                                                 A.grad.as<double>(), s->nmat, n + 1 < (int64_t)n1, st);
             if (e == cudaSuccess) {
@@ -3542,6 +3602,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
             if (e != cudaSuccess) return cuda_fail(e, "adjoint step");
             t ^= 1;
         }
+        if (beside) VIRS_CUDA(cudaEventRecord(A.used[w], st));
     }
     VIRS_CUDA(cudaStreamSynchronize(st));
     VIRS_TRY(check_err(s));
