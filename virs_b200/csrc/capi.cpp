@@ -3545,6 +3545,10 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     VIRS_CUDA(launch_adj_inject(A.buf[t].as<float>(), s->code.as<uint8_t>(), s->rcv.as<uint64_t>(), s->nrcv,
                                 A.dl.as<float>(), steps, steps - 1, s->src.as<uint64_t>(), s->nsrc,
                                 A.gsig.as<float>(), steps, st));
+    // up to four sections: a reverse step is one launch
+    const bool one = s->nsec <= 4;
+    AdjSlots slots{nullptr, nullptr, A.ast.as<float4>(), A.dbar.as<float>(), A.rr[0].as<float>(), A.grad.as<double>(), ncoef};
+    if (one) VIRS_CUDA(launch_adj_open(step_args(s, 0), slots, A.buf[t].as<float>(), st));
     for (int64_t c = (int64_t)A.nck - 1; c >= 0; --c) {
         const uint64_t n0 = (uint64_t)c * every, n1 = std::min<uint64_t>(n0 + every, steps);
         // rebuild the segment: restore the checkpoint and run forward, keeping
@@ -3587,18 +3591,19 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
         for (int64_t n = (int64_t)n1 - 1; n >= (int64_t)n0; --n) {
             const uint64_t k = (uint64_t)n - n0;
             StepArgs a = step_args(s, 0);
-            cudaError_t e = launch_adj_boundary(a, A.buf[t].as<float>(), segrec + k * nb,
-                                                reinterpret_cast<const float *>(segst + k * sb),
-                                                A.ast.as<float4>(), A.dbar.as<float>(), A.rr[t ^ 1].as<float>(),
-                                                A.grad.as<double>(), s->nmat, n + 1 < (int64_t)n1, st);
-            if (e == cudaSuccess) {
-                a.p = A.buf[t].ptr;
-                a.q = A.buf[t ^ 1].ptr;
-                a.nhard = 0;
-                const AdjPost po{s->probe.as<Probe>(), s->nsrc, s->nrcv, A.rr[t].as<float>(), A.dbar.as<float>(),
-                                 A.dl.as<float>(), A.gsig.as<float>(), steps, n - 1};
-                e = launch_adj_step(a, po, s->geo, st);
-            }
+            slots.rec = segrec + k * nb;
+            slots.fst = reinterpret_cast<const float *>(segst + k * sb);
+            const AdjPost po{s->probe.as<Probe>(), s->nsrc, s->nrcv, A.rr[t].as<float>(), A.dbar.as<float>(),
+                             A.dl.as<float>(), A.gsig.as<float>(), steps, n - 1};
+            cudaError_t e = cudaSuccess;
+            if (!one)
+                e = launch_adj_boundary(a, A.buf[t].as<float>(), slots.rec, slots.fst, slots.ast, A.dbar.as<float>(),
+                                        A.rr[t ^ 1].as<float>(), slots.grad, s->nmat, st);
+            a.p = A.buf[t].ptr;
+            a.q = A.buf[t ^ 1].ptr;
+            a.nhard = 0;
+            if (e == cudaSuccess)
+                e = one ? launch_adj_one(a, po, slots, s->geo, n + 1 < (int64_t)n1, st) : launch_adj_step(a, po, s->geo, st);
             if (e != cudaSuccess) return cuda_fail(e, "adjoint step");
             t ^= 1;
         }

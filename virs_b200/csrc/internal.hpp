@@ -220,6 +220,21 @@ struct AdjPost {
     uint64_t stride;
     int64_t n;              // the next reverse step (-1: none)
 };
+// per boundary slot: the forward records and states before the step (slot of
+// the segment), the state adjoints [S][nb], T' and its RR, and the sums
+struct AdjSlots {
+    const float4 *rec;
+    const float *fst;
+    float4 *ast;
+    float *traw, *rr;
+    double *grad;           // [M][S][5]
+    uint32_t ncoef;
+};
+// a reverse step of up to four sections in one launch; overlap: the kernel
+// before it in the stream is one too (nothing that wrote rec or fst)
+cudaError_t launch_adj_open(const StepArgs &a, const AdjSlots &x, float *T, cudaStream_t s);
+cudaError_t launch_adj_one(const StepArgs &a, const AdjPost &po, const AdjSlots &x, const FusedGeo &g, bool overlap,
+                           cudaStream_t s);
 cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, const FusedGeo &g, cudaStream_t s);
 cudaError_t launch_probe_blocks(Probe *probe, uint32_t n, const uint32_t *bpos, uint64_t nb, uint32_t plane,
                                 uint32_t nz, const FusedGeo &g, uint8_t *has_probe, cudaStream_t s);
@@ -325,10 +340,9 @@ cudaError_t launch_hard_list(const uint8_t *code, uint64_t n, uint32_t *count, u
 cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv, uint32_t nrcv, const float *dl,
                               uint64_t dl_stride, uint64_t n, const uint64_t *src, uint32_t nsrc, float *gsig,
                               uint64_t gs_stride, cudaStream_t s);
-// f: the forward step's arguments; overlap: the kernel before on the stream
-// is launch_adj_step (nothing that wrote rec or fst)
+// f: the forward step's arguments
 cudaError_t launch_adj_boundary(const StepArgs &f, float *T, const float4 *rec, const float *fst, float4 *ast,
-                                float *dbar, float *rr, double *grad, uint32_t nmat, bool overlap, cudaStream_t s);
+                                float *dbar, float *rr, double *grad, uint32_t nmat, cudaStream_t s);
 cudaError_t launch_set_u32(uint32_t *p, uint32_t v, cudaStream_t s);
 cudaError_t launch_zero_at(float *f, const uint32_t *pos, uint32_t n, cudaStream_t s);
 

@@ -21,10 +21,11 @@
 // The forward values the cascade needs (p - q and the states before step n)
 // come from a recomputation of the segment from the last checkpoint.
 //
-// 128x128x96 voxels, 79 K slots of two sections: a reverse step was five
-// launches of 28.7 us and their gaps, two of 12 us in all now.
+// Cascades of up to four sections take both in one launch (k_adj_one,
+// kernels_fused.cu).  128x128x96 voxels, 79 K slots of two sections: a reverse
+// step was five launches of 28.7 us and their gaps, then two of 12, now one.
+#include "adjoint.cuh"
 #include "pdl.cuh"
-#include "step_common.cuh"
 
 namespace virs {
 namespace {
@@ -49,7 +50,7 @@ struct AdjArgs {
     float *T;                  // adjoint field (p role)
     const uint32_t *bpos, *bmeta; // as StepArgs
     const BndWeight *wtab;
-    const float *coef, *coefp; // [M][S][5], and padded to vectors (StepArgs)
+    const float *coef;         // [M][S][5]
     const float4 *rec;         // forward records of this step {free, p, q, 0}
     const float *fst;          // forward states before this step (the cascade's layout, state_index)
     float4 *ast;               // state adjoints, one vector per section [S][nb]
@@ -61,29 +62,6 @@ struct AdjArgs {
     double kg, mix_y, mix_d;   // K * gain
 };
 
-// the transposed correction of one slot: the value F left in the adjoint
-// field, the cascade output's adjoint and what dbar and RR' take beyond it
-struct AdjCorr {
-    double fr, ybar, db, cq;
-};
-__device__ __forceinline__ AdjCorr adj_correct(const AdjArgs &a, float f, uint32_t meta)
-{
-    const BndWeight e = a.wtab[meta >> 16];
-    AdjCorr c;
-    if (a.form == VIRS_BOUNDARY_REFERENCE) {
-        const double kgw = a.kg * e.kgw; // the weight itself
-        c.fr = f;
-        c.ybar = -kgw * a.mix_y * f;
-        c.db = -kgw * a.mix_d * f;
-        c.cq = 0.0;
-    } else {
-        c.fr = quotient((double)f, e.den, e.rden);
-        c.ybar = -e.kgw * a.mix_y * c.fr;
-        c.db = 0.0;
-        c.cq = e.ac * c.fr;
-    }
-    return c;
-}
 // the slot's results: F into the field, dbar, and RR' = F + dbar - cq
 __device__ __forceinline__ void adj_store(const AdjArgs &a, uint64_t b, uint32_t pos, const AdjCorr &c, double yb)
 {
@@ -126,7 +104,7 @@ __global__ void __launch_bounds__(AB) k_adj_boundary(const AdjArgs a)
     const uint64_t b = (uint64_t)blockIdx.x * AB + threadIdx.x;
     if (b < a.nb) {
         const uint32_t pos = a.bpos[b], meta = a.bmeta[b];
-        const AdjCorr c = adj_correct(a, a.T[pos], meta);
+        const AdjCorr c = adj_correct(a.wtab, a.form, a.kg, a.mix_y, a.mix_d, a.T[pos], meta);
         // forward inputs of every section at this step
         const uint32_t S = a.nsec, m = (meta >> 8) & 0xffu;
         const float *kc = a.coef + (uint64_t)m * S * 5;
@@ -183,131 +161,6 @@ __global__ void __launch_bounds__(AB) k_adj_boundary(const AdjArgs a)
         if (gsm[k] != 0.0) atomicAdd(a.grad + k, gsm[k]);
 }
 
-// The sums of v[0..N) over a warp (N a power of two): each exchange halves
-// the values a lane holds, so N values cost N - 1 + log2(32 / N) shuffles
-// instead of 5 N.  Returns the sum of value *idx, the same on every lane of
-// a group of 32 / N.
-template <int N> __device__ __forceinline__ double warp_sums(double (&v)[N], int *idx)
-{
-    const int lane = (int)(threadIdx.x & 31u);
-    int k = 0;
-    int n = N;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        if (n > 1) {
-            n /= 2;
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int j = 0; j < N / 2; ++j)
-                if (j < n) {
-                    const double give = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
-                    v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                }
-            k += up ? n : 0;
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-        }
-    }
-    *idx = k;
-    return v[0];
-}
-
-// Cascades of S = 1..4 sections, unrolled: the forward section inputs and
-// the filter states stay in registers.  What the forward recomputation and
-// the set-up wrote (records, states, positions) is read before the wait for
-// the kernel before; the launch that opens a segment does not overlap with
-// the recomputation (launch_adj_boundary).  The 5 S gradient terms of a
-// warp's slots are summed one material at a time, nearly always one or two
-// per warp.  A shuffle tree per term, records and states after the wait and
-// a double-precision division made it 15.4 us at 79 K slots of two sections,
-// 7.6 us now.
-template <int S> __global__ void __launch_bounds__(AB) k_adj_boundary_s(const __grid_constant__ AdjArgs a)
-{
-    constexpr int NG = (2 * (S + 1) + 3) / 4, NC = (5 * S + 3) / 4, NV = 5 * S;
-    constexpr int NP = NV <= 8 ? 8 : NV <= 16 ? 16 : 32;
-    extern __shared__ double gsm[]; // block partial sums of the coefficient gradients
-    pdl_trigger();
-    const uint64_t b = (uint64_t)blockIdx.x * AB + threadIdx.x;
-    const bool act = b < a.nb;
-    const uint64_t bl = act ? b : a.nb - 1; // idle lanes of the last block repeat its last slot, unstored
-    const uint32_t pos = __ldg(a.bpos + bl), meta = __ldg(a.bmeta + bl), m = (meta >> 8) & 0xffu;
-    const float4 rec = a.rec[bl];
-    float h[4 * NG], kc[4 * NC];
-#pragma unroll
-    for (int g = 0; g < NG; ++g) {
-        const float4 v = reinterpret_cast<const float4 *>(a.fst)[(uint64_t)g * a.nb + bl];
-        h[4 * g] = v.x;
-        h[4 * g + 1] = v.y;
-        h[4 * g + 2] = v.z;
-        h[4 * g + 3] = v.w;
-    }
-#pragma unroll
-    for (int g = 0; g < NC; ++g) {
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(a.coefp) + m * NC + g);
-        kc[4 * g] = v.x;
-        kc[4 * g + 1] = v.y;
-        kc[4 * g + 2] = v.z;
-        kc[4 * g + 3] = v.w;
-    }
-    for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB) gsm[k] = 0.0;
-    // forward inputs of every section at this step
-    float xin[S];
-    float in = __fsub_rn(rec.y, rec.z);
-#pragma unroll
-    for (int q = 0; q < S; ++q) {
-        xin[q] = in;
-        float yv = __fmaf_rn(kc[5 * q], in, __fmul_rn(kc[5 * q + 1], h[2 * q]));
-        yv = __fmaf_rn(kc[5 * q + 2], h[2 * q + 1], yv);
-        yv = __fmaf_rn(-kc[5 * q + 3], h[2 * q + 2], yv);
-        in = __fmaf_rn(-kc[5 * q + 4], h[2 * q + 3], yv);
-    }
-    pdl_wait();
-    float4 aq[S];
-#pragma unroll
-    for (int q = 0; q < S; ++q) aq[q] = a.ast[(uint64_t)q * a.nb + bl];
-    const AdjCorr c = adj_correct(a, a.T[pos], meta);
-    double yb = c.ybar, gv[NP];
-#pragma unroll
-    for (int j = NV; j < NP; ++j) gv[j] = 0.0;
-#pragma unroll
-    for (int q = S - 1; q >= 0; --q) {
-        const double yt = yb + (double)aq[q].z;
-        gv[5 * q] = yt * (double)xin[q];
-        gv[5 * q + 1] = yt * (double)h[2 * q];
-        gv[5 * q + 2] = yt * (double)h[2 * q + 1];
-        gv[5 * q + 3] = -yt * (double)h[2 * q + 2];
-        gv[5 * q + 4] = -yt * (double)h[2 * q + 3];
-        const double xbar = (double)kc[5 * q] * yt + (double)aq[q].x;
-        const double x1 = (double)kc[5 * q + 1] * yt + (double)aq[q].y;
-        const double x2 = (double)kc[5 * q + 2] * yt;
-        const double y1 = -(double)kc[5 * q + 3] * yt + (double)aq[q].w;
-        const double y2 = -(double)kc[5 * q + 4] * yt;
-        aq[q] = make_float4((float)x1, (float)x2, (float)y1, (float)y2);
-        yb = xbar;
-    }
-    if (act) {
-#pragma unroll
-        for (int q = 0; q < S; ++q) a.ast[(uint64_t)q * a.nb + b] = aq[q];
-        adj_store(a, b, pos, c, yb);
-    }
-    __syncthreads(); // gsm is zero
-    unsigned left = __ballot_sync(0xffffffffu, act);
-    while (left) {
-        const uint32_t mm = __shfl_sync(0xffffffffu, m, __ffs(left) - 1);
-        const bool mine = act && m == mm;
-        left &= ~__ballot_sync(0xffffffffu, mine);
-        double v[NP];
-#pragma unroll
-        for (int j = 0; j < NP; ++j) v[j] = mine ? gv[j] : 0.0;
-        int idx;
-        const double sum = warp_sums<NP>(v, &idx);
-        if (idx < NV && (threadIdx.x & (32 / NP - 1)) == 0) atomicAdd(gsm + mm * NV + idx, sum);
-    }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < a.ncoef; k += AB)
-        if (gsm[k] != 0.0) atomicAdd(a.grad + k, gsm[k]);
-}
-
 } // namespace
 
 cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv, uint32_t nrcv, const float *dl,
@@ -319,25 +172,12 @@ cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv
 }
 
 cudaError_t launch_adj_boundary(const StepArgs &f, float *T, const float4 *rec, const float *fst, float4 *ast,
-                                float *dbar, float *rr, double *grad, uint32_t nmat, bool overlap, cudaStream_t s)
+                                float *dbar, float *rr, double *grad, uint32_t nmat, cudaStream_t s)
 {
     if (f.nb == 0) return cudaSuccess;
-    const AdjArgs a{T, f.bpos, f.bmeta, f.wtab, f.coef, f.coefp, rec, fst, ast, dbar, rr, grad, f.nb, f.nsec,
+    const AdjArgs a{T, f.bpos, f.bmeta, f.wtab, f.coef, rec, fst, ast, dbar, rr, grad, f.nb, f.nsec,
                     nmat * f.nsec * 5, f.form, f.K * f.gain, f.mix_y, f.mix_d};
-    const size_t sm = (size_t)a.ncoef * sizeof(double);
-    const unsigned g = (unsigned)((f.nb + AB - 1) / AB);
-    const auto run = [&](void (*kern)(AdjArgs)) {
-        if (overlap) return launch_overlapped(kern, g, AB, sm, s, a);
-        kern<<<g, AB, sm, s>>>(a);
-        return cudaGetLastError();
-    };
-    switch (f.nsec) {
-    case 1: return run(k_adj_boundary_s<1>);
-    case 2: return run(k_adj_boundary_s<2>);
-    case 3: return run(k_adj_boundary_s<3>);
-    case 4: return run(k_adj_boundary_s<4>);
-    default: return run(k_adj_boundary);
-    }
+    return launch_overlapped(k_adj_boundary, (unsigned)((f.nb + AB - 1) / AB), AB, (size_t)a.ncoef * sizeof(double), s, a);
 }
 
 namespace {

@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "adjoint.cuh"
 #include "pdl.cuh"
 #include "step_voxel.cuh"
 
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(FB, fused_min_blocks<PL>()) k_fused(const __gr
 }
 
 // One step of the adjoint fields after the transposed correction
-// (kernels_adjoint.cu): the stencil T' = A F - RR (F in a.p, RR and then T'
+// (k_adj_boundary, kernels_adjoint.cu; cascades of more than four sections): the stencil T' = A F - RR (F in a.p, RR and then T'
 // in a.q), at a boundary slot T' = (the mirrored leapfrog on F with the
 // slot's own RR) + dbar, and on what a block wrote the sources' gradients
 // and the receivers' loss gradients of the next reverse step n (n < 0: none).
@@ -329,6 +330,216 @@ __global__ void __launch_bounds__(FB, fused_min_blocks<PL>()) k_adj_step(const _
         const Probe p = po.probe[k];
         if (p.blk == blk) po.gsig[(uint64_t)k * po.stride + (uint64_t)po.n] = T[p.pos];
     }
+}
+
+// One reverse step in one launch, for cascades of S = 1..4 sections: as
+// k_adj_step, with a slot's transposed correction and cascade run by the
+// thread that then updates its voxel.  That needs no value of another slot of
+// this step, because what the neighbours read at a boundary voxel, F, depends
+// on T there alone: the thread that makes T' leaves F' = the transposed
+// correction of T' in the field and T' itself in an array per slot (traw).
+// Records and states, which the recomputation wrote, are read before the wait
+// for the kernel before; the launch that opens a segment does not overlap
+// with what came before it.  The gradient terms of a warp's slots are summed
+// in FP64 one material at a time, nearly always one or two per warp.  A
+// gradient over 256 steps of 128x128x96 (79 K slots of two sections), the
+// recomputation beside it: 5.60 ms with the cascade in a launch of its own
+// before the stencil's, 4.78 now; over 128 steps of 300x200x160 (three
+// sections) 12.78 and 12.38.
+//
+// adj_sections: sections [q0, q0 + N) of a slot, transposed, and their sums.
+template <int N, int NH, int NK, int S>
+__device__ __forceinline__ void adj_sections(const StepArgs &a, const AdjSlots &x, uint64_t b, bool act, uint32_t m, int q0,
+                                             const float (&h)[NH], const float (&kc)[NK], const float (&xin)[S],
+                                             const float4 (&aq)[S], double &yb, double *gsm)
+{
+    constexpr int NV = 5 * N, NP = NV <= 8 ? 8 : 16;
+    double gv[NP];
+#pragma unroll
+    for (int j = NV; j < NP; ++j) gv[j] = 0.0;
+#pragma unroll
+    for (int n = N - 1; n >= 0; --n) {
+        const int q = q0 + n;
+        const double yt = yb + (double)aq[q].z;
+        gv[5 * n] = yt * (double)xin[q];
+        gv[5 * n + 1] = yt * (double)h[2 * q];
+        gv[5 * n + 2] = yt * (double)h[2 * q + 1];
+        gv[5 * n + 3] = -yt * (double)h[2 * q + 2];
+        gv[5 * n + 4] = -yt * (double)h[2 * q + 3];
+        const double xbar = (double)kc[5 * q] * yt + (double)aq[q].x;
+        const double x1 = (double)kc[5 * q + 1] * yt + (double)aq[q].y;
+        const double x2 = (double)kc[5 * q + 2] * yt;
+        const double y1 = -(double)kc[5 * q + 3] * yt + (double)aq[q].w;
+        const double y2 = -(double)kc[5 * q + 4] * yt;
+        if (act) x.ast[(uint64_t)q * a.nb + b] = make_float4((float)x1, (float)x2, (float)y1, (float)y2);
+        yb = xbar;
+    }
+    unsigned left = __ballot_sync(0xffffffffu, act);
+    while (left) {
+        const uint32_t mm = __shfl_sync(0xffffffffu, m, __ffs(left) - 1);
+        const bool mine = act && m == mm;
+        left &= ~__ballot_sync(0xffffffffu, mine);
+        double v[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) v[j] = mine ? gv[j] : 0.0;
+        int idx;
+        const double sum = warp_sums<NP>(v, &idx);
+        if (idx < NV && (threadIdx.x & (32 / NP - 1)) == 0) atomicAdd(gsm + (mm * S + q0) * 5 + idx, sum);
+    }
+}
+
+template <int S>
+__device__ __forceinline__ void adj_slot(const StepArgs &a, const AdjSlots &x, uint64_t b, bool first, double *gsm)
+{
+    constexpr int NG = (2 * (S + 1) + 3) / 4, NC = (5 * S + 3) / 4;
+    const bool act = b < a.nb;
+    const uint64_t bl = act ? b : a.nb - 1; // idle lanes of the last block repeat its last slot, unstored
+    const uint32_t pos = __ldg(a.bpos + bl), meta = __ldg(a.bmeta + bl), m = (meta >> 8) & 0xffu;
+    const float4 rec = x.rec[bl];
+    float h[4 * NG], kc[4 * NC];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const float4 v = reinterpret_cast<const float4 *>(x.fst)[(uint64_t)g * a.nb + bl];
+        h[4 * g] = v.x;
+        h[4 * g + 1] = v.y;
+        h[4 * g + 2] = v.z;
+        h[4 * g + 3] = v.w;
+    }
+#pragma unroll
+    for (int g = 0; g < NC; ++g) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(a.coefp) + m * NC + g);
+        kc[4 * g] = v.x;
+        kc[4 * g + 1] = v.y;
+        kc[4 * g + 2] = v.z;
+        kc[4 * g + 3] = v.w;
+    }
+    // forward inputs of every section at this step
+    float xin[S];
+    float in = __fsub_rn(rec.y, rec.z);
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+        xin[q] = in;
+        float yv = __fmaf_rn(kc[5 * q], in, __fmul_rn(kc[5 * q + 1], h[2 * q]));
+        yv = __fmaf_rn(kc[5 * q + 2], h[2 * q + 1], yv);
+        yv = __fmaf_rn(-kc[5 * q + 3], h[2 * q + 2], yv);
+        in = __fmaf_rn(-kc[5 * q + 4], h[2 * q + 3], yv);
+    }
+    if (first) {
+        pdl_wait();
+        __syncthreads(); // gsm is zero
+    }
+    const float *P = static_cast<const float *>(a.p);
+    const uint32_t sy = a.px, sz = a.px * a.ny;
+    const float t = x.traw[bl], rr = x.rr[bl];
+    float4 aq[S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) aq[q] = x.ast[(uint64_t)q * a.nb + bl];
+    const float n0 = P[pos + 1], n1 = P[pos - 1], n2 = P[pos + sy], n3 = P[pos - sy], n4 = P[pos + sz], n5 = P[pos - sz];
+    const double kg = a.K * a.gain;
+    const AdjCorr c = adj_correct(a.wtab, a.form, kg, a.mix_y, a.mix_d, t, meta);
+    const float fr = (float)c.fr;
+    const float r = leapfrog((uint8_t)meta, fr, n0, n1, n2, n3, n4, n5, rr, a.c2dt2, a.inv_h2);
+    double yb = c.ybar;
+#pragma unroll
+    for (int q0 = (S - 1) / 2 * 2; q0 >= 0; q0 -= 2) { // two sections at a time: more terms at once cost registers
+        if (q0 + 1 < S) adj_sections<2, 4 * NG, 4 * NC, S>(a, x, b, act, m, q0, h, kc, xin, aq, yb, gsm);
+        else adj_sections<1, 4 * NG, 4 * NC, S>(a, x, b, act, m, q0, h, kc, xin, aq, yb, gsm);
+    }
+    if (act) {
+        const float db = (float)(c.db + yb), tn = __fadd_rn(r, db);
+        x.rr[b] = __fsub_rn(__fadd_rn(fr, db), (float)c.cq);
+        x.traw[b] = tn;
+        static_cast<float *>(a.q)[pos] = (float)adj_correct(a.wtab, a.form, kg, a.mix_y, a.mix_d, tn, meta).fr;
+    }
+}
+
+// the slot at a position a slot block owns
+__device__ __forceinline__ uint64_t slot_of(const StepArgs &a, uint32_t pos, uint64_t lo, uint64_t hi)
+{
+    while (hi - lo > 1) {
+        const uint64_t mid = (lo + hi) / 2;
+        if (a.bpos[mid] <= pos) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// sources and receivers at the voxels this block wrote; `slots`: it owns slots
+// [s0, s1), whose T' is in traw and whose F' is in the field
+__device__ __noinline__ void adj_owned(const StepArgs &a, const AdjPost &po, const AdjSlots &x, uint32_t blk, bool slots,
+                                       uint64_t s0, uint64_t s1)
+{
+    __syncthreads();
+    float *T = static_cast<float *>(a.q);
+    for (uint32_t k = threadIdx.x; k < po.nrcv; k += FB) {
+        const Probe p = po.probe[po.nsrc + k];
+        // a receiver on a voxel that no step updates reads a constant
+        if (p.blk == blk && a.code[p.pos] < CODE_HARD)
+            atomicAdd(slots ? x.traw + slot_of(a, p.pos, s0, s1) : T + p.pos,
+                      po.dl[(uint64_t)k * po.stride + (uint64_t)po.n]);
+    }
+    __syncthreads();
+    if (slots)
+        for (uint32_t k = threadIdx.x; k < po.nrcv; k += FB) {
+            const Probe p = po.probe[po.nsrc + k];
+            if (p.blk != blk) continue;
+            const uint64_t b = slot_of(a, p.pos, s0, s1);
+            T[p.pos] = (float)adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, x.traw[b], a.bmeta[b]).fr;
+        }
+    for (uint32_t k = threadIdx.x; k < po.nsrc; k += FB) {
+        const Probe p = po.probe[k];
+        if (p.blk == blk)
+            po.gsig[(uint64_t)k * po.stride + (uint64_t)po.n] = slots ? x.traw[slot_of(a, p.pos, s0, s1)] : T[p.pos];
+    }
+}
+
+// blocks per SM the register allocation must allow.  Grids of one plane per
+// thread do not fill more.  Else four where that spills at most 24 bytes (three
+// sections, 128 steps of 300x200x160: 13.06 ms with three blocks, 12.38 with
+// four); with four sections it would spill 112 (170x120x110, 0.5 M slots: 9.21
+// against 9.03 with three).
+template <int PL, int S> constexpr int adj_min_blocks() { return PL == 2 && S <= 3 ? 4 : 3; }
+
+template <int PL, int S>
+__global__ void __launch_bounds__(FB, adj_min_blocks<PL, S>()) k_adj_one(const __grid_constant__ StepArgs a,
+                                                                     const __grid_constant__ AdjPost po,
+                                                                     const __grid_constant__ AdjSlots x,
+                                                                     const __grid_constant__ FusedGeo g)
+{
+    extern __shared__ double gsm[]; // a slot block's sums of the coefficient gradients
+    pdl_trigger();
+    const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+    const bool probes = po.n >= 0 && __ldg(g.has_probe + blk) != 0;
+    const uint64_t s0 = (uint64_t)blk * PL * FB;
+    if (blk < g.gb) {
+        for (uint32_t k = tid; k < x.ncoef; k += FB) gsm[k] = 0.0;
+#pragma unroll 1
+        for (int k = 0; k < PL; ++k) adj_slot<S>(a, x, s0 + k * FB + tid, k == 0, gsm);
+        __syncthreads();
+        for (uint32_t k = tid; k < x.ncoef; k += FB)
+            if (gsm[k] != 0.0) atomicAdd(x.grad + k, gsm[k]);
+    } else {
+        const Site st = stencil_site(blk, g);
+        const uint32_t plane = a.px * a.ny, o = (st.bx * FB + tid) * V;
+        const bool act = o < plane;
+        StencilVecs<float, PL> s;
+        s.site(a, st.z, act ? o : plane - V, plane);
+        pdl_wait();
+        s.values(a, plane);
+        stencil_update<float, PL, false>(a, s, act, st.z);
+    }
+    if (probes) adj_owned(a, po, x, blk, blk < g.gb, s0, s0 + PL * FB < a.nb ? s0 + PL * FB : a.nb);
+}
+
+// before the first reverse step: T of the slots' voxels into traw, F in its place
+__global__ void k_adj_open(const StepArgs a, const AdjSlots x, float *T)
+{
+    const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= a.nb) return;
+    const uint32_t pos = a.bpos[b];
+    const float t = T[pos];
+    x.traw[b] = t;
+    T[pos] = (float)adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, t, a.bmeta[b]).fr;
 }
 
 // Many simulations in one launch.  The members' arguments are kernel
@@ -446,6 +657,30 @@ cudaError_t launch_fused(int storage, int mode, const StepArgs &a, const PostArg
 cudaError_t launch_adj_step(const StepArgs &a, const AdjPost &po, const FusedGeo &g, cudaStream_t s)
 {
     return g.pl == 1 ? launch_pdl(k_adj_step<1>, g.blocks, s, a, po, g) : launch_pdl(k_adj_step<2>, g.blocks, s, a, po, g);
+}
+
+cudaError_t launch_adj_open(const StepArgs &a, const AdjSlots &x, float *T, cudaStream_t s)
+{
+    if (a.nb) k_adj_open<<<(unsigned)((a.nb + 255) / 256), 256, 0, s>>>(a, x, T);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adj_one(const StepArgs &a, const AdjPost &po, const AdjSlots &x, const FusedGeo &g, bool overlap,
+                           cudaStream_t s)
+{
+    const size_t sm = (size_t)x.ncoef * sizeof(double);
+    const auto run = [&](auto *k1, auto *k2) {
+        const auto kern = g.pl == 1 ? k1 : k2;
+        if (overlap) return launch_overlapped(kern, g.blocks, FB, sm, s, a, po, x, g);
+        kern<<<g.blocks, FB, sm, s>>>(a, po, x, g);
+        return cudaGetLastError();
+    };
+    switch (a.nsec) {
+    case 1: return run(k_adj_one<1, 1>, k_adj_one<2, 1>);
+    case 2: return run(k_adj_one<1, 2>, k_adj_one<2, 2>);
+    case 3: return run(k_adj_one<1, 3>, k_adj_one<2, 3>);
+    default: return run(k_adj_one<1, 4>, k_adj_one<2, 4>);
+    }
 }
 
 cudaError_t launch_fused_batch(int storage, int sections, const FusedBatch &b, cudaStream_t s, bool sr)
