@@ -411,7 +411,7 @@ struct virs_sim {
     struct {
         uint64_t steps = 0, nck = 0, gen = 0;
         uint32_t every = 0;
-        bool ready = false;
+        bool ready = false, kept = false; // kept: the last segment's records and states are in segrec[0], segst[0]
         DevBuf ckp, ckq, cks, segrec[2], segst[2], buf[2], ast, dbar, rr[2], grad, dl, gsig;
         cudaEvent_t built[2] = {}, used[2] = {}; // a segment's buffers are filled, and read
     } adj;
@@ -3433,6 +3433,61 @@ VIRS_EXPORT virs_status virs_batch_autotune(virs_batch *b, uint32_t trial_steps,
 // adjoint
 // ============================================================================
 
+namespace {
+// The next n steps of a segment from buffer parity s->cur, keeping the
+// boundary pass's records and the states before every step in segment buffers
+// w: the pass writes its records straight into slot k, reads the states
+// before the step from slot k and writes those after it to slot k + 1 (the
+// last step's to the handle's own states).
+virs_status keep_steps(virs_sim *s, int w, uint64_t n, cudaStream_t st)
+{
+    auto &A = s->adj;
+    const size_t sb = state_bytes(s);
+    char *segst = A.segst[w].as<char>();
+    for (uint64_t k = 0; k < n; ++k) {
+        const int par = s->cur ^ (int)(k & 1);
+        StepArgs ka = step_args(s, par);
+        ka.side = A.segrec[w].as<float4>() + k * s->nb;
+        ka.state = reinterpret_cast<float *>(segst + k * sb);
+        ka.state_out = k + 1 < n ? reinterpret_cast<float *>(segst + (k + 1) * sb) : s->state.as<float>();
+        cudaError_t e;
+        if (fused_on(s)) {
+            e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, par), s->geo, st);
+        } else {
+            e = launch_stencil(s, par, st);
+            if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, st);
+            if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, par), st);
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "adjoint segment");
+    }
+    return VIRS_OK;
+}
+
+size_t segment_bytes(const virs_sim *s)
+{
+    return s->adj.every * (std::max<uint64_t>(s->nb, 1) * sizeof(float4) + state_bytes(s));
+}
+virs_status alloc_segment(virs_sim *s, int w)
+{
+    auto &A = s->adj;
+    VIRS_TRY(A.segrec[w].alloc(A.every * std::max<uint64_t>(s->nb, 1) * sizeof(float4), "adjoint segment records",
+                               s->stream, false));
+    return A.segst[w].alloc(A.every * state_bytes(s), "adjoint segment states", s->stream, false);
+}
+
+// Whether the forward pass keeps its last segment, so that the reverse pass
+// need not recompute it: where a step is one launch, which the records do not
+// slow down (9.4 and 9.3 us at 128x128x96), and up to 1 GiB.
+bool keep_last(virs_sim *s)
+{
+    if (!fused_on(s) || (pair_on(s) && pairs_pay(s)) || segment_bytes(s) > (1u << 30)) return false;
+    if (alloc_segment(s, 0) == VIRS_OK) return true;
+    s->adj.segrec[0].release();
+    s->adj.segst[0].release();
+    return false;
+}
+} // namespace
+
 VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, uint32_t every, void *stream)
 {
     if (!s) return fail(VIRS_E_ARG, "virs_forward_checkpointed: null");
@@ -3455,11 +3510,22 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
     VIRS_TRY(A.cks.alloc(A.nck * sb, "checkpoints", s->stream, false));
     VIRS_CUDA(cudaEventRecord(s->done, s->stream));
     VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    A.kept = keep_last(s);
     for (uint64_t c = 0; c < A.nck; ++c) {
         VIRS_CUDA(cudaMemcpyAsync(A.ckp.as<char>() + c * fb, s->field[s->cur].ptr, fb, cudaMemcpyDeviceToDevice, st));
         VIRS_CUDA(cudaMemcpyAsync(A.ckq.as<char>() + c * fb, s->field[s->cur ^ 1].ptr, fb, cudaMemcpyDeviceToDevice, st));
         VIRS_CUDA(cudaMemcpyAsync(A.cks.as<char>() + c * sb, s->state.ptr, sb, cudaMemcpyDeviceToDevice, st));
-        VIRS_TRY(run_steps(s, std::min<uint64_t>(every, steps - c * every), st));
+        const uint64_t n = std::min<uint64_t>(every, steps - c * every);
+        if (!A.kept || c + 1 < A.nck) {
+            VIRS_TRY(run_steps(s, n, st));
+            continue;
+        }
+        VIRS_CUDA(cudaMemcpyAsync(A.segst[0].ptr, s->state.ptr, sb, cudaMemcpyDeviceToDevice, st));
+        VIRS_TRY(keep_steps(s, 0, n, st));
+        s->cur ^= (int)(n & 1);
+        s->steps_done += n;
+        s->ctr_at += n;
+        VIRS_CUDA(cudaEventRecord(s->done, st));
     }
     A.gen = s->gen;
     A.ready = true;
@@ -3468,20 +3534,16 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
 
 namespace {
 // Whether a segment is recomputed beside the reverse steps of the segment
-// after it, on a second stream with a second set of segment buffers (`extra`
-// bytes).  On small grids both chains are bound by latency (128x128x96, 256
+// after it, on a second stream with a second set of segment buffers.  On small grids both chains are bound by latency (128x128x96, 256
 // steps, 64 or 16 to a segment: a gradient 6.44 -> 5.60 and 7.10 -> 5.62 ms;
 // 80x64x60 2.37 -> 1.95, 170x120x110 with 0.5 M slots 9.67 -> 9.3); on large ones little is left
 // to gain (400x300x250 19.07 -> 18.82) and the buffers grow, hence the 1 GiB.
 // Without the memory for them the two take turns in one stream.
-bool adj_beside(virs_sim *s, size_t extra)
+bool adj_beside(virs_sim *s)
 {
     auto &A = s->adj;
-    if (A.nck < 2 || extra > (1u << 30)) return false;
-    const uint64_t every = A.every;
-    if (A.segrec[1].alloc(every * std::max<uint64_t>(s->nb, 1) * sizeof(float4), "adjoint segment records", s->stream,
-                          false) != VIRS_OK ||
-        A.segst[1].alloc(every * state_bytes(s), "adjoint segment states", s->stream, false) != VIRS_OK) {
+    if (A.nck < 2 || segment_bytes(s) > (1u << 30)) return false;
+    if (alloc_segment(s, 1) != VIRS_OK) {
         A.segrec[1].release();
         A.segst[1].release();
         return false;
@@ -3521,9 +3583,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     // adjoints, four per section
     const size_t fb = s->nvox * 4, sb = state_bytes(s), sba = std::max<uint64_t>(nb, 1) * s->nsec * 4 * 4;
     const uint32_t ncoef = s->nmat * s->nsec * 5;
-    const size_t rb = every * std::max<uint64_t>(nb, 1) * sizeof(float4);
-    VIRS_TRY(A.segrec[0].alloc(rb, "adjoint segment records", st, false));
-    VIRS_TRY(A.segst[0].alloc(every * sb, "adjoint segment states", st, false));
+    if (!A.kept) VIRS_TRY(alloc_segment(s, 0));
     for (int k = 0; k < 2; ++k) VIRS_TRY(A.buf[k].alloc(fb, "adjoint field", st));
     VIRS_TRY(A.ast.alloc(sba, "adjoint filter states", st));
     VIRS_TRY(A.dbar.alloc(std::max<uint64_t>(nb, 1) * 4, "adjoint boundary terms", st));
@@ -3534,7 +3594,7 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     if (s->nrcv) VIRS_CUDA(copy_on(s->stream, A.dl.ptr, dl_dir, (size_t)s->nrcv * steps * 4, cudaMemcpyHostToDevice));
     VIRS_TRY(ready_to_run(s));
     if (!s->probe_ok) VIRS_TRY(build_probes(s));
-    const bool beside = adj_beside(s, rb + every * sb);
+    const bool beside = adj_beside(s);
     AdjBeside both{beside ? s->xstream : nullptr};
     cudaStream_t rst = beside ? s->xstream : st; // the recomputation's stream
     if (beside) {
@@ -3551,41 +3611,24 @@ VIRS_EXPORT virs_status virs_adjoint(virs_sim *s, const float *dl_dir, double *g
     if (one) VIRS_CUDA(launch_adj_open(step_args(s, 0), slots, A.buf[t].as<float>(), st));
     for (int64_t c = (int64_t)A.nck - 1; c >= 0; --c) {
         const uint64_t n0 = (uint64_t)c * every, n1 = std::min<uint64_t>(n0 + every, steps);
-        // rebuild the segment: restore the checkpoint and run forward, keeping
-        // the states before every step and the stencil's boundary records
-        const int w = beside ? (int)(c & 1) : 0;
+        // rebuild the segment, unless the forward pass kept it: restore the
+        // checkpoint and run forward, keeping states and records
+        const int w = beside ? (int)((A.nck - 1 - (uint64_t)c) & 1) : 0;
         float4 *segrec = A.segrec[w].as<float4>();
         char *segst = A.segst[w].as<char>();
-        s->cur = 0;
-        if (beside && c + 2 < (int64_t)A.nck) VIRS_CUDA(cudaStreamWaitEvent(rst, A.used[w], 0));
-        VIRS_CUDA(cudaMemcpyAsync(s->field[0].ptr, A.ckp.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
-        VIRS_CUDA(cudaMemcpyAsync(s->field[1].ptr, A.ckq.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
-        VIRS_CUDA(cudaMemcpyAsync(segst, A.cks.as<char>() + c * sb, sb, cudaMemcpyDeviceToDevice, rst));
-        VIRS_CUDA(launch_set_u32(s->ctr.as<uint32_t>(), (uint32_t)n0, rst));
-        for (uint64_t n = n0; n < n1; ++n) {
-            const uint64_t k = n - n0;
-            // the boundary pass keeps its records straight in the segment's
-            // slot k, and reads the states before the step from slot k and
-            // writes those after it to slot k + 1 (the last step's to the
-            // handle's own states)
-            StepArgs ka = step_args(s, s->cur);
-            ka.side = segrec + k * nb;
-            ka.state = reinterpret_cast<float *>(segst + k * sb);
-            ka.state_out = k + 1 < every ? reinterpret_cast<float *>(segst + (k + 1) * sb) : s->state.as<float>();
-            cudaError_t e;
-            if (fused_on(s)) {
-                e = launch_fused(s->prm.storage, BND_KEEP, ka, post_args(s, s->cur), s->geo, rst);
-            } else {
-                e = launch_stencil(s, s->cur, rst);
-                if (e == cudaSuccess) e = launch_boundary(s->prm.storage, ka, BND_KEEP, rst);
-                if (e == cudaSuccess) e = launch_post(s->prm.storage, post_args(s, s->cur), rst);
+        if (!A.kept || c + 1 < (int64_t)A.nck) {
+            s->cur = 0;
+            if (beside && c + 2 < (int64_t)A.nck) VIRS_CUDA(cudaStreamWaitEvent(rst, A.used[w], 0));
+            VIRS_CUDA(cudaMemcpyAsync(s->field[0].ptr, A.ckp.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
+            VIRS_CUDA(cudaMemcpyAsync(s->field[1].ptr, A.ckq.as<char>() + c * fb, fb, cudaMemcpyDeviceToDevice, rst));
+            VIRS_CUDA(cudaMemcpyAsync(segst, A.cks.as<char>() + c * sb, sb, cudaMemcpyDeviceToDevice, rst));
+            VIRS_CUDA(launch_set_u32(s->ctr.as<uint32_t>(), (uint32_t)n0, rst));
+            VIRS_TRY(keep_steps(s, w, n1 - n0, rst));
+            s->cur ^= (int)((n1 - n0) & 1);
+            if (beside) {
+                VIRS_CUDA(cudaEventRecord(A.built[w], rst));
+                VIRS_CUDA(cudaStreamWaitEvent(st, A.built[w], 0));
             }
-            if (e != cudaSuccess) return cuda_fail(e, "adjoint recomputation");
-            s->cur ^= 1;
-        }
-        if (beside) {
-            VIRS_CUDA(cudaEventRecord(A.built[w], rst));
-            VIRS_CUDA(cudaStreamWaitEvent(st, A.built[w], 0));
         }
         // reverse steps of the segment
         for (int64_t n = (int64_t)n1 - 1; n >= (int64_t)n0; --n) {
