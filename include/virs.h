@@ -394,7 +394,7 @@ virs_status virs_set_tiling(virs_sim *sim, int tile_rows, int planes_per_block, 
  * first step is complete, so the results are bit-identical to single steps.  tile_rows 12, 14, 16 or 32 (0 = 14; with
  * 12, 14 and 16 rows 4, 3 and 2 planes are in flight), planes per block
  * 0 = all.  With both 0 the library chooses the tile, and takes single steps
- * where they are faster (FP32 below 28 M voxels, 16-bit storage).  Off (1) by
+ * where they are faster (FP32 below 31 M voxels, 16-bit storage).  Off (1) by
  * default; not used with the register-streaming kernel (pipeline depth 0).  With the device stop rule, a run that stops
  * inside a group of four steps leaves the stop step's fields in the usual
  * buffers, as single steps do.  *active tells whether the current settings

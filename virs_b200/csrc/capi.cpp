@@ -889,19 +889,20 @@ uint64_t sr_base(const virs_sim *s) { return s->slab ? (s->slab_lo - 1) * (uint6
 // 1 / 4 / 16, three sections; the first two rows 1 / 8, two sections):
 //   0.07 M voxels FP32   8.6 /   9.3 against   3.2 /   3.6 us   BF16  10.0 / 10.1 against 3.1 / 3.5 us
 //   3.7 M               18.9 /  26.3           9.5 /  18.3            17.5 / 24.0         9.2 / 17.6
-//   24 M                79.1 /  99.5 / 169    66.7 /  87.9 / 163     63.0 / 82.2 / 152   59.4 / 78.9 / 152
-//   38 M               103.4 / 131.4 / 235    95.2 / 128.5 / 241     80.7 / 110  / 213   81.8 / 116  / 226
-//   60 M               169.6 / 203.4 / 344   158.1 / 195.2 / 343    121   / 155  / 294  137   / 175  / 321
-//   118 M              296.2 / 345.9 / 570   290.9 / 353.0 / 588    192   / 242  / 457  252   / 320  / 550
-// so the line lies at 64 M voxels in FP32, 24 M in 16-bit storage, 20 M with
-// stochastic rounding (24 M: 70.5 against 71.5 us), and at 8 M boundary slots
-// (24 M voxels, sponge 16: 7.6 M slots; 38 M: 10.7 M), whose states stream
-// better through a kernel of their own.  A tiling set by the
-// caller names the stencil kernel; the stop rule and the timing of the parts
-// need the separate kernels.
+//   24 M                77.8 /  99.2 / 170    62.0 /  83.1 / 162     65.1 / 81.9 / 152   53.0 / 72.9 / 148
+//   38 M               102.6 / 131.3 / 235    90.9 / 121.7 / 240     79.2 / 109  / 214   76.0 / 107  / 219
+//   60 M               169.6 / 203.0 / 342   146.9 / 185.9 / 347     121  / 156  / 292   120  / 159  / 307
+//   118 M              296.5 / 348.1 / 571   278   / 343   / 580
+//   181 M              426.4 / 487.5 / 779   422   / 493   / 829
+// so the line lies at 96 M voxels in FP32, 48 M in 16-bit storage, 26 M with
+// stochastic rounding (FP16, 24 M 69.7 against 65.5 us, 38 M 86.5 against
+// 92.4), and at 8 M boundary slots (24 M voxels, sponge 16: 7.1 M slots; 38 M:
+// 10.6 M), whose states stream better through a kernel of their own.  A tiling
+// set by the caller names the stencil kernel; the stop rule and the timing of
+// the parts need the separate kernels.
 bool fused_on(const virs_sim *s)
 {
-    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 64u << 20 : sr_on(s) ? 20u << 20 : 24u << 20;
+    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 96u << 20 : sr_on(s) ? 26u << 20 : 48u << 20;
     return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most && s->nb <= (8u << 20);
 }
 
@@ -1089,14 +1090,14 @@ PairTile pair_tile(const virs_sim *s)
 
 // Whether a run takes its groups of four steps two at a time.  With the tile
 // left to the library, only where that is the faster way to the same bits: in
-// FP32 above 28 M voxels (per step, one launch a step against two steps per
-// pass: 24 M 66.7 and 66 us, 38 M 95.0 and 88.3, 60 M 159 and 143), not in
+// FP32 above 31 M voxels (per step, one launch a step against two steps per
+// pass: 24 M 62.0 and 66 us, 38 M 90.9 and 88.3, 60 M 147 and 143), not in
 // 16-bit storage, where the two-step kernel is bound by issue (the hall 515
 // against 600 us, 701x517x333 187 against 211).  The timing of the parts
 // takes two steps as asked.
 bool pairs_pay(const virs_sim *s)
 {
-    return !s->pair_auto || s->timing || (s->prm.storage == VIRS_STORAGE_F32 && (!fused_on(s) || s->nvox > (28u << 20)));
+    return !s->pair_auto || s->timing || (s->prm.storage == VIRS_STORAGE_F32 && (!fused_on(s) || s->nvox > (31u << 20)));
 }
 
 // the voxels whose p^{n+2} the two-step kernel leaves provisional, for the

@@ -29,8 +29,8 @@
 // flag), then waits for the previous step's grid.
 //
 // 160x120x100 voxels with a sponge of 8 (0.64 M boundary slots): 17.4 us a
-// step in three launches, 10.4 with one plane and slot per thread, 9.4 now;
-// 300x200x130 with a sponge of 1: 28.6, 24.4 and 20.2.  Where the lines to the
+// step in three launches, 10.4 with one plane and slot per thread, 8.8 now;
+// 300x200x130 with a sponge of 1: 28.6, 24.4 and 19.0.  Where the lines to the
 // staged kernels lie: fused_on and batch_fused in capi.cpp.
 #include <algorithm>
 #include <type_traits>
