@@ -3104,20 +3104,20 @@ virs_status batch_check(const virs_batch *b)
 // against one (sponge 1-2, three sections):
 //   4 rooms, 0.6 M voxels in all    FP32   29.5 against    6.3 us   BF16  33.6 against  6.1 us
 //   12, 2.9 M                              44.0            22.0           46.9           21.3
-//   24, 26 M (1.1 M each)                 148             110            127            109
-//   100, 97 M (0.97 M each)               551             454            448            445
-//   8, 42 M (5.2 M each)                  160             136            132            135
-//   16, 79 M (4.9 M each)                 298             263            240            259
-//   40, 277 M (6.9 M each)                947             918            745            899
+//   24, 26 M (1.1 M each)                 148             110            127             99
+//   12 of 3.1 M, 37 M                                                    150            117
+//   40 of 3.9 M, 155 M                                                   532            488
+//   12 of 1 M and 6 of 8 M, 65 M                                         187            192
+//   8, 42 M (5.2 M each)                  160             136
 //   8, 184 M (23 M each)                  533             528            393            512
 //   12, 541 M (45 M each)                1450            1510           1041           1458
-// so the line lies at 24 M voxels per member in FP32, 1.5 M in 16-bit storage
-// (row padding included), and at 12 M in all for fewer, larger members.
+// so the line lies at 24 M voxels per member in FP32, 3.5 M in 16-bit storage
+// (1.5 M with stochastic rounding; row padding included), and at 12 M in all for fewer, larger members.
 bool batch_fused(const virs_batch *b)
 {
     size_t n = 0;
     for (const virs_sim *s : b->mem) n += s->nvox;
-    const size_t each = b->storage == VIRS_STORAGE_F32 ? 24u << 20 : 3u << 19;
+    const size_t each = b->storage == VIRS_STORAGE_F32 ? 24u << 20 : sr_on(b->mem[0]) ? 3u << 19 : 7u << 19;
     return !b->tiling_set && n <= std::max<size_t>(12u << 20, each * b->mem.size());
 }
 
