@@ -291,6 +291,7 @@ struct virs_sim {
     DevBuf segnz;                  // [nseg] 1 if a 128-voxel row segment holds a non-zero code
     DevBuf field[2];
     int cur = 0;
+    bool given_boundary = false;   // the grid came with boundary voxels (flag 2), as a classified one exported has them
 
     // z-slab of a larger grid (virs_set_grid_slab): flags_raw / wall_mat
     // hold ext_nz planes, classified together; the grid kept (nz planes,
@@ -590,13 +591,17 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
     if (!finite_pos(h)) return fail(VIRS_E_ARG, "cell size must be finite and positive");
     const size_t n = nx * ny * nz;
     uint8_t mx = 0;
+    bool given = false;
     if (flags)
-        for (size_t i = 0; i < n; ++i)
+        for (size_t i = 0; i < n; ++i) {
             if (flags[i] > 3) return fail(VIRS_E_ARG, "flags must be 0..3 (flag " + std::to_string(flags[i]) + " at " + std::to_string(i) + ")");
+            given |= flags[i] == 2;
+        }
     if (wmat)
         for (size_t i = 0; i < n; ++i) mx = std::max(mx, wmat[i]);
     s->drop_graphs();
     s->has_grid = s->classified = false;
+    s->given_boundary = given;
     s->slab = keep != 0;
     s->ext_nz = (uint32_t)nz;
     s->slab_drop = (uint32_t)drop;
@@ -1680,8 +1685,10 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
         VIRS_TRY(bits.alloc(nvc / 8, "sponge scratch", st, false));
         VIRS_TRY(near2.alloc(nvc * 2, "sponge scratch", st, false));
         VIRS_TRY(live.alloc(sponge_live_tiles(s->px, s->ny, s->ext_nz), "sponge scratch", st, false));
-        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch", st, false));
-        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch", st, false));
+        // read at every boundary voxel: those that came with the grid have
+        // material 0 and distance 0, the sponge kernels write the others
+        VIRS_TRY(bmat_full.alloc(nvc, "sponge scratch", st, s->given_boundary));
+        VIRS_TRY(bd2_full.alloc(nvc * 2, "sponge scratch", st, s->given_boundary));
         if (s->slab) VIRS_TRY(flags_ext.alloc(nvc, "sponge scratch", st, false));
         ClassifyArgs ca{};
         ca.flags_in = s->flags_raw.as<uint8_t>();

@@ -286,8 +286,8 @@ struct ClassifyArgs {
     const uint8_t *flags_in;   // padded
     const uint8_t *wall_mat;   // padded
     uint8_t *flags_out;        // padded
-    uint8_t *bmat_full;        // padded scratch, set at boundary voxels
-    uint16_t *bd2_full;        // padded scratch, set at boundary voxels
+    uint8_t *bmat_full;        // padded scratch, set at the voxels that become boundary voxels
+    uint16_t *bd2_full;        // ... both zeroed by the caller if flags_in holds some already
     uint32_t *bits;            // padded voxels / 32 words: walls
     uint16_t *near2;           // padded: the nearest wall in the plane
     uint8_t *live;             // sponge_live_tiles(): tiles of near2 with any
