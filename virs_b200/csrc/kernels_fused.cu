@@ -502,7 +502,9 @@ __device__ __noinline__ void adj_owned(const StepArgs &a, const AdjPost &po, con
     if (slots)
         for (uint32_t k = threadIdx.x; k < po.nrcv; k += FB) {
             const Probe p = po.probe[po.nsrc + k];
-            if (p.blk != blk) continue;
+            // a receiver on a border plane, which comes to the first block
+            // too, has no slot (sources are interior)
+            if (p.blk != blk || a.code[p.pos] >= CODE_HARD) continue;
             const uint64_t b = slot_of(a, p.pos, s0, s1);
             T[p.pos] = (float)adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, x.traw[b], a.bmeta[b]).fr;
         }
