@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
         const double s2 = sn * a.rot_c - cs * a.rot_s;
         cs = cs * a.rot_c + sn * a.rot_s;
         sn = s2;
-        if (!(fabs(u) < 1.0)) continue;
+        if (!(fabs(tau) < (double)a.half)) continue; // not |u| < 1: 49 * (1 / 49) rounds below 1
         const double v = 1.0 - u * u;
         double w = 0.0;
 #pragma unroll 4
