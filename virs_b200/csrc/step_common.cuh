@@ -330,13 +330,14 @@ __device__ __forceinline__ float2 leapfrog_air2(float2 ce, float2 x2, float2 yp,
 // den in [1, 2^1000]: num * rden and two corrections with the exact residual.
 // The last one is correctly rounded when the value before is within an ulp
 // (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990).  Infinities and NaN as the division gives
-// them.
+// System/6000 processor", 1990).  The residual is taken as q den - num: a
+// zero then keeps the division's sign (with num - q den, -0 would become
+// +0).  Infinities and NaN as the division gives them.
 __device__ __forceinline__ double quotient(double num, double den, double rden)
 {
     const double q0 = __dmul_rn(num, rden);
-    const double q1 = __fma_rn(__fma_rn(-q0, den, num), rden, q0);
-    const double q2 = __fma_rn(__fma_rn(-q1, den, num), rden, q1);
+    const double q1 = __fma_rn(-__fma_rn(q0, den, -num), rden, q0);
+    const double q2 = __fma_rn(-__fma_rn(q1, den, -num), rden, q1);
     return fabs(q0) <= 1.7976931348623157e308 ? q2 : q0;
 }
 
