@@ -58,7 +58,8 @@ virs_status cuda_fail(cudaError_t e, const char *what)
 // them back and tries again; when the last handle on the device is destroyed,
 // the blocks go that nobody took since the last time that happened.  A block
 // enters only from a Recycle scope, whose owner has waited for the work that
-// used it; every access is under the mutex.
+// used it (a handle's completion event follows all of it: take_up, Follow);
+// every access is under the mutex.
 namespace {
 struct DevPool {
     struct Block {
@@ -577,6 +578,23 @@ virs_status wait_done(const virs_sim *s)
     VIRS_CUDA(cudaEventSynchronize(s->done));
     return VIRS_OK;
 }
+
+// st takes up after everything queued for the handle, on its own stream or a
+// caller's
+virs_status take_up(const virs_sim *s, cudaStream_t st)
+{
+    VIRS_CUDA(cudaStreamWaitEvent(s->stream, s->done, 0));
+    VIRS_CUDA(cudaEventRecord(s->done, s->stream));
+    VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    return VIRS_OK;
+}
+// on every way out, a failed call's too, the handle's completion event follows
+// what was queued on st
+struct Follow {
+    const virs_sim *s;
+    cudaStream_t st;
+    ~Follow() { cudaEventRecord(s->done, st); }
+};
 
 // allocate the grid-sized buffers and upload flags / wall materials.  For a
 // slab (keep > 0) the nz planes uploaded are classified together and the
@@ -1420,7 +1438,6 @@ virs_status run_steps(virs_sim *s, uint64_t n, cudaStream_t st)
     s->cur ^= (int)(n & 1);
     s->steps_done += n;
     s->ctr_at += n;
-    VIRS_CUDA(cudaEventRecord(s->done, st));
     if (s->stop_rule) {
         // how many of the n steps ran before the rule fired
         uint32_t sb[2] = {0, 0};
@@ -2089,8 +2106,8 @@ VIRS_EXPORT virs_status virs_run(virs_sim *s, uint64_t steps, void *stream)
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
     if (steps == 0) return VIRS_OK;
     if (s->steps_done + steps >= (1ull << 32)) return fail(VIRS_E_ARG, "step counter would pass 2^32");
-    VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-    VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    VIRS_TRY(take_up(s, st));
+    Follow f{s, st};
     return run_steps(s, steps, st);
 }
 
@@ -2445,8 +2462,8 @@ VIRS_EXPORT virs_status virs_run_host(virs_sim *s, uint64_t steps, const float *
     VIRS_TRY(use_device(s));
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
     const uint64_t first = s->steps_done;
-    VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-    VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    VIRS_TRY(take_up(s, st));
+    Follow f{s, st};
     if (signal && s->nsrc) {
         if (first + steps > s->siglen)
             return fail(VIRS_E_ARG, "virs_run_host: source signals were set for fewer steps than requested");
@@ -3044,11 +3061,7 @@ virs_status energy_inputs(virs_sim *s, void *stream, EnergyInputs *in)
     in->scale2 = (double)s->inv_scale * (double)s->inv_scale;
     in->stream = stream ? (cudaStream_t)stream : s->stream;
     in->done = s->done;
-    if (in->stream != s->stream) {
-        VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-        VIRS_CUDA(cudaStreamWaitEvent(in->stream, s->done, 0));
-    }
-    return VIRS_OK;
+    return take_up(s, in->stream);
 }
 
 } // namespace virs
@@ -3253,10 +3266,16 @@ virs_status batch_steps(virs_batch *b, uint64_t n, cudaStream_t st, bool use_gra
         if (s->steps_done + n > s->ircap)
             return fail(VIRS_E_ARG, "a batch member has receiver storage for fewer steps: reserve them with "
                                     "virs_start_simulation");
-    for (virs_sim *s : b->mem) {
-        VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-        VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
-    }
+    for (virs_sim *s : b->mem) VIRS_TRY(take_up(s, st));
+    struct AllFollow { // as Follow, for the batch and its members
+        const virs_batch *b;
+        cudaStream_t st;
+        ~AllFollow()
+        {
+            for (const virs_sim *s : b->mem) cudaEventRecord(s->done, st);
+            cudaEventRecord(b->done, st);
+        }
+    } f{b, st};
     if (!b->fused) b->waits = true;
     const int cur = m0->cur;
     uint64_t i = 0;
@@ -3273,9 +3292,7 @@ virs_status batch_steps(virs_batch *b, uint64_t n, cudaStream_t st, bool use_gra
         s->cur ^= (int)(n & 1);
         s->steps_done += n;
         s->ctr_at += n;
-        VIRS_CUDA(cudaEventRecord(s->done, st));
     }
-    VIRS_CUDA(cudaEventRecord(b->done, st));
     return VIRS_OK;
 }
 
@@ -3516,8 +3533,8 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
     VIRS_TRY(A.ckp.alloc(A.nck * fb, "checkpoints", s->stream, false));
     VIRS_TRY(A.ckq.alloc(A.nck * fb, "checkpoints", s->stream, false));
     VIRS_TRY(A.cks.alloc(A.nck * sb, "checkpoints", s->stream, false));
-    VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-    VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    VIRS_TRY(take_up(s, st));
+    Follow f{s, st};
     A.kept = keep_last(s);
     for (uint64_t c = 0; c < A.nck; ++c) {
         VIRS_CUDA(cudaMemcpyAsync(A.ckp.as<char>() + c * fb, s->field[s->cur].ptr, fb, cudaMemcpyDeviceToDevice, st));
@@ -3533,7 +3550,6 @@ VIRS_EXPORT virs_status virs_forward_checkpointed(virs_sim *s, uint64_t steps, u
         s->cur ^= (int)(n & 1);
         s->steps_done += n;
         s->ctr_at += n;
-        VIRS_CUDA(cudaEventRecord(s->done, st));
     }
     A.gen = s->gen;
     A.ready = true;
