@@ -1,0 +1,50 @@
+"""Freed device memory goes back to CUDA: a slab's buffers at once (a
+neighbour's pull may still read them, which cudaFree waits for).  In a process
+of its own, where no other handle or library allocates."""
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import numpy as np, torch
+from virs_b200 import capi, slabs
+def room(shape, slab=False):
+    s = capi.Simulation(capi.default_params())
+    flags = np.zeros(shape[::-1], np.uint8)
+    flags[:, :, 0] = 1
+    if slab:
+        slabs.setup_slab(s, shape, 0.05, flags.reshape(-1), np.zeros(flags.size, np.uint8), 0, 2, 1)
+    else:
+        s.set_grid(shape, 0.05, flags.reshape(-1))
+    s.classify()
+    s.set_receivers([shape[0] * (shape[1] + 1) + 5])
+    s.start(8)
+    if not slab:
+        s.run(4)
+        s.synchronize()
+    return s
+free = lambda: torch.cuda.mem_get_info()[0]
+room((64, 32, 16)).close()      # context and kernels
+"""
+
+
+def _child(code):
+    p = subprocess.run([sys.executable, "-c", HEAD + code], cwd=Path(__file__).resolve().parent.parent,
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stdout + p.stderr
+
+
+def test_a_slabs_buffers_are_not_kept():
+    """Both fields of a slab of 32 M voxels at the least, while another handle lives."""
+    _child("""
+other = room((64, 32, 16))
+s = room((512, 512, 246), slab=True)
+before = free()
+s.close()
+got = free() - before
+assert got >= 2 * 4 * 512 * 512 * 122, got
+""")

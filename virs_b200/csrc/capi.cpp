@@ -58,8 +58,9 @@ virs_status cuda_fail(cudaError_t e, const char *what)
 // them back and tries again; when the last handle on the device is destroyed,
 // the blocks go that nobody took since the last time that happened.  A block
 // enters only from a Recycle scope, whose owner has waited for the work that
-// used it (a handle's completion event follows all of it: take_up, Follow);
-// every access is under the mutex.
+// used it: a handle's completion event follows all of it (take_up, Follow)
+// but the reads of a slab's planes by its neighbours, so a slab's buffers go
+// to cudaFree, which waits for the device.  Every access is under the mutex.
 namespace {
 struct DevPool {
     struct Block {
@@ -116,11 +117,12 @@ DevPool *dev_pool()
 }
 thread_local int g_recycle = 0;
 
-// device buffers released in this scope go to the pool; no work in flight
-// may use them
+// device buffers released in this scope go to the pool (on); no work in
+// flight may use them
 struct Recycle {
-    Recycle() { ++g_recycle; }
-    ~Recycle() { --g_recycle; }
+    const bool on;
+    explicit Recycle(bool on_ = true) : on(on_) { g_recycle += on; }
+    ~Recycle() { g_recycle -= on; }
     Recycle(const Recycle &) = delete;
     Recycle &operator=(const Recycle &) = delete;
 };
@@ -1538,7 +1540,9 @@ VIRS_EXPORT virs_status virs_destroy(virs_sim *s)
     cudaStreamSynchronize(s->stream);
     if (s->xstream) cudaStreamSynchronize(s->xstream);
     {
-        Recycle r;
+        // a neighbour's pull, or a caller's through virs_slab_planes, may
+        // still read a slab's fields
+        Recycle r(!s->slab);
         delete s;
     }
     pool_handle(-1);
