@@ -105,6 +105,13 @@ virs_status virs_create(const virs_params *p, virs_sim **out);
  * simulator_gpu.cpp:237-305).  NULL is accepted. */
 virs_status virs_destroy(virs_sim *sim);
 
+/* Device memory that handles have freed is kept for the next allocation, at
+ * most a sixteenth of the device's.  All of it goes when the last handle on
+ * the device is destroyed for the first time; a program that comes back keeps
+ * what it takes again each time.  This call gives all of it back to CUDA, for
+ * another library or process; handles are not touched. */
+virs_status virs_trim_memory(int device);
+
 /* Message of the last failed call on this thread ("" if none). */
 const char *virs_last_error(void);
 

@@ -1,6 +1,8 @@
-"""Freed device memory goes back to CUDA: a slab's buffers at once (a
-neighbour's pull may still read them, which cudaFree waits for).  In a process
-of its own, where no other handle or library allocates."""
+"""Freed device memory goes back to CUDA: all of it when a program's only
+handles are gone, or when it asks (virs_trim_memory); a slab's buffers at once
+(a neighbour's pull may still read them, which cudaFree waits for).  Each in a
+process of its own, where no other handle or library allocates; 64 MiB of
+slack for modules loaded late."""
 import subprocess
 import sys
 from pathlib import Path
@@ -28,7 +30,7 @@ def room(shape, slab=False):
         s.synchronize()
     return s
 free = lambda: torch.cuda.mem_get_info()[0]
-room((64, 32, 16)).close()      # context and kernels
+small = room((64, 32, 16))      # context and kernels
 """
 
 
@@ -38,10 +40,38 @@ def _child(code):
     assert p.returncode == 0, p.stdout + p.stderr
 
 
+def test_the_only_room_gives_its_memory_back():
+    """80 M voxels: about 1.7 GB."""
+    _child("""
+before = free()
+a = room((512, 512, 306))
+held = before - free()
+assert held > 1000 << 20, held
+a.close()
+small.close()
+left = before - free()
+assert left <= 64 << 20, left
+""")
+
+
+def test_rooms_after_rooms_give_it_back_when_asked():
+    _child("""
+small.close()
+before = free()
+for _ in range(3):
+    room((512, 512, 100)).close()
+other = room((64, 32, 16))
+capi.trim_memory()
+left = before - free()
+assert left <= 64 << 20, left
+other.run(4)
+assert np.isfinite(other.ir()).all()
+""")
+
+
 def test_a_slabs_buffers_are_not_kept():
     """Both fields of a slab of 32 M voxels at the least, while another handle lives."""
     _child("""
-other = room((64, 32, 16))
 s = room((512, 512, 246), slab=True)
 before = free()
 s.close()

@@ -62,6 +62,7 @@ _SIGS = {
     "virs_params_default": ([_P], C.c_int),
     "virs_create": ([_P, _P], C.c_int),
     "virs_destroy": ([_P], C.c_int),
+    "virs_trim_memory": ([C.c_int], C.c_int),
     "virs_set_material_roles": ([_P, _P, C.c_size_t], C.c_int),
     "virs_load_obj": ([_P, C.c_char_p], C.c_int),
     "virs_set_mesh": ([_P, _P, C.c_size_t, _P, _P, C.c_size_t], C.c_int),
@@ -189,6 +190,11 @@ def default_params(**kw) -> Params:
             raise AttributeError(f"no parameter {k}")
         setattr(p, k, v)
     return p
+
+
+def trim_memory(device: int = 0) -> None:
+    """Give the device memory kept for the next handles back to CUDA."""
+    check(lib().virs_trim_memory(device))
 
 
 def design_highpass(fs: float, cutoff: float, q: float, gain: float = 1.0) -> np.ndarray:

@@ -55,8 +55,10 @@ virs_status cuda_fail(cudaError_t e, const char *what)
 // each per room: 14 of 20 ms for a 320x240x160 one, 36 of 50 ms for a hall of
 // 403 M voxels).  Bounds: the blocks of a device total at most a sixteenth of
 // its memory (the oldest go first); an allocation that fails gives all of
-// them back and tries again; when the last handle on the device is destroyed,
-// the blocks go that nobody took since the last time that happened.  A block
+// them back and tries again; when the last handle on the device is destroyed
+// for the first time, all of them go (one room says nothing of a next), and
+// each time after it the blocks that nobody took since the time before;
+// virs_trim_memory gives all of them back for other users of the memory.  A block
 // enters only from a Recycle scope, whose owner has waited for the work that
 // used it: a handle's completion event follows all of it (take_up, Follow)
 // but the reads of a slab's planes by its neighbours, so a slab's buffers go
@@ -148,7 +150,7 @@ struct Scratch {
     };
 };
 
-// handles on a device: the last one's end ages the pool
+// handles on a device: the last one's end gives blocks back and ages the pool
 void pool_handle(int step)
 {
     DevPool *p = dev_pool();
@@ -158,7 +160,7 @@ void pool_handle(int step)
     if (p->handles > 0 || step > 0) return;
     for (auto it = p->blocks.begin(); it != p->blocks.end();) {
         auto next = std::next(it);
-        if (it->age < p->age) p->drop(it);
+        if (it->age < p->age || p->age == 0) p->drop(it);
         it = next;
     }
     ++p->age;
@@ -1546,6 +1548,16 @@ VIRS_EXPORT virs_status virs_destroy(virs_sim *s)
         delete s;
     }
     pool_handle(-1);
+    return VIRS_OK;
+}
+
+VIRS_EXPORT virs_status virs_trim_memory(int device)
+{
+    VIRS_CUDA(cudaSetDevice(device));
+    if (DevPool *p = dev_pool()) {
+        std::lock_guard<std::mutex> g(p->mu);
+        while (!p->blocks.empty()) p->drop(p->blocks.begin());
+    }
     return VIRS_OK;
 }
 
