@@ -921,12 +921,15 @@ uint64_t sr_base(const virs_sim *s) { return s->slab ? (s->slab_lo - 1) * (uint6
 //   60 M               169.6 / 203.0 / 342   146.9 / 185.9 / 347     121  / 156  / 292   120  / 159  / 307
 //   118 M              296.5 / 348.1 / 571   278   / 343   / 580
 //   181 M              426.4 / 487.5 / 779   422   / 493   / 829
-// so the line lies at 96 M voxels in FP32, 48 M in 16-bit storage, 26 M with
-// stochastic rounding (FP16, 24 M 69.7 against 65.5 us, 38 M 86.5 against
-// 92.4), and at 8 M boundary slots (24 M voxels, sponge 16: 7.1 M slots; 38 M:
-// 10.6 M), whose states stream better through a kernel of their own.  A tiling
-// set by the caller names the stencil kernel; the stop rule and the timing of
-// the parts need the separate kernels.
+// so with a layer of 1 to 4 one launch is the faster up to 118 M voxels in FP32
+// and no more at 181 M, up to 38 M (with a layer of 4) in 16-bit storage and
+// no more at 60 M, up to 24 M with stochastic rounding (FP16, 24 M 69.7
+// against 65.5 us, 38 M 86.5 against 92.4).  The lines lie between, in FP32
+// short of what 118 M would still gain, at 96 M, 48 M and 26 M; and at 8 M
+// boundary slots (24 M voxels, sponge 16: 7.1 M slots; 38 M: 10.6 M), whose
+// states stream better through a kernel of their own.  A tiling set by the
+// caller names the stencil kernel; the stop rule and the timing of the parts
+// need the separate kernels.
 bool fused_on(const virs_sim *s)
 {
     const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 96u << 20 : sr_on(s) ? 26u << 20 : 48u << 20;
@@ -3147,8 +3150,11 @@ virs_status batch_check(const virs_batch *b)
 //   8, 42 M (5.2 M each)                  160             136
 //   8, 184 M (23 M each)                  533             528            393            512
 //   12, 541 M (45 M each)                1450            1510           1041           1458
-// so the line lies at 24 M voxels per member in FP32, 3.5 M in 16-bit storage
-// (1.5 M with stochastic rounding; row padding included), and at 12 M in all for fewer, larger members.
+// so the line lies at a mean of 24 M voxels per member in FP32, 3.5 M in 16-bit
+// storage (1.5 M with stochastic rounding; row padding included), and at 12 M
+// in all for fewer, larger members.  The mean is coarse: 40 even rooms of
+// 3.9 M would gain in one launch and take three, so that the mixed batch,
+// whose mean is close to theirs and which loses in one launch, stays out.
 bool batch_fused(const virs_batch *b)
 {
     size_t n = 0;

@@ -344,7 +344,6 @@ cudaError_t launch_adj_inject(float *T, const uint8_t *code, const uint64_t *rcv
 cudaError_t launch_adj_boundary(const StepArgs &f, float *T, const float4 *rec, const float *fst, float4 *ast,
                                 float *dbar, float *rr, double *grad, uint32_t nmat, cudaStream_t s);
 cudaError_t launch_set_u32(uint32_t *p, uint32_t v, cudaStream_t s);
-cudaError_t launch_zero_at(float *f, const uint32_t *pos, uint32_t n, cudaStream_t s);
 
 // mesh voxelisation (kernels_voxelize.cu)
 size_t voxelize_tri_bytes();

@@ -53,7 +53,6 @@ template <typename T> struct Vec {
     using Raw = std::conditional_t<sizeof(T) == 4, uint4, uint2>;
     Raw v;
     __device__ void load(const T *p) { v = *reinterpret_cast<const Raw *>(p); }
-    __device__ void zero() { v = Raw{}; }
     __device__ void get(float (&r)[V]) const
     {
         const T *h = reinterpret_cast<const T *>(&v);

@@ -160,16 +160,6 @@ __global__ void __launch_bounds__(32 * TY, 1024 / (32 * TY)) k_step(const __grid
     }
 }
 
-// The compacted boundary pass (simulator_gpu.cu:105-150): one thread per
-// boundary voxel in list order.  The stencil kernels left these voxels
-// untouched (p^{n-1} in place); the pass gathers the seven p values and
-// p^{n-1} of its voxel, computes the leapfrog update with the wall mirror,
-// then the filter correction.  Consecutive slots are consecutive voxels of
-// a row (floor, ceiling and y walls) or the same x of consecutive rows
-// (x walls), so the gathers of a warp share lines.
-//   BND_UPDATE  leapfrog + filters, the result written to p^{n+1}
-//   BND_KEEP    the same, and the record {free value, p, p^{n-1}} of the
-//               slot kept in a.side (the adjoint's recomputation)
 // The compacted boundary pass (simulator_gpu.cu:105-150), in list order.
 // The stencil kernels left these voxels untouched (p^{n-1} in place); the
 // pass gathers the seven p values from the p^n buffer (not written during

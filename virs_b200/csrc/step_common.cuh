@@ -287,24 +287,9 @@ __device__ __forceinline__ float leapfrog(uint8_t c, float ce, float xp, float x
     return __fmaf_rn(c2dt2, lap, t);
 }
 
-// the same update for an air voxel without wall neighbours (code 0): no
-// selects; bit-identical to leapfrog(0, ...)
-__device__ __forceinline__ float leapfrog_air(float ce, float xp, float xm, float yp, float ym, float zp, float zm,
-                                              float qv, float c2dt2, float inv_h2)
-{
-    float s = __fadd_rn(xp, xm);
-    s = __fadd_rn(s, yp);
-    s = __fadd_rn(s, ym);
-    s = __fadd_rn(s, zp);
-    s = __fadd_rn(s, zm);
-    const float lap = __fmul_rn(__fmaf_rn(-6.0f, ce, s), inv_h2);
-    const float t = __fsub_rn(__fmul_rn(2.0f, ce), qv);
-    return __fmaf_rn(c2dt2, lap, t);
-}
-
 // two air voxels at once with the packed FP32 instructions of sm_100, whose
 // components round exactly like the scalar __fadd_rn / __fmul_rn /
-// __fmaf_rn: bit-identical to two leapfrog_air calls.  The first sum
+// __fmaf_rn: bit-identical to two leapfrog(0, ...) calls.  The first sum
 // (xp + xm) comes in as x2: its operands straddle the register pairs of a
 // loaded vector, so it is two scalar adds.  2*ce is exact, so
 // fma(2, ce, -qv) rounds like fsub(2*ce, qv) (they part only where 2*ce
