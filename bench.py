@@ -105,6 +105,14 @@ def stencil_roofline(r, storage: str):
             ROOT / "profiles" / "k_step_tma_dram_traffic.txt")
 
 
+def own_step(r):
+    """Whether the timed region took the step as the library runs it without
+    a tiling (the tuner's candidate of 0 planes): on grids up to its size
+    limits one launch for everything, which the per-kernel pass, made of the
+    separate kernels, does not show."""
+    return r["tiling"]["planes_per_block"] == 0 and not r["time_blocking"]["active"]
+
+
 def host_threads():
     try:
         return len(os.sched_getaffinity(0))
@@ -202,7 +210,8 @@ def time_run(sim, steps, stream):
 
 def bench_storage(sc, storage, args, stream, dev, world, dist, want_e2e, rounding=0):
     """Warm up, then time K steps: device-resident graph run, a per-kernel
-    CUDA-event pass, and (optionally) the end-to-end host run.  rounding:
+    CUDA-event pass (its own run, always through the separate kernels), and
+    (optionally) the end-to-end host run.  rounding:
     the 16-bit stores' rounding (virs_set_rounding)."""
     import torch
     from virs_b200 import scenes
@@ -291,7 +300,9 @@ def bench_storage(sc, storage, args, stream, dev, world, dist, want_e2e, roundin
 
 def bench_batch(storage, args, stream, dev, dist=None):
     """The batched workload: 64 source positions in a 256^3 room plus 16 rooms
-    of 96^3..320^3, advanced by three launches per step (virs_batch)."""
+    of 96^3..320^3, advanced together (virs_batch): three launches per step,
+    or one per 64 members where the tuner keeps the library's own step (0
+    planes) and the members are small enough for it."""
     import torch
     from virs_b200 import capi, scenes
     steps, warm = args.batch_steps, GRAPH_WARMUP
@@ -318,7 +329,7 @@ def bench_batch(storage, args, stream, dev, dist=None):
         s.close()
     return {"value": nvox * steps / (ms * 1e-3) / 1e9, "ms_per_step": ms / steps, "members": len(scs),
             "voxels_per_step": nvox, "steps": steps, "tiling": [t.tile_rows, t.planes_per_block, t.pipeline_depth],
-            "ir_finite": ok, "launches_per_step": 3}
+            "ir_finite": ok, "launches_per_step": 3 if t.planes_per_block else None}
 
 
 CPU_CROP_PLANES = 16   # planes of the hall crop both CPU figures time
@@ -598,6 +609,9 @@ def run_virs(args):
             "boundary_pass_note": ("per step: a two-step pass's two boundary launches (the second also recomputes "
                                    "the voxels next to sources), halved" if steps_per_launch == 2
                                    else "per step"),
+            "kernel_pass": "events around the separate kernels, in a run of its own" +
+                           ("; the timed region took the library's own step, one launch where the grid is within "
+                            "its limits" if own_step(r32) else ""),
         },
         "e2e": {
             "value": round(nvox * args.steps / (r32["e2e_ms"] * 1e-3) / 1e9 * world, 3),
@@ -607,7 +621,8 @@ def run_virs(args):
             "api": "virs_run_host (pinned host buffers)",
             "wall_ms": r32["e2e_wall_ms"],
         },
-        "gpu_launches": round(r32.get("launches_per_step", 3) * args.steps),
+        # of the library's own step at least one per step
+        "gpu_launches": round((1 if own_step(r32) else r32.get("launches_per_step", 3)) * args.steps),
         "clocks": r32["clocks"],
         "variants": variants,
     }

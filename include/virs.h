@@ -398,14 +398,16 @@ virs_status virs_set_tiling(virs_sim *sim, int tile_rows, int planes_per_block, 
  * kernel reads p^n and p^{n-1} once and writes p^{n+1} and p^{n+2}, over two
  * more field buffers allocated on first use (a grid for which they do not fit
  * runs single steps).  The voxels next to sources are recomputed after the
- * first step is complete, so the results are bit-identical to single steps.  tile_rows 12, 14, 16 or 32 (0 = 14; with
- * 12, 14 and 16 rows 4, 3 and 2 planes are in flight), planes per block
- * 0 = all.  With both 0 the library chooses the tile, and takes single steps
- * where they are faster (FP32 below 31 M voxels, 16-bit storage).  Off (1) by
- * default; not used with the register-streaming kernel (pipeline depth 0).  With the device stop rule, a run that stops
- * inside a group of four steps leaves the stop step's fields in the usual
- * buffers, as single steps do.  *active tells whether the current settings
- * allow two steps per pass. */
+ * first step is complete, so the results are bit-identical to single steps.
+ * tile_rows 12, 14, 16 or 32 (0 = 14; with 12, 14 and 16 rows 4, 3 and 2
+ * planes are in flight), planes per block 0 = all.  With both 0 the library
+ * chooses the tile, and takes single steps where they are faster (FP32 below
+ * 31 M voxels, 16-bit storage).  Off (1) by default; not used with the
+ * register-streaming kernel (pipeline depth 0).  With the device stop rule, a
+ * run that stops inside a group of four steps leaves the stop step's fields in
+ * the usual buffers, as single steps do.  *active tells whether the current
+ * settings allow two steps per pass; with a named tile, whether a run takes
+ * them. */
 virs_status virs_set_time_blocking(virs_sim *sim, int steps_per_pass, int tile_rows, int planes_per_block);
 virs_status virs_get_time_blocking(const virs_sim *sim, int *steps_per_pass, int *tile_rows, int *planes_per_block,
                                    int *active);
@@ -432,8 +434,9 @@ typedef struct virs_tiling {
 } virs_tiling;
 
 /* Autotuner (no reference counterpart): right after virs_start_simulation,
- * times `trial_steps` steps of each TMA variant (tile rows 4/8/16, depth
- * 1..3, 8..64 planes per block) and then of the two-step variants (time
+ * times `trial_steps` steps of the step as it runs without a tiling (one launch
+ * on grids up to the library's limits), of each TMA variant (tile rows 4/8/16,
+ * depth 1..3, 8..64 planes per block) and then of the two-step variants (time
  * blocking: tile rows 14/16/12, 32..102 planes per block, trial_steps
  * rounded up to a multiple of four, at least eight) on this handle's own
  * grid and keeps the fastest: the tiling it returns, and the steps per pass
@@ -441,7 +444,10 @@ typedef struct virs_tiling {
  * forward and then reverse order, because a sustained load reaches the
  * GPU's power cap within about a second and would favour the candidates
  * timed first.  The simulation is then back at rest.  Results are cached
- * per device, storage and grid shape for the life of the process.
+ * per device, storage and grid shape for the life of the process.  A returned
+ * tiling of 0 planes per block stands for the step without a tiling, in force
+ * on this handle: on another, virs_set_tiling(h, 0, 0, -1) gives it, while
+ * the returned rows and depth would name the staged kernels.
  * virs_batch_autotune does the same for a batch's tilings (one tile per
  * block or persistent). */
 virs_status virs_autotune(virs_sim *sim, uint32_t trial_steps, virs_tiling *best);
