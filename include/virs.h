@@ -133,7 +133,8 @@ virs_status virs_set_mesh(virs_sim *sim, const float *verts, size_t nverts, cons
 
 /* Replaces updateGPUFromGrid for the flags (simulator_dispatch.cpp:70-81):
  * set the grid directly.  flags [nx*ny*nz] with values 0..3 (reference
- * layout); wall_material [nx*ny*nz] or NULL (all absorber 0). */
+ * layout); wall_material [nx*ny*nz] or NULL (all absorber 0).  Voxels given as
+ * 2 stay boundary voxels, of material 0 at wall distance 0. */
 virs_status virs_set_grid(virs_sim *sim, uint64_t nx, uint64_t ny, uint64_t nz, float cell_size,
                           const uint8_t *flags, const uint8_t *wall_material);
 
