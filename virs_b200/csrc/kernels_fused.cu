@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(FB, fused_min_blocks<PL>()) k_adj_step(const _
             const BVox<float, 0> &x = v[k];
             const float r = leapfrog((uint8_t)x.meta, x.ce, x.nb[0], x.nb[1], x.nb[2], x.nb[3], x.nb[4], x.nb[5],
                                      po.rr[s], a.c2dt2, a.inv_h2);
-            static_cast<float *>(a.q)[x.i] = __fadd_rn(r, po.dbar[s]);
+            static_cast<float *>(a.q)[x.i] = keep::add(r, po.dbar[s]);
         }
     } else {
         const Site st = stencil_site(blk, g);
@@ -379,18 +379,20 @@ __device__ __forceinline__ void adj_sections(const StepArgs &a, const AdjSlots &
 #pragma unroll
     for (int n = N - 1; n >= 0; --n) {
         const int q = q0 + n;
-        const double yt = yb + (double)aq[q].z;
-        gv[5 * n] = yt * (double)xin[q];
+        const double yt = yb + keep::wide(aq[q].z);
+        gv[5 * n] = yt * keep::wide(xin[q]);
         gv[5 * n + 1] = yt * (double)h[2 * q];
         gv[5 * n + 2] = yt * (double)h[2 * q + 1];
         gv[5 * n + 3] = -yt * (double)h[2 * q + 2];
         gv[5 * n + 4] = -yt * (double)h[2 * q + 3];
-        const double xbar = (double)kc[5 * q] * yt + (double)aq[q].x;
-        const double x1 = (double)kc[5 * q + 1] * yt + (double)aq[q].y;
+        const double xbar = (double)kc[5 * q] * yt + keep::wide(aq[q].x);
+        const double x1 = (double)kc[5 * q + 1] * yt + keep::wide(aq[q].y);
         const double x2 = (double)kc[5 * q + 2] * yt;
-        const double y1 = -(double)kc[5 * q + 3] * yt + (double)aq[q].w;
+        const double y1 = -(double)kc[5 * q + 3] * yt + keep::wide(aq[q].w);
         const double y2 = -(double)kc[5 * q + 4] * yt;
-        if (act) x.ast[(uint64_t)q * a.nb + b] = make_float4((float)x1, (float)x2, (float)y1, (float)y2);
+        if (act)
+            x.ast[(uint64_t)q * a.nb + b] =
+                make_float4(keep::narrow(x1), keep::narrow(x2), keep::narrow(y1), keep::narrow(y2));
         yb = xbar;
     }
     unsigned left = __ballot_sync(0xffffffffu, act);
@@ -434,14 +436,14 @@ __device__ __forceinline__ void adj_slot(const StepArgs &a, const AdjSlots &x, u
     }
     // forward inputs of every section at this step
     float xin[S];
-    float in = __fsub_rn(rec.y, rec.z);
+    float in = keep::sub(rec.y, rec.z);
 #pragma unroll
     for (int q = 0; q < S; ++q) {
         xin[q] = in;
-        float yv = __fmaf_rn(kc[5 * q], in, __fmul_rn(kc[5 * q + 1], h[2 * q]));
-        yv = __fmaf_rn(kc[5 * q + 2], h[2 * q + 1], yv);
-        yv = __fmaf_rn(-kc[5 * q + 3], h[2 * q + 2], yv);
-        in = __fmaf_rn(-kc[5 * q + 4], h[2 * q + 3], yv);
+        float yv = keep::fma(kc[5 * q], in, keep::mul(kc[5 * q + 1], h[2 * q]));
+        yv = keep::fma(kc[5 * q + 2], h[2 * q + 1], yv);
+        yv = keep::fma(-kc[5 * q + 3], h[2 * q + 2], yv);
+        in = keep::fma(-kc[5 * q + 4], h[2 * q + 3], yv);
     }
     if (first) {
         pdl_wait();
@@ -456,7 +458,7 @@ __device__ __forceinline__ void adj_slot(const StepArgs &a, const AdjSlots &x, u
     const float n0 = P[pos + 1], n1 = P[pos - 1], n2 = P[pos + sy], n3 = P[pos - sy], n4 = P[pos + sz], n5 = P[pos - sz];
     const double kg = a.K * a.gain;
     const AdjCorr c = adj_correct(a.wtab, a.form, kg, a.mix_y, a.mix_d, t, meta);
-    const float fr = (float)c.fr;
+    const float fr = keep::narrow(c.fr);
     const float r = leapfrog((uint8_t)meta, fr, n0, n1, n2, n3, n4, n5, rr, a.c2dt2, a.inv_h2);
     double yb = c.ybar;
 #pragma unroll
@@ -465,10 +467,10 @@ __device__ __forceinline__ void adj_slot(const StepArgs &a, const AdjSlots &x, u
         else adj_sections<1, 4 * NG, 4 * NC, S>(a, x, b, act, m, q0, h, kc, xin, aq, yb, gsm);
     }
     if (act) {
-        const float db = (float)(c.db + yb), tn = __fadd_rn(r, db);
-        x.rr[b] = __fsub_rn(__fadd_rn(fr, db), (float)c.cq);
+        const float db = keep::narrow(c.db + yb), tn = keep::add(r, db);
+        x.rr[b] = keep::sub(keep::add(fr, db), keep::narrow(c.cq));
         x.traw[b] = tn;
-        static_cast<float *>(a.q)[pos] = (float)adj_correct(a.wtab, a.form, kg, a.mix_y, a.mix_d, tn, meta).fr;
+        static_cast<float *>(a.q)[pos] = keep::narrow(adj_correct(a.wtab, a.form, kg, a.mix_y, a.mix_d, tn, meta).fr);
     }
 }
 
@@ -505,7 +507,7 @@ __device__ __noinline__ void adj_owned(const StepArgs &a, const AdjPost &po, con
             // too, has no slot (sources are interior)
             if (p.blk != blk || a.code[p.pos] >= CODE_HARD) continue;
             const uint64_t b = slot_of(a, p.pos, s0, s1);
-            T[p.pos] = (float)adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, x.traw[b], a.bmeta[b]).fr;
+            T[p.pos] = keep::narrow(adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, x.traw[b], a.bmeta[b]).fr);
         }
     for (uint32_t k = threadIdx.x; k < po.nsrc; k += FB) {
         const Probe p = po.probe[k];
@@ -560,7 +562,7 @@ __global__ void k_adj_open(const StepArgs a, const AdjSlots x, float *T)
     const uint32_t pos = a.bpos[b];
     const float t = T[pos];
     x.traw[b] = t;
-    T[pos] = (float)adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, t, a.bmeta[b]).fr;
+    T[pos] = keep::narrow(adj_correct(a.wtab, a.form, a.K * a.gain, a.mix_y, a.mix_d, t, a.bmeta[b]).fr);
 }
 
 // Many simulations in one launch.  The members' arguments are kernel
