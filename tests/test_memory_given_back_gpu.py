@@ -1,5 +1,5 @@
 """Freed device memory goes back to CUDA: all of it when a program's only
-handles are gone, or when it asks (virs_trim_memory); a slab's buffers at once
+handles are gone, or when it asks (virs_trim_memory); a slab's fields at once
 (a neighbour's pull may still read them, which cudaFree waits for).  Each in a
 process of its own, where no other handle or library allocates; 64 MiB of
 slack for modules loaded late."""
@@ -69,7 +69,7 @@ assert np.isfinite(other.ir()).all()
 """)
 
 
-def test_a_slabs_buffers_are_not_kept():
+def test_a_slabs_fields_are_not_kept():
     """Both fields of a slab of 32 M voxels at the least, while another handle lives."""
     _child("""
 s = room((512, 512, 246), slab=True)

@@ -61,8 +61,8 @@ virs_status cuda_fail(cudaError_t e, const char *what)
 // virs_trim_memory gives all of them back for other users of the memory.  A block
 // enters only from a Recycle scope, whose owner has waited for the work that
 // used it: a handle's completion event follows all of it (take_up, Follow)
-// but the reads of a slab's planes by its neighbours, so a slab's buffers go
-// to cudaFree, which waits for the device.  Every access is under the mutex.
+// but the reads of a slab's planes by its neighbours, so a slab's fields go to
+// cudaFree, which waits for the device.  Every access is under the mutex.
 namespace {
 struct DevPool {
     struct Block {
@@ -119,12 +119,11 @@ DevPool *dev_pool()
 }
 thread_local int g_recycle = 0;
 
-// device buffers released in this scope go to the pool (on); no work in
-// flight may use them
+// device buffers released in this scope go to the pool; no work in flight
+// may use them
 struct Recycle {
-    const bool on;
-    explicit Recycle(bool on_ = true) : on(on_) { g_recycle += on; }
-    ~Recycle() { g_recycle -= on; }
+    Recycle() { ++g_recycle; }
+    ~Recycle() { --g_recycle; }
     Recycle(const Recycle &) = delete;
     Recycle &operator=(const Recycle &) = delete;
 };
@@ -1547,7 +1546,9 @@ VIRS_EXPORT virs_status virs_destroy(virs_sim *s)
     {
         // a neighbour's pull, or a caller's through virs_slab_planes, may
         // still read a slab's fields
-        Recycle r(!s->slab);
+        if (s->slab)
+            for (DevBuf &f : s->field) f.release();
+        Recycle r;
         delete s;
     }
     pool_handle(-1);
