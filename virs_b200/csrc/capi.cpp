@@ -279,6 +279,8 @@ struct virs_sim {
     virs_params prm{};
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
+    static constexpr unsigned long long ANY_STREAM = ~0ull;
+    unsigned long long done_on = ANY_STREAM; // the stream whose order covers what `done` follows beyond the handle's own
     std::unique_ptr<SlabGraph> slab_graph;
 
     // geometry
@@ -582,14 +584,29 @@ virs_status wait_done(const virs_sim *s)
     return VIRS_OK;
 }
 
-// st takes up after everything queued for the handle, on its own stream or a
-// caller's
-virs_status take_up(const virs_sim *s, cudaStream_t st)
+// the driver's number of a stream, never given twice (a handle may be)
+virs_status stream_id(cudaStream_t st, unsigned long long *id)
 {
-    VIRS_CUDA(cudaStreamWaitEvent(s->stream, s->done, 0));
+    VIRS_CUDA(cudaStreamGetId(st, id));
+    return VIRS_OK;
+}
+// st (its number: id) takes up after everything queued for the handle, on its
+// own stream or a caller's; the caller of this records the event on st (Follow)
+virs_status take_up(virs_sim *s, cudaStream_t st, unsigned long long id)
+{
+    // the order on st itself is given
+    if (s->done_on != id) VIRS_CUDA(cudaStreamWaitEvent(s->stream, s->done, 0));
+    s->done_on = virs_sim::ANY_STREAM;
     VIRS_CUDA(cudaEventRecord(s->done, s->stream));
     VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    s->done_on = id;
     return VIRS_OK;
+}
+virs_status take_up(virs_sim *s, cudaStream_t st)
+{
+    unsigned long long id = 0;
+    VIRS_TRY(stream_id(st, &id));
+    return take_up(s, st, id);
 }
 // on every way out, a failed call's too, the handle's completion event follows
 // what was queued on st
@@ -2463,6 +2480,7 @@ VIRS_EXPORT virs_status virs_slab_step_end(virs_sim *s, void *stream)
     s->cur ^= 1;
     s->steps_done += 1;
     s->ctr_at += 1;
+    s->done_on = virs_sim::ANY_STREAM;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     return VIRS_OK;
 }
@@ -3289,7 +3307,9 @@ virs_status batch_steps(virs_batch *b, uint64_t n, cudaStream_t st, bool use_gra
         if (s->steps_done + n > s->ircap)
             return fail(VIRS_E_ARG, "a batch member has receiver storage for fewer steps: reserve them with "
                                     "virs_start_simulation");
-    for (virs_sim *s : b->mem) VIRS_TRY(take_up(s, st));
+    unsigned long long id = 0;
+    VIRS_TRY(stream_id(st, &id));
+    for (virs_sim *s : b->mem) VIRS_TRY(take_up(s, st, id));
     struct AllFollow { // as Follow, for the batch and its members
         const virs_batch *b;
         cudaStream_t st;
