@@ -279,6 +279,7 @@ struct virs_sim {
     virs_params prm{};
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
+    cudaEvent_t own = nullptr;         // take_up: the work queued on `stream`
     static constexpr unsigned long long ANY_STREAM = ~0ull;
     unsigned long long done_on = ANY_STREAM; // the stream whose order covers what `done` follows beyond the handle's own
     std::unique_ptr<SlabGraph> slab_graph;
@@ -430,6 +431,7 @@ struct virs_sim {
         drop_graphs();
         slab_graph.reset();
         if (done) cudaEventDestroy(done);
+        if (own) cudaEventDestroy(own);
         if (xdone) cudaEventDestroy(xdone);
         for (cudaEvent_t e : {adj.built[0], adj.built[1], adj.used[0], adj.used[1]})
             if (e) cudaEventDestroy(e);
@@ -591,14 +593,15 @@ virs_status stream_id(cudaStream_t st, unsigned long long *id)
     return VIRS_OK;
 }
 // st (its number: id) takes up after everything queued for the handle, on its
-// own stream or a caller's; the caller of this records the event on st (Follow)
+// own stream or a caller's; the caller of this records the event on st
+// (Follow).  A call refused between the two leaves the event where it was: it
+// must not lose what is in flight.
 virs_status take_up(virs_sim *s, cudaStream_t st, unsigned long long id)
 {
     // the order on st itself is given
     if (s->done_on != id) VIRS_CUDA(cudaStreamWaitEvent(s->stream, s->done, 0));
-    s->done_on = virs_sim::ANY_STREAM;
-    VIRS_CUDA(cudaEventRecord(s->done, s->stream));
-    VIRS_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    VIRS_CUDA(cudaEventRecord(s->own, s->stream));
+    VIRS_CUDA(cudaStreamWaitEvent(st, s->own, 0));
     s->done_on = id;
     return VIRS_OK;
 }
@@ -1541,6 +1544,7 @@ VIRS_EXPORT virs_status virs_create(const virs_params *p, virs_sim **out)
     // of the setup calls, which run on the legacy default stream
     VIRS_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     VIRS_CUDA(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming));
+    VIRS_CUDA(cudaEventCreateWithFlags(&s->own, cudaEventDisableTiming));
     VIRS_CUDA(cudaEventRecord(s->done, s->stream));
     s->roles.assign(2, VIRS_ROLE_IGNORE);
     s->roles[0] = 0;

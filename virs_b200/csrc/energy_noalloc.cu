@@ -144,10 +144,11 @@ VIRS_EXPORT virs_status virs_energy_noalloc(virs_sim *sim, double *d_out, void *
         break;
     }
     k_energy_planes_sum<<<1, 32, 0, in.stream>>>(scratch, in.nz, in.scale2, d_out);
-    VIRS_CUDA(cudaGetLastError());
+    const cudaError_t e = cudaGetLastError();
     // the handle's completion event now follows these reads of its fields, so
     // virs_synchronize and virs_destroy wait for them (also on a caller's
     // stream) before the fields can be freed
     VIRS_CUDA(cudaEventRecord(in.done, in.stream));
+    if (e != cudaSuccess) return cuda_fail(e, "energy kernels");
     return VIRS_OK;
 }
