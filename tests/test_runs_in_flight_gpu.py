@@ -40,3 +40,26 @@ def test_a_refused_energy_on_the_runs_stream_does_not_hide_it():
     sim.synchronize()
     assert st.query()
     sim.close()
+
+
+def test_more_receiver_samples_than_reserved_keep_those_of_a_run_in_flight():
+    """1024 are reserved at least; the second run grows them while the first one records."""
+    import torch
+    shape = (40, 32, 24)
+    want = _room(shape, 40)
+    want.run(1000)
+    want.run(100)
+    for second in (None, "the same stream"):
+        sim = _room(shape, 40)
+        sim.run(4)
+        sim.synchronize()
+        st = torch.cuda.Stream()
+        sim.run(4, st.cuda_stream)
+        with torch.cuda.stream(st):
+            torch.cuda._sleep(SLEEP)
+        sim.run(992, st.cuda_stream)
+        sim.run(100, st.cuda_stream if second else None)
+        sim.synchronize()
+        assert np.array_equal(sim.ir().view(np.uint32), want.ir().view(np.uint32))
+        sim.close()
+    want.close()

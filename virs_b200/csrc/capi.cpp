@@ -783,6 +783,7 @@ virs_status ensure_ir(virs_sim *s, uint64_t need)
     uint64_t cap = std::max<uint64_t>(need, s->ircap ? s->ircap * 2 : 1024);
     DevBuf nb;
     VIRS_TRY(nb.alloc(std::max<uint32_t>(s->nrcv, 1) * cap * sizeof(float), "receiver samples"));
+    VIRS_TRY(wait_done(s)); // a run in flight on a caller's stream still records into the old ones
     if (s->ircap && s->nrcv)
         VIRS_CUDA(copy2d_on(s->stream, nb.ptr, cap * sizeof(float), s->ir.ptr, s->ircap * sizeof(float),
                                s->ircap * sizeof(float), s->nrcv, cudaMemcpyDeviceToDevice));
