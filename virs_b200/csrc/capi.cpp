@@ -947,13 +947,40 @@ uint64_t sr_base(const virs_sim *s) { return s->slab ? (s->slab_lo - 1) * (uint6
 // against 65.5 us, 38 M 86.5 against 92.4).  The lines lie between, in FP32
 // short of what 118 M would still gain, at 96 M, 48 M and 26 M; and at 8 M
 // boundary slots (24 M voxels, sponge 16: 7.1 M slots; 38 M: 10.6 M), whose
-// states stream better through a kernel of their own.  A tiling set by the
-// caller names the stencil kernel; the stop rule and the timing of the parts
-// need the separate kernels.
+// states stream better through a kernel of their own.
+//
+// More sections move the lines: four fill the registers, and longer cascades,
+// which run section by section, have two thirds of the boundary pass's warps
+// in flight.  Three launches against one, FP32 unless stated:
+//   4 sections    7.8 M voxels, 3.3 M slots    90.9 against  88.9 us   BF16  84   against 82 us
+//                38 M, 0.7 M / 2.7 M / 5.2 M  121 / 154 / 195   114 / 152 / 203   91 / 125 / 166   91 / 131 / 181
+//                58 M, 3.5 M and 76 M, 1.1 M  208 / 207         212 / 213
+//   6 / 16        1.3 M, 0.74 M                30.9 /  70.1      30.4 /  82.5
+//   8 / 16        1.9 M, 1.1 M                 52   /  82        48   /  88
+//   6 / 12        7.8 M, 1.8 M                 85   / 117        84   / 122             78   / 110        77   / 115
+//   5 / 12        7.8 M, 3.3 M                111   / 183       120   / 206            104   / 176       113   / 199
+//   6 / 12       38 M, 1.3 M                  147   / 174       135   / 165            119   / 146       114   / 145
+//   6 / 12       38 M, 2.7 M                  182   / 231       181   / 238            156   / 204       162   / 218
+//   8 / 12       76 M, 2.1 M                  259   / 287       256   / 289
+// so four sections take one launch up to 48 M voxels (32 M in 16-bit storage)
+// and 4 M slots, and more of them up to 12 M slots times sections, in FP32 a
+// sixth of the voxels (up to 40 M) more, and on grids of few planes or rows
+// (below 1.6 M voxels), whose slots' blocks end in a part-filled wave, 5 M.
+//
+// A tiling set by the caller names the stencil kernel; the stop rule and the
+// timing of the parts need the separate kernels.
 bool fused_on(const virs_sim *s)
 {
-    const size_t most = s->prm.storage == VIRS_STORAGE_F32 ? 96u << 20 : sr_on(s) ? 26u << 20 : 48u << 20;
-    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most && s->nb <= (8u << 20);
+    const bool f32 = s->prm.storage == VIRS_STORAGE_F32;
+    uint64_t most = f32 ? 96u << 20 : sr_on(s) ? 26u << 20 : 48u << 20, slots = 8u << 20;
+    if (s->nsec == 4) {
+        most = std::min<uint64_t>(most, f32 ? 48u << 20 : 32u << 20);
+        slots = 4u << 20;
+    } else if (s->nsec > 4) {
+        const uint64_t states = s->nvox < 1600000 ? 5000000 : 12000000 + (f32 ? std::min<uint64_t>(s->nvox, 40000000) / 6 : 0);
+        slots = states / s->nsec;
+    }
+    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most && s->nb <= slots;
 }
 
 // the probes and block flags of the one-launch step, pl as fused_geo; `buf`
@@ -3179,12 +3206,31 @@ virs_status batch_check(const virs_batch *b)
 // in all for fewer, larger members.  The mean is coarse: 40 even rooms of
 // 3.9 M would gain in one launch and take three, so that the mixed batch,
 // whose mean is close to theirs and which loses in one launch, stays out.
+// Cascades of more than four sections lose where they have many slots (as in
+// fused_on; three launches against one, FP32 and BF16):
+//   16 of 1.9 M voxels, 33 M slots times sections   292 against  283 us    271 against  265 us
+//                       66 M                        395          401       372          383
+//                      107 M                        678          722       658          709
+//   24 of 0.9 M,        24 M                        223          214       193          198
+//                       49 M                        298          302       267          283
+//   24 of 0.13 M,       30 M                        168          159       171          158
+//    8 of 8.3 M,        45 M                        434          437
+//                       90 M                        574          604
+// so they take one launch up to 40 M slots times sections, 32 M in 16-bit storage.
 bool batch_fused(const virs_batch *b)
 {
     size_t n = 0;
-    for (const virs_sim *s : b->mem) n += s->nvox;
-    const size_t each = b->storage == VIRS_STORAGE_F32 ? 24u << 20 : sr_on(b->mem[0]) ? 3u << 19 : 7u << 19;
-    return !b->tiling_set && n <= std::max<size_t>(12u << 20, each * b->mem.size());
+    uint64_t states = 0;
+    uint32_t sections = 0;
+    for (const virs_sim *s : b->mem) {
+        n += s->nvox;
+        states += s->nb * s->nsec;
+        sections = std::max(sections, s->nsec);
+    }
+    const bool f32 = b->storage == VIRS_STORAGE_F32;
+    const size_t each = f32 ? 24u << 20 : sr_on(b->mem[0]) ? 3u << 19 : 7u << 19;
+    return !b->tiling_set && n <= std::max<size_t>(12u << 20, each * b->mem.size()) &&
+           (sections <= 4 || states <= (f32 ? 40000000u : 32000000u));
 }
 
 // descriptors of every member for the batch's tiling
