@@ -343,6 +343,7 @@ struct virs_sim {
     DevBuf probe;                  // sources and receivers for the one-launch step (kernels_fused.cu)
     FusedGeo geo{};
     bool probe_ok = false;
+    bool scattered = false;        // sources and receivers too many and too far apart for that step (make_probes)
     uint64_t ctr_at = 0;           // the step the counter word of parity `cur` holds
     mutable std::atomic<bool> waits{false}; // kernels with bounded waits queued since check_err
     float *host_word = nullptr, *host_word_dev = nullptr; // pinned: virs_step's sample
@@ -448,6 +449,7 @@ struct virs_sim {
                 g = nullptr;
             }
     }
+    void drop_probes() { probe_ok = scattered = false; }
     void drop_graphs()
     {
         destroy_graphs();
@@ -683,7 +685,7 @@ virs_status install_grid(virs_sim *s, uint64_t nx, uint64_t ny, uint64_t nz, flo
     s->pair_nomem = false;
     // sources and receivers refer to voxel indices of the previous grid
     s->nsrc = s->nrcv = 0;
-    s->probe_ok = false;
+    s->drop_probes();
     s->src_ref.clear();
     s->rcv_ref.clear();
     s->has_grid = true;
@@ -980,12 +982,21 @@ bool fused_on(const virs_sim *s)
         const uint64_t states = s->nvox < 1600000 ? 5000000 : 12000000 + (f32 ? std::min<uint64_t>(s->nvox, 40000000) / 6 : 0);
         slots = states / s->nsec;
     }
-    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && s->nvox <= most && s->nb <= slots;
+    return !s->tiling_set && s->depth > 0 && !s->stop_rule && !s->timing && !s->scattered && s->nvox <= most && s->nb <= slots;
 }
 
-// the probes and block flags of the one-launch step, pl as fused_geo; `buf`
-// holds the probes, then a flag per block
-virs_status make_probes(const virs_sim *s, int pl, DevBuf &buf, FusedGeo *geo)
+constexpr uint32_t MANY_PROBES = 6000;
+// The probes and block flags of the one-launch step, pl as fused_geo; `buf`
+// holds the probes, then a flag per block.
+// A block with a probe goes through the whole list for its own, so the work
+// grows with the probes times the blocks that have any; the post kernel of
+// three launches takes them in one block.  Receivers at random, three launches
+// against one, FP32 (a plane of receivers in brackets): 7.8 M voxels, 4096
+// 37.7 against 32.3 us (34.8 and 18.8), 16384 73 against 114 (59 and 31);
+// 38 M, 4096 131 against 110, 16384 188 against 336 (171 and 103); 1.9 M, whose
+// step has 1115 blocks, 16384 54 against 36.  The two cross at about 6000 in
+// 3000 to 5000 blocks.  `scattered`: more than that in more than 2048 blocks.
+virs_status make_probes(const virs_sim *s, int pl, DevBuf &buf, FusedGeo *geo, bool *scattered)
 {
     const uint32_t n = s->nsrc + s->nrcv;
     FusedGeo g = fused_geo(s->px, s->ny, s->nz, s->nb, sm_count(s->prm.device), pl);
@@ -998,11 +1009,17 @@ virs_status make_probes(const virs_sim *s, int pl, DevBuf &buf, FusedGeo *geo)
     VIRS_CUDA(launch_probe_blocks(buf.as<Probe>(), n, s->bpos.as<uint32_t>(), s->nb, s->px * s->ny, s->nz, g,
                                   buf.as<uint8_t>() + n * sizeof(Probe), s->stream));
     *geo = g;
+    *scattered = false;
+    if (n > MANY_PROBES) {
+        std::vector<uint8_t> has(g.blocks);
+        VIRS_CUDA(copy_on(s->stream, has.data(), g.has_probe, g.blocks, cudaMemcpyDeviceToHost));
+        *scattered = std::count(has.begin(), has.end(), (uint8_t)1) > 2048;
+    }
     return VIRS_OK;
 }
 virs_status build_probes(virs_sim *s)
 {
-    VIRS_TRY(make_probes(s, 0, s->probe, &s->geo));
+    VIRS_TRY(make_probes(s, 0, s->probe, &s->geo, &s->scattered));
     VIRS_CUDA(cudaStreamSynchronize(s->stream)); // the run may take a caller's stream
     s->probe_ok = true;
     s->graph_dirty = true;
@@ -1880,7 +1897,7 @@ VIRS_EXPORT virs_status virs_classify(virs_sim *s)
     s->pm_rows = 0;
     s->pzm_zc = -1;
     s->pl_ok = false;
-    s->probe_ok = false;
+    s->drop_probes();
     s->classified = true;
     VIRS_CUDA(cudaEventRecord(s->done, st));
     return VIRS_OK;
@@ -2092,7 +2109,7 @@ VIRS_EXPORT virs_status virs_set_sources(virs_sim *s, uint32_t n, const uint64_t
     s->src_ref.assign(idx, idx + n);
     s->sig.release();
     s->pl_ok = false;
-    s->probe_ok = false;
+    s->drop_probes();
     s->graph_dirty = true;
     ++s->gen;
     return VIRS_OK;
@@ -2115,7 +2132,7 @@ VIRS_EXPORT virs_status virs_set_receivers(virs_sim *s, uint32_t n, const uint64
     s->rcv_ref.assign(idx, idx + n);
     s->ir.release();
     s->ircap = 0;
-    s->probe_ok = false;
+    s->drop_probes();
     s->graph_dirty = true;
     ++s->gen;
     return VIRS_OK;
@@ -3238,6 +3255,15 @@ virs_status batch_build(virs_batch *b)
 {
     b->drop_graphs();
     b->fused = batch_fused(b);
+    for (virs_sim *s : b->mem) {
+        if (!b->fused || s->nsrc + s->nrcv <= MANY_PROBES) continue;
+        VIRS_TRY(ready_to_run(s));
+        DevBuf probes;
+        FusedGeo geo{};
+        bool scattered = false;
+        VIRS_TRY(make_probes(s, 2, probes, &geo, &scattered));
+        b->fused = !scattered;
+    }
     for (auto &l : b->launches) l.clear();
     b->zmasks.clear();
     b->probes.clear();
@@ -3263,7 +3289,8 @@ virs_status batch_build(virs_batch *b)
         FusedGeo geo{};
         if (b->fused) {
             b->probes.emplace_back();
-            VIRS_TRY(make_probes(s, 2, b->probes.back(), &geo));
+            bool scattered = false; // of no member, as looked at above
+            VIRS_TRY(make_probes(s, 2, b->probes.back(), &geo, &scattered));
             VIRS_CUDA(cudaStreamSynchronize(s->stream));
         }
         if (!b->fused && zero_masks_useful(s)) {
