@@ -131,24 +131,30 @@ __global__ void __launch_bounds__(LB) k_ir_resample(const float *__restrict in, 
 // w(tau) = I0(beta sqrt(1 - (tau / half)^2)) / I0(beta).  FP64 throughout.
 //
 // The weights are the work (channels share them): a warp takes one output
-// sample of up to CH channels, its lanes every 32nd tap.  The window is the
+// sample of up to CH channels (G = 32), its lanes every G-th tap.  The window is the
 // power series of I0 in 1 - (tau / half)^2 itself, sum_k c_k v^k with
 // c_k = (beta / 2)^(2k) / (k!)^2 / I0(beta) (all terms positive: no
 // cancellation), from the kernel's parameters; the sine of
-// a lane's next tap follows from the last by the rotation by 32 taps, except
+// a lane's next tap follows from the last by the rotation by G taps, except
 // near tau = 0, where its relative error would matter.  8 channels, 4000 to
 // 5049 samples, 490 taps: 1463 us with the series, a sine and a division per
 // tap and channel, one output per thread; 46 us in this form (two chains of
 // half the length, odd and even powers, were no faster: the FP64 rate bounds
-// it, not the chain).
+// it, not the chain).  Short windows leave most of 32 lanes idle, and the sums
+// over the lanes become the work: there four lanes take a sample, a warp
+// eight (8 channels, 6300 samples, 2 to 32 taps: 213 to 250 us a call with a
+// thread per output and channel, 257 with a warp, 176 with four lanes; 1000
+// channels, 2 taps: 2.9, 3.9 and 2.2 ms).
 constexpr int CH = 8;            // channels per warp
 constexpr int SINC_TERMS = 128;  // of the series (beta <= 50 needs 80)
 struct SincArgs {
-    double step_ratio, fc2, inv_half, rot_s, rot_c; // sine and cosine of pi * fc2 * 32
+    double step_ratio, fc2, inv_half, rot_s, rot_c; // sine and cosine of pi * fc2 * G
     int half, terms;
     double c[SINC_TERMS];
 };
 
+// G: the lanes of an output sample
+template <int G>
 __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint64_t in_stride, uint64_t len,
                                                 const __grid_constant__ SincArgs a, float *__restrict out,
                                                 uint64_t out_len, uint32_t channels, uint32_t *__restrict peak)
@@ -159,9 +165,10 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
     for (int j = threadIdx.x; j < SINC_TERMS / 2; j += RB)
         cf[j] = make_double2(2 * j < a.terms ? a.c[2 * j] : 0.0, 2 * j + 1 < a.terms ? a.c[2 * j + 1] : 0.0);
     __syncthreads();
-    const int lane = threadIdx.x & 31, pairs = (a.terms + 1) / 2;
-    const uint64_t k = (uint64_t)blockIdx.x * (RB / 32) + threadIdx.x / 32;
-    if (k >= out_len) return; // the whole warp
+    const int lane = threadIdx.x & (G - 1), pairs = (a.terms + 1) / 2;
+    const uint64_t kg = (uint64_t)blockIdx.x * (RB / G) + threadIdx.x / G;
+    if (G == 32 && kg >= out_len) return;                // the whole warp
+    const uint64_t k = kg < out_len ? kg : out_len - 1;  // idle groups repeat the last sample, unstored
     const uint32_t c0 = blockIdx.y * CH, nc = min(channels - c0, (uint32_t)CH);
     const float *f = in + (uint64_t)c0 * in_stride;
     const double t = (double)k * a.step_ratio;
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
     for (int c = 0; c < CH; ++c) acc[c] = 0.0;
     double sn, cs;
     sincospi(a.fc2 * (t - (n0 + (double)lane)), &sn, &cs);
-    for (double n = n0 + (double)lane; n <= n1; n += 32.0) {
+    for (double n = n0 + (double)lane; n <= n1; n += (double)G) {
         const double tau = t - n, u = tau * a.inv_half, x = a.fc2 * tau;
         const double s = fabs(x) < 0.5 ? sinpi(x) : sn;
         // sin(x - d) and cos(x - d) for the next tap
@@ -196,8 +203,8 @@ __global__ void __launch_bounds__(RB) k_ir_sinc(const float *__restrict in, uint
     for (int c = 0; c < CH; ++c) {
         if (c >= (int)nc) break;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(FULL, acc[c], o);
-        if (lane == 0) {
+        for (int o = G / 2; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(FULL, acc[c], o);
+        if (lane == 0 && kg < out_len) {
             const float v = (float)acc[c];
             out[(uint64_t)(c0 + c) * out_len + k] = v;
             if (peak) atomicMax(peak + c0 + c, __float_as_uint(fabsf(v))); // non-negative floats order as integers
@@ -224,7 +231,12 @@ cudaError_t launch_ir_sinc(const float *in, uint64_t in_stride, uint64_t len, do
     a.fc2 = cutoff * fmin(fs_in, rate) / fs_in; // 2 fc
     a.half = half;
     a.inv_half = 1.0 / (double)half;
-    const double turn = fmod(32.0 * a.fc2, 2.0);
+    // Four lanes per output sample for short windows, as long as those fill
+    // the device (one channel of 380 samples, 32 taps: 41 us with 32 lanes, 44
+    // with four; of 6300 samples, 64 taps: 70 and 70, 128 taps 77 and 81).
+    const uint64_t warps = out_len * ((channels + CH - 1) / CH);
+    const int G = half <= 32 && warps >= 4096 ? 4 : 32;
+    const double turn = fmod((double)G * a.fc2, 2.0);
     a.rot_s = sin(M_PI * turn);
     a.rot_c = cos(M_PI * turn);
     // I0(beta) and the window's coefficients, as many as change the sum
@@ -240,12 +252,13 @@ cudaError_t launch_ir_sinc(const float *in, uint64_t in_stride, uint64_t len, do
         a.terms = k + 1;
     }
     for (int k = 0; k < a.terms; ++k) a.c[k] /= i0b;
-    const dim3 g((unsigned)((out_len + RB / 32 - 1) / (RB / 32)), (channels + CH - 1) / CH);
+    const unsigned per = (unsigned)(RB / G); // output samples per block
+    const dim3 g((unsigned)((out_len + per - 1) / per), (channels + CH - 1) / CH);
     if (peak) {
         cudaError_t e = cudaMemsetAsync(peak, 0, channels * sizeof(uint32_t), s);
         if (e != cudaSuccess) return e;
     }
-    k_ir_sinc<<<g, RB, 0, s>>>(in, in_stride, len, a, out, out_len, channels, peak);
+    (G == 4 ? k_ir_sinc<4> : k_ir_sinc<32>)<<<g, RB, 0, s>>>(in, in_stride, len, a, out, out_len, channels, peak);
     if (peak)
         k_ir_normalize<<<dim3((unsigned)((out_len + RB - 1) / RB), channels), RB, 0, s>>>(out, out_len, peak);
     return cudaGetLastError();
