@@ -2230,8 +2230,10 @@ virs_status slab_exchange(virs_sim *lo, virs_sim *hi)
 {
     const size_t pb = (size_t)lo->px * lo->ny * lo->storage_bytes();
     VIRS_TRY(use_device(lo));
+    VIRS_CUDA(cudaStreamWaitEvent(lo->stream, lo->done, 0)); // its own on a caller's stream
     VIRS_CUDA(cudaStreamWaitEvent(lo->stream, hi->done, 0));
     VIRS_TRY(use_device(hi));
+    VIRS_CUDA(cudaStreamWaitEvent(hi->stream, hi->done, 0));
     VIRS_CUDA(cudaStreamWaitEvent(hi->stream, lo->done, 0));
     VIRS_TRY(use_device(lo));
     VIRS_CUDA(cudaMemcpyAsync(slab_plane(lo, lo->nz - 1), slab_plane(hi, 1), pb, cudaMemcpyDefault, lo->stream));
@@ -2443,6 +2445,7 @@ VIRS_EXPORT virs_status virs_slab_run(virs_sim *const *slabs, uint32_t n, uint64
         if (s->stop_rule && s->stopped) return fail(VIRS_E_STATE, "virs_slab_run: the stop rule fired");
         VIRS_TRY(ready_to_run(s));
         VIRS_TRY(ensure_ir(s, s->steps_done + steps));
+        VIRS_CUDA(cudaStreamWaitEvent(s->stream, s->done, 0)); // what runs on a caller's stream
         if (s->depth > 0 && zero_masks_useful(s) && s->nz > 5 &&
             (s->zmi_rows != s->tile_rows || s->zmi_zc != eff_planes(s))) {
             s->zmi_rows = s->zmi_zc = 0;
