@@ -1,6 +1,7 @@
 """Slabs that ran on callers' streams, one of them still busy (torch's sleep
 kernel, about a third of a second): an exchange and a run of all slabs follow
-them, as the handles' completion events do."""
+them, as the handles' completion events do; and a stream in capture, which
+cannot wait for such work, is refused."""
 import numpy as np
 import pytest
 
@@ -72,3 +73,27 @@ def test_exchange_and_run_follow_what_is_in_flight(how):
         assert np.array_equal(got.view(np.uint32), want.reshape(-1)[lo * plane:hi * plane].view(np.uint32))
     for s in (whole, *sims):
         s.close()
+
+
+def test_a_stream_in_capture_is_refused():
+    import torch
+    sim = capi.Simulation(capi.default_params())
+    sim.set_grid(SHAPE, 0.05, _flags())
+    _start(sim, _p0())
+    st = torch.cuda.Stream()
+    sim.run(4, st.cuda_stream)
+    sim.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    x = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        graph.capture_begin(capture_error_mode="thread_local")
+        x += 1
+        with pytest.raises(capi.VirsError) as e:
+            sim.run(4, st.cuda_stream)
+        graph.capture_end()
+    assert e.value.status == capi.E_CUDA
+    sim.run(4, st.cuda_stream)
+    sim.synchronize()
+    assert int(sim.info().steps_done) == 8
+    sim.close()
